@@ -12,6 +12,8 @@
 //   log  uint64[K][V][W]   ring of K levels: log[L-base][v] = bits found at level L
 //   jf   int32[2][V]       joint frontier (vertices with any new bit), ping-pong
 //   heavy int32[2][V]      joint-frontier vertices of degree >= opts.batch_heavy
+//   smask uint16[V]        which log slots hold bits of the vertex: the flush
+//                          reads and clears only those
 //   done bit per vertex    every source has visited it (bottom-up skips it)
 //   jfb  bit per vertex    [2] joint-frontier membership of levels L and L+1:
 //                          dedups top-down claims and lets bottom-up skip the
@@ -23,9 +25,11 @@
 // rebuilds the frontier from its bitmap) or bottom-up (every unfinished
 // vertex ORs its neighbours' frontier words, stopping once all bits of the
 // active sources it lacks are covered; light, mid and large degree tiers).
-// Depths are never scattered during the traversal: a flush kernel decodes the
-// log into a byte tile per span of vertices, zeroing the slots as it reads
-// them, and writes the source-major depth rows with coalesced vector stores.
+// All of it is in the graph's traversal ids (descending degree). Depths are
+// never scattered during the traversal: a flush kernel takes spans of
+// consecutive caller ids, gathers and decodes their log words into a byte tile,
+// zeroing the slots as it reads them, and writes the source-major depth rows
+// with coalesced vector stores.
 #include <algorithm>
 #include <string.h>
 #include <vector>
@@ -76,11 +80,15 @@ struct BatchArgs {
   const int4* lead;     // adj[off[v] .. off[v]+3] per vertex (-1 past the row)
   const int32_t* deg;
   const uint32_t* active;
+  const int32_t* inv;   // traversal id of each caller id (null: the same)
+  const int64_t* coff;  // row offsets in caller order (degrees of the rows a flush writes)
   int64_t V, E;
+  int64_t n_active;     // vertices with a row have ids below this
   int32_t W, lgW;       // words per vertex and log2(W)
   int32_t K;            // log slots in use
   unsigned long long* X;
   unsigned long long* log;
+  uint16_t* smask;      // [V] bit k set iff the vertex has bits in log slot k
   const unsigned long long* mask;  // [W] valid source bits
   // [2][W] active sources: act[cur] holds the sources whose level-L frontier
   // is non-empty, act[nxt] collects those found at level L+1. A source that
@@ -124,6 +132,9 @@ __device__ __forceinline__ T bsum(T x, T* s_red) {
     for (int w = 0; w < BB / 32; ++w) r += s_red[w];
   return r;
 }
+
+// The traversal id of caller id v.
+__device__ __forceinline__ int in_id(const BatchArgs& a, int v) { return a.inv ? a.inv[v] : v; }
 
 // Warp-aggregated append of v (when `want`) to list, counter *n.
 __device__ __forceinline__ void wappend(bool want, int v, int32_t* list, int32_t* n) {
@@ -178,14 +189,17 @@ __global__ void __launch_bounds__(SEED_THREADS) k_b_seed(BatchArgs a) {
     bool fresh = false;
     int v = 0, d = 0;
     if (i < n_seed) {
-      v = a.src[i];
+      v = in_id(a, a.src[i]);
       const int s = a.seed_slot ? a.seed_slot[i] : i;
       const unsigned long long bit = 1ull << (s & 63);
       atomicOr(&a.X[(size_t)v * a.W + (s >> 6)], bit);
       atomicOr(&s0[(size_t)v * a.W + (s >> 6)], bit);
       const uint32_t tb = 1u << (v & 31);
       fresh = !(atomicOr(&a.jfb[0][v >> 5], tb) & tb);
-      if (fresh) d = a.deg[v];
+      if (fresh) {
+        d = a.deg[v];
+        a.smask[v] = 1;
+      }
     }
     const unsigned mf = __ballot_sync(FULL, fresh);
     if (!mf) continue;
@@ -339,11 +353,12 @@ __device__ __forceinline__ void load_words(const unsigned long long* p, unsigned
 }
 
 // Records the outcome of one bottom-up vertex (called by the lane that owns
-// the vertex): frontier append, counters, completion bit.
-__device__ __forceinline__ void bu_finish_vertex(const BatchArgs& a, BatchCtl* c, int v, int nxt, bool gany,
-                                                 bool gfull, int64_t d, unsigned long long& my_m,
+// the vertex): frontier append, the slot's mark (sbit), counters, completion bit.
+__device__ __forceinline__ void bu_finish_vertex(const BatchArgs& a, BatchCtl* c, int v, int nxt, uint32_t sbit,
+                                                 bool gany, bool gfull, int64_t d, unsigned long long& my_m,
                                                  unsigned long long& my_md) {
   if (gany) {
+    a.smask[v] = (uint16_t)(a.smask[v] | sbit);
     my_m += (unsigned long long)d;
     atomicOr(&a.jfb[nxt][v >> 5], 1u << (v & 31));
     a.jf[nxt][atomicAdd(&c->n_jf[nxt], 1)] = v;
@@ -409,6 +424,7 @@ __device__ void b_bu_mid(const BatchArgs& a, BatchCtl* c, const unsigned long lo
   const int gw = (blockIdx.x * BB + threadIdx.x) >> 5, nw = (gridDim.x * BB) >> 5;
   const unsigned long long* ac = a.act[c->cur] + gl * WPT;
   const uint32_t* jfc = a.jfb[c->cur];
+  const uint32_t sbit = 2u << (c->level - c->base);
   for (int i = gw; i < a.n_mid; i += nw) {
     const int v = a.mid[i];
     if ((a.donebits[v >> 5] >> (v & 31)) & 1u) continue;
@@ -422,7 +438,7 @@ __device__ void b_bu_mid(const BatchArgs& a, BatchCtl* c, const unsigned long lo
       any |= need[j] != 0;
     }
     if (!__any_sync(FULL, any)) {  // every source it still lacks has finished
-      if (lane == 0) bu_finish_vertex(a, c, v, nxt, false, true, a.deg[v], my_m, my_md);
+      if (lane == 0) bu_finish_vertex(a, c, v, nxt, sbit, false, true, a.deg[v], my_m, my_md);
       continue;
     }
     const int64_t beg = a.off[v], end = a.off[v + 1];
@@ -459,7 +475,7 @@ __device__ void b_bu_mid(const BatchArgs& a, BatchCtl* c, const unsigned long lo
     }
     const bool gany = __any_sync(FULL, got);
     const bool gfull = __all_sync(FULL, full);
-    if (lane == 0) bu_finish_vertex(a, c, v, nxt, gany, gfull, end - beg, my_m, my_md);
+    if (lane == 0) bu_finish_vertex(a, c, v, nxt, sbit, gany, gfull, end - beg, my_m, my_md);
   }
 }
 
@@ -477,6 +493,7 @@ __device__ void b_bu_large(const BatchArgs& a, BatchCtl* c, const unsigned long 
   const int nxt = c->cur ^ 1;
   const uint32_t* jfc = a.jfb[c->cur];
   const unsigned long long* ac = a.act[c->cur];
+  const uint32_t sbit = 2u << (c->level - c->base);
   for (int i = blockIdx.x; i < a.n_large; i += gridDim.x) {
     const int v = a.large[i];
     __syncthreads();
@@ -488,7 +505,7 @@ __device__ void b_bu_large(const BatchArgs& a, BatchCtl* c, const unsigned long 
     __syncthreads();
     if (s_skip) continue;
     if (!__syncthreads_or(t < W && s_need[t] != 0)) {  // every source it still lacks has finished
-      if (t == 0) bu_finish_vertex(a, c, v, nxt, false, true, a.deg[v], my_m, my_md);
+      if (t == 0) bu_finish_vertex(a, c, v, nxt, sbit, false, true, a.deg[v], my_m, my_md);
       continue;
     }
     unsigned long long need[WPT], acc[WPT];
@@ -534,7 +551,7 @@ __device__ void b_bu_large(const BatchArgs& a, BatchCtl* c, const unsigned long 
     }
     const bool gany = __syncthreads_or(got);
     const bool gfull = !__syncthreads_or(!full);
-    if (t == 0) bu_finish_vertex(a, c, v, nxt, gany, gfull, end - beg, my_m, my_md);
+    if (t == 0) bu_finish_vertex(a, c, v, nxt, sbit, gany, gfull, end - beg, my_m, my_md);
   }
 }
 
@@ -554,7 +571,7 @@ __device__ void b_bu_expand(const BatchArgs& a, BatchCtl* c, unsigned long long*
   const unsigned gmask = (G == 32) ? FULL : (((1u << G) - 1) << (grp * G));
   const int64_t gtid = blockIdx.x * (int64_t)BB + threadIdx.x, nth = (int64_t)gridDim.x * BB;
   const int64_t gw = gtid >> 5, nw = nth >> 5;
-  const int64_t Wd = (a.V + 31) >> 5;
+  const int64_t Wd = (a.n_active + 31) >> 5;
   unsigned long long mk[WPL];
 #pragma unroll
   for (int j = 0; j < WPL; ++j) mk[j] = a.act[cur][gl * WPL + j];
@@ -643,6 +660,7 @@ __device__ void b_bu_expand(const BatchArgs& a, BatchCtl* c, unsigned long long*
         }
         // append v to the next joint frontier (one lane per group)
         if (gl == 0 && gany) {
+          a.smask[v] = (uint16_t)(a.smask[v] | (2u << slot));
           const int at = atomicAdd(&c->n_jf[nxt], 1);
           a.jf[nxt][at] = (int)v;
           front_bits |= 1u << vl;
@@ -748,13 +766,15 @@ __device__ void join_sources(const BatchArgs& a, volatile BatchCtl* vc, int L, i
   int32_t* rows = const_cast<int32_t*>(vc->row_map);
   for (int j = 0; j < nj && j < JOIN_MAX; ++j) {
     const int s = *(volatile int32_t*)&box->pos[j];
-    const int v = *(volatile int32_t*)&box->src[j];
+    const int cv = *(volatile int32_t*)&box->src[j];
     const int r = *(volatile int32_t*)&box->row[j];
-    if (s < 0 || s >= a.W * 64 || v < 0 || v >= a.V) continue;  // the host never posts these
+    if (s < 0 || s >= a.W * 64 || cv < 0 || cv >= a.V) continue;  // the host never posts these
+    const int v = in_id(a, cv);
     const unsigned long long bit = 1ull << (s & 63);
     const size_t at = (size_t)v * a.W + (s >> 6);
     a.X[at] |= bit;
     F[at] |= bit;
+    a.smask[v] = (uint16_t)(a.smask[v] | (1u << (L - vc->base)));
     a.act[nxt][s >> 6] |= bit;
     a.join[s] = L;
     if (rows) rows[s] = r;
@@ -812,6 +832,7 @@ __global__ void __launch_bounds__(BB) k_b_commit(BatchArgs a) {
     const auto vertex_done = [&](int v, bool got, bool full) {
       if (!got) return;
       const int d = a.deg[v];
+      a.smask[v] = (uint16_t)(a.smask[v] | (2u << slot));
       my_m += d;
       if (full) {
         atomicOr(&a.donebits[v >> 5], 1u << (v & 31));
@@ -904,7 +925,7 @@ __global__ void __launch_bounds__(BB) k_b_commit(BatchArgs a) {
 // ----------------------------------------------------------- flush --------
 // Converts log slots [first, last] (levels base+first .. base+last) into the
 // source-major depth rows and recycles the slots in the same pass. A CTA takes
-// a span of 1024 vertices and walks the W word columns in groups of
+// a span of 1024 vertices (caller ids) and walks the W word columns in groups of
 // CG = min(W, 4), VS = 1024 / CG vertices per pass.
 // Decode (thread per vertex): the slots of a vertex are disjoint bit sets, so
 // the vertex's CG words of every slot fold into a found mask and four bit
@@ -1037,47 +1058,69 @@ struct FlushState {
 template <int CG, bool BYTES>
 __device__ void flush_span(const BatchArgs& a, const FlushState& fs, int64_t v0, int nv) {
   constexpr int VS = 1024 / CG;  // vertices per pass
+  constexpr int Q = VS / BB;     // ... and per thread
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int first = fs.first, last = fs.last;
+  // the slots decoded: [first, last]
+  const uint32_t decoded = ((2u << fs.last) - 1u) & ~((1u << fs.first) - 1u);
+  // The thread's vertices of this pass (traversal ids) and their slot marks.
+  // Both reads for the next pass are issued during this one: the ids before
+  // the decode, the marks (gathered at those ids) before the rows are written.
+  int iv[Q], next_iv[Q];
+  uint32_t mk[Q];
+  const auto load_ids = [&](int sub, int (&id)[Q]) {
+#pragma unroll
+    for (int q = 0; q < Q; ++q) {
+      const int vi = sub + (int)threadIdx.x + q * BB;
+      id[q] = vi < nv ? (a.inv ? __ldg(a.inv + v0 + vi) : (int)(v0 + vi)) : -1;
+    }
+  };
+  const auto load_marks = [&](const int (&id)[Q]) {
+#pragma unroll
+    for (int q = 0; q < Q; ++q) mk[q] = id[q] >= 0 ? a.smask[id[q]] : 0u;
+  };
+  load_ids(0, iv);
+  load_marks(iv);
   for (int sub = 0; sub < nv; sub += VS) {
     const int nsub = min(VS, nv - sub);
+    load_ids(sub + VS, next_iv);
     for (int cg = 0; cg < a.W; cg += CG) {
       if (cg * 64 >= fs.nsrc) break;  // words of no source: never set, so already zero
       __syncthreads();  // the previous tile has been written out
-      for (int vi = threadIdx.x; vi < VS; vi += BB) {
-        const bool in = vi < nsub;
-        const size_t at = (size_t)(v0 + sub + vi) * a.W + cg;
+      const bool last_cols = cg + CG >= a.W || (cg + CG) * 64 >= fs.nsrc;
+#pragma unroll
+      for (int q = 0; q < Q; ++q) {
+        const int vi = (int)threadIdx.x + q * BB;
+        const uint32_t marks = mk[q], md = marks & decoded;
+        const size_t at = (size_t)(marks ? iv[q] : 0) * a.W + cg;
         unsigned long long f[CG], p0[CG], p1[CG], p2[CG], p3[CG];
 #pragma unroll
         for (int cc = 0; cc < CG; ++cc) f[cc] = p0[cc] = p1[cc] = p2[cc] = p3[cc] = 0;
         // loads and folds only: no store or warp-collective may sit between
-        // the slot loads, which the compiler then keeps in flight together
-        if (in) {
-          // slots in groups of four from a multiple of 4: bits 0 and 1 of a
-          // slot's index follow from its place in the group, bits 2 and 3 are
-          // the group's
-          for (int k0 = 0; k0 <= last; k0 += 4) {
+        // the slot loads, which the compiler then keeps in flight together.
+        // Slots in groups of four from a multiple of 4: bits 0 and 1 of a
+        // slot's index follow from its place in the group, bits 2 and 3 are
+        // the group's. Only marked slots are read (about a third of them).
+        for (int k0 = 0; md >> k0; k0 += 4) {
 #pragma unroll
-            for (int h = 0; h < 2; ++h) {
-              const int ka = k0 + 2 * h, kb = ka + 1;
-              unsigned long long wa[CG], wb[CG];
-              if (ka >= first && ka <= last) load_cols<CG>(slot_ptr(a, ka) + at, wa);
-              else
+          for (int h = 0; h < 2; ++h) {
+            const int ka = k0 + 2 * h, kb = ka + 1;
+            unsigned long long wa[CG], wb[CG];
+            if ((md >> ka) & 1u) load_cols<CG>(slot_ptr(a, ka) + at, wa);
+            else
 #pragma unroll
-                for (int cc = 0; cc < CG; ++cc) wa[cc] = 0;
-              if (kb >= first && kb <= last) load_cols<CG>(slot_ptr(a, kb) + at, wb);
-              else
+              for (int cc = 0; cc < CG; ++cc) wa[cc] = 0;
+            if ((md >> kb) & 1u) load_cols<CG>(slot_ptr(a, kb) + at, wb);
+            else
 #pragma unroll
-                for (int cc = 0; cc < CG; ++cc) wb[cc] = 0;
+              for (int cc = 0; cc < CG; ++cc) wb[cc] = 0;
 #pragma unroll
-              for (int cc = 0; cc < CG; ++cc) {
-                const unsigned long long u = wa[cc] | wb[cc];
-                f[cc] |= u;
-                p0[cc] |= wb[cc];
-                if (h) p1[cc] |= u;
-                if (k0 & 4) p2[cc] |= u;
-                if (k0 & 8) p3[cc] |= u;
-              }
+            for (int cc = 0; cc < CG; ++cc) {
+              const unsigned long long u = wa[cc] | wb[cc];
+              f[cc] |= u;
+              p0[cc] |= wb[cc];
+              if (h) p1[cc] |= u;
+              if (k0 & 4) p2[cc] |= u;
+              if (k0 & 8) p3[cc] |= u;
             }
           }
         }
@@ -1093,19 +1136,25 @@ __device__ void flush_span(const BatchArgs& a, const FlushState& fs, int64_t v0,
             for (int n = 0; n < 8; ++n) fs.tile[tile_word<CG>(vi, cc * 16 + hw * 8 + n)] = o[n];
           }
         }
-        if (in) {
-          // recycle: a window flush carries slot K-1 (the next window's
-          // frontier) into slot 0 and zeroes slots 1..K-1; the final flush
-          // zeroes slots 0..last (slot 0 too after a window flush)
-          int z0 = 0;
-          if (!fs.final_flush) {
+        if (marks) {
+          // recycle the marked slots: a window flush carries the last slot
+          // (K-1, the next window's frontier) into slot 0, all others end zero
+          uint32_t z = marks;
+          const bool carry = !fs.final_flush && ((marks >> fs.last) & 1u);
+          if (carry) {
             unsigned long long x[CG];
-            load_cols<CG>(slot_ptr(a, last) + at, x);
+            load_cols<CG>(slot_ptr(a, fs.last) + at, x);
             store_cols<CG>(slot_ptr(a, 0) + at, x[0], x[CG > 1 ? 1 : 0], x[CG > 2 ? 2 : 0], x[CG > 2 ? 3 : 0]);
-            z0 = 1;
+            z &= ~1u;
           }
-          for (int k = z0; k <= last; ++k) store_cols<CG>(slot_ptr(a, k) + at, 0ull, 0ull, 0ull, 0ull);
+          for (; z; z &= z - 1) store_cols<CG>(slot_ptr(a, __ffs(z) - 1) + at, 0ull, 0ull, 0ull, 0ull);
+          if (last_cols) a.smask[iv[q]] = carry ? 1 : 0;
         }
+      }
+      if (last_cols) {  // this pass has used its marks: fetch the next one's
+#pragma unroll
+        for (int q = 0; q < Q; ++q) iv[q] = next_iv[q];
+        load_marks(iv);
       }
       __syncthreads();
       for (int r0 = warp * 4; r0 < 64 * CG; r0 += BB / 32 * 4) {
@@ -1245,7 +1294,8 @@ __global__ void __launch_bounds__(BB, 3) k_b_flush(BatchArgs a, int final_flush)
       const int64_t v0 = u * 1024;
       const int nv = (int)min((int64_t)1024, a.V - v0);
       __syncthreads();
-      for (int i = threadIdx.x; i < 1024; i += BB) s_deg[i] = i < nv ? a.deg[v0 + i] : 0;
+      for (int i = threadIdx.x; i < 1024; i += BB)
+        s_deg[i] = i < nv ? (int)(a.coff[v0 + i + 1] - a.coff[v0 + i]) : 0;
       __syncthreads();
       if (bytes) {
         if (a.W == 1) flush_span<1, true>(a, fs, v0, nv);
@@ -1456,8 +1506,9 @@ int create_batch_workspace(ent_graph* g, int n_src, BatchWorkspace** out) {
   const size_t sz_q = al(sizeof(int32_t) * (V + 4));
   const size_t sz_mask = al(sizeof(unsigned long long) * W);
   const size_t sz_src = al(sizeof(int32_t) * w->cap_src);
+  const size_t sz_marks = al(sizeof(uint16_t) * V);
   const size_t sz_st = al(sizeof(unsigned long long) * w->cap_src) * 2 + 2 * al(sizeof(int32_t) * w->cap_src);
-  const size_t total = sz_x + sz_log + 4 * sz_bits + 6 * sz_q + 3 * sz_mask + sz_src + sz_st + 256;
+  const size_t total = sz_x + sz_log + 4 * sz_bits + 6 * sz_q + 3 * sz_mask + sz_src + sz_st + sz_marks + 256;
   cudaError_t e = cudaMalloc(&w->slab, total);
   if (e != cudaSuccess) { destroy_batch_workspace(w); return fail(ENT_ERR_OOM, "batch workspace (%zu bytes) failed", total); }
   // Initialise on the graph's stream and wait (see create_workspace in
@@ -1474,11 +1525,14 @@ int create_batch_workspace(ent_graph* g, int n_src, BatchWorkspace** out) {
   BatchArgs& a = w->args;
   memset(&a, 0, sizeof(a));
   a.ctl = w->ctl;
-  a.off = g->off;
+  a.off = g->toff;
   a.adj = g->trav;
   a.lead = g->lead;
   a.deg = g->deg;
   a.active = g->active;
+  a.inv = g->inv;
+  a.coff = g->off;
+  a.n_active = g->n_active;
   a.V = V;
   a.E = g->E;
   a.W = W;
@@ -1488,6 +1542,7 @@ int create_batch_workspace(ent_graph* g, int n_src, BatchWorkspace** out) {
   a.K = w->K;
   a.X = (unsigned long long*)p; w->x_ptr = p; w->x_bytes = sz_x; p += sz_x;
   a.log = (unsigned long long*)p; p += sz_log;
+  a.smask = (uint16_t*)p; p += sz_marks;
   a.donebits = (uint32_t*)p; w->small_ptr = p; w->small_bytes = 3 * sz_bits; p += sz_bits;
   a.jfb[0] = (uint32_t*)p; p += sz_bits;
   a.jfb[1] = (uint32_t*)p; p += sz_bits;

@@ -14,6 +14,13 @@
 //    chunk_edges edges), claim vertices with atomicOr on `vis`, and append
 //    discoveries to a raw queue with warp-aggregated atomics
 //    (reference expanders K2-K4, expander.cuh:74-423).
+//  * Vertices carry traversal ids, descending degree (dev_graph.h): the sweeps
+//    end at the last vertex that has a row, a warp's vertices have equal
+//    degrees and adjacent rows, and the hubs' status bits share a few lines
+//    that stay in L1. The caller's ids appear where the source comes in and
+//    where depths and parents are stored. R-MAT s24: 0.51 -> 0.35 ms a
+//    traversal (first bottom-up level 0.22 -> 0.10); uniform graphs gain
+//    nothing from it and lose nothing measurable (ER 2^24 d32 1.90 -> 1.89 ms).
 //  * Bottom-up (BU) levels sweep the status bitmaps: a warp owns one word
 //    (32 consecutive ids) and checks only unvisited, non-isolated vertices,
 //    each lane serially for small degrees, the whole warp together for large
@@ -22,8 +29,7 @@
 //    (reference K5-K7, expander.cuh:431-819; hub cache comm.h:172-177).
 //    Rows are ordered by descending neighbour degree, so the first check
 //    usually meets a hub; each vertex's first four neighbours are also kept
-//    in a `lead` array read coalesced beside its row offsets, so that check
-//    costs no scattered row read.
+//    in a `lead` array read coalesced, so that check costs no row read.
 //  * The inspector (reference K8/K9/K11, inspector.cuh:36-432) classifies the
 //    next frontier into small/mid/large queues with one single-pass
 //    decoupled look-back scan, order-preserving: from the raw discovery queue
@@ -120,7 +126,10 @@ struct LevelArgs {
   const int4* lead;        // adj[off[v] .. off[v]+3] per vertex (-1 past the row)
   const int32_t* deg;
   const uint32_t* active;
+  const int32_t* perm;     // caller id of each traversal id, null where they are the same
+  const int32_t* inv;      // traversal id of each caller id, null likewise
   int64_t V, E;
+  int64_t n_active;        // vertices with a row have ids below this: the range of a bottom-up sweep
   uint32_t* vis;
   uint32_t* fb[2];
   int32_t* q[2][3];
@@ -148,6 +157,22 @@ __device__ __forceinline__ uint32_t n_chunks_of(int d, const LevelArgs& a) {
   return (uint32_t)((d + a.chunk - 1) / a.chunk);
 }
 __device__ __forceinline__ uint32_t hub_slot(uint32_t v, int shift) { return (v * 0x9E3779B1u) >> shift; }
+
+// The caller's id of traversal id v (depths and parents are indexed by it).
+__device__ __forceinline__ int out_id(const LevelArgs& a, int v) { return a.perm ? __ldg(a.perm + v) : v; }
+
+// Stores a depth under a caller id. The stores of a bottom-up level are
+// scattered (its vertices are in traversal order): their lines are asked to
+// stay in L2, which otherwise evicts them half-written under the level's
+// streams (s24: 0.363 -> 0.344 ms; at s22 and below they stay anyway).
+__device__ __forceinline__ void st_keep(int32_t* p, int32_t x) {
+  asm volatile(
+      "{\n .reg .b64 pol;\n createpolicy.fractional.L2::evict_last.b64 pol, 1.0;\n"
+      " st.global.L2::cache_hint.b32 [%0], %1, pol;\n}" ::"l"(p),
+      "r"(x)
+      : "memory");
+}
+__device__ __forceinline__ void st_keep(uint8_t* p, uint8_t x) { *p = x; }  // a byte row is small enough to stay
 
 // Direct-mapped table of the frontier's highest-degree vertices (the
 // reference keeps the max-degree vertex per slot, inspector.cuh:218-224, but
@@ -239,12 +264,13 @@ __device__ __forceinline__ void fill_unreached(uint8_t* p, int64_t n, int64_t ti
 // by degree). Written by one thread of k_reset while the others fill; no fill
 // touches the control block or the queues.
 template <class DT>
-__device__ void init_state(const LevelArgs& a, int32_t src, DT* depth, int32_t* parent) {
+__device__ void init_state(const LevelArgs& a, int32_t caller_src, DT* depth, int32_t* parent) {
+  const int32_t src = a.inv ? a.inv[caller_src] : caller_src;
   BfsCtl* c = a.ctl;
   const int d = a.deg[src];
   const int cl = cls_of(d, a);
   a.q[0][cl][0] = src;
-  c->src = src;
+  c->src = caller_src;
   c->depth = reinterpret_cast<int32_t*>(depth);  // the level kernels of this DT cast it back
   c->parent = parent;
   c->level = 0;
@@ -284,8 +310,9 @@ __device__ void init_state(const LevelArgs& a, int32_t src, DT* depth, int32_t* 
 }
 
 // The first kernel of a traversal: depths unreached but depth[src] = 0,
-// parents -1 but parent[src] = src, the visited and frontier-0 bitmaps holding
-// src alone, hub tables clear, and the loop state (one thread). The level
+// parents -1 but parent[src] = src (caller ids), the visited and frontier-0
+// bitmaps (traversal ids) holding src alone, hub tables clear, and the loop
+// state (one thread). The level
 // kernels are instantiated for int32 depths and for the reference's byte
 // depths (DT = uint8_t: written directly, no conversion pass).
 template <class DT>
@@ -294,8 +321,9 @@ __global__ void __launch_bounds__(BT) k_reset(LevelArgs a, int32_t src, DT* dept
   if (tid == 0) init_state(a, src, depth, parent);
   fill_unreached(depth, a.V, tid, nth, src);
   if (parent) fill_neg1(parent, a.V, tid, nth, src, src);
-  const int64_t W = (a.V + 31) >> 5, sw = src >> 5;
-  const uint32_t sb = 1u << (src & 31);
+  const int32_t isrc = a.inv ? __ldg(a.inv + src) : src;
+  const int64_t W = (a.V + 31) >> 5, sw = isrc >> 5;
+  const uint32_t sb = 1u << (isrc & 31);
   for (int64_t i = tid; i < W; i += nth) {
     const uint32_t x = i == sw ? sb : 0u;
     a.vis[i] = x;
@@ -309,18 +337,23 @@ __global__ void __launch_bounds__(BT) k_reset(LevelArgs a, int32_t src, DT* dept
 }
 
 // ------------------------------------------------------------ top-down ----
-template <class DT>
-__device__ __forceinline__ void td_visit(const LevelArgs& a, BfsCtl* c, int v, int u, bool valid, int ln,
-                                         DT* depth, int32_t* parent, uint32_t* fbn) {
+// Claims v for frontier vertex u. The depth is written by the inspector, which
+// goes over the claimed vertices anyway: the caller's id it is stored under is
+// one more dependent read, kept out of this loop.
+__device__ __forceinline__ void td_visit(const LevelArgs& a, BfsCtl* c, int v, int u, bool valid, int32_t* parent,
+                                         uint32_t* fbn) {
   bool mine = false;
   if (valid) {
     const uint32_t w = (uint32_t)v >> 5, b = 1u << (v & 31);
-    if (!(ld_cg(a.vis + w) & b)) {
+    // A look through L1: the hubs, which most edges lead to, share a few
+    // words, and reading those in L2 for every edge serialises there (R-MAT
+    // s22 all top-down: 1.77 ms, 0.98 ms through L1). A stale word only costs
+    // the atomic, which decides.
+    if (!(__ldca(a.vis + w) & b)) {
       const uint32_t old = atomicOr(a.vis + w, b);
       if (!(old & b)) {
         mine = true;
-        depth[v] = (DT)ln;
-        if (parent) parent[v] = u;
+        if (parent) parent[out_id(a, v)] = out_id(a, u);
         red_or(fbn + w, b);
       }
     }
@@ -336,8 +369,7 @@ __device__ __forceinline__ void td_visit(const LevelArgs& a, BfsCtl* c, int v, i
   }
 }
 
-template <class DT>
-__device__ void td_expand(const LevelArgs& a, BfsCtl* c, int L, DT* depth, int32_t* parent) {
+__device__ void td_expand(const LevelArgs& a, BfsCtl* c, int L, int32_t* parent) {
   const int qc = c->qcur;
   const int ns = c->n_q[0], nm = c->n_q[1], nl = c->n_q[2], nch = c->n_chunks;
   const int32_t* __restrict__ qs = a.q[qc][0];
@@ -348,7 +380,6 @@ __device__ void td_expand(const LevelArgs& a, BfsCtl* c, int L, DT* depth, int32
   const int lane = threadIdx.x & 31;
   const int gw = (int)((blockIdx.x * (int64_t)BT + threadIdx.x) >> 5);
   const int nw = (int)(((int64_t)gridDim.x * BT) >> 5);
-  const int ln = L + 1;
 
   // Large tier: one CTA per chunk of a high-degree vertex.
   __shared__ int s_vi;
@@ -371,7 +402,7 @@ __device__ void td_expand(const LevelArgs& a, BfsCtl* c, int L, DT* depth, int32
       const int64_t e = e0 + threadIdx.x;
       const bool valid = e < end;
       const int v = valid ? __ldg(a.adj + e) : 0;
-      td_visit(a, c, v, u, valid, ln, depth, parent, fbn);
+      td_visit(a, c, v, u, valid, parent, fbn);
     }
   }
   // Mid tier: one warp per vertex.
@@ -382,7 +413,7 @@ __device__ void td_expand(const LevelArgs& a, BfsCtl* c, int L, DT* depth, int32
       const int64_t e = e0 + lane;
       const bool valid = e < end;
       const int v = valid ? __ldg(a.adj + e) : 0;
-      td_visit(a, c, v, u, valid, ln, depth, parent, fbn);
+      td_visit(a, c, v, u, valid, parent, fbn);
     }
   }
   // Small tier: a warp gathers the adjacency lists of 32 vertices and
@@ -418,7 +449,7 @@ __device__ void td_expand(const LevelArgs& a, BfsCtl* c, int L, DT* depth, int32
       const int ej = __shfl_sync(FULL, excl, j);
       const int uj = __shfl_sync(FULL, u, j);
       const int v = valid ? __ldg(a.adj + sj + (k - ej)) : 0;
-      td_visit(a, c, v, uj, valid, ln, depth, parent, fbn);
+      td_visit(a, c, v, uj, valid, parent, fbn);
     }
   }
 }
@@ -460,7 +491,7 @@ __device__ void bu_expand(const LevelArgs& a, BfsCtl* c, int L, DT* depth, int32
   const int64_t gtid = blockIdx.x * (int64_t)BT + threadIdx.x, nth = (int64_t)gridDim.x * BT;
   const int64_t gw = gtid >> 5, nw = nth >> 5;
   const int ln = L + 1;
-  const int64_t W = (a.V + 31) >> 5;
+  const int64_t W = (a.n_active + 31) >> 5;
   unsigned long long my_n = 0, my_m = 0;
   // A warp owns one status word: 32 consecutive vertex ids.
   for (int64_t wi = gw; wi < W; wi += nw) {
@@ -476,11 +507,12 @@ __device__ void bu_expand(const LevelArgs& a, BfsCtl* c, int L, DT* depth, int32
     if (todo) {
       // The lead neighbour (the highest-degree one) is the parent of most
       // vertices found: the first 4 neighbours are read coalesced, beside the
-      // row offsets, and the first is probed before anything else, whatever
-      // the vertex's degree.
-      ld = __ldg(a.lead + v);
-      e0 = a.off[v];
-      d = (int)(a.off[v + 1] - e0);
+      // degrees, and the first is probed before anything else, whatever
+      // the vertex's degree. These arrays are read once a level and far larger
+      // than L2 at s24: marked as streaming, they leave it to the bitmaps and
+      // the depths (s24 median 0.418 -> 0.367 ms).
+      ld = __ldcs(a.lead + v);
+      d = __ldcs(a.deg + v);
       if (is_front(ld.x)) { found = true; pu = ld.x; }
     }
     if (todo && !found && d > 1) {
@@ -490,6 +522,7 @@ __device__ void bu_expand(const LevelArgs& a, BfsCtl* c, int L, DT* depth, int32
       else if (f2) found = true, pu = ld.z;
       else if (f3) found = true, pu = ld.w;
     }
+    if (todo && !found && d > 4) e0 = __ldcs(a.off + v);
     if (todo && !found && d < a.small_max) {
       // A light vertex that keeps scanning is usually not adjacent to the
       // frontier at all: it checks BU_ILP neighbours per step, their reads
@@ -506,7 +539,7 @@ __device__ void bu_expand(const LevelArgs& a, BfsCtl* c, int L, DT* depth, int32
           if (!found && f[i]) { found = true; pu = u[i]; }
       }
     }
-    unsigned heavy = __ballot_sync(FULL, todo && !found && d >= a.small_max);
+    unsigned heavy = __ballot_sync(FULL, todo && !found && d > 4 && d >= a.small_max);
     while (heavy) {
       const int j = __ffs(heavy) - 1;
       heavy &= heavy - 1;
@@ -522,8 +555,9 @@ __device__ void bu_expand(const LevelArgs& a, BfsCtl* c, int L, DT* depth, int32
       if (lane == j && hit >= 0) { found = true; pu = hit; }
     }
     if (found) {
-      depth[v] = (DT)ln;
-      if (parent) parent[v] = pu;
+      const int o = a.perm ? __ldcs(a.perm + v) : (int)v;
+      st_keep(depth + o, (DT)ln);
+      if (parent) parent[o] = out_id(a, pu);
       my_n++;
       my_m += (unsigned long long)d;
       hub_insert(a, hub_next, (int)v, d);
@@ -583,7 +617,7 @@ __global__ void __launch_bounds__(BT, 8) k_expand(LevelArgs a) {
   if (c->done || c->skip) return;
   const int L = c->level;
   DT* depth = reinterpret_cast<DT*>(c->depth);
-  if (c->dir == TD) td_expand(a, c, L, depth, c->parent);
+  if (c->dir == TD) td_expand(a, c, L, c->parent);
   else bu_expand(a, c, L, depth, c->parent, s_hub, s_red);
 }
 
@@ -622,6 +656,7 @@ struct QueueOut {
   }
 };
 
+template <class DT>
 __global__ void __launch_bounds__(BT) k_inspect(LevelArgs a) {
   __shared__ uint32_t s_scan[32 * KS];
   __shared__ uint32_t s_excl[KS];
@@ -662,7 +697,8 @@ __global__ void __launch_bounds__(BT) k_inspect(LevelArgs a) {
       const int32_t* qk = a.q[qcur][k];
       for (int64_t i = gtid; i < c->n_q[k]; i += nth) fbo[(uint32_t)qk[i] >> 5] = 0;
     }
-    // Classify the raw next frontier into q[qcur^1].
+    // Classify the raw next frontier into q[qcur^1], and write its depths.
+    DT* depth = reinterpret_cast<DT*>(c->depth);
     const int64_t n = c->n_raw;
     const uint32_t ntiles = (uint32_t)((n + TILE - 1) / TILE);
     unsigned long long* hub_next = a.hub[(L + 1) & 1];
@@ -671,13 +707,18 @@ __global__ void __launch_bounds__(BT) k_inspect(LevelArgs a) {
       if (tile >= ntiles) break;
       int32_t v[IPT];
       load_tile(a.raw, (int64_t)tile * TILE, n, v);
-      int dg[IPT], cl[IPT];
+      int dg[IPT], cl[IPT], oid[IPT];
       uint32_t cnt[4] = {0, 0, 0, 0};
 #pragma unroll
+      for (int j = 0; j < IPT; ++j) {  // both reads of every item in flight together
+        dg[j] = v[j] >= 0 ? __ldg(a.deg + v[j]) : 0;
+        oid[j] = v[j] >= 0 ? out_id(a, v[j]) : 0;
+      }
+#pragma unroll
       for (int j = 0; j < IPT; ++j) {
-        dg[j] = v[j] >= 0 ? a.deg[v[j]] : 0;
         cl[j] = v[j] >= 0 ? cls_of(dg[j], a) : -1;
         if (cl[j] >= 0) {
+          depth[oid[j]] = (DT)(L + 1);
           cnt[cl[j]]++;
           my_m += dg[j];
           my_maxd = max(my_maxd, (uint32_t)dg[j]);
@@ -746,6 +787,8 @@ __global__ void __launch_bounds__(BT) k_inspect(LevelArgs a) {
       // Hand over to TD: classify the frontier bitmap (ascending ids) into
       // q[qcur^1]. A tile is BT*WPT words, WPT consecutive words per thread
       // (the frontier is sparse here: few look-back tiles, not few words).
+      // A bottom-up level finds vertices with rows only: ids below n_active.
+      const int64_t W = (a.n_active + 31) >> 5;
       const uint32_t ntiles = (uint32_t)((W + BT * WPT - 1) / (BT * WPT));
       while (true) {
         const uint32_t tile = acquire_tile(c, &s_tile);
@@ -975,6 +1018,10 @@ __device__ __forceinline__ void narrow_append(const LevelArgs& a, BfsCtl* c, boo
 //    shared-memory entries) and arrives.
 // Every CTA takes the same decisions from the same counts, so all reach the
 // same barriers; there are no spin waits.
+// A vertex's depth is written when its entry is expanded, not when it is
+// claimed: the caller's id it is stored under is read beside the entry's row,
+// off the level's critical path (a frontier handed over gets its depths from
+// the inspector).
 template <class DT>
 __global__ void __launch_bounds__(NT, 1) k_narrow(LevelArgs a) {
   extern __shared__ int4 s_q[];  // [2][NQCAP]
@@ -1058,7 +1105,6 @@ __global__ void __launch_bounds__(NT, 1) k_narrow(LevelArgs a) {
 
     if (!coord) {
       const NarrowOut o{s_q + nxt * NQCAP, &s_cnt[nxt], &s_m[nxt], &s_flag[nxt], spill};
-      const int ln = L + 1;
       int k = (int)((n_all + nwt - 1) / nwt);
       if (k > 32) k = 32;
       for (int first = gw * k; first < (int)n_all; first += nwt * k) {
@@ -1071,13 +1117,14 @@ __global__ void __launch_bounds__(NT, 1) k_narrow(LevelArgs a) {
           if (r + step <= nc - 1 && (uint32_t)i >= e_end) r += step;
         }
         const uint32_t base = __shfl_sync(FULL, incl, (r + 31) & 31);  // end of CTA r-1 (unused for r = 0)
-        int u = -1, d = 0;
+        int u = -1, d = 0, out = -1;
         int64_t st = 0;
         if (lane < k && i < (int)n_all) {
           const int4 e = *(cl.map_shared_rank(s_q + cur * NQCAP, r) + (i - (r ? (int)base : 0)));
           u = e.x;
           d = e.y;
           st = (int64_t)(((uint64_t)(uint32_t)e.w << 32) | (uint32_t)e.z);
+          out = out_id(a, u);
         }
         int dincl = d;
 #pragma unroll
@@ -1129,8 +1176,7 @@ __global__ void __launch_bounds__(NT, 1) k_narrow(LevelArgs a) {
                 // the next level walks this row: start its first sector towards L2 now
                 // (an empty row may start one past the array: nothing to fetch)
                 if (o1 > o0) asm volatile("prefetch.global.L2 [%0];" ::"l"(a.adj + o0));
-                depth[x] = (DT)ln;
-                if (parent) parent[x] = uj[q];
+                if (parent) parent[out_id(a, x)] = out_id(a, uj[q]);
               }
             }
           }
@@ -1138,6 +1184,7 @@ __global__ void __launch_bounds__(NT, 1) k_narrow(LevelArgs a) {
           for (int q = 0; q < NROUND; ++q)
             if (r0 + 32 * q < total) narrow_append(a, c, mine[q], v[q], vd[q], vst[q], o);
         }
+        if (out >= 0) depth[out] = (DT)L;
       }
       bar1_arrive();  // this warp's appends are complete
       cluster_arrive_relaxed();
@@ -1335,7 +1382,7 @@ static int build_graph(ent_graph* g, BfsWorkspace* w) {
     bp.kernelParams = largs;
     cudaGraphNode_t n_expand, n_inspect;
     ENT_CUDA(cudaGraphAddKernelNode(&n_expand, body, prev ? &prev : nullptr, prev ? 1 : 0, &bp));
-    bp.func = (void*)k_inspect;
+    bp.func = (void*)k_inspect<DT>;
     bp.gridDim = dim3(w->grid_inspect);
     bp.sharedMemBytes = 0;
     ENT_CUDA(cudaGraphAddKernelNode(&n_inspect, body, &n_expand, 1, &bp));
@@ -1442,11 +1489,14 @@ static int create_workspace(ent_graph* g, BfsWorkspace** out, bool force_graph =
   LevelArgs& a = w->args;
   memset(&a, 0, sizeof(a));
   a.ctl = w->ctl;
-  a.off = g->off;
+  a.off = g->toff;
   a.adj = g->trav;
   a.lead = g->lead;
   a.deg = g->deg;
   a.active = g->active;
+  a.perm = g->perm;
+  a.inv = g->inv;
+  a.n_active = g->n_active;
   a.V = V;
   a.E = g->E;
   a.vis = (uint32_t*)p; p += sz_bits;
@@ -1476,7 +1526,7 @@ static int create_workspace(ent_graph* g, BfsWorkspace** out, bool force_graph =
   w->smem_expand = sizeof(int32_t) * (hub > 0 ? hub : 1);
   int occ_e = 0, occ_i = 0;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_e, k_expand<int32_t>, BT, w->smem_expand);
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_i, k_inspect, BT, 0);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_i, k_inspect<int32_t>, BT, 0);
   if (occ_e < 1) occ_e = 1;
   if (occ_i < 1) occ_i = 1;
   if (o.blocks_per_sm > 0) occ_e = std::min(occ_e, o.blocks_per_sm);
@@ -1574,7 +1624,7 @@ static int run_bfs_typed(ent_graph* g, int32_t src, DT* depth, int32_t* parent, 
     int32_t* flags_h = &w->ctl_h->done;  // done, narrow
     for (int64_t it = 0;; ++it) {
       k_expand<DT><<<w->grid_expand, BT, w->smem_expand, s>>>(la);
-      k_inspect<<<w->grid_inspect, BT, 0, s>>>(la);
+      k_inspect<DT><<<w->grid_inspect, BT, 0, s>>>(la);
       g_kernel_launches += 2;
       ENT_CUDA(cudaGetLastError());
       ENT_CUDA(cudaMemcpyAsync(flags_h, &w->ctl->done, 2 * sizeof(int32_t), cudaMemcpyDeviceToHost, s));
@@ -1853,7 +1903,7 @@ int ent_bfs_trace(ent_graph* g, int32_t src, ent_level_trace* out, int32_t max_l
     ENT_CUDA(cudaEventRecord(e[0], s));
     k_expand<int32_t><<<w->grid_expand, BT, w->smem_expand, s>>>(la);
     ENT_CUDA(cudaEventRecord(e[1], s));
-    k_inspect<<<w->grid_inspect, BT, 0, s>>>(la);
+    k_inspect<int32_t><<<w->grid_inspect, BT, 0, s>>>(la);
     ENT_CUDA(cudaEventRecord(e[2], s));
     g_kernel_launches += 2;
     ENT_CUDA(cudaGetLastError());

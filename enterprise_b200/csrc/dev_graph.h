@@ -17,12 +17,21 @@ void destroy_deep_lanes(DeepLanes* l);
 // Device memory layout of one graph (all on `device`):
 //   off  int64[V+1]   row offsets (reference strt_pos + adj_card, allocator.cuh:107-114)
 //   adj  int32[E]     column ids, rows ascending (reference adj_list, allocator.cuh:116-120)
+// and the traversal's own arrays (one slab), in traversal ids: vertices by
+// descending degree, ties by caller id. The vertices without a row come last,
+// so a bottom-up sweep covers the first n_active ids without idle lanes; a
+// warp's 32 vertices have (nearly) equal degrees and adjacent rows; and the
+// hubs, which most probes hit, share a few cache lines of every per-vertex
+// array. Caller ids appear only where sources come in and results go out.
+//   perm int32[V]     caller id of each traversal id (null: caller order, when
+//                     E >= 2^31 or E == 0; toff and trav are then off and adj)
+//   inv  int32[V]     traversal id of each caller id
+//   toff int64[V+1]   row offsets
+//   trav int32[E]     the rows, ascending: the highest-degree neighbours first.
+//                     A bottom-up check then meets the likeliest parent, a hub,
+//                     first.
 //   deg  int32[V]     degrees, read by the classifier (reference adj_card)
 //   active uint32[V/32] bit v set iff deg(v) > 0 (bottom-up skips isolated vertices)
-//   trav int32[E]     the rows of adj re-ordered by descending neighbour degree
-//                     (ties by id): the traversal's adjacency. A bottom-up check
-//                     then meets the likeliest parent, a hub, first. Equal to
-//                     adj when E >= 2^31 (no re-ordering).
 //   lead int4[V]      first 4 entries of each trav row (the highest-degree
 //                     neighbours), -1 past the row's end: a bottom-up sweep
 //                     reads them coalesced instead of a random row sector per
@@ -33,10 +42,15 @@ struct ent_graph {
   int64_t V = 0, E = 0;
   int64_t* off = nullptr;
   int32_t* adj = nullptr;
+  void* slab = nullptr;  // the arrays below (toff and trav may alias off and adj)
+  int32_t* perm = nullptr;
+  int32_t* inv = nullptr;
+  int64_t* toff = nullptr;
+  int32_t* trav = nullptr;
   int32_t* deg = nullptr;
   uint32_t* active = nullptr;
-  int32_t* trav = nullptr;
   int4* lead = nullptr;
+  int64_t n_active = 0;  // vertices with a row are traversal ids [0, n_active); V in caller order
   cudaStream_t stream = nullptr;
   ent_bfs_opts opts;
   std::mutex mu;

@@ -19,17 +19,11 @@ RmatParams make_rmat_params(int scale, int ef, double a, double b, double c, uin
 GridParams make_grid_params(int64_t w, int64_t h, double drop, uint64_t seed);
 ErParams make_er_params(int64_t n, double mean_degree, uint64_t seed);
 
-__global__ void k_degrees(const int64_t* __restrict__ off, int32_t* __restrict__ deg, int64_t V) {
-  for (int64_t v = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; v < V; v += (int64_t)gridDim.x * blockDim.x)
-    deg[v] = (int32_t)(off[v + 1] - off[v]);
-}
-
 int graph_alloc(ent_graph* g, int64_t V, int64_t E) {
   g->V = V;
   g->E = E;
   ENT_CUDA(cudaMalloc(&g->off, sizeof(int64_t) * (V + 1)));
   ENT_CUDA(cudaMalloc(&g->adj, sizeof(int32_t) * (E > 0 ? E : 1)));
-  ENT_CUDA(cudaMalloc(&g->deg, sizeof(int32_t) * V));
   return ENT_OK;
 }
 
@@ -45,18 +39,64 @@ __global__ void k_active_bits(const int32_t* __restrict__ deg, uint32_t* __restr
   }
 }
 
-// Key that orders a row by descending neighbour degree, then ascending id.
-__global__ void k_degree_keys(const int32_t* __restrict__ adj, const int32_t* __restrict__ deg, int64_t E,
-                              unsigned long long* __restrict__ keys) {
-  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < E; e += (int64_t)gridDim.x * blockDim.x) {
-    const int32_t u = adj[e];
-    keys[e] = ((unsigned long long)(uint32_t)(0x7fffffff - deg[u]) << 32) | (uint32_t)u;
+// Degrees in caller order, and the sort keys that order vertices by descending
+// degree (ties keep ascending ids: the sort is stable).
+__global__ void k_degrees(const int64_t* __restrict__ off, int64_t V, int32_t* __restrict__ deg,
+                          uint32_t* __restrict__ key, int32_t* __restrict__ id) {
+  for (int64_t v = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; v < V; v += (int64_t)gridDim.x * blockDim.x) {
+    const int32_t d = (int32_t)(off[v + 1] - off[v]);
+    if (deg) deg[v] = d;
+    if (key) {
+      key[v] = ~(uint32_t)d;
+      id[v] = (int32_t)v;
+    }
   }
 }
 
-__global__ void k_keys_to_ids(const unsigned long long* __restrict__ keys, int64_t E, int32_t* __restrict__ out) {
-  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < E; e += (int64_t)gridDim.x * blockDim.x)
-    out[e] = (int32_t)(uint32_t)keys[e];
+// From the sorted keys: degrees in traversal order, the inverse labelling, and
+// the number of vertices with a row (the first n_active traversal ids).
+__global__ void k_labels(const uint32_t* __restrict__ key, const int32_t* __restrict__ perm, int64_t V,
+                         int32_t* __restrict__ deg, int32_t* __restrict__ inv, int64_t* __restrict__ n_active) {
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < V; i += (int64_t)gridDim.x * blockDim.x) {
+    const int32_t d = (int32_t)~key[i];
+    deg[i] = d;
+    inv[perm[i]] = (int32_t)i;
+    if (d > 0 && (i == V - 1 || ~key[i + 1] == 0)) *n_active = i + 1;
+  }
+}
+
+// The rows in traversal order with traversal ids, still in caller column
+// order. A warp takes ROW_CHUNK consecutive entries of the output, so hubs
+// are split over warps: the chunk's first and last rows are searched once, and
+// each lane's entry then searches only between them (no step inside a hub).
+constexpr int ROW_CHUNK = 1024;
+__global__ void __launch_bounds__(256) k_relabel_rows(const int64_t* __restrict__ off, const int32_t* __restrict__ adj,
+                                                      const int64_t* __restrict__ toff,
+                                                      const int32_t* __restrict__ perm,
+                                                      const int32_t* __restrict__ inv, int64_t V, int64_t E,
+                                                      int32_t* __restrict__ out) {
+  const int lane = threadIdx.x & 31;
+  const int64_t gw = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
+  const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
+  // the row holding entry e lies in [lo, hi]
+  const auto row_of = [&](int64_t e, int64_t lo, int64_t hi) {
+    while (lo < hi) {
+      const int64_t mid = (lo + hi + 1) >> 1;
+      if (toff[mid] <= e) lo = mid;
+      else hi = mid - 1;
+    }
+    return lo;
+  };
+  for (int64_t c0 = gw * ROW_CHUNK; c0 < E; c0 += nw * ROW_CHUNK) {
+    const int64_t c1 = min(E, c0 + ROW_CHUNK);
+    // lane 0 searches the first row, lane 1 the last
+    const int64_t mine = row_of(lane == 0 ? c0 : c1 - 1, 0, V - 1);
+    const int64_t r0 = __shfl_sync(0xffffffffu, mine, 0), r1 = __shfl_sync(0xffffffffu, mine, 1);
+    for (int64_t e = c0 + lane; e < c1; e += 32) {
+      const int64_t r = row_of(e, r0, r1);
+      out[e] = inv[adj[off[perm[r]] + (e - toff[r])]];
+    }
+  }
 }
 
 // lead[v] = the first 4 neighbours of v in the traversal adjacency (its
@@ -70,61 +110,114 @@ __global__ void k_lead(const int64_t* __restrict__ off, const int32_t* __restric
   }
 }
 
-// Builds the traversal adjacency (rows by descending neighbour degree).
-static int build_traversal_order(ent_graph* g) {
-  const int64_t E = g->E, V = g->V;
-  if (E == 0 || E > 0x7fffffffll || V > 0x7ffffffell) {
-    g->trav = g->adj;  // no re-ordering: traverse the canonical rows
-    return ENT_OK;
-  }
-  ENT_CUDA(cudaMalloc(&g->trav, sizeof(int32_t) * E));
-  unsigned long long *k0 = nullptr, *k1 = nullptr;
-  void* tmp = nullptr;
-  size_t tmp_bytes = 0;
-  cudaError_t e = cudaMalloc(&k0, sizeof(unsigned long long) * E);
-  if (e == cudaSuccess) e = cudaMalloc(&k1, sizeof(unsigned long long) * E);
+// Whether a graph of this size gets its own traversal order (the sorts take
+// 32-bit counts).
+static bool relabelled(int64_t V, int64_t E) { return E > 0 && E <= 0x7fffffffll && V <= 0x7ffffffell; }
+
+// Bytes of the traversal arrays (one slab): degrees, active bits and lead
+// entries, and with an order of its own, offsets, rows and the labelling.
+struct TravLayout {
+  size_t toff, deg, perm, inv, active, lead, trav, total;
+};
+static TravLayout trav_layout(int64_t V, int64_t E) {
+  TravLayout l{};
+  size_t at = 0;
+  const auto put = [&](size_t bytes) {
+    const size_t p = at;
+    at = (at + bytes + 255) & ~(size_t)255;
+    return p;
+  };
+  const bool own = relabelled(V, E);
+  l.lead = put(sizeof(int4) * V);
+  l.toff = put(own ? sizeof(int64_t) * (V + 1) : 0);
+  l.deg = put(sizeof(int32_t) * V);
+  l.perm = put(own ? sizeof(int32_t) * V : 0);
+  l.inv = put(own ? sizeof(int32_t) * V : 0);
+  l.active = put(sizeof(uint32_t) * (((V + 31) >> 5) + 1));
+  l.trav = put(own ? sizeof(int32_t) * E : 0);
+  l.total = at;
+  return l;
+}
+
+// Builds the traversal order: vertices by descending degree, rows by ascending
+// traversal id (that is, by descending neighbour degree).
+static cudaError_t build_traversal_order(ent_graph* g) {
+  const int64_t V = g->V, E = g->E;
   const int blocks = g->num_sms * 16;
-  if (e == cudaSuccess) {
-    k_degree_keys<<<blocks, 256, 0, g->stream>>>(g->adj, g->deg, E, k0);
-    g_kernel_launches++;
-    e = cub::DeviceSegmentedSort::SortKeys(nullptr, tmp_bytes, k0, k1, (int)E, (int)V, g->off, g->off + 1,
-                                           g->stream);
-  }
-  if (e == cudaSuccess) e = cudaMalloc(&tmp, tmp_bytes);
+  cudaStream_t s = g->stream;
+  size_t t_sort = 0, t_scan = 0, t_seg = 0;
+  uint32_t *nk = nullptr, *nk2 = nullptr;
+  int32_t *ni = nullptr, *ni2 = nullptr;
+  cudaError_t e = cub::DeviceRadixSort::SortPairs(nullptr, t_sort, nk, nk2, ni, ni2, V, 0, 32, s);
+  if (e == cudaSuccess) e = cub::DeviceScan::InclusiveSum(nullptr, t_scan, g->deg, g->toff + 1, V, s);
   if (e == cudaSuccess)
-    e = cub::DeviceSegmentedSort::SortKeys(tmp, tmp_bytes, k0, k1, (int)E, (int)V, g->off, g->off + 1, g->stream);
+    e = cub::DeviceSegmentedSort::SortKeys(nullptr, t_seg, ni, ni2, (int)E, (int)V, g->toff, g->toff + 1, s);
+  if (e != cudaSuccess) return e;
+  const auto al = [](size_t x) { return (x + 255) & ~(size_t)255; };
+  const size_t sz_v = al(sizeof(int32_t) * V);
+  // the vertex sort's buffers and the row sort's share their memory
+  const size_t sz_a = 3 * sz_v, sz_b = al(sizeof(int32_t) * E);
+  const size_t t_cub = al(std::max(std::max(t_sort, t_scan), t_seg));
+  char* tmp = nullptr;
+  e = cudaMalloc(&tmp, 256 + std::max(sz_a, sz_b) + t_cub);
+  if (e != cudaSuccess) return e;
+  int64_t* n_active = (int64_t*)tmp;
+  uint32_t* key = (uint32_t*)(tmp + 256);
+  uint32_t* key2 = (uint32_t*)(tmp + 256 + sz_v);
+  int32_t* id = (int32_t*)(tmp + 256 + 2 * sz_v);
+  int32_t* rows = (int32_t*)(tmp + 256);
+  void* cub_tmp = tmp + 256 + std::max(sz_a, sz_b);
+  k_degrees<<<blocks, 256, 0, s>>>(g->off, V, nullptr, key, id);
+  e = cub::DeviceRadixSort::SortPairs(cub_tmp, t_sort, key, key2, id, g->perm, V, 0, 32, s);
   if (e == cudaSuccess) {
-    k_keys_to_ids<<<blocks, 256, 0, g->stream>>>(k1, E, g->trav);
-    g_kernel_launches++;
-    e = cudaStreamSynchronize(g->stream);
+    k_labels<<<blocks, 256, 0, s>>>(key2, g->perm, V, g->deg, g->inv, n_active);
+    e = cudaMemsetAsync(g->toff, 0, sizeof(int64_t), s);
   }
-  if (k0) cudaFree(k0);
-  if (k1) cudaFree(k1);
-  if (tmp) cudaFree(tmp);
-  if (e != cudaSuccess)
-    return fail(e == cudaErrorMemoryAllocation ? ENT_ERR_OOM : ENT_ERR_CUDA, "traversal order build failed: %s",
-                cudaGetErrorString(e));
-  return ENT_OK;
+  if (e == cudaSuccess) e = cub::DeviceScan::InclusiveSum(cub_tmp, t_scan, g->deg, g->toff + 1, V, s);
+  if (e == cudaSuccess) {
+    k_relabel_rows<<<blocks, 256, 0, s>>>(g->off, g->adj, g->toff, g->perm, g->inv, V, E, rows);
+    e = cub::DeviceSegmentedSort::SortKeys(cub_tmp, t_seg, rows, g->trav, (int)E, (int)V, g->toff, g->toff + 1, s);
+  }
+  g_kernel_launches += 3;
+  if (e == cudaSuccess) e = cudaMemcpyAsync(&g->n_active, n_active, sizeof(int64_t), cudaMemcpyDeviceToHost, s);
+  const cudaError_t e2 = cudaStreamSynchronize(s);
+  cudaFree(tmp);
+  return e != cudaSuccess ? e : e2;
 }
 
 int graph_finish(ent_graph* g) {
   ENT_CUDA(cudaDeviceGetAttribute(&g->num_sms, cudaDevAttrMultiProcessorCount, g->device));
   if (!g->stream) ENT_CUDA(cudaStreamCreateWithFlags(&g->stream, cudaStreamNonBlocking));
-  int blocks = (int)std::min<int64_t>((g->V + 255) / 256, (int64_t)g->num_sms * 16);
-  k_degrees<<<blocks, 256, 0, g->stream>>>(g->off, g->deg, g->V);
-  g_kernel_launches++;
-  ENT_CUDA(cudaGetLastError());
-  const int64_t W = (g->V + 31) >> 5;
-  ENT_CUDA(cudaMalloc(&g->active, sizeof(uint32_t) * (W + 1)));
+  const int64_t V = g->V, E = g->E;
+  const TravLayout l = trav_layout(V, E);
+  ENT_CUDA(cudaMalloc(&g->slab, l.total));
+  char* p = (char*)g->slab;
+  g->lead = (int4*)(p + l.lead);
+  g->deg = (int32_t*)(p + l.deg);
+  g->active = (uint32_t*)(p + l.active);
+  const int blocks = (int)std::min<int64_t>((V + 255) / 256, (int64_t)g->num_sms * 16);
+  if (relabelled(V, E)) {
+    g->toff = (int64_t*)(p + l.toff);
+    g->perm = (int32_t*)(p + l.perm);
+    g->inv = (int32_t*)(p + l.inv);
+    g->trav = (int32_t*)(p + l.trav);
+    const cudaError_t e = build_traversal_order(g);
+    if (e != cudaSuccess)
+      return fail(e == cudaErrorMemoryAllocation ? ENT_ERR_OOM : ENT_ERR_CUDA, "traversal order build failed: %s",
+                  cudaGetErrorString(e));
+  } else {  // caller order: the canonical rows
+    g->toff = g->off;
+    g->trav = g->adj;
+    g->n_active = V;
+    k_degrees<<<blocks, 256, 0, g->stream>>>(g->off, V, g->deg, nullptr, nullptr);
+    g_kernel_launches++;
+    ENT_CUDA(cudaGetLastError());
+  }
+  const int64_t W = (V + 31) >> 5;
   k_active_bits<<<(int)std::min<int64_t>((W + 255) / 256, (int64_t)g->num_sms * 16), 256, 0, g->stream>>>(
-      g->deg, g->active, g->V);
-  g_kernel_launches++;
-  ENT_CUDA(cudaGetLastError());
-  int rc = build_traversal_order(g);
-  if (rc != ENT_OK) return rc;
-  ENT_CUDA(cudaMalloc(&g->lead, sizeof(int4) * (g->V > 0 ? g->V : 1)));
-  k_lead<<<blocks, 256, 0, g->stream>>>(g->off, g->trav, g->V, g->lead);
-  g_kernel_launches++;
+      g->deg, g->active, V);
+  k_lead<<<blocks, 256, 0, g->stream>>>(g->toff, g->trav, V, g->lead);
+  g_kernel_launches += 2;
   ENT_CUDA(cudaGetLastError());
   ENT_CUDA(cudaStreamSynchronize(g->stream));
   ent_bfs_opts_default(&g->opts);
@@ -138,12 +231,9 @@ static void graph_free(ent_graph* g) {
   if (g->bws) destroy_batch_workspace(g->bws);
   if (g->lanes) destroy_deep_lanes(g->lanes);
   if (g->stage) cudaFree(g->stage);
-  if (g->trav && g->trav != g->adj) cudaFree(g->trav);
-  if (g->active) cudaFree(g->active);
-  if (g->lead) cudaFree(g->lead);
+  if (g->slab) cudaFree(g->slab);
   if (g->off) cudaFree(g->off);
   if (g->adj) cudaFree(g->adj);
-  if (g->deg) cudaFree(g->deg);
   if (g->stream) cudaStreamDestroy(g->stream);
   delete g;
 }
@@ -500,10 +590,7 @@ int64_t ent_graph_edge_count(const ent_graph* g) { return g ? g->E : -1; }
 int32_t ent_graph_device(const ent_graph* g) { return g ? g->device : -1; }
 int64_t ent_graph_device_bytes(const ent_graph* g) {
   if (!g) return -1;
-  const int64_t V = g->V, E = g->E, W = (V + 31) >> 5;
-  int64_t b = 8 * (V + 1) + 4 * std::max<int64_t>(E, 1) + 4 * V + 4 * (W + 1) + 16 * std::max<int64_t>(V, 1);
-  if (g->trav && g->trav != g->adj) b += 4 * E;
-  return b;
+  return 8 * (g->V + 1) + 4 * std::max<int64_t>(g->E, 1) + (int64_t)trav_layout(g->V, g->E).total;
 }
 
 int ent_device_alloc(int32_t gpu, size_t bytes, void** out) {
