@@ -11,7 +11,8 @@
 //   X    uint64[V][W]      visited bits
 //   log  uint64[K][V][W]   ring of K levels: log[L-base][v] = bits found at level L
 //   jf   int32[2][V]       joint frontier (vertices with any new bit), ping-pong
-//   heavy int32[2][V]      joint-frontier vertices of degree >= opts.batch_heavy
+//   heavy int2[2][]        chunks (vertex, index) of the joint-frontier vertices of
+//                          degree >= min(opts.batch_heavy, TD_CHUNK)
 //   smask uint16[V]        which log slots hold bits of the vertex: the flush
 //                          reads and clears only those
 //   done bit per vertex    every source has visited it (bottom-up skips it)
@@ -45,6 +46,7 @@ constexpr int KMAX = 16;       // log slots (levels per flush window)
 constexpr int LOOP_UNROLL = 2; // level-loop bodies per while-node iteration of the CUDA-graph loop
 constexpr int SEED_THREADS = 1024;  // the one seeding CTA: a multi-graph plan seeds thousands of entries
 constexpr int WMAX = 32;       // words per vertex per launch (2048 sources)
+constexpr int TD_CHUNK = 512;  // row entries of a heavy vertex that one warp takes, top-down
 
 struct BatchCtl {
   int32_t level;     // level of the frontier being expanded
@@ -101,7 +103,7 @@ struct BatchArgs {
   const int32_t* large;       // degree >= batch_large_min
   int32_t n_mid, n_large;
   int32_t* jf[2];
-  int32_t* heavy[2];
+  int2* heavy[2];       // (vertex, chunk) per TD_CHUNK entries of each heavy frontier vertex
   const int32_t* src;   // [n_src], or the seed vertices of a seed list
   const int32_t* seed_slot;  // source of each seed-list entry (null: entry i seeds source i)
   unsigned long long* st_edges;  // per source: sum of degrees of reached vertices
@@ -110,7 +112,7 @@ struct BatchArgs {
   int32_t* join;                 // per source: the level of its depth 0 (0 unless it joined later)
   JoinBox* box;                  // mapped mailbox of sources joining at a level boundary, or null
   double alpha;      // bottom-up when frontier edges * alpha > unfinished edges
-  int32_t heavy_deg; // top-down: from this degree every CTA takes a slice of a vertex
+  int32_t heavy_deg; // top-down: from this degree a vertex is split into chunks
   cudaGraphConditionalHandle cond;
   int32_t use_cond;
   int32_t max_levels;
@@ -145,6 +147,16 @@ __device__ __forceinline__ void wappend(bool want, int v, int32_t* list, int32_t
   if (lane == leader) base = atomicAdd(n, __popc(m));
   base = __shfl_sync(FULL, base, leader);
   if (want) list[base + __popc(m & lanemask_lt())] = v;
+}
+
+// Lists the chunks of heavy vertex v (degree d) at heavy[at].
+__device__ __forceinline__ int heavy_chunks(int64_t d) { return (int)((d + TD_CHUNK - 1) / TD_CHUNK); }
+__device__ __forceinline__ void list_heavy(const BatchArgs& a, int idx, int at, int v, int64_t d) {
+  const int n = heavy_chunks(d);
+  for (int i = 0; i < n; ++i) a.heavy[idx][at + i] = make_int2(v, i);
+}
+__device__ __forceinline__ void add_heavy(const BatchArgs& a, BatchCtl* c, int idx, int v, int64_t d) {
+  if (d >= a.heavy_deg) list_heavy(a, idx, atomicAdd(&c->n_heavy[idx], heavy_chunks(d)), v, d);
 }
 
 // Adds found source bits to the CTA's active-source word; the atomic is only
@@ -208,15 +220,7 @@ __global__ void __launch_bounds__(SEED_THREADS) k_b_seed(BatchArgs a) {
     if (lane == leader) at = atomicAdd(&s_n, __popc(mf));
     at = __shfl_sync(FULL, at, leader);
     if (fresh) a.jf[0][at + __popc(mf & lanemask_lt())] = v;
-    const bool hv = fresh && d >= a.heavy_deg;
-    const unsigned mh = __ballot_sync(FULL, hv);
-    if (mh) {
-      const int lh = __ffs(mh) - 1;
-      int ah = 0;
-      if (lane == lh) ah = atomicAdd(&s_h, __popc(mh));
-      ah = __shfl_sync(FULL, ah, lh);
-      if (hv) a.heavy[0][ah + __popc(mh & lanemask_lt())] = v;
-    }
+    if (fresh && d >= a.heavy_deg) list_heavy(a, 0, atomicAdd(&s_h, heavy_chunks(d)), v, d);
     // degrees are below 2^31: split in 16-bit halves, each sums over 32 lanes without overflow
     const unsigned dlo = __reduce_add_sync(FULL, (unsigned)d & 0xFFFFu);
     const unsigned dhi = __reduce_add_sync(FULL, (unsigned)d >> 16);
@@ -253,48 +257,67 @@ __global__ void __launch_bounds__(SEED_THREADS) k_b_seed(BatchArgs a) {
 }
 
 // ----------------------------------------------------------- top-down -----
-// Claims the bits of frontier vertex u (frontier words fu) for neighbour v.
-// With `scan` (uniform) the words and the frontier bit are ORed by atomics
-// whose results are not used, so nothing waits on memory; the commit then
-// drops the bits v already had. Otherwise v's visited words filter the bits
-// and the first claimant appends v to the next frontier.
-__device__ __forceinline__ void td_edge(const BatchArgs& a, BatchCtl* c, const unsigned long long* fu, int v,
-                                        bool valid, unsigned long long* nb, int nxt, bool scan) {
-  if (scan) {
-    if (valid) {
-      bool any = false;
-      for (int w = 0; w < a.W; ++w) {
-        const unsigned long long f = fu[w];
-        if (f) {
-          atomicOr(nb + (size_t)v * a.W + w, f);
-          any = true;
-        }
-      }
-      if (any) atomicOr(&a.jfb[nxt][v >> 5], 1u << (v & 31));
+// Claims the bits of a frontier vertex (its words fu, in shared memory) for
+// the vertices of its row entries [beg, end): one warp, TD_ILP entries per lane
+// in flight together. With `scan` (uniform) the words and the frontier bit are
+// ORed by atomics whose results are not used, so nothing waits on them; the
+// commit then drops the bits a vertex already had. Otherwise a vertex's
+// visited words filter the bits and the first claimant appends it to the next
+// frontier. The frontier bit is looked at through L1 before its atomic: the
+// hubs, which most entries lead to, share a few words of it, where atomics of
+// every entry would serialise (a stale word only costs the atomic).
+constexpr int TD_ILP = 2;
+__device__ __forceinline__ void td_entries(const BatchArgs& a, BatchCtl* c, const unsigned long long* fu, int64_t beg,
+                                           int64_t end, unsigned long long* nb, int nxt, bool scan) {
+  const int lane = threadIdx.x & 31;
+  uint32_t* jn = a.jfb[nxt];
+  for (int64_t e0 = beg; e0 < end; e0 += 32 * TD_ILP) {
+    int v[TD_ILP];
+    bool any[TD_ILP];
+#pragma unroll
+    for (int u = 0; u < TD_ILP; ++u) {
+      const int64_t e = e0 + 32 * u + lane;
+      v[u] = e < end ? __ldg(a.adj + e) : -1;
+      any[u] = scan && v[u] >= 0;
     }
-    return;
-  }
-  bool first = false;
-  if (valid) {
-    const unsigned long long* xv = a.X + (size_t)v * a.W;
-    bool any = false;
     for (int w = 0; w < a.W; ++w) {
       const unsigned long long f = fu[w];
       if (!f) continue;
-      const unsigned long long b = f & ~__ldg(xv + w);
-      if (b) {
-        atomicOr(nb + (size_t)v * a.W + w, b);
-        any = true;
-      }
+      unsigned long long b[TD_ILP];
+#pragma unroll
+      for (int u = 0; u < TD_ILP; ++u)
+        b[u] = v[u] < 0 ? 0ull : (scan ? f : f & ~__ldg(a.X + (size_t)v[u] * a.W + w));
+#pragma unroll
+      for (int u = 0; u < TD_ILP; ++u)
+        if (b[u]) {
+          atomicOr(nb + (size_t)v[u] * a.W + w, b[u]);
+          any[u] = true;
+        }
     }
-    if (any) {
-      const uint32_t tb = 1u << (v & 31);
-      first = !(atomicOr(&a.jfb[nxt][v >> 5], tb) & tb);
+#pragma unroll
+    for (int u = 0; u < TD_ILP; ++u) {
+      bool first = false;
+      if (any[u]) {
+        const uint32_t tb = 1u << (v[u] & 31);
+        uint32_t* word = jn + (v[u] >> 5);
+        if (!(__ldca(word) & tb)) {
+          if (scan) atomicOr(word, tb);
+          else first = !(atomicOr(word, tb) & tb);
+        }
+      }
+      if (!scan) wappend(first, v[u], a.jf[nxt], &c->n_jf[nxt]);
     }
   }
-  wappend(first, v, a.jf[nxt], &c->n_jf[nxt]);
 }
 
+// A warp takes one item at a time: a chunk of TD_CHUNK entries of a heavy
+// vertex (degree >= heavy_deg, listed chunk by chunk), or the whole row of a
+// light one. The vertex's W words are kept in shared memory for all its
+// entries. Splitting a hub's row over warps matters from the first level on:
+// with whole rows up to 4095 entries per warp, and larger ones shared by all
+// CTAs one vertex after another, s22 x 256 spent 0.21 ms on a first level of
+// 15k entries and 1.3-1.9 ms on the second (19-28M entries); this takes 0.04
+// and 0.26-0.38 ms.
 __device__ void b_td_expand(const BatchArgs& a, BatchCtl* c, unsigned long long* s_f) {
   const int cur = c->cur, nxt = cur ^ 1;
   const int slot = c->level - c->base;
@@ -302,37 +325,27 @@ __device__ void b_td_expand(const BatchArgs& a, BatchCtl* c, unsigned long long*
   unsigned long long* NB = slot_ptr(a, slot + 1);
   const bool scan = c->td_scan != 0;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  // Heavy frontier vertices: every CTA takes an interleaved slice of the edges.
-  const int nh = c->n_heavy[cur];
-  for (int h = 0; h < nh; ++h) {
-    const int u = a.heavy[cur][h];
-    __syncthreads();
-    for (int w = threadIdx.x; w < a.W; w += BB) s_f[w] = F[(size_t)u * a.W + w];
-    __syncthreads();
-    const int64_t beg = a.off[u], end = a.off[u + 1];
-    for (int64_t e0 = beg + (int64_t)blockIdx.x * BB; e0 < end; e0 += (int64_t)gridDim.x * BB) {
-      const int64_t e = e0 + threadIdx.x;
-      const bool valid = e < end;
-      td_edge(a, c, s_f, valid ? __ldg(a.adj + e) : 0, valid, NB, nxt, scan);
-    }
-  }
-  // Light frontier vertices: one warp each; the warp keeps F[u] in shared memory.
-  __syncthreads();
   unsigned long long* fw = s_f + (size_t)warp * a.W;
-  const int n = c->n_jf[cur];
+  const int nh = c->n_heavy[cur], n = nh + c->n_jf[cur];
   const int gw = (blockIdx.x * BB + threadIdx.x) >> 5, nw = (gridDim.x * BB) >> 5;
   for (int i = gw; i < n; i += nw) {
-    const int u = a.jf[cur][i];
-    const int64_t beg = a.off[u], end = a.off[u + 1];
-    if (end - beg >= a.heavy_deg) continue;
+    int u;
+    int64_t beg, end;
+    if (i < nh) {
+      const int2 h = a.heavy[cur][i];
+      u = h.x;
+      beg = a.off[u] + (int64_t)h.y * TD_CHUNK;
+      end = min(a.off[u + 1], beg + TD_CHUNK);
+    } else {
+      u = a.jf[cur][i - nh];
+      beg = a.off[u];
+      end = a.off[u + 1];
+      if (end - beg >= a.heavy_deg) continue;
+    }
     __syncwarp();
     for (int w = lane; w < a.W; w += 32) fw[w] = F[(size_t)u * a.W + w];
     __syncwarp();
-    for (int64_t e0 = beg; e0 < end; e0 += 32) {
-      const int64_t e = e0 + lane;
-      const bool valid = e < end;
-      td_edge(a, c, fw, valid ? __ldg(a.adj + e) : 0, valid, NB, nxt, scan);
-    }
+    td_entries(a, c, fw, beg, end, NB, nxt, scan);
   }
 }
 
@@ -362,7 +375,6 @@ __device__ __forceinline__ void bu_finish_vertex(const BatchArgs& a, BatchCtl* c
     my_m += (unsigned long long)d;
     atomicOr(&a.jfb[nxt][v >> 5], 1u << (v & 31));
     a.jf[nxt][atomicAdd(&c->n_jf[nxt], 1)] = v;
-    if (d >= a.heavy_deg) a.heavy[nxt][atomicAdd(&c->n_heavy[nxt], 1)] = v;
   }
   if (gfull) {
     atomicOr(&a.donebits[v >> 5], 1u << (v & 31));
@@ -654,10 +666,6 @@ __device__ void b_bu_expand(const BatchArgs& a, BatchCtl* c, unsigned long long*
           full_bits |= 1u << vl;
           my_md += (unsigned long long)(e1 - e0);
         }
-        if (gl == 0 && gany && e1 - e0 >= a.heavy_deg) {
-          const int at = atomicAdd(&c->n_heavy[nxt], 1);
-          a.heavy[nxt][at] = (int)v;
-        }
         // append v to the next joint frontier (one lane per group)
         if (gl == 0 && gany) {
           a.smask[v] = (uint16_t)(a.smask[v] | (2u << slot));
@@ -785,7 +793,10 @@ __device__ void join_sources(const BatchArgs& a, volatile BatchCtl* vc, int L, i
       a.jf[nxt][n_next++] = v;
       const int d = a.deg[v];
       m_next += d;
-      if (d >= a.heavy_deg) a.heavy[nxt][vc->n_heavy[nxt]++] = v;
+      if (d >= a.heavy_deg) {
+        list_heavy(a, nxt, vc->n_heavy[nxt], v, d);
+        vc->n_heavy[nxt] = vc->n_heavy[nxt] + heavy_chunks(d);
+      }
     }
   }
   vc->n_jf[nxt] = (int32_t)n_next;
@@ -794,6 +805,12 @@ __device__ void join_sources(const BatchArgs& a, volatile BatchCtl* vc, int L, i
   vc->m_done = 0;
   __threadfence();
   st_release_sys(&box->taken, seq);
+}
+
+// The next level's direction: m_next frontier edges against the edges of
+// vertices not yet complete.
+__device__ __forceinline__ bool goes_bottom_up(const BatchArgs& a, int64_t m_next, int64_t m_done) {
+  return (double)m_next * a.alpha > (double)(a.E - m_done);
 }
 
 // Top-down: fold the claimed bits into X and count. Both directions: clear
@@ -817,6 +834,18 @@ __global__ void __launch_bounds__(BB) k_b_commit(BatchArgs a) {
     const int64_t gtid = blockIdx.x * (int64_t)BB + threadIdx.x, nth = (int64_t)gridDim.x * BB;
     const int nc = c->n_jf[cur];
     for (int64_t i = gtid; i < nc; i += nth) a.jfb[cur][(uint32_t)a.jf[cur][i] >> 5] = 0;
+    // A bottom-up level leaves the heavy chunks of its finds to this kernel
+    // (listing them there spilled registers in the tiers' loops), and only a
+    // level that turns top-down needs them. The counts are final, so every CTA
+    // takes the finisher's decision by itself; sources joining may change it,
+    // so a batch with a mailbox always lists.
+    if (dir == 1 && (a.box || !goes_bottom_up(a, (int64_t)c->acc_m, c->m_done + (int64_t)c->acc_mdone))) {
+      const int nn = c->n_jf[nxt];
+      for (int64_t i = gtid; i < nn; i += nth) {
+        const int v = a.jf[nxt][i];
+        add_heavy(a, c, nxt, v, a.deg[v]);
+      }
+    }
   }
   if (dir == 0) {
     const int slot = c->level - c->base;
@@ -838,29 +867,26 @@ __global__ void __launch_bounds__(BB) k_b_commit(BatchArgs a) {
         atomicOr(&a.donebits[v >> 5], 1u << (v & 31));
         my_md += d;
       }
-      if (d >= a.heavy_deg) a.heavy[nxt][atomicAdd(&c->n_heavy[nxt], 1)] = v;
+      add_heavy(a, c, nxt, v, d);
     };
     if (c->td_scan) {
-      // a warp takes 32 consecutive jfb words (lane = word) and walks their
-      // set bits in rounds, one vertex per lane per round
+      // a warp takes one jfb word, a vertex per lane: the words of 32
+      // neighbouring vertices are read together, and the hubs' dense words are
+      // spread over all warps (32 words per warp, a set bit per lane and round,
+      // took 0.22 ms at s22 x 256, this 0.11)
       uint32_t* jn = a.jfb[nxt];
       const int64_t Wd = (a.V + 31) >> 5;
-      for (int64_t wb = gtid - lane; wb < Wd; wb += nth) {
-        const int64_t wi = wb + lane;
-        const uint32_t orig = wi < Wd ? jn[wi] : 0u;
-        uint32_t bits = orig, keep = orig;
-        while (__any_sync(FULL, bits != 0)) {
-          const bool valid = bits != 0;
-          const int b = valid ? __ffs(bits) - 1 : 0;
-          bits &= bits - 1;
-          const int v = (int)(wi * 32 + b);
-          bool got, full;
-          td_commit_words(a, NB, ac, v, valid, s_act, got, full);
-          if (valid && !got) keep &= ~(1u << b);
-          wappend(valid && got, v, a.jf[nxt], &c->n_jf[nxt]);
-          if (valid) vertex_done(v, got, full);
-        }
-        if (keep != orig) jn[wi] = keep;
+      for (int64_t wi = gtid >> 5; wi < Wd; wi += nth >> 5) {
+        const uint32_t bits = jn[wi];
+        if (!bits) continue;
+        const bool valid = (bits >> lane) & 1u;
+        const int v = (int)(wi * 32 + lane);
+        bool got, full;
+        td_commit_words(a, NB, ac, v, valid, s_act, got, full);
+        wappend(got, v, a.jf[nxt], &c->n_jf[nxt]);
+        if (valid) vertex_done(v, got, full);
+        const uint32_t keep = __ballot_sync(FULL, got);
+        if (lane == 0 && keep != bits) jn[wi] = keep;
       }
     } else {
       // warp-uniform trip count: the claimed words are OR-reduced across the warp
@@ -903,8 +929,7 @@ __global__ void __launch_bounds__(BB) k_b_commit(BatchArgs a) {
   vc->n_jf[cur] = 0;
   vc->n_heavy[cur] = 0;
   vc->m_f = m_next;
-  const double m_u = (double)(a.E - vc->m_done);
-  vc->dir = ((double)m_next * a.alpha > m_u) ? 1 : 0;
+  vc->dir = goes_bottom_up(a, m_next, vc->m_done) ? 1 : 0;
   // a top-down level over at least V/4 edges claims without waiting on memory
   vc->td_scan = vc->dir == 0 && m_next * 4 >= a.V;
   int done = n_next == 0;
@@ -1506,9 +1531,12 @@ int create_batch_workspace(ent_graph* g, int n_src, BatchWorkspace** out) {
   const size_t sz_q = al(sizeof(int32_t) * (V + 4));
   const size_t sz_mask = al(sizeof(unsigned long long) * W);
   const size_t sz_src = al(sizeof(int32_t) * w->cap_src);
+  // chunks of heavy vertices: at most one per TD_CHUNK edges and one per vertex
+  const int32_t heavy_deg = std::min(g->opts.batch_heavy, TD_CHUNK);
+  const size_t sz_heavy = al(sizeof(int2) * (g->E / TD_CHUNK + std::min(V, g->E / heavy_deg) + 1));
   const size_t sz_marks = al(sizeof(uint16_t) * V);
   const size_t sz_st = al(sizeof(unsigned long long) * w->cap_src) * 2 + 2 * al(sizeof(int32_t) * w->cap_src);
-  const size_t total = sz_x + sz_log + 4 * sz_bits + 6 * sz_q + 3 * sz_mask + sz_src + sz_st + sz_marks + 256;
+  const size_t total = sz_x + sz_log + 4 * sz_bits + 4 * sz_q + 2 * sz_heavy + 3 * sz_mask + sz_src + sz_st + sz_marks + 256;
   cudaError_t e = cudaMalloc(&w->slab, total);
   if (e != cudaSuccess) { destroy_batch_workspace(w); return fail(ENT_ERR_OOM, "batch workspace (%zu bytes) failed", total); }
   // Initialise on the graph's stream and wait (see create_workspace in
@@ -1547,7 +1575,7 @@ int create_batch_workspace(ent_graph* g, int n_src, BatchWorkspace** out) {
   a.jfb[0] = (uint32_t*)p; p += sz_bits;
   a.jfb[1] = (uint32_t*)p; p += sz_bits;
   for (int i = 0; i < 2; ++i) { a.jf[i] = (int32_t*)p; p += sz_q; }
-  for (int i = 0; i < 2; ++i) { a.heavy[i] = (int32_t*)p; p += sz_q; }
+  for (int i = 0; i < 2; ++i) { a.heavy[i] = (int2*)p; p += sz_heavy; }
   uint32_t* lightbits = (uint32_t*)p; p += sz_bits;
   int32_t* mid = (int32_t*)p; p += sz_q;
   int32_t* large = (int32_t*)p; p += sz_q;
@@ -1567,7 +1595,7 @@ int create_batch_workspace(ent_graph* g, int n_src, BatchWorkspace** out) {
   a.join = (int32_t*)p; p += al(sizeof(int32_t) * w->cap_src);  // zeroed with the statistics
   a.box = nullptr;
   a.alpha = g->opts.batch_alpha;
-  a.heavy_deg = g->opts.batch_heavy;
+  a.heavy_deg = heavy_deg;
   a.max_levels = (int32_t)std::min<int64_t>(V + 2, 0x7ffffff0);
   w->smem = sizeof(unsigned long long) * std::max(W * (BB / 32), W);
   {

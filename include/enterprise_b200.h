@@ -83,7 +83,7 @@ typedef struct ent_bfs_opts {
   double batch_alpha;      /* bottom-up when frontier edges*alpha > unfinished edges */
   int32_t batch_small_max; /* bottom-up: degree < this -> lane group per vertex     */
   int32_t batch_large_min; /* bottom-up: degree >= this -> CTA per vertex           */
-  int32_t batch_heavy;     /* top-down: degree >= this -> all CTAs share the vertex */
+  int32_t batch_heavy;     /* top-down: degree >= min(this, 512) -> warps share the vertex */
   /* small-frontier ("narrow") mode of the single-source traversal: while the
      top-down frontier stays small, one thread-block cluster runs level after
      level inside a single launch. Entered when the frontier has at most
