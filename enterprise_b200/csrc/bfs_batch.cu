@@ -912,8 +912,15 @@ __global__ void __launch_bounds__(BB) k_b_commit(BatchArgs a) {
     s_last = atomicAdd(&c->finished, 1u) == gridDim.x - 1;
   }
   __syncthreads();
-  if (!s_last || threadIdx.x != 0) return;
+  if (!s_last) return;
   __threadfence();
+  // The sources with a frontier at the new level have reached that depth (a
+  // source that joins below starts at depth 0, as the statistics were zeroed).
+  for (int s = threadIdx.x; s < a.W * 64; s += BB)
+    if (((unsigned long long)__ldcg(reinterpret_cast<const long long*>(a.act[nxt] + (s >> 6))) >> (s & 63)) & 1ull)
+      a.st_maxd[s] = c->level + 1 - a.join[s];
+  __syncthreads();
+  if (threadIdx.x != 0) return;
   volatile BatchCtl* vc = c;
   int64_t n_next = vc->n_jf[nxt];
   int64_t m_next = (int64_t)vc->acc_m;
@@ -963,8 +970,8 @@ __global__ void __launch_bounds__(BB) k_b_commit(BatchArgs a) {
 // (the first window: -1 where not found) and the rows allow it, a lane takes
 // 4 consecutive vertices and stores each row's 4 depths as one vector;
 // otherwise (later windows write only the pairs they found) a lane takes a
-// vertex. Reached vertices, the sum of their degrees and the deepest level
-// are kept per row.
+// vertex. Reached vertices and the sum of their degrees are kept per row (the
+// deepest level follows from the levels' active sources, k_b_commit).
 constexpr int TILE_BYTES = 64 * 1024;  // VS vertices x 64*CG source bytes
 constexpr int FLUSH_TILE_BYTES = TILE_BYTES + 1024 * 4;  // + the span's degrees
 
@@ -1061,15 +1068,10 @@ __device__ __forceinline__ int sext_byte(uint32_t w, uint32_t j) {
   return (int)r;
 }
 
-// The low bytes of a, b, c, d as one word, a in byte 0.
-__device__ __forceinline__ uint32_t pack_low_bytes(int a, int b, int c, int d) {
-  return __byte_perm(__byte_perm((uint32_t)a, (uint32_t)b, 0x0040u), __byte_perm((uint32_t)c, (uint32_t)d, 0x0040u),
-                     0x5410u);
-}
-
 struct FlushState {
   int first, last, base, windows, nsrc;
   bool final_flush;
+  bool joined;              // some source started later than level 0
   bool vec;                 // whole-window rows take 16-byte (int32) or 4-byte (u8) vector stores
   int32_t* depth;
   const int32_t* row_map;
@@ -1077,14 +1079,141 @@ struct FlushState {
   const int* s_deg;         // [1024] degrees of the span
   unsigned* s_cnt;          // [W*64] reached vertices per source
   unsigned long long* s_edg;  // [W*64] their degrees
-  int* s_maxd;              // [W*64] deepest level
+  // Per column group: the found mask most vertices of this CTA share, and the
+  // vertices and degrees counted under it (added to its sources at the end)
+  unsigned long long* s_pat;  // [W]
+  unsigned long long* s_pe;   // [W / CG] degree sums
+  unsigned* s_pn;             // [W / CG] vertices
+  int* s_claim;               // one mismatching thread proposes a new mask in s_cand
+  unsigned long long* s_cand; // [4]
 };
+
+// Adds column group cg's vertices counted under the shared mask to the mask's
+// sources. Called by every thread; the caller synchronises around it.
+template <int CG>
+__device__ __forceinline__ void settle_pattern(const FlushState& fs, int cg) {
+  const int t = threadIdx.x;
+  if (t < 64 * CG && ((fs.s_pat[cg + (t >> 6)] >> (t & 63)) & 1ull)) {
+    fs.s_cnt[cg * 64 + t] += fs.s_pn[cg / CG];
+    fs.s_edg[cg * 64 + t] += fs.s_pe[cg / CG];
+  }
+}
+
+// Writes the rows of column group cg for the nsub vertices of the tile: a warp
+// per 4 sources. With STATS, each pair also counts towards its source's
+// reached vertices and their degrees; without, the caller has counted the
+// tile's vertices under the shared mask.
+template <int CG, bool BYTES, bool STATS>
+__device__ __forceinline__ void write_rows(const BatchArgs& a, const FlushState& fs, int64_t v0, int sub, int nsub,
+                                           int cg) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (int r0 = warp * 4; r0 < 64 * CG; r0 += BB / 32 * 4) {
+    const int s0 = cg * 64 + r0;
+    if (s0 >= fs.nsrc) break;
+    const int c4 = r0 >> 2;
+    size_t ofs[4];  // element offset of each row's segment (int32 or byte rows)
+    bool rv[4];
+    int rb[4];      // depth of log slot 0 for the row: the window's base level less the source's start
+    bool wide = false;   // a byte row whose depths could pass 254 here: checked one by one
+    bool plain = true;   // the slot index is the depth
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      rv[j] = s0 + j < fs.nsrc;
+      ofs[j] = rv[j] ? (size_t)(fs.row_map ? fs.row_map[s0 + j] : s0 + j) * a.V + v0 + sub : 0;
+      rb[j] = fs.base - (fs.joined && rv[j] ? a.join[s0 + j] : 0);
+      if (BYTES && rv[j] && rb[j] > 239) wide = true;
+      plain &= rb[j] == 0;
+    }
+    unsigned cnt[4] = {0, 0, 0, 0};
+    unsigned long long edg[4] = {0, 0, 0, 0};
+    if (fs.vec && !wide) {
+      for (int vi = lane * 4; vi < nsub; vi += 128) {
+        uint32_t wv[4], x[4];
+#pragma unroll
+        for (int t = 0; t < 4; ++t) wv[t] = fs.tile[tile_word<CG>(vi + t, c4)];
+        if constexpr (BYTES) byte_transpose4(wv[0], wv[1], wv[2], wv[3], x[0], x[1], x[2], x[3]);
+        int4 dg = make_int4(0, 0, 0, 0);
+        if constexpr (STATS) dg = *reinterpret_cast<const int4*>(fs.s_deg + sub + vi);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          if (!rv[j]) continue;
+          int d[4];
+          if constexpr (!BYTES || STATS) {
+#pragma unroll
+            for (int t = 0; t < 4; ++t) d[t] = sext_byte(wv[t], j);  // -1 where not found
+          }
+          if constexpr (STATS) {
+            cnt[j] += 4 + (d[0] >> 31) + (d[1] >> 31) + (d[2] >> 31) + (d[3] >> 31);
+            // two degrees below 2^31 each cannot overflow 32 bits
+            const uint32_t e01 = (uint32_t)(dg.x & ~(d[0] >> 31)) + (uint32_t)(dg.y & ~(d[1] >> 31));
+            const uint32_t e23 = (uint32_t)(dg.z & ~(d[2] >> 31)) + (uint32_t)(dg.w & ~(d[3] >> 31));
+            edg[j] += (unsigned long long)e01 + e23;
+          }
+          if constexpr (BYTES) {
+            // four depths at once: slot (0..15) + base stays below 255 (no
+            // carry into the next byte), and not found stays 0xFF
+            uint32_t o = x[j];
+            if (!plain) o = ((o & 0x0F0F0F0Fu) + (uint32_t)rb[j] * 0x01010101u) | (((o >> 7) & 0x01010101u) * 0xFFu);
+            *reinterpret_cast<uint32_t*>(reinterpret_cast<uint8_t*>(fs.depth) + ofs[j] + vi) = o;
+          } else {
+            if (!plain) {
+#pragma unroll
+              for (int t = 0; t < 4; ++t) d[t] += rb[j] & ~(d[t] >> 31);
+            }
+            *reinterpret_cast<int4*>(fs.depth + ofs[j] + vi) = make_int4(d[0], d[1], d[2], d[3]);
+          }
+        }
+      }
+    } else {
+      bool deep = false;  // a depth above 254 met in byte rows
+      for (int vi = lane; vi < nsub; vi += 32) {
+        const uint32_t wv = fs.tile[tile_word<CG>(vi, c4)];
+        const int dg = STATS ? fs.s_deg[sub + vi] : 0;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          if (!rv[j]) continue;
+          const int d = sext_byte(wv, j);
+          const int m = d >> 31;
+          const int v = d + (rb[j] & ~m);
+          if (fs.windows == 0 || d >= 0) {
+            if constexpr (BYTES) {
+              reinterpret_cast<uint8_t*>(fs.depth)[ofs[j] + vi] = (uint8_t)v;  // -1 -> 255
+              deep |= v > 254;
+            } else {
+              fs.depth[ofs[j] + vi] = v;
+            }
+          }
+          if constexpr (STATS) {
+            cnt[j] += 1 + m;
+            edg[j] += (uint32_t)(dg & ~m);
+          }
+        }
+      }
+      if constexpr (BYTES)
+        if (__any_sync(FULL, deep) && lane == 0) atomicOr(&a.ctl->err, 16);
+    }
+    if constexpr (STATS) {
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        // a lane's degree sum is below 2^36 (at most 32 vertices), so both
+        // 16-bit-split halves sum over 32 lanes without overflow
+        const unsigned c = __reduce_add_sync(FULL, cnt[j]);
+        const unsigned elo = __reduce_add_sync(FULL, (unsigned)(edg[j] & 0xFFFFu));
+        const unsigned ehi = __reduce_add_sync(FULL, (unsigned)(edg[j] >> 16));
+        if (lane == 0 && rv[j] && c) {  // a source's rows are always this warp's
+          fs.s_cnt[s0 + j] += c;
+          fs.s_edg[s0 + j] += ((unsigned long long)ehi << 16) + elo;
+        }
+      }
+    }
+  }
+}
 
 template <int CG, bool BYTES>
 __device__ void flush_span(const BatchArgs& a, const FlushState& fs, int64_t v0, int nv) {
   constexpr int VS = 1024 / CG;  // vertices per pass
   constexpr int Q = VS / BB;     // ... and per thread
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31;
   // the slots decoded: [first, last]
   const uint32_t decoded = ((2u << fs.last) - 1u) & ~((1u << fs.first) - 1u);
   // The thread's vertices of this pass (traversal ids) and their slot marks.
@@ -1112,6 +1241,12 @@ __device__ void flush_span(const BatchArgs& a, const FlushState& fs, int64_t v0,
       if (cg * 64 >= fs.nsrc) break;  // words of no source: never set, so already zero
       __syncthreads();  // the previous tile has been written out
       const bool last_cols = cg + CG >= a.W || (cg + CG) * 64 >= fs.nsrc;
+      // Statistics. Nearly all found vertices of a batch share one found mask
+      // (every source of the giant component): those are counted once here,
+      // and only a pass with another mask counts pair by pair.
+      unsigned pn = 0;
+      unsigned long long pe = 0;
+      bool mis = false;
 #pragma unroll
       for (int q = 0; q < Q; ++q) {
         const int vi = (int)threadIdx.x + q * BB;
@@ -1122,30 +1257,29 @@ __device__ void flush_span(const BatchArgs& a, const FlushState& fs, int64_t v0,
         for (int cc = 0; cc < CG; ++cc) f[cc] = p0[cc] = p1[cc] = p2[cc] = p3[cc] = 0;
         // loads and folds only: no store or warp-collective may sit between
         // the slot loads, which the compiler then keeps in flight together.
-        // Slots in groups of four from a multiple of 4: bits 0 and 1 of a
-        // slot's index follow from its place in the group, bits 2 and 3 are
-        // the group's. Only marked slots are read (about a third of them).
-        for (int k0 = 0; md >> k0; k0 += 4) {
+        // Only marked slots are read (about a third of them), two at a time
+        // (three or four spill: s22 x 256 1.29 -> 1.36 and 1.50 ms).
+        for (uint32_t z = md; z;) {
+          unsigned long long w[2][CG];
+          int k[2];
 #pragma unroll
-          for (int h = 0; h < 2; ++h) {
-            const int ka = k0 + 2 * h, kb = ka + 1;
-            unsigned long long wa[CG], wb[CG];
-            if ((md >> ka) & 1u) load_cols<CG>(slot_ptr(a, ka) + at, wa);
+          for (int i = 0; i < 2; ++i) {
+            k[i] = z ? __ffs(z) - 1 : 0;
+            if (z) load_cols<CG>(slot_ptr(a, k[i]) + at, w[i]);
             else
 #pragma unroll
-              for (int cc = 0; cc < CG; ++cc) wa[cc] = 0;
-            if ((md >> kb) & 1u) load_cols<CG>(slot_ptr(a, kb) + at, wb);
-            else
+              for (int cc = 0; cc < CG; ++cc) w[i][cc] = 0;
+            if (z) z &= z - 1;
+          }
 #pragma unroll
-              for (int cc = 0; cc < CG; ++cc) wb[cc] = 0;
+          for (int i = 0; i < 2; ++i) {
 #pragma unroll
             for (int cc = 0; cc < CG; ++cc) {
-              const unsigned long long u = wa[cc] | wb[cc];
-              f[cc] |= u;
-              p0[cc] |= wb[cc];
-              if (h) p1[cc] |= u;
-              if (k0 & 4) p2[cc] |= u;
-              if (k0 & 8) p3[cc] |= u;
+              f[cc] |= w[i][cc];
+              if (k[i] & 1) p0[cc] |= w[i][cc];
+              if (k[i] & 2) p1[cc] |= w[i][cc];
+              if (k[i] & 4) p2[cc] |= w[i][cc];
+              if (k[i] & 8) p3[cc] |= w[i][cc];
             }
           }
         }
@@ -1159,6 +1293,23 @@ __device__ void flush_span(const BatchArgs& a, const FlushState& fs, int64_t v0,
                                  (uint32_t)(p3[cc] >> (32 * hw)), o);
 #pragma unroll
             for (int n = 0; n < 8; ++n) fs.tile[tile_word<CG>(vi, cc * 16 + hw * 8 + n)] = o[n];
+          }
+        }
+        if (md) {
+          bool eq = true;
+#pragma unroll
+          for (int cc = 0; cc < CG; ++cc) eq &= f[cc] == fs.s_pat[cg + cc];
+          unsigned long long any = 0;
+#pragma unroll
+          for (int cc = 0; cc < CG; ++cc) any |= f[cc];
+          if (eq && any) {
+            pn += 1;
+            pe += (unsigned)fs.s_deg[sub + vi];
+          } else if (any) {
+            mis = true;
+            if (atomicExch(fs.s_claim, 1) == 0)
+#pragma unroll
+              for (int cc = 0; cc < CG; ++cc) fs.s_cand[cc] = f[cc];
           }
         }
         if (marks) {
@@ -1181,95 +1332,27 @@ __device__ void flush_span(const BatchArgs& a, const FlushState& fs, int64_t v0,
         for (int q = 0; q < Q; ++q) iv[q] = next_iv[q];
         load_marks(iv);
       }
-      __syncthreads();
-      for (int r0 = warp * 4; r0 < 64 * CG; r0 += BB / 32 * 4) {
-        const int s0 = cg * 64 + r0;
-        if (s0 >= fs.nsrc) break;
-        const int c4 = r0 >> 2;
-        size_t ofs[4];  // element offset of each row's segment (int32 or byte rows)
-        bool rv[4];
-        int rb[4];      // depth of log slot 0 for the row: the window's base level less the source's start
-        bool wide = false;  // a byte row whose depths could pass 254 here: checked one by one
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          rv[j] = s0 + j < fs.nsrc;
-          ofs[j] = rv[j] ? (size_t)(fs.row_map ? fs.row_map[s0 + j] : s0 + j) * a.V + v0 + sub : 0;
-          rb[j] = fs.base - (rv[j] ? a.join[s0 + j] : 0);
-          if (BYTES && rv[j] && rb[j] > 239) wide = true;
+      const int odd = __syncthreads_count(mis);  // the tile is complete
+      if (odd == 0) {
+        const unsigned n = __reduce_add_sync(FULL, pn);
+        // a lane's degree sum is below 2^33: both halves sum over 32 lanes without overflow
+        const unsigned elo = __reduce_add_sync(FULL, (unsigned)(pe & 0xFFFFu));
+        const unsigned ehi = __reduce_add_sync(FULL, (unsigned)(pe >> 16));
+        if (lane == 0 && n) {
+          atomicAdd(fs.s_pn + cg / CG, n);
+          atomicAdd(fs.s_pe + cg / CG, ((unsigned long long)ehi << 16) + elo);
         }
-        unsigned cnt[4] = {0, 0, 0, 0};
-        unsigned long long edg[4] = {0, 0, 0, 0};
-        int mx[4] = {-1, -1, -1, -1};
-        if (fs.vec && !wide) {
-          for (int vi = lane * 4; vi < nsub; vi += 128) {
-            uint32_t wv[4];
-#pragma unroll
-            for (int t = 0; t < 4; ++t) wv[t] = fs.tile[tile_word<CG>(vi + t, c4)];
-            const int4 dg = *reinterpret_cast<const int4*>(fs.s_deg + sub + vi);
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-              if (!rv[j]) continue;
-              int v[4], m[4];
-#pragma unroll
-              for (int t = 0; t < 4; ++t) {
-                const int d = sext_byte(wv[t], j);
-                m[t] = d >> 31;  // -1 where not found
-                v[t] = d + (rb[j] & ~m[t]);
-                cnt[j] += 1 + m[t];
-                mx[j] = max(mx[j], v[t]);
-              }
-              // two degrees below 2^31 each cannot overflow 32 bits
-              const uint32_t e01 = (uint32_t)(dg.x & ~m[0]) + (uint32_t)(dg.y & ~m[1]);
-              const uint32_t e23 = (uint32_t)(dg.z & ~m[2]) + (uint32_t)(dg.w & ~m[3]);
-              edg[j] += (unsigned long long)e01 + e23;
-              if constexpr (BYTES)
-                *reinterpret_cast<uint32_t*>(reinterpret_cast<uint8_t*>(fs.depth) + ofs[j] + vi) =
-                    pack_low_bytes(v[0], v[1], v[2], v[3]);
-              else
-                *reinterpret_cast<int4*>(fs.depth + ofs[j] + vi) = make_int4(v[0], v[1], v[2], v[3]);
-            }
-          }
-        } else {
-          bool deep = false;  // a depth above 254 met in byte rows
-          for (int vi = lane; vi < nsub; vi += 32) {
-            const uint32_t wv = fs.tile[tile_word<CG>(vi, c4)];
-            const int dg = fs.s_deg[sub + vi];
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-              if (!rv[j]) continue;
-              const int d = sext_byte(wv, j);
-              const int m = d >> 31;
-              const int v = d + (rb[j] & ~m);
-              if (fs.windows == 0 || d >= 0) {
-                if constexpr (BYTES) {
-                  reinterpret_cast<uint8_t*>(fs.depth)[ofs[j] + vi] = (uint8_t)v;  // -1 -> 255
-                  deep |= v > 254;
-                } else {
-                  fs.depth[ofs[j] + vi] = v;
-                }
-              }
-              cnt[j] += 1 + m;
-              edg[j] += (uint32_t)(dg & ~m);
-              mx[j] = max(mx[j], v);
-            }
-          }
-          if constexpr (BYTES)
-            if (__any_sync(FULL, deep) && lane == 0) atomicOr(&a.ctl->err, 16);
+        write_rows<CG, BYTES, false>(a, fs, v0, sub, nsub, cg);
+      } else {
+        write_rows<CG, BYTES, true>(a, fs, v0, sub, nsub, cg);
+        __syncthreads();
+        if (odd >= BB / 4) {  // most vertices differ: take the proposed mask from here on
+          settle_pattern<CG>(fs, cg);
+          __syncthreads();
+          if ((int)threadIdx.x < CG) fs.s_pat[cg + threadIdx.x] = fs.s_cand[threadIdx.x];
+          if (threadIdx.x == 0) fs.s_pn[cg / CG] = 0, fs.s_pe[cg / CG] = 0;
         }
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          // a lane's degree sum is below 2^36 (at most 32 vertices), so both
-          // 16-bit-split halves sum over 32 lanes without overflow
-          const unsigned c = __reduce_add_sync(FULL, cnt[j]);
-          const unsigned elo = __reduce_add_sync(FULL, (unsigned)(edg[j] & 0xFFFFu));
-          const unsigned ehi = __reduce_add_sync(FULL, (unsigned)(edg[j] >> 16));
-          const int dmax = __reduce_max_sync(FULL, mx[j]);
-          if (lane == 0 && rv[j] && c) {  // a source's rows are always this warp's
-            fs.s_cnt[s0 + j] += c;
-            fs.s_edg[s0 + j] += ((unsigned long long)ehi << 16) + elo;
-            fs.s_maxd[s0 + j] = max(fs.s_maxd[s0 + j], dmax);
-          }
-        }
+        if (threadIdx.x == 0) *fs.s_claim = 0;
       }
     }
   }
@@ -1300,6 +1383,7 @@ __global__ void __launch_bounds__(BB, 3) k_b_flush(BatchArgs a, int final_flush)
     fs.first = fs.windows == 0 ? 0 : 1;
     fs.nsrc = c->n_src;
     fs.final_flush = final_flush != 0;
+    fs.joined = c->joined != 0;
     fs.depth = c->depth;
     fs.row_map = c->row_map;
     const bool bytes = c->out_bytes != 0;
@@ -1311,9 +1395,19 @@ __global__ void __launch_bounds__(BB, 3) k_b_flush(BatchArgs a, int final_flush)
     fs.s_deg = reinterpret_cast<const int*>(s_flush + TILE_BYTES);
     fs.s_cnt = reinterpret_cast<unsigned*>(s_flush + FLUSH_TILE_BYTES);
     fs.s_edg = reinterpret_cast<unsigned long long*>(fs.s_cnt + NSRC);  // NSRC is a multiple of 64: 8-byte aligned
-    fs.s_maxd = reinterpret_cast<int*>(fs.s_edg + NSRC);
+    fs.s_pat = fs.s_edg + NSRC;
+    fs.s_pe = fs.s_pat + a.W;
+    fs.s_cand = fs.s_pe + a.W;
+    fs.s_pn = reinterpret_cast<unsigned*>(fs.s_cand + 4);
+    fs.s_claim = reinterpret_cast<int*>(fs.s_pn + a.W);
+    if ((int)threadIdx.x < a.W) {
+      fs.s_pat[threadIdx.x] = a.mask[threadIdx.x];  // until a pass proposes another
+      fs.s_pe[threadIdx.x] = 0;
+      fs.s_pn[threadIdx.x] = 0;
+    }
+    if (threadIdx.x == 0) *fs.s_claim = 0;
     int* s_deg = reinterpret_cast<int*>(s_flush + TILE_BYTES);
-    for (int i = threadIdx.x; i < NSRC; i += BB) { fs.s_cnt[i] = 0; fs.s_edg[i] = 0; fs.s_maxd[i] = -1; }
+    for (int i = threadIdx.x; i < NSRC; i += BB) { fs.s_cnt[i] = 0; fs.s_edg[i] = 0; }
     const int64_t units = (a.V + 1023) / 1024;
     for (int64_t u = blockIdx.x; u < units; u += gridDim.x) {
       const int64_t v0 = u * 1024;
@@ -1333,11 +1427,16 @@ __global__ void __launch_bounds__(BB, 3) k_b_flush(BatchArgs a, int final_flush)
       }
     }
     __syncthreads();
+    for (int cg = 0; cg < a.W; cg += a.W >= 4 ? 4 : a.W) {
+      if (a.W == 1) settle_pattern<1>(fs, cg);
+      else if (a.W == 2) settle_pattern<2>(fs, cg);
+      else settle_pattern<4>(fs, cg);
+    }
+    __syncthreads();
     for (int s = threadIdx.x; s < fs.nsrc; s += BB) {
       if (fs.s_cnt[s]) {
         atomicAdd(&a.st_verts[s], (unsigned long long)fs.s_cnt[s]);
         atomicAdd(&a.st_edges[s], fs.s_edg[s]);
-        atomicMax(&a.st_maxd[s], fs.s_maxd[s]);
       }
     }
   }
@@ -1618,8 +1717,9 @@ int create_batch_workspace(ent_graph* g, int n_src, BatchWorkspace** out) {
   const int64_t want = std::max<int64_t>(1, (V + BB * 8 - 1) / (BB * 8));
   w->grid = (int)std::min<int64_t>((int64_t)g->num_sms * occ, want);
   w->grid_flush = (int)std::min<int64_t>((int64_t)g->num_sms * 3, std::max<int64_t>(1, (V + 1023) / 1024));
-  // tile and degrees; per source: reached vertices, their degree sum, deepest level
-  w->smem_flush = FLUSH_TILE_BYTES + (size_t)W * 64 * (4 + 8 + 4) + 16;
+  // tile and degrees; per source: reached vertices, their degree sum
+  // per word: its part of the shared mask, its counts; and the proposed mask
+  w->smem_flush = FLUSH_TILE_BYTES + (size_t)W * 64 * (4 + 8) + (size_t)W * (8 + 8 + 4) + 4 * 8 + 16;
   {
     e = cudaFuncSetAttribute(k_b_flush, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)w->smem_flush);
     if (e != cudaSuccess) { destroy_batch_workspace(w); return fail(ENT_ERR_CUDA, "flush smem attribute failed"); }
