@@ -11,23 +11,31 @@
 // __device__ array that exists on every GPU that loads this library, for the
 // lifetime of the process.
 //
-// The scratch holds a visited bitmap, two frontier queues and two counters
+// The scratch holds a visited bitmap, two frontier queues and a control block
 // for at most NOALLOC_MAX_VERTICES vertices (about 8.5 MB per GPU). Larger
 // graphs are rejected with ENT_ERR_INVALID_ARG. The traversal is level-
-// synchronous top-down; each level's kernel reads one frontier queue and
-// appends the next with warp-aggregated atomics, exactly the depths every
-// other entry point of this library produces.
+// synchronous top-down (the caller's rows need not hold both directions of an
+// edge, which bottom-up levels would rely on) and gives exactly the depths
+// every other entry point of this library produces.
+//
+// The whole traversal is one cooperative launch: its CTAs go from level to
+// level through a grid-wide barrier (bounded waits), so the host neither
+// launches nor waits per level. While the frontier is small, CTA 0 runs the
+// levels alone with its frontier in shared memory and the others wait at the
+// barrier.
 //
 // Sharing: every call uses the same array and leaves its last contents
 // behind; each call clears the visited bitmap and the counters before it
 // starts. Two calls whose work overlaps on the same GPU (for example from two
 // host threads at once, or on two streams) race on the shared scratch and
 // produce wrong results: callers must serialise them.
+#include <algorithm>
 #include <cuda_runtime.h>
 #include <mutex>
 #include <stdint.h>
 #include <vector>
 
+#include "dev_common.cuh"
 #include "ent_internal.h"
 
 namespace ent {
@@ -38,83 +46,316 @@ constexpr int64_t NOALLOC_WORDS = NOALLOC_MAX_VERTICES / 32;
 // Layout inside the scratch array (all offsets 256-byte aligned):
 //   [0]                       uint32 visited[NOALLOC_WORDS]
 //   [NOALLOC_WORDS*4]         int32  queue[2][NOALLOC_MAX_VERTICES]
-//   [.. + 8*MAX]              int32  count[2]  (frontier sizes)
+//   [.. + 8*MAX]              NaCtl
+// A queue holds light vertices from its front and heavy ones from its back
+// (together at most V entries).
 constexpr size_t NA_OFF_QUEUE = NOALLOC_WORDS * 4;
-constexpr size_t NA_OFF_COUNT = NA_OFF_QUEUE + 2 * NOALLOC_MAX_VERTICES * 4;
-constexpr size_t NA_BYTES = NA_OFF_COUNT + 256;
+constexpr size_t NA_OFF_CTL = NA_OFF_QUEUE + 2 * NOALLOC_MAX_VERTICES * 4;
+
+constexpr int NA_T = 1024;        // threads per CTA, one per SM
+constexpr int NA_ILP = 4;         // entries a lane has in flight together
+constexpr int NA_HEAVY = 256;     // degree from which a CTA takes a vertex's row
+constexpr int NA_HUGE = 1 << 15;  // ... and from which all CTAs share it
+constexpr int NA_HUGE_CAP = 1024; // listed ones per level (more are rows of one CTA)
+constexpr int NA_SOLO = 1024;     // light frontier vertices up to which CTA 0 runs alone
+constexpr int NA_SOLO_CAP = 2048; // frontier entries it keeps in shared memory
+constexpr int NA_SOLO_LEVELS = 4096;  // levels it runs before it meets the others again
+
+struct NaCtl {
+  uint32_t arrived;   // barrier arrivals, all barriers of a launch together
+  int32_t err;        // a wait ran out
+  int32_t level[2];   // per phase (mod 2): the level CTA 0 reached running alone
+  int32_t n[3][4];    // per phase (mod 3): light, heavy, huge frontier vertices
+  int32_t huge[2][NA_HUGE_CAP];
+};
+constexpr size_t NA_BYTES = (NA_OFF_CTL + sizeof(NaCtl) + 255) / 256 * 256;
 
 static __device__ __align__(256) unsigned char g_noalloc_scratch[NA_BYTES];
 
-struct NaView {
+struct NaArgs {
   uint32_t* visited;
   int32_t* queue[2];
-  int32_t* count;
+  NaCtl* ctl;
+  const int64_t* off;
+  const int32_t* adj;
+  int32_t* depth;
+  int64_t V;
+  int32_t src;
 };
 
-__host__ __device__ inline NaView na_view(unsigned char* base) {
-  NaView v;
-  v.visited = reinterpret_cast<uint32_t*>(base);
-  v.queue[0] = reinterpret_cast<int32_t*>(base + NA_OFF_QUEUE);
-  v.queue[1] = v.queue[0] + NOALLOC_MAX_VERTICES;
-  v.count = reinterpret_cast<int32_t*>(base + NA_OFF_COUNT);
-  return v;
-}
-
-// Clears what must start at zero (visited bits, counters) and fills depth with -1.
-__global__ void k_na_clear(unsigned char* scratch, int64_t V, int32_t* depth) {
-  NaView s = na_view(scratch);
-  const int64_t tid = blockIdx.x * (int64_t)blockDim.x + threadIdx.x, nth = (int64_t)gridDim.x * blockDim.x;
-  const int64_t W = (V + 31) / 32;
-  for (int64_t i = tid; i < W; i += nth) s.visited[i] = 0;
-  for (int64_t i = tid; i < V; i += nth) depth[i] = -1;
-  if (tid < 2) s.count[tid] = 0;
-}
-
-__global__ void k_na_seed(unsigned char* scratch, int32_t src, int32_t* depth) {
-  NaView s = na_view(scratch);
-  depth[src] = 0;
-  s.visited[src >> 5] = 1u << (src & 31);
-  s.queue[0][0] = src;
-  s.count[0] = 1;
-  s.count[1] = 0;
-}
-
-// One top-down level: a warp per frontier vertex, lanes over its neighbours.
-__global__ void k_na_expand(unsigned char* scratch, const int64_t* __restrict__ off, const int32_t* __restrict__ adj,
-                            int cur, int32_t next_level, int32_t* depth) {
-  NaView s = na_view(scratch);
-  const int32_t* q = s.queue[cur];
-  int32_t* qn = s.queue[cur ^ 1];
-  int32_t* cn = &s.count[cur ^ 1];
-  const int n = s.count[cur];
-  const int lane = threadIdx.x & 31;
-  const int gw = (int)((blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5);
-  const int nw = (int)(((int64_t)gridDim.x * blockDim.x) >> 5);
-  for (int i = gw; i < n; i += nw) {
-    const int u = q[i];
-    const int64_t beg = off[u], end = off[u + 1];
-    for (int64_t e0 = beg; e0 < end; e0 += 32) {
-      const int64_t e = e0 + lane;
-      bool mine = false;
-      int v = 0;
-      if (e < end) {
-        v = adj[e];
-        const uint32_t b = 1u << (v & 31);
-        if (!(s.visited[v >> 5] & b) && !(atomicOr(&s.visited[v >> 5], b) & b)) {
-          mine = true;
-          depth[v] = next_level;
-        }
-      }
-      const unsigned m = __ballot_sync(0xffffffffu, mine);
-      if (m) {
-        const int leader = __ffs(m) - 1;
-        int base = 0;
-        if (lane == leader) base = atomicAdd(cn, __popc(m));
-        base = __shfl_sync(0xffffffffu, base, leader);
-        if (mine) qn[base + __popc(m & ((1u << lane) - 1))] = v;
+// One CTA's arrival at the grid-wide barrier and the wait for all: target is
+// the number of arrivals after which it opens. False when a wait ran out
+// anywhere (every CTA then leaves).
+__device__ bool na_barrier(NaCtl* c, uint32_t target) {
+  __shared__ int s_ok;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    atomicAdd(&c->arrived, 1u);
+    int ok = 1;
+    for (int spins = 0;; ++spins) {
+      uint32_t x;
+      asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(x) : "l"(&c->arrived) : "memory");
+      if (x >= target) break;
+      if (spins > 64) __nanosleep(64);
+      if (spins >= SPIN_LIMIT * 4 || ((spins & 63) == 63 && *(volatile int32_t*)&c->err)) {
+        *(volatile int32_t*)&c->err = 1;
+        ok = 0;
+        break;
       }
     }
+    __threadfence();
+    s_ok = ok && !*(volatile int32_t*)&c->err;
   }
+  __syncthreads();
+  return s_ok != 0;
+}
+
+// Where the claimed vertices of a level go.
+struct NaOut {
+  int32_t* q;        // the next level's queue
+  int32_t* n;        // its global counts
+  int32_t* huge;     // its huge list
+  // CTA 0 alone: light vertices go to shared memory while they fit
+  int4* s_q;
+  int32_t* s_n;      // [3]: light, heavy, huge
+};
+
+// Claims the neighbours v[] (negative: none) of frontier vertices for `ln` and
+// queues the won ones by degree. One warp, converged.
+template <bool SOLO>
+__device__ __forceinline__ void na_claim(const NaArgs& a, const int (&v)[NA_ILP], int ln, const NaOut& o) {
+  const int lane = threadIdx.x & 31;
+  bool open[NA_ILP], mine[NA_ILP];
+  int64_t st[NA_ILP];
+  int d[NA_ILP];
+  // A look through L1 saves most atomics (a stale word only costs one); a
+  // small frontier claims at once: the look would lengthen its chain.
+#pragma unroll
+  for (int i = 0; i < NA_ILP; ++i)
+    open[i] = v[i] >= 0 && (SOLO || !((__ldca(a.visited + (v[i] >> 5)) >> (v[i] & 31)) & 1u));
+#pragma unroll
+  for (int i = 0; i < NA_ILP; ++i) {
+    mine[i] = false;
+    st[i] = 0;
+    d[i] = 0;
+    if (open[i]) {  // the row is read beside the claim
+      const int64_t o0 = __ldg(a.off + v[i]), o1 = __ldg(a.off + v[i] + 1);
+      const uint32_t b = 1u << (v[i] & 31);
+      mine[i] = !(atomicOr(a.visited + (v[i] >> 5), b) & b);
+      st[i] = o0;
+      d[i] = (int)min(o1 - o0, (int64_t)INT32_MAX);
+    }
+  }
+  int n_light = 0;
+#pragma unroll
+  for (int i = 0; i < NA_ILP; ++i) {
+    if (mine[i]) a.depth[v[i]] = ln;
+    n_light += __popc(__ballot_sync(FULL, mine[i] && d[i] > 0 && d[i] < NA_HEAVY));
+  }
+  int base = 0;
+  if (n_light) {
+    if (lane == 0) base = atomicAdd(SOLO ? o.s_n : o.n, n_light);
+    base = __shfl_sync(FULL, base, 0);
+  }
+#pragma unroll
+  for (int i = 0; i < NA_ILP; ++i) {
+    const bool light = mine[i] && d[i] > 0 && d[i] < NA_HEAVY;
+    const unsigned m = __ballot_sync(FULL, light);
+    if (light) {
+      const int at = base + __popc(m & lanemask_lt());
+      if (SOLO && at < NA_SOLO_CAP)
+        o.s_q[at] = make_int4(v[i], d[i], (int)(uint32_t)st[i], (int)(uint32_t)((uint64_t)st[i] >> 32));
+      else
+        o.q[at] = v[i];
+    }
+    base += __popc(m);
+    if (mine[i] && d[i] >= NA_HEAVY) {  // few: one atomic each
+      const int h = d[i] >= NA_HUGE ? atomicAdd((SOLO ? o.s_n : o.n) + 2, 1) : NA_HUGE_CAP;
+      if (h < NA_HUGE_CAP) o.huge[h] = v[i];
+      else o.q[NOALLOC_MAX_VERTICES - 1 - atomicAdd((SOLO ? o.s_n : o.n) + 1, 1)] = v[i];
+    }
+  }
+}
+
+// The concatenated rows of a warp's light vertices (lane: one row of d entries
+// from st, d = 0: none), NA_ILP rounds of 32 entries together.
+template <bool SOLO>
+__device__ __forceinline__ void na_rows(const NaArgs& a, int d, int64_t st, int ln, const NaOut& o) {
+  const int lane = threadIdx.x & 31;
+  int incl = d;
+#pragma unroll
+  for (int ofs = 1; ofs < 32; ofs <<= 1) {
+    const int y = __shfl_up_sync(FULL, incl, ofs);
+    if (lane >= ofs) incl += y;
+  }
+  const int total = __shfl_sync(FULL, incl, 31), excl = incl - d;
+  for (int r0 = 0; r0 < total; r0 += 32 * NA_ILP) {
+    int v[NA_ILP];
+#pragma unroll
+    for (int i = 0; i < NA_ILP; ++i) {
+      v[i] = -1;
+      if (r0 + 32 * i < total) {  // warp-uniform
+        const int k = r0 + 32 * i + lane;
+        int j = 0;
+#pragma unroll
+        for (int step = 16; step > 0; step >>= 1) {
+          const int ev = __shfl_sync(FULL, excl, (j + step) & 31);
+          if (j + step < 32 && ev <= k) j += step;
+        }
+        const int64_t sj = __shfl_sync(FULL, st, j);
+        const int ej = __shfl_sync(FULL, excl, j);
+        if (k < total) v[i] = __ldg(a.adj + sj + (k - ej));
+      }
+    }
+    na_claim<SOLO>(a, v, ln, o);
+  }
+}
+
+// Entries first, first + step, ... below end of one long row, 32 * NA_ILP
+// consecutive ones per warp and turn.
+__device__ __forceinline__ void na_slice(const NaArgs& a, int64_t first, int64_t step, int64_t end, int ln,
+                                         const NaOut& o) {
+  const int lane = threadIdx.x & 31;
+  for (int64_t e0 = first; e0 < end; e0 += step) {
+    int v[NA_ILP];
+#pragma unroll
+    for (int i = 0; i < NA_ILP; ++i) {
+      const int64_t e = e0 + 32 * i + lane;
+      v[i] = e < end ? __ldg(a.adj + e) : -1;
+    }
+    na_claim<false>(a, v, ln, o);
+  }
+}
+
+// CTA 0 alone, from level L on: runs levels while all frontier vertices are
+// light and fit, at most NA_SOLO_LEVELS, and leaves the next frontier in the
+// queues, its counts in `out` and its level in *level.
+__device__ void na_solo(const NaArgs& a, int L, int n, int4 (*s_q)[NA_SOLO_CAP], int32_t (*s_n)[3], int32_t* out,
+                        int32_t* level) {
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  constexpr int NWARP = NA_T / 32;
+  const int32_t* q0 = a.queue[L & 1];
+  for (int i = tid; i < n; i += NA_T) {
+    const int u = __ldcg(q0 + i);
+    const int64_t st = a.off[u];
+    s_q[L & 1][i] = make_int4(u, (int)(a.off[u + 1] - st), (int)(uint32_t)st, (int)(uint32_t)((uint64_t)st >> 32));
+  }
+  if (tid < 3) s_n[0][tid] = s_n[1][tid] = 0;
+  __syncthreads();
+  int n2 = 0, n3 = 0;
+  for (int run = 0;; ++run) {
+    const int cur = L & 1, nxt = cur ^ 1;
+    const NaOut o{a.queue[nxt], nullptr, a.ctl->huge[nxt], s_q[nxt], s_n[nxt]};
+    // up to 32 rows per warp, spread over all warps
+    const int k = min(32, (n + NWARP - 1) / NWARP);
+    for (int first = warp * k; first < n; first += NWARP * k) {
+      int d = 0;
+      int64_t st = 0;
+      if (lane < k && first + lane < n) {
+        const int4 e = s_q[cur][first + lane];
+        d = e.y;
+        st = (int64_t)(((uint64_t)(uint32_t)e.w << 32) | (uint32_t)e.z);
+      }
+      na_rows<true>(a, d, st, L + 1, o);
+    }
+    __syncthreads();
+    n = s_n[nxt][0];
+    n2 = s_n[nxt][1];
+    n3 = s_n[nxt][2];
+    ++L;
+    if (n == 0 || n > NA_SOLO_CAP || n2 || n3 || run + 1 >= NA_SOLO_LEVELS) break;
+    if (tid < 3) s_n[cur][tid] = 0;  // takes the counts of the level after
+    __syncthreads();
+  }
+  // hand over: stored entries to the queue (the rest are there), counts
+  int32_t* q = a.queue[L & 1];
+  for (int i = tid; i < min(n, NA_SOLO_CAP); i += NA_T) q[i] = s_q[L & 1][i].x;
+  if (tid == 0) {
+    out[0] = n;
+    out[1] = n2;
+    out[2] = n3;
+    *level = L;
+  }
+}
+
+// The whole traversal (cooperative launch; the control block is zeroed before).
+// Bound by the atomics and scattered reads of the entries on wide levels and
+// by the barrier and the chain entry -> row -> claim on narrow ones. R-MAT
+// s18: 0.23 ms; a 700 x 700 grid: 4.2 ms, 2.6 us a level (a launch and a host
+// wait per level, a warp per vertex: 1.17 and 18.8 ms). 1024 threads and one
+// CTA per SM beat two of 512 (grid 5.2 ms: CTA 0 alone has more lanes); rows
+// of one CTA from 256 entries beat 64 and 1024 (0.28 ms at s18), four entries
+// per lane two (0.27 ms).
+// A phase is one level of all CTAs, or several of CTA 0 alone; a barrier ends
+// it. Phase p reads the counts n[p % 3], fills n[(p + 1) % 3] and clears
+// n[(p + 2) % 3], which no CTA reads any more once it is past the barrier
+// before: a CTA that is late to read n[p % 3] still finds it unchanged.
+__global__ void __launch_bounds__(NA_T, 1) k_na_run(NaArgs a) {
+  extern __shared__ int4 s_dyn[];
+  int4(*s_q)[NA_SOLO_CAP] = reinterpret_cast<int4(*)[NA_SOLO_CAP]>(s_dyn);
+  __shared__ int32_t s_n[2][3];
+  NaCtl* c = a.ctl;
+  const int64_t tid = blockIdx.x * (int64_t)NA_T + threadIdx.x, nth = (int64_t)gridDim.x * NA_T;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  constexpr int NWARP = NA_T / 32;
+  const int64_t W = (a.V + 31) >> 5;
+  for (int64_t i = tid; i < W; i += nth) a.visited[i] = i == (a.src >> 5) ? 1u << (a.src & 31) : 0u;
+  for (int64_t i = tid; i < a.V; i += nth) a.depth[i] = i == a.src ? 0 : -1;
+  if (tid == 0) {
+    const int64_t d = a.off[a.src + 1] - a.off[a.src];
+    if (d > 0 && d < NA_HEAVY) {
+      a.queue[0][0] = a.src;
+      c->n[0][0] = 1;
+    } else if (d >= NA_HEAVY) {
+      a.queue[0][NOALLOC_MAX_VERTICES - 1] = a.src;
+      c->n[0][1] = 1;
+    }
+  }
+  uint32_t target = 0;
+  if (!na_barrier(c, target += gridDim.x)) return;
+  int L = 0;
+  for (int p = 0; L <= a.V; ++p) {
+    const int32_t* cnt = c->n[p % 3];
+    int32_t* next = c->n[(p + 1) % 3];
+    const int n_l = __ldcg(cnt), n_h = __ldcg(cnt + 1), n_g = min(__ldcg(cnt + 2), NA_HUGE_CAP);
+    if (n_l + n_h + n_g == 0) return;
+    if (tid < 3) c->n[(p + 2) % 3][tid] = 0;
+    if (n_l <= NA_SOLO && n_h + n_g == 0) {
+      if (blockIdx.x == 0) na_solo(a, L, n_l, s_q, s_n, next, &c->level[p & 1]);
+      if (!na_barrier(c, target += gridDim.x)) return;
+      L = __ldcg(&c->level[p & 1]);
+      continue;
+    }
+    const int32_t* q = a.queue[L & 1];
+    const NaOut o{a.queue[(L + 1) & 1], next, c->huge[(L + 1) & 1], nullptr, nullptr};
+    const int64_t gw = (int64_t)blockIdx.x * NWARP + warp, nw = (int64_t)gridDim.x * NWARP;
+    for (int i = 0; i < n_g; ++i) {  // rows shared by all CTAs
+      const int u = __ldcg(c->huge[L & 1] + i);
+      const int64_t beg = a.off[u], end = a.off[u + 1];
+      na_slice(a, beg + gw * 32 * NA_ILP, nw * 32 * NA_ILP, end, L + 1, o);
+    }
+    for (int i = blockIdx.x; i < n_h; i += gridDim.x) {  // rows of one CTA
+      const int u = __ldcg(q + NOALLOC_MAX_VERTICES - 1 - i);
+      const int64_t beg = a.off[u], end = a.off[u + 1];
+      na_slice(a, beg + warp * 32 * NA_ILP, NWARP * 32 * NA_ILP, end, L + 1, o);
+    }
+    // up to 32 light rows per warp, spread over all warps
+    const int k = (int)min((int64_t)32, (n_l + nw - 1) / nw);
+    for (int64_t first = gw * k; first < n_l; first += nw * k) {
+      int d = 0;
+      int64_t st = 0;
+      if (lane < k && first + lane < n_l) {
+        const int u = __ldcg(q + first + lane);
+        st = a.off[u];
+        d = (int)(a.off[u + 1] - st);
+      }
+      na_rows<false>(a, d, st, L + 1, o);
+    }
+    ++L;
+    if (!na_barrier(c, target += gridDim.x)) return;
+  }
+  if (tid == 0) c->err = 2;  // more levels than vertices
 }
 
 // Device address of the scratch array, looked up once per device and CUDA
@@ -183,30 +424,43 @@ extern "C" int ent_bfs_noalloc(const int64_t* beg_pos_dev, const int32_t* csr_de
   int rc = na_scratch_for_current_device(&scratch);
   if (rc != ENT_OK) return rc;
   cudaStream_t s = (cudaStream_t)stream;
-  int dev_sms = 148;
-  int dev = 0;
+  int dev = 0, sms = 148, per_sm = 1;
   cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&dev_sms, cudaDevAttrMultiProcessorCount, dev);
-  const int blocks = dev_sms * 8;
-  k_na_clear<<<blocks, 256, 0, s>>>(scratch, vert_count, depth_dev);
-  k_na_seed<<<1, 1, 0, s>>>(scratch, src, depth_dev);
-  g_kernel_launches += 2;
-  NaView view = na_view(scratch);
-  int cur = 0;
-  for (int64_t level = 0; level <= vert_count; ++level) {
-    k_na_expand<<<blocks, 256, 0, s>>>(scratch, beg_pos_dev, csr_dev, cur, (int32_t)(level + 1), depth_dev);
-    g_kernel_launches++;
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return fail(ENT_ERR_CUDA, "level kernel launch failed: %s", cudaGetErrorString(e));
-    int32_t next = 0;
-    // 4-byte read of the next frontier size into a host variable (no allocation)
-    e = cudaMemcpyAsync(&next, view.count + (cur ^ 1), sizeof(int32_t), cudaMemcpyDeviceToHost, s);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-    if (e != cudaSuccess) return fail(ENT_ERR_CUDA, "level sync failed: %s", cudaGetErrorString(e));
-    if (next == 0) return ENT_OK;
-    e = cudaMemsetAsync(view.count + cur, 0, sizeof(int32_t), s);
-    if (e != cudaSuccess) return fail(ENT_ERR_CUDA, "counter reset failed: %s", cudaGetErrorString(e));
-    cur ^= 1;
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  constexpr size_t smem = 2 * NA_SOLO_CAP * sizeof(int4);
+  cudaError_t e = cudaFuncSetAttribute(k_na_run, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_na_run, NA_T, smem);
+  if (e != cudaSuccess) return fail(ENT_ERR_CUDA, "kernel setup failed: %s", cudaGetErrorString(e));
+  NaArgs a;
+  a.visited = reinterpret_cast<uint32_t*>(scratch);
+  a.queue[0] = reinterpret_cast<int32_t*>(scratch + NA_OFF_QUEUE);
+  a.queue[1] = a.queue[0] + NOALLOC_MAX_VERTICES;
+  a.ctl = reinterpret_cast<NaCtl*>(scratch + NA_OFF_CTL);
+  a.off = beg_pos_dev;
+  a.adj = csr_dev;
+  a.depth = depth_dev;
+  a.V = vert_count;
+  a.src = src;
+  e = cudaMemsetAsync(a.ctl, 0, sizeof(NaCtl), s);
+  if (e != cudaSuccess) return fail(ENT_ERR_CUDA, "control reset failed: %s", cudaGetErrorString(e));
+  // Every CTA must be resident (they wait on one another): as many as fit, fewer
+  // for small graphs, whose barriers are then cheaper. Where part of the GPU is
+  // set aside (MPS, a partition) the launch is refused and tried smaller.
+  void* args[1] = {&a};
+  int grid = (int)std::min<int64_t>((int64_t)sms * std::max(1, std::min(per_sm, 1)), (vert_count + 255) / 256);
+  for (;; grid >>= 1) {
+    e = cudaLaunchCooperativeKernel((const void*)k_na_run, dim3(grid), dim3(NA_T), args, smem, s);
+    if (e != cudaErrorCooperativeLaunchTooLarge || grid <= 1) break;
+    cudaGetLastError();
   }
-  return fail(ENT_ERR_INTERNAL, "level loop did not terminate");
+  if (e != cudaSuccess) return fail(ENT_ERR_CUDA, "traversal launch failed: %s", cudaGetErrorString(e));
+  g_kernel_launches++;
+  int32_t err = 0;
+  // 4-byte read of the status into a host variable (no allocation)
+  e = cudaMemcpyAsync(&err, &a.ctl->err, sizeof(int32_t), cudaMemcpyDeviceToHost, s);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+  if (e != cudaSuccess) return fail(ENT_ERR_CUDA, "traversal failed: %s", cudaGetErrorString(e));
+  if (err == 1) return fail(ENT_ERR_TIMEOUT, "a wait between the traversal's CTAs ran out");
+  if (err) return fail(ENT_ERR_INTERNAL, "level loop did not terminate");
+  return ENT_OK;
 }
