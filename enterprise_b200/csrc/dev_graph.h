@@ -51,6 +51,7 @@ struct ent_graph {
   uint32_t* active = nullptr;
   int4* lead = nullptr;
   int64_t n_active = 0;  // vertices with a row are traversal ids [0, n_active); V in caller order
+  bool rows_sorted = false;  // every adj row is ascending (known with an order of its own)
   cudaStream_t stream = nullptr;
   ent_bfs_opts opts;
   std::mutex mu;
@@ -60,6 +61,7 @@ struct ent_graph {
   int32_t probe_levels = -1;  // depth of the graph as probed by its first auto-mode batch (-1: not yet)
   void* stage = nullptr;      // device rows of batches whose results go to host memory
   size_t stage_cap = 0;
+  void* val = nullptr;        // ent_validate's scratch: its result words, a depth per vertex
 };
 
 namespace ent {

@@ -74,7 +74,7 @@ __global__ void __launch_bounds__(256) k_relabel_rows(const int64_t* __restrict_
                                                       const int64_t* __restrict__ toff,
                                                       const int32_t* __restrict__ perm,
                                                       const int32_t* __restrict__ inv, int64_t V, int64_t E,
-                                                      int32_t* __restrict__ out) {
+                                                      int32_t* __restrict__ out, int64_t* __restrict__ unsorted) {
   const int lane = threadIdx.x & 31;
   const int64_t gw = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
   const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
@@ -94,7 +94,10 @@ __global__ void __launch_bounds__(256) k_relabel_rows(const int64_t* __restrict_
     const int64_t r0 = __shfl_sync(0xffffffffu, mine, 0), r1 = __shfl_sync(0xffffffffu, mine, 1);
     for (int64_t e = c0 + lane; e < c1; e += 32) {
       const int64_t r = row_of(e, r0, r1);
-      out[e] = inv[adj[off[perm[r]] + (e - toff[r])]];
+      const int64_t at = off[perm[r]] + (e - toff[r]);
+      const int32_t u = adj[at];
+      if (e > toff[r] && adj[at - 1] > u) *unsorted = 1;  // a caller's row (validation searches sorted rows)
+      out[e] = inv[u];
     }
   }
 }
@@ -161,26 +164,30 @@ static cudaError_t build_traversal_order(ent_graph* g) {
   char* tmp = nullptr;
   e = cudaMalloc(&tmp, 256 + std::max(sz_a, sz_b) + t_cub);
   if (e != cudaSuccess) return e;
-  int64_t* n_active = (int64_t*)tmp;
+  int64_t* n_active = (int64_t*)tmp;  // [0], and [1]: some row is not sorted
   uint32_t* key = (uint32_t*)(tmp + 256);
   uint32_t* key2 = (uint32_t*)(tmp + 256 + sz_v);
   int32_t* id = (int32_t*)(tmp + 256 + 2 * sz_v);
   int32_t* rows = (int32_t*)(tmp + 256);
   void* cub_tmp = tmp + 256 + std::max(sz_a, sz_b);
-  k_degrees<<<blocks, 256, 0, s>>>(g->off, V, nullptr, key, id);
-  e = cub::DeviceRadixSort::SortPairs(cub_tmp, t_sort, key, key2, id, g->perm, V, 0, 32, s);
+  int64_t h[2] = {0, 0};
+  e = cudaMemsetAsync(n_active, 0, sizeof(h), s);
+  if (e == cudaSuccess) k_degrees<<<blocks, 256, 0, s>>>(g->off, V, nullptr, key, id);
+  if (e == cudaSuccess) e = cub::DeviceRadixSort::SortPairs(cub_tmp, t_sort, key, key2, id, g->perm, V, 0, 32, s);
   if (e == cudaSuccess) {
     k_labels<<<blocks, 256, 0, s>>>(key2, g->perm, V, g->deg, g->inv, n_active);
     e = cudaMemsetAsync(g->toff, 0, sizeof(int64_t), s);
   }
   if (e == cudaSuccess) e = cub::DeviceScan::InclusiveSum(cub_tmp, t_scan, g->deg, g->toff + 1, V, s);
   if (e == cudaSuccess) {
-    k_relabel_rows<<<blocks, 256, 0, s>>>(g->off, g->adj, g->toff, g->perm, g->inv, V, E, rows);
+    k_relabel_rows<<<blocks, 256, 0, s>>>(g->off, g->adj, g->toff, g->perm, g->inv, V, E, rows, n_active + 1);
     e = cub::DeviceSegmentedSort::SortKeys(cub_tmp, t_seg, rows, g->trav, (int)E, (int)V, g->toff, g->toff + 1, s);
   }
   g_kernel_launches += 3;
-  if (e == cudaSuccess) e = cudaMemcpyAsync(&g->n_active, n_active, sizeof(int64_t), cudaMemcpyDeviceToHost, s);
+  if (e == cudaSuccess) e = cudaMemcpyAsync(h, n_active, sizeof(h), cudaMemcpyDeviceToHost, s);
   const cudaError_t e2 = cudaStreamSynchronize(s);
+  g->n_active = h[0];
+  g->rows_sorted = h[1] == 0;
   cudaFree(tmp);
   return e != cudaSuccess ? e : e2;
 }
@@ -231,6 +238,7 @@ static void graph_free(ent_graph* g) {
   if (g->bws) destroy_batch_workspace(g->bws);
   if (g->lanes) destroy_deep_lanes(g->lanes);
   if (g->stage) cudaFree(g->stage);
+  if (g->val) cudaFree(g->val);
   if (g->slab) cudaFree(g->slab);
   if (g->off) cudaFree(g->off);
   if (g->adj) cudaFree(g->adj);
