@@ -41,7 +41,7 @@ SOURCES = [
     "replicas.cpp",
     "tune.cpp",
 ]
-HEADERS = ["gen_common.h", "ent_internal.h", "dev_graph.h", "dev_common.cuh", "batch_internal.h"]
+HEADERS = ["gen_common.h", "ent_internal.h", "dev_graph.h", "dev_common.cuh", "batch_internal.h", "bfs_resident.cuh"]
 
 
 def nvcc() -> str:

@@ -83,34 +83,6 @@ struct NaArgs {
   int32_t src;
 };
 
-// One CTA's arrival at the grid-wide barrier and the wait for all: target is
-// the number of arrivals after which it opens. False when a wait ran out
-// anywhere (every CTA then leaves).
-__device__ bool na_barrier(NaCtl* c, uint32_t target) {
-  __shared__ int s_ok;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    __threadfence();
-    atomicAdd(&c->arrived, 1u);
-    int ok = 1;
-    for (int spins = 0;; ++spins) {
-      uint32_t x;
-      asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(x) : "l"(&c->arrived) : "memory");
-      if (x >= target) break;
-      if (spins > 64) __nanosleep(64);
-      if (spins >= SPIN_LIMIT * 4 || ((spins & 63) == 63 && *(volatile int32_t*)&c->err)) {
-        *(volatile int32_t*)&c->err = 1;
-        ok = 0;
-        break;
-      }
-    }
-    __threadfence();
-    s_ok = ok && !*(volatile int32_t*)&c->err;
-  }
-  __syncthreads();
-  return s_ok != 0;
-}
-
 // Where the claimed vertices of a level go.
 struct NaOut {
   int32_t* q;        // the next level's queue
@@ -313,7 +285,7 @@ __global__ void __launch_bounds__(NA_T, 1) k_na_run(NaArgs a) {
     }
   }
   uint32_t target = 0;
-  if (!na_barrier(c, target += gridDim.x)) return;
+  if (!grid_barrier(&c->arrived, &c->err, target += gridDim.x, [] {})) return;
   int L = 0;
   for (int p = 0; L <= a.V; ++p) {
     const int32_t* cnt = c->n[p % 3];
@@ -323,7 +295,7 @@ __global__ void __launch_bounds__(NA_T, 1) k_na_run(NaArgs a) {
     if (tid < 3) c->n[(p + 2) % 3][tid] = 0;
     if (n_l <= NA_SOLO && n_h + n_g == 0) {
       if (blockIdx.x == 0) na_solo(a, L, n_l, s_q, s_n, next, &c->level[p & 1]);
-      if (!na_barrier(c, target += gridDim.x)) return;
+      if (!grid_barrier(&c->arrived, &c->err, target += gridDim.x, [] {})) return;
       L = __ldcg(&c->level[p & 1]);
       continue;
     }
@@ -353,7 +325,7 @@ __global__ void __launch_bounds__(NA_T, 1) k_na_run(NaArgs a) {
       na_rows<false>(a, d, st, L + 1, o);
     }
     ++L;
-    if (!na_barrier(c, target += gridDim.x)) return;
+    if (!grid_barrier(&c->arrived, &c->err, target += gridDim.x, [] {})) return;
   }
   if (tid == 0) c->err = 2;  // more levels than vertices
 }

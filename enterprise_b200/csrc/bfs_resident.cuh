@@ -1,0 +1,625 @@
+// The whole single-source traversal as one cooperative kernel, for graphs that
+// the level kernels of bfs_single.cu cannot keep busy (included there).
+//
+// On a small graph the level loop costs more than the levels: a level is three
+// kernel nodes and half a while-node iteration, about 20 us whatever it does
+// (R-MAT s12: 124 us a traversal, 16 us of them in kernels; s20: 138 us). Here
+// the CTAs stay resident and go from level to level through a grid-wide
+// barrier, and every CTA takes the level's decision by itself from the counts
+// that the barrier published, so no level ends in one CTA's chain.
+//
+// A phase is one of
+//   * a top-down level: rows split by degree over lane groups, CTAs and the
+//     whole grid (as in bfs_noalloc.cu); a claim queues its vertex by degree
+//     and sets its frontier bit, so that either direction can follow;
+//   * a bottom-up level: a warp per status word, as in k_expand;
+//   * a queue build, from the frontier bitmap, where a bottom-up level hands
+//     over to top-down;
+//   * a run of small top-down levels by CTA 0 alone, its frontier in shared
+//     memory (counted as small-frontier levels), while the others wait.
+// Phase p reads the counts n[p % 3] and acc[p % 3], fills those of p + 1 and
+// clears those of p + 2, which no CTA reads any more once it is past the
+// barrier before; frontier bitmaps rotate the same way per level. All waits
+// are bounded: one that runs out sets the error bit and every CTA leaves.
+//
+// Not here: parents, hub tables and runs with the small-frontier mode off stay
+// with the level kernels.
+#pragma once
+
+constexpr int RT = 1024;          // threads per CTA, one per SM (64 registers a thread)
+constexpr int RW = RT / 32;
+constexpr int R_ILP = 4;          // row entries a lane has in flight together
+constexpr int R_BW = 3;           // bottom-up: status words a warp has in flight together
+constexpr int R_BILP = 2;         // ... and row entries of each per step
+constexpr int R_HEAVY = 256;      // degree from which a CTA takes a vertex's row
+constexpr int R_HUGE = 1 << 15;   // ... and from which all CTAs share it
+constexpr int R_SOLO = 2048;      // frontier up to which CTA 0 starts to run alone
+constexpr int R_SOLO_M = 16384;   // ... and its degree sum; it leaves above twice that
+constexpr int R_SOLO_CAP = 4096;  // frontier entries it keeps in shared memory
+constexpr int R_SOLO_LEVELS = 4096;  // levels it runs before it meets the others again
+
+struct ResCtl {
+  uint32_t arrived;  // barrier arrivals of this launch
+  int32_t err;       // a wait ran out
+  int32_t pad[2];
+  int32_t n[3][4];   // light, heavy, huge frontier vertices of a phase
+  unsigned long long acc[3][2];  // vertices and degree sum that a phase found
+  struct {
+    int64_t n_f, m_f, n_vis, m_vis;
+    int32_t level, pad;
+  } solo[2];         // where CTA 0 got to alone, by phase parity
+};
+
+struct ResArgs {
+  ResCtl* rc;
+  uint32_t* fb[3];
+  int32_t* queue[2];  // light vertices from the front, heavy ones from the back (V entries)
+  int32_t* huge[2];
+};
+
+enum { RK_TD, RK_BU, RK_QUEUE, RK_SOLO, RK_DONE };
+
+// What every CTA knows about the phase to come (thread 0 keeps it current).
+struct ResState {
+  int32_t kind, L, f, p;      // f: fb index of the frontier
+  int32_t n_l, n_h, n_g;
+  int32_t td_levels, bu_levels, narrow_levels, err;
+  int64_t n_f, m_f, n_vis, m_vis;
+};
+
+__device__ __forceinline__ int64_t ldcg64(const void* p) {
+  return (int64_t)__ldcg(reinterpret_cast<const long long*>(p));
+}
+
+// The kind of a top-down level over the queued frontier.
+__device__ __forceinline__ int res_td_kind(const LevelArgs& a, const ResState& s) {
+  return s.n_h + s.n_g == 0 && s.n_l <= R_SOLO && s.n_f <= a.narrow_f && s.m_f <= min(a.narrow_m, (int64_t)R_SOLO_M)
+             ? RK_SOLO
+             : RK_TD;
+}
+
+// After phase s.p (thread 0): the next one, from the counts the barrier
+// published. The rules are k_inspect's.
+__device__ void res_advance(const LevelArgs& a, const ResArgs& r, ResState& s) {
+  const ResCtl* c = r.rc;
+  const int q = (s.p + 1) % 3;
+  const int kind = s.kind;
+  const int32_t n_l = __ldcg(&c->n[q][0]), n_h = __ldcg(&c->n[q][1]), n_g = __ldcg(&c->n[q][2]);
+  int64_t n_next = 0, m_next = 0;
+  if (kind == RK_SOLO) {
+    const auto* so = &c->solo[s.p & 1];
+    const int L = __ldcg(&so->level);
+    n_next = ldcg64(&so->n_f);
+    m_next = ldcg64(&so->m_f);
+    s.n_vis = ldcg64(&so->n_vis);
+    s.m_vis = ldcg64(&so->m_vis);
+    s.td_levels += L - s.L;
+    s.narrow_levels += L - s.L;
+    s.L = L;
+  } else if (kind != RK_QUEUE) {
+    n_next = ldcg64(&c->acc[q][0]);
+    m_next = ldcg64(&c->acc[q][1]);
+    s.n_vis += n_next;
+    s.m_vis += m_next;
+    s.L += 1;
+    if (kind == RK_TD) s.td_levels += 1;
+    else s.bu_levels += 1;
+  }
+  s.p += 1;
+  s.n_l = n_l;
+  s.n_h = n_h;
+  s.n_g = n_g;
+  if (kind == RK_QUEUE) {
+    s.kind = res_td_kind(a, s);
+    return;
+  }
+  const int64_t n_before = s.n_f;
+  s.f = (s.f + 1) % 3;
+  s.n_f = n_next;
+  s.m_f = m_next;
+  bool done = n_next == 0;
+  if (s.L >= a.max_levels && !done) {
+    s.err |= 4;
+    done = true;
+  }
+  if (s.n_vis > a.V) {
+    s.err |= 8;
+    done = true;
+  }
+  if (done) {
+    s.kind = RK_DONE;
+    return;
+  }
+  if (kind == RK_BU) {
+    const bool to_td = a.policy == ENT_POLICY_BEAMER && (double)n_next < (double)a.V / a.beta && n_next < n_before;
+    s.kind = to_td ? RK_QUEUE : RK_BU;
+    return;
+  }
+  bool bu = a.policy == ENT_POLICY_BU_ONLY;
+  if (a.policy == ENT_POLICY_BEAMER) bu = (double)m_next > (double)(a.E - s.m_vis) / a.alpha;
+  if (a.policy == ENT_POLICY_REFERENCE) bu = (double)m_next >= a.ref_ratio * (double)a.E;
+  s.kind = bu ? RK_BU : res_td_kind(a, s);
+}
+
+// Where the claims of a top-down phase go, and what they add up to.
+struct ResOut {
+  uint32_t* fb;      // the next frontier's bits (not while CTA 0 runs alone)
+  int32_t* q;
+  int32_t* huge;
+  int32_t* n;        // counts: global, or CTA 0's own in shared memory
+  int4* s_q;         // CTA 0 alone: entries in shared memory while they fit
+};
+
+// Queues vertex v (degree d, row start st) of a converged warp by degree;
+// n_light: the warp's light ones in all R_ILP rounds were counted at `base`.
+__device__ __forceinline__ void res_put_heavy(const LevelArgs& a, const ResOut& o, int v, int d) {
+  if (d >= R_HUGE) o.huge[atomicAdd(o.n + 2, 1)] = v;
+  else o.q[a.V - 1 - atomicAdd(o.n + 1, 1)] = v;
+}
+
+template <class DT, bool SOLO>
+__device__ __forceinline__ void res_claim(const LevelArgs& a, const int (&v)[R_ILP], int ln, DT* depth, const ResOut& o,
+                                          unsigned& my_n, unsigned long long& my_m) {
+  const int lane = threadIdx.x & 31;
+  bool open[R_ILP], mine[R_ILP];
+  int64_t st[R_ILP];
+  int d[R_ILP], id[R_ILP];
+#pragma unroll
+  for (int i = 0; i < R_ILP; ++i)
+    open[i] = v[i] >= 0 && (SOLO || !((__ldca(a.vis + (v[i] >> 5)) >> (v[i] & 31)) & 1u));
+#pragma unroll
+  for (int i = 0; i < R_ILP; ++i) {
+    mine[i] = false;
+    st[i] = 0;
+    d[i] = id[i] = 0;
+    if (open[i]) {  // row and degree, or degree and caller id, are read beside the claim
+      if (SOLO) {
+        st[i] = __ldg(a.off + v[i]);
+        d[i] = (int)(__ldg(a.off + v[i] + 1) - st[i]);
+      } else {
+        d[i] = __ldg(a.deg + v[i]);
+        id[i] = out_id(a, v[i]);
+      }
+      const uint32_t b = 1u << (v[i] & 31);
+      mine[i] = !(atomicOr(a.vis + (v[i] >> 5), b) & b);
+    }
+  }
+  int n_light = 0;
+#pragma unroll
+  for (int i = 0; i < R_ILP; ++i) {
+    if (mine[i]) {
+      if (!SOLO) {  // alone, depths and bits are written later: off the level's chain
+        depth[id[i]] = (DT)ln;
+        red_or(o.fb + (v[i] >> 5), 1u << (v[i] & 31));
+      }
+      my_n += 1;
+      my_m += (unsigned)d[i];
+    }
+    n_light += __popc(__ballot_sync(FULL, mine[i] && d[i] < R_HEAVY));
+  }
+  if (__any_sync(FULL, mine[0] || mine[1] || mine[2] || mine[3])) {
+    int base = 0;
+    if (n_light) {
+      if (lane == 0) base = atomicAdd(o.n, n_light);
+      base = __shfl_sync(FULL, base, 0);
+    }
+#pragma unroll
+    for (int i = 0; i < R_ILP; ++i) {
+      const bool light = mine[i] && d[i] < R_HEAVY;
+      const unsigned m = __ballot_sync(FULL, light);
+      if (light) {
+        const int at = base + __popc(m & lanemask_lt());
+        if (SOLO && at < R_SOLO_CAP)
+          o.s_q[at] = make_int4(v[i], d[i], (int)(uint32_t)st[i], (int)(uint32_t)((uint64_t)st[i] >> 32));
+        else
+          o.q[at] = v[i];
+      }
+      base += __popc(m);
+      if (mine[i] && d[i] >= R_HEAVY) res_put_heavy(a, o, v[i], d[i]);  // few: an atomic each
+    }
+  }
+}
+
+// The concatenated rows of a warp's light vertices (lane: d entries from st).
+template <class DT, bool SOLO>
+__device__ __forceinline__ void res_rows(const LevelArgs& a, int d, int64_t st, int ln, DT* depth, const ResOut& o,
+                                         unsigned& my_n, unsigned long long& my_m) {
+  const int lane = threadIdx.x & 31;
+  int incl = d;
+#pragma unroll
+  for (int ofs = 1; ofs < 32; ofs <<= 1) {
+    const int y = __shfl_up_sync(FULL, incl, ofs);
+    if (lane >= ofs) incl += y;
+  }
+  const int total = __shfl_sync(FULL, incl, 31), excl = incl - d;
+  for (int r0 = 0; r0 < total; r0 += 32 * R_ILP) {
+    int v[R_ILP];
+#pragma unroll
+    for (int i = 0; i < R_ILP; ++i) {
+      v[i] = -1;
+      if (r0 + 32 * i < total) {  // warp-uniform
+        const int k = r0 + 32 * i + lane;
+        int j = 0;
+#pragma unroll
+        for (int step = 16; step > 0; step >>= 1) {
+          const int ev = __shfl_sync(FULL, excl, (j + step) & 31);
+          if (j + step < 32 && ev <= k) j += step;
+        }
+        const int64_t sj = __shfl_sync(FULL, st, j);
+        const int ej = __shfl_sync(FULL, excl, j);
+        if (k < total) v[i] = __ldg(a.adj + sj + (k - ej));
+      }
+    }
+    res_claim<DT, SOLO>(a, v, ln, depth, o, my_n, my_m);
+  }
+}
+
+// Entries first, first + step, ... of one long row, 32 * R_ILP per warp and turn.
+template <class DT>
+__device__ __forceinline__ void res_slice(const LevelArgs& a, int64_t first, int64_t step, int64_t end, int ln,
+                                          DT* depth, const ResOut& o, unsigned& my_n, unsigned long long& my_m) {
+  const int lane = threadIdx.x & 31;
+  for (int64_t e0 = first; e0 < end; e0 += step) {
+    int v[R_ILP];
+#pragma unroll
+    for (int i = 0; i < R_ILP; ++i) {
+      const int64_t e = e0 + 32 * i + lane;
+      v[i] = e < end ? __ldg(a.adj + e) : -1;
+    }
+    res_claim<DT, false>(a, v, ln, depth, o, my_n, my_m);
+  }
+}
+
+template <class DT>
+__device__ void res_td(const LevelArgs& a, const ResArgs& r, const ResState& s, DT* depth, const ResOut& o,
+                       unsigned& my_n, unsigned long long& my_m) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int32_t* q = r.queue[s.L & 1];
+  const int ln = s.L + 1;
+  const int64_t gw = (int64_t)blockIdx.x * RW + warp, nw = (int64_t)gridDim.x * RW;
+  for (int i = 0; i < s.n_g; ++i) {  // rows shared by all CTAs
+    const int u = __ldcg(r.huge[s.L & 1] + i);
+    res_slice(a, a.off[u] + gw * 32 * R_ILP, nw * 32 * R_ILP, a.off[u + 1], ln, depth, o, my_n, my_m);
+  }
+  for (int i = blockIdx.x; i < s.n_h; i += gridDim.x) {  // rows of one CTA
+    const int u = __ldcg(q + a.V - 1 - i);
+    res_slice(a, a.off[u] + warp * 32 * R_ILP, (int64_t)RW * 32 * R_ILP, a.off[u + 1], ln, depth, o, my_n, my_m);
+  }
+  // up to 32 light rows per warp, spread over all warps
+  const int k = (int)min((int64_t)32, (s.n_l + nw - 1) / nw);
+  for (int64_t first = gw * k; first < s.n_l; first += nw * k) {
+    int d = 0;
+    int64_t st = 0;
+    if (lane < k && first + lane < s.n_l) {
+      const int u = __ldcg(q + first + lane);
+      st = a.off[u];
+      d = a.deg[u];
+    }
+    res_rows<DT, false>(a, d, st, ln, depth, o, my_n, my_m);
+  }
+}
+
+// One bottom-up level over the words of vertices that have rows (bu_expand
+// with nothing to list).
+template <class DT>
+__device__ void res_bu(const LevelArgs& a, const ResArgs& r, const ResState& s, DT* depth, unsigned& my_n,
+                       unsigned long long& my_m) {
+  const uint32_t* fbc = r.fb[s.f];
+  uint32_t* fbn = r.fb[(s.f + 1) % 3];
+  // read through L1: the barrier before this phase made it current
+  const auto is_front = [&](int u) { return (__ldca(fbc + (u >> 5)) >> (u & 31)) & 1u; };
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int64_t gw = (int64_t)blockIdx.x * RW + warp, nw = (int64_t)gridDim.x * RW;
+  const int64_t W = (a.n_active + 31) >> 5;
+  // R_BW words at a time through every stage together: a CTA of 64-register
+  // threads holds half the warps of k_expand, so each has to keep more reads in
+  // flight (R-MAT s24, whole traversal: 1 word 0.43 ms, 2 0.38, 3 0.355, 4 0.35;
+  // ER 2^23 d16: 0.65, 0.58, 0.55, 0.59).
+  for (int64_t w0 = gw; w0 < W; w0 += R_BW * nw) {
+    uint32_t vis[R_BW], mask[R_BW];
+    int4 ld[R_BW];
+    int d[R_BW], id[R_BW];
+    bool todo[R_BW];  // still to be found
+    bool found[R_BW];
+#pragma unroll
+    for (int t = 0; t < R_BW; ++t) {
+      const int64_t wi = w0 + t * nw;
+      vis[t] = wi < W ? __ldcg(a.vis + wi) : 0u;
+      mask[t] = wi < W ? a.active[wi] & ~vis[t] : 0u;
+    }
+#pragma unroll
+    for (int t = 0; t < R_BW; ++t) {
+      ld[t] = make_int4(-1, -1, -1, -1);
+      d[t] = id[t] = 0;
+      todo[t] = (mask[t] >> lane) & 1u;
+      if (todo[t]) {
+        const int64_t v = (w0 + t * nw) * 32 + lane;
+        ld[t] = __ldcs(a.lead + v);
+        d[t] = __ldcs(a.deg + v);
+        id[t] = a.perm ? __ldcs(a.perm + v) : (int)v;
+      }
+    }
+#pragma unroll
+    for (int t = 0; t < R_BW; ++t) {
+      found[t] = todo[t] && is_front(ld[t].x);
+      todo[t] &= !found[t];
+    }
+#pragma unroll
+    for (int t = 0; t < R_BW; ++t)
+      if (todo[t] && d[t] > 1) {
+        found[t] = is_front(ld[t].y) | (ld[t].z >= 0 && is_front(ld[t].z)) | (ld[t].w >= 0 && is_front(ld[t].w));
+        todo[t] = !found[t];
+      }
+    uint32_t e0[R_BW];
+#pragma unroll
+    for (int t = 0; t < R_BW; ++t) {
+      todo[t] &= d[t] > 4;  // shorter rows have been looked through
+      e0[t] = 0;
+      if (todo[t]) e0[t] = (uint32_t)__ldcs(a.off + (w0 + t * nw) * 32 + lane);
+    }
+    // light rows: R_BILP entries of each word per step
+    for (int k = 4;; k += R_BILP) {
+      bool more = false;
+      int u[R_BW][R_BILP];
+#pragma unroll
+      for (int t = 0; t < R_BW; ++t) {
+        const bool go = todo[t] && d[t] < a.small_max && k < d[t];
+        more |= go;
+#pragma unroll
+        for (int i = 0; i < R_BILP; ++i) u[t][i] = go && k + i < d[t] ? __ldg(a.adj + e0[t] + k + i) : -1;
+      }
+      if (!more) break;
+#pragma unroll
+      for (int t = 0; t < R_BW; ++t) {
+        bool f = false;
+#pragma unroll
+        for (int i = 0; i < R_BILP; ++i) f |= u[t][i] >= 0 && is_front(u[t][i]);
+        if (f) found[t] = true, todo[t] = false;
+      }
+    }
+    // heavy rows: the warp together
+#pragma unroll
+    for (int t = 0; t < R_BW; ++t) {
+      unsigned heavy = __ballot_sync(FULL, todo[t] && d[t] >= a.small_max);
+      while (heavy) {
+        const int j = __ffs(heavy) - 1;
+        heavy &= heavy - 1;
+        const uint32_t beg = __shfl_sync(FULL, e0[t], j);
+        const int n = __shfl_sync(FULL, d[t], j);
+        bool hit = false;
+        for (int b0 = 0; b0 < n && !hit; b0 += 64) {
+          const int e = b0 + lane;
+          const int u0 = e < n ? __ldg(a.adj + beg + e) : -1, u1 = e + 32 < n ? __ldg(a.adj + beg + e + 32) : -1;
+          hit = __any_sync(FULL, (u0 >= 0 && is_front(u0)) || (u1 >= 0 && is_front(u1)));
+        }
+        if (lane == j) found[t] = hit;
+      }
+    }
+#pragma unroll
+    for (int t = 0; t < R_BW; ++t) {
+      if (found[t]) {
+        st_keep(depth + id[t], (DT)(s.L + 1));
+        my_n += 1;
+        my_m += (unsigned)d[t];
+      }
+      const unsigned fm = __ballot_sync(FULL, found[t]);
+      const int64_t wi = w0 + t * nw;
+      if (lane == 0 && fm) {  // this warp is the only writer of word wi during the level
+        a.vis[wi] = vis[t] | fm;
+        fbn[wi] = fm;
+      }
+    }
+  }
+}
+
+// Queues the frontier in fb[s.f], left by a bottom-up level (vertices with rows).
+__device__ void res_queue(const LevelArgs& a, const ResArgs& r, const ResState& s, const ResOut& o) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int64_t gw = (int64_t)blockIdx.x * RW + warp, nw = (int64_t)gridDim.x * RW;
+  const int64_t W = (a.n_active + 31) >> 5;
+  for (int64_t w0 = gw * 32; w0 < W; w0 += nw * 32) {
+    uint32_t bits = w0 + lane < W ? __ldcg(r.fb[s.f] + w0 + lane) : 0u;
+    while (__any_sync(FULL, bits != 0)) {
+      const int v = bits ? (int)((w0 + lane) * 32 + __ffs(bits) - 1) : -1;
+      bits &= bits - 1;
+      const int d = v >= 0 ? __ldg(a.deg + v) : 0;
+      const bool light = v >= 0 && d < R_HEAVY;
+      const unsigned m = __ballot_sync(FULL, light);
+      int base = 0;
+      if (lane == 0 && m) base = atomicAdd(o.n, __popc(m));
+      base = __shfl_sync(FULL, base, 0);
+      if (light) o.q[base + __popc(m & lanemask_lt())] = v;
+      if (v >= 0 && !light) res_put_heavy(a, o, v, d);
+    }
+  }
+}
+
+// CTA 0 alone: top-down levels while the frontier is light and small, at most
+// R_SOLO_LEVELS and no further than the direction rule allows; leaves the next
+// frontier queued, its bits set in fbn, its counts in `n` and the totals in so.
+template <class DT, class Solo>
+__device__ void res_solo(const LevelArgs& a, const ResArgs& r, const ResState& s0, DT* depth, uint32_t* fbn, int32_t* n,
+                         Solo* so, int4 (*s_q)[R_SOLO_CAP]) {
+  __shared__ int32_t s_n[2][3];
+  __shared__ unsigned long long s_m[2], s_v[2];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  int L = s0.L, cnt = s0.n_l;
+  int64_t n_vis = s0.n_vis, m_vis = s0.m_vis, n_f = s0.n_f, m_f = s0.m_f;
+  for (int i = tid; i < cnt; i += RT) {
+    const int u = __ldcg(r.queue[L & 1] + i);
+    const int64_t st = a.off[u];
+    s_q[L & 1][i] = make_int4(u, a.deg[u], (int)(uint32_t)st, (int)(uint32_t)((uint64_t)st >> 32));
+  }
+  if (tid < 3) s_n[0][tid] = s_n[1][tid] = 0;
+  if (tid < 2) s_m[tid] = s_v[tid] = 0;
+  __syncthreads();
+  int n2 = 0, n3 = 0;
+  for (int run = 0;; ++run) {
+    const int cur = L & 1, nxt = cur ^ 1;
+    const ResOut o{nullptr, r.queue[nxt], r.huge[nxt], s_n[nxt], s_q[nxt]};
+    const int k = min(32, (cnt + RW - 1) / RW);
+    unsigned my_n = 0;
+    unsigned long long my_m = 0;
+    for (int first = warp * k; first < cnt; first += RW * k) {
+      int d = 0, id = -1;
+      int64_t st = 0;
+      if (lane < k && first + lane < cnt) {
+        const int4 e = s_q[cur][first + lane];
+        d = e.y;
+        st = (int64_t)(((uint64_t)(uint32_t)e.w << 32) | (uint32_t)e.z);
+        id = out_id(a, e.x);
+      }
+      res_rows<DT, true>(a, d, st, L + 1, depth, o, my_n, my_m);
+      if (id >= 0) depth[id] = (DT)L;
+    }
+    my_n = __reduce_add_sync(FULL, my_n);
+    if (my_n) {
+      // a lane's claims in one level hold fewer than 2^32 entries of light rows; heavy ones may be any
+#pragma unroll
+      for (int ofs = 16; ofs > 0; ofs >>= 1) my_m += __shfl_xor_sync(FULL, my_m, ofs);
+      if (lane == 0) {
+        atomicAdd(&s_v[nxt], (unsigned long long)my_n);
+        atomicAdd(&s_m[nxt], my_m);
+      }
+    }
+    __syncthreads();
+    cnt = s_n[nxt][0];
+    n2 = s_n[nxt][1];
+    n3 = s_n[nxt][2];
+    n_f = (int64_t)s_v[nxt];
+    m_f = (int64_t)s_m[nxt];
+    n_vis += n_f;
+    m_vis += m_f;
+    ++L;
+    const bool bu = (a.policy == ENT_POLICY_BEAMER && (double)m_f > (double)(a.E - m_vis) / a.alpha) ||
+                    (a.policy == ENT_POLICY_REFERENCE && (double)m_f >= a.ref_ratio * (double)a.E);
+    if (n_f == 0 || cnt > R_SOLO_CAP || n_f > 2 * (int64_t)a.narrow_f || m_f > min(a.exit_m, 2 * (int64_t)R_SOLO_M) || n2 || n3 || bu ||
+        run + 1 >= R_SOLO_LEVELS || L >= a.max_levels)
+      break;
+    if (tid < 3) s_n[cur][tid] = 0;  // takes the counts of the level after
+    if (tid == 3) s_m[cur] = s_v[cur] = 0;
+    __syncthreads();
+  }
+  // hand over: stored entries to the queue (the rest are there), depths, bits, counts
+  int32_t* q = r.queue[L & 1];
+  for (int i = tid; i < min(cnt, R_SOLO_CAP); i += RT) q[i] = s_q[L & 1][i].x;
+  __syncthreads();
+  const auto hand = [&](int v) {
+    depth[out_id(a, v)] = (DT)L;
+    red_or(fbn + (v >> 5), 1u << (v & 31));
+  };
+  for (int i = tid; i < cnt; i += RT) hand(q[i]);
+  for (int i = tid; i < n2; i += RT) hand(q[a.V - 1 - i]);
+  for (int i = tid; i < n3; i += RT) hand(r.huge[L & 1][i]);
+  if (tid == 0) {
+    n[0] = cnt;
+    n[1] = n2;
+    n[2] = n3;
+    so->n_f = n_f;
+    so->m_f = m_f;
+    so->n_vis = n_vis;
+    so->m_vis = m_vis;
+    so->level = L;
+  }
+}
+
+template <class DT>
+__global__ void __launch_bounds__(RT, 1) k_resident(LevelArgs a, ResArgs r, int32_t src, DT* depth) {
+  extern __shared__ int4 s_dyn[];
+  int4(*s_q)[R_SOLO_CAP] = reinterpret_cast<int4(*)[R_SOLO_CAP]>(s_dyn);
+  __shared__ ResState s_st;
+  __shared__ unsigned long long s_red[2];
+  ResCtl* c = r.rc;
+  const int64_t tid = blockIdx.x * (int64_t)RT + threadIdx.x, nth = (int64_t)gridDim.x * RT;
+  const int64_t W = (a.V + 31) >> 5;
+  const int32_t isrc = a.inv ? __ldg(a.inv + src) : src;
+  fill_unreached(depth, a.V, tid, nth, src);
+  for (int64_t i = tid; i < W; i += nth) {
+    const uint32_t x = i == (isrc >> 5) ? 1u << (isrc & 31) : 0u;
+    a.vis[i] = x;
+    r.fb[0][i] = x;
+    r.fb[1][i] = 0;
+    r.fb[2][i] = 0;
+  }
+  if (threadIdx.x == 0) {
+    const int d = a.deg[isrc];
+    ResState s;
+    s.L = s.f = s.p = 0;
+    s.td_levels = s.bu_levels = s.narrow_levels = s.err = 0;
+    s.n_f = s.n_vis = 1;
+    s.m_f = s.m_vis = d;
+    s.n_l = d < R_HEAVY;
+    s.n_g = d >= R_HUGE;
+    s.n_h = 1 - s.n_l - s.n_g;
+    s.kind = a.policy == ENT_POLICY_BU_ONLY ? RK_BU : res_td_kind(a, s);
+    s_st = s;
+    s_red[0] = s_red[1] = 0;
+    if (blockIdx.x == 0) {
+      if (s.n_l) r.queue[0][0] = isrc;
+      else if (s.n_h) r.queue[0][a.V - 1] = isrc;
+      else r.huge[0][0] = isrc;
+    }
+  }
+  uint32_t target = 0;
+  if (!grid_barrier(&c->arrived, &c->err, target += gridDim.x, [] {})) {
+    if (tid == 0) atomicOr(&a.ctl->err, 2);
+    return;
+  }
+  for (;;) {
+    const ResState& s = s_st;  // thread 0 changes it inside the barrier only
+    if (s.kind == RK_DONE) break;
+    int32_t* n_next = c->n[(s.p + 1) % 3];
+    unsigned long long* acc = c->acc[(s.p + 1) % 3];
+    if (tid < 3) c->n[(s.p + 2) % 3][tid] = 0;
+    if (tid < 2) c->acc[(s.p + 2) % 3][tid] = 0;
+    if (s.kind != RK_QUEUE) {  // the bits of the frontier before this one
+      uint32_t* old = r.fb[(s.f + 2) % 3];
+      for (int64_t i = tid; i < W; i += nth) old[i] = 0;
+    }
+    unsigned my_n = 0;
+    unsigned long long my_m = 0;
+    uint32_t* fbn = r.fb[(s.f + 1) % 3];
+    const int nq = s.kind == RK_QUEUE ? s.L & 1 : (s.L + 1) & 1;
+    const ResOut o{fbn, r.queue[nq], r.huge[nq], n_next, nullptr};
+    if (s.kind == RK_TD) res_td(a, r, s, depth, o, my_n, my_m);
+    else if (s.kind == RK_BU) res_bu(a, r, s, depth, my_n, my_m);
+    else if (s.kind == RK_QUEUE) res_queue(a, r, s, o);
+    else if (blockIdx.x == 0) res_solo(a, r, s, depth, fbn, n_next, &c->solo[s.p & 1], s_q);
+    if (s.kind <= RK_BU) {
+      const unsigned wn = __reduce_add_sync(FULL, my_n);
+      if (wn) {
+#pragma unroll
+        for (int ofs = 16; ofs > 0; ofs >>= 1) my_m += __shfl_xor_sync(FULL, my_m, ofs);
+        if ((threadIdx.x & 31) == 0) {
+          atomicAdd(&s_red[0], (unsigned long long)wn);
+          atomicAdd(&s_red[1], my_m);
+        }
+      }
+      __syncthreads();
+      if (threadIdx.x == 0 && s_red[0]) {
+        atomicAdd(&acc[0], s_red[0]);
+        atomicAdd(&acc[1], s_red[1]);
+        s_red[0] = s_red[1] = 0;
+      }
+    }
+    if (!grid_barrier(&c->arrived, &c->err, target += gridDim.x, [&] { res_advance(a, r, s_st); })) {
+      if (tid == 0) atomicOr(&a.ctl->err, 2);
+      return;
+    }
+  }
+  if (tid == 0) {
+    const ResState& s = s_st;
+    BfsCtl* k = a.ctl;
+    k->src = src;
+    k->level = s.L;
+    k->done = 1;
+    k->err = s.err;
+    k->td_levels = s.td_levels;
+    k->bu_levels = s.bu_levels;
+    k->narrow_levels = s.narrow_levels;
+    k->iters = 0;
+    k->narrow_calls = 0;
+    k->n_vis = s.n_vis;
+    k->m_vis = s.m_vis;
+  }
+}

@@ -47,6 +47,9 @@
 //    each queue entry carries the vertex's row start and degree, read while
 //    its visit was being claimed, so a level costs one adjacency read, one
 //    status probe and one claim on its critical path.
+//  * Graphs of up to 2^23 vertices run as one cooperative kernel instead
+//    (bfs_resident.cuh) unless they are road-like or parents are asked for;
+//    what follows is the rest.
 //  * The whole traversal is one CUDA graph: a reset kernel (which also writes
 //    the loop state), then a while node whose body is two copies of
 //    [expand, inspect, narrow]; the inspector sets the loop condition and the
@@ -1261,6 +1264,8 @@ __global__ void __launch_bounds__(NT, 1) k_narrow(LevelArgs a) {
   __threadfence();
 }
 
+#include "bfs_resident.cuh"
+
 // Pulls a finished byte-depth row into L2 (kept there preferentially) before
 // its copy to the host: the traversal wrote it as bytes scattered over all its
 // levels, mostly evicted since, and the copy engine would otherwise read it
@@ -1291,6 +1296,13 @@ struct BfsWorkspace {
   cudaGraphExec_t exec[2] = {nullptr, nullptr};
   cudaGraphNode_t reset_node[2] = {nullptr, nullptr};
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
+  // the one-kernel traversal of small graphs (null rc: not for this workspace)
+  ResArgs res = {};
+  int grid_res = 0;
+  // traversals of one workspace run one after another, whatever streams they
+  // are launched on: the end of the latest one, and its stream
+  cudaEvent_t ev_order = nullptr;
+  cudaStream_t last_stream = nullptr;
   // ent_bfs_many: a second depth buffer, a copy stream and pinned per-source
   // copies of the control block (created on first use)
   int32_t* depth_b = nullptr;
@@ -1318,6 +1330,7 @@ void destroy_bfs_workspace(BfsWorkspace* w) {
   if (w->parent) cudaFree(w->parent);
   if (w->ev0) cudaEventDestroy(w->ev0);
   if (w->ev1) cudaEventDestroy(w->ev1);
+  if (w->ev_order) cudaEventDestroy(w->ev_order);
   if (w->depth_b) cudaFree(w->depth_b);
   for (int i = 0; i < 2; ++i)
     if (w->depth8[i]) cudaFree(w->depth8[i]);
@@ -1453,6 +1466,32 @@ static int pick_narrow_cluster(int limit, size_t smem) {
   return 0;
 }
 
+constexpr size_t RES_SMEM = 2 * R_SOLO_CAP * sizeof(int4);
+
+// Whether this graph's traversals (without parents) run as one kernel,
+// k_resident, instead of the level kernels. Measured, level kernels -> one
+// kernel, ms: R-MAT s16 0.146 -> 0.068, s20 0.158 -> 0.101, s22 0.235 -> 0.16,
+// s23 0.272 -> 0.228; ER 2^22 d16 0.41 -> 0.29, 2^23 d16 0.70 -> 0.55. At 2^24
+// vertices the bottom-up levels outweigh the launches and want k_expand's
+// occupancy: R-MAT 0.340 -> 0.355, ER d32 1.89 -> 2.43. Graphs of low mean
+// degree (grids, roads) are deep, and their levels belong in the cluster of
+// k_narrow: a 300^2 grid 1.5 -> 2.1 ms, 1024^2 5.4 -> 13 ms.
+constexpr int64_t RES_MAX_V = 1 << 23;
+constexpr int64_t RES_MIN_DEGREE = 5;
+static bool resident_fits(const ent_graph* g, const BfsWorkspace* w) {
+  const ent_bfs_opts& o = g->opts;
+  if (g->V > RES_MAX_V || g->E < RES_MIN_DEGREE * g->V || !g->perm) return false;
+  if (o.loop != ENT_LOOP_GRAPH || w->narrow_nc == 0 || o.hub_slots > 0 || o.fault_inject) return false;
+  int n = 0;
+  for (const void* f : {(const void*)k_resident<int32_t>, (const void*)k_resident<uint8_t>})
+    if (cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)RES_SMEM) != cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, f, RT, RES_SMEM) != cudaSuccess || n < 1) {
+      cudaGetLastError();
+      return false;
+    }
+  return true;
+}
+
 static int create_workspace(ent_graph* g, BfsWorkspace** out, bool force_graph = false, int32_t cluster = 0) {
   BfsWorkspace* w = new BfsWorkspace();
   w->device = g->device;
@@ -1469,7 +1508,7 @@ static int create_workspace(ent_graph* g, BfsWorkspace** out, bool force_graph =
   size_t sz_q = al(sizeof(int32_t) * (V + 4));
   size_t sz_hub = al(sizeof(unsigned long long) * (hub > 0 ? hub : 1));
   size_t sz_tiles = al(sizeof(unsigned long long) * tiles * KS);
-  size_t total = 3 * sz_bits + 9 * sz_q + 2 * sz_hub + sz_tiles;
+  size_t total = 4 * sz_bits + 9 * sz_q + 2 * sz_hub + sz_tiles + al(sizeof(ResCtl));
   cudaError_t e = cudaMalloc(&w->slab, total);
   if (e != cudaSuccess) { destroy_bfs_workspace(w); return fail(ENT_ERR_OOM, "workspace allocation (%zu bytes) failed", total); }
   // Initialise on the graph's stream and wait: the traversal runs on
@@ -1484,6 +1523,7 @@ static int create_workspace(ent_graph* g, BfsWorkspace** out, bool force_graph =
   if (e == cudaSuccess) e = cudaMalloc(&w->parent, sizeof(int32_t) * V);
   if (e == cudaSuccess) e = cudaEventCreate(&w->ev0);
   if (e == cudaSuccess) e = cudaEventCreate(&w->ev1);
+  if (e == cudaSuccess) e = cudaEventCreateWithFlags(&w->ev_order, cudaEventDisableTiming);
   if (e != cudaSuccess) { destroy_bfs_workspace(w); return fail(ENT_ERR_OOM, "workspace setup failed: %s", cudaGetErrorString(e)); }
   char* p = (char*)w->slab;
   LevelArgs& a = w->args;
@@ -1509,6 +1549,8 @@ static int create_workspace(ent_graph* g, BfsWorkspace** out, bool force_graph =
   a.hub[0] = (unsigned long long*)p; p += sz_hub;
   a.hub[1] = (unsigned long long*)p; p += sz_hub;
   a.tiles = (unsigned long long*)p; p += sz_tiles;
+  uint32_t* fb2 = (uint32_t*)p; p += sz_bits;
+  ResCtl* rc = (ResCtl*)p; p += al(sizeof(ResCtl));
   a.small_max = o.small_max;
   a.large_min = o.large_min;
   a.chunk = o.chunk_edges;
@@ -1543,9 +1585,22 @@ static int create_workspace(ent_graph* g, BfsWorkspace** out, bool force_graph =
     a.exit_m = 2 * (int64_t)o.narrow_max_edges;
     a.narrow_deg = o.narrow_max_degree;
   }
-  if (o.loop == ENT_LOOP_GRAPH || force_graph) {
-    int rc = build_graph<int32_t>(g, w);
-    if (rc != ENT_OK) { destroy_bfs_workspace(w); return rc; }
+  if (!force_graph && resident_fits(g, w)) {
+    w->res.rc = rc;
+    w->res.fb[0] = a.fb[0];
+    w->res.fb[1] = a.fb[1];
+    w->res.fb[2] = fb2;
+    for (int i = 0; i < 2; ++i) {
+      w->res.queue[i] = a.q[i][0];
+      w->res.huge[i] = a.qc[i];
+    }
+    // small graphs: fewer CTAs, cheaper barriers, and room for other streams' work
+    const int64_t want = std::max<int64_t>((V + 4 * RT - 1) / (4 * RT), g->E / (8 * RT));
+    w->grid_res = (int)std::max<int64_t>(1, std::min<int64_t>(g->num_sms, want));
+  }
+  if (force_graph) {  // else built on first use
+    int rcode = build_graph<int32_t>(g, w);
+    if (rcode != ENT_OK) { destroy_bfs_workspace(w); return rcode; }
   }
   *out = w;
   return ENT_OK;
@@ -1571,7 +1626,7 @@ static void fill_stats(const BfsCtl& h, float ms, ent_stats* stats) {
 template <class DT>
 static int launch_graph(ent_graph* g, BfsWorkspace* w, int32_t src, DT* depth, int32_t* parent, cudaStream_t s) {
   const int k = depth_kind<DT>();
-  if (!w->exec[k]) {  // the byte-depth graph is built on first use
+  if (!w->exec[k]) {  // built on first use
     int rc = build_graph<DT>(g, w);
     if (rc != ENT_OK) return rc;
   }
@@ -1589,6 +1644,26 @@ static int launch_graph(ent_graph* g, BfsWorkspace* w, int32_t src, DT* depth, i
   return ENT_OK;
 }
 
+// One launch of the resident traversal on stream s (no parents).
+// ENT_ERR_UNSUPPORTED when the GPU cannot hold all its CTAs at once (part of
+// it set aside, by MPS or a partition): the level kernels take over.
+template <class DT>
+static int launch_resident(BfsWorkspace* w, int32_t src, DT* depth, cudaStream_t s) {
+  LevelArgs a = w->args;
+  a.use_cond = 0;
+  void* args[4] = {&a, &w->res, &src, &depth};
+  ENT_CUDA(cudaMemsetAsync(w->res.rc, 0, sizeof(ResCtl), s));
+  const cudaError_t e =
+      cudaLaunchCooperativeKernel((const void*)k_resident<DT>, dim3(w->grid_res), dim3(RT), args, RES_SMEM, s);
+  if (e == cudaErrorCooperativeLaunchTooLarge) {
+    cudaGetLastError();
+    w->res.rc = nullptr;
+    return ENT_ERR_UNSUPPORTED;
+  }
+  ENT_CUDA(e);
+  return ENT_OK;
+}
+
 int launch_bfs_single(BfsWorkspace* w, int32_t src, int32_t* depth_dev, cudaStream_t s) {
   g_kernel_launches += 1;  // reset; the level kernels are counted by bfs_single_stats
   return launch_graph(nullptr, w, src, depth_dev, nullptr, s);  // int32 graph: built with the workspace
@@ -1603,17 +1678,27 @@ int bfs_single_stats(BfsWorkspace* w, cudaStream_t s, ent_stats* stats) {
   return ENT_OK;
 }
 
-template <class DT>
-static int run_bfs_typed(ent_graph* g, int32_t src, DT* depth, int32_t* parent, cudaStream_t stream, ent_stats* stats) {
+// One traversal on `stream`. With stats it waits for the end; `queued` (device
+// to host copies of the results) then runs between the launch and the wait.
+static int nothing_queued() { return ENT_OK; }
+template <class DT, class Queued = int (*)()>
+static int run_bfs_typed(ent_graph* g, int32_t src, DT* depth, int32_t* parent, cudaStream_t stream, ent_stats* stats,
+                         Queued queued = nothing_queued) {
   if (!g->ws) {
     int rc = create_workspace(g, &g->ws);
     if (rc != ENT_OK) return rc;
   }
   BfsWorkspace* w = g->ws;
   cudaStream_t s = stream ? stream : g->stream;
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusActive;
+  if (cudaStreamIsCapturing(s, &cap) != cudaSuccess) cudaGetLastError();
+  const bool capturing = cap != cudaStreamCaptureStatusNone;  // the launches below refuse it
+  if (!capturing && w->last_stream && w->last_stream != s) ENT_CUDA(cudaStreamWaitEvent(s, w->ev_order, 0));
   if (stats) ENT_CUDA(cudaEventRecord(w->ev0, s));
   if (g->opts.loop == ENT_LOOP_GRAPH) {
-    int rc = launch_graph(g, w, src, depth, parent, s);
+    int rc = ENT_ERR_UNSUPPORTED;
+    if (w->res.rc && !parent && !capturing) rc = launch_resident(w, src, depth, s);
+    if (rc == ENT_ERR_UNSUPPORTED) rc = launch_graph(g, w, src, depth, parent, s);
     if (rc != ENT_OK) return rc;
   } else {
     LevelArgs la = w->args;
@@ -1637,9 +1722,15 @@ static int run_bfs_typed(ent_graph* g, int32_t src, DT* depth, int32_t* parent, 
       if (it > w->V + 2) return fail(ENT_ERR_INTERNAL, "level loop did not terminate");
     }
   }
+  if (!capturing) {
+    ENT_CUDA(cudaEventRecord(w->ev_order, s));
+    w->last_stream = s;
+  }
   if (stats) {
     ENT_CUDA(cudaEventRecord(w->ev1, s));
     ENT_CUDA(cudaMemcpyAsync(w->ctl_h, w->ctl, sizeof(BfsCtl), cudaMemcpyDeviceToHost, s));
+    const int rc = queued();
+    if (rc != ENT_OK) return rc;
     ENT_CUDA(cudaStreamSynchronize(s));
     float ms = 0.f;
     cudaEventElapsedTime(&ms, w->ev0, w->ev1);
@@ -1942,14 +2033,16 @@ int ent_bfs(ent_graph* g, int32_t src, int32_t* depth_out, int32_t* parent_out, 
   }
   BfsWorkspace* w = g->ws;
   ent_stats local;
-  int rc = run_bfs_single(g, src, w->depth, parent_out ? w->parent : nullptr, g->stream, stats ? stats : &local);
-  if (rc != ENT_OK) return rc;
-  if (depth_out)
-    ENT_CUDA(cudaMemcpyAsync(depth_out, w->depth, sizeof(int32_t) * g->V, cudaMemcpyDeviceToHost, g->stream));
-  if (parent_out)
-    ENT_CUDA(cudaMemcpyAsync(parent_out, w->parent, sizeof(int32_t) * g->V, cudaMemcpyDeviceToHost, g->stream));
-  ENT_CUDA(cudaStreamSynchronize(g->stream));
-  return ENT_OK;
+  // the copies are queued behind the traversal, before its statistics are waited for
+  const auto copies = [&]() -> int {
+    if (depth_out)
+      ENT_CUDA(cudaMemcpyAsync(depth_out, w->depth, sizeof(int32_t) * g->V, cudaMemcpyDeviceToHost, g->stream));
+    if (parent_out)
+      ENT_CUDA(cudaMemcpyAsync(parent_out, w->parent, sizeof(int32_t) * g->V, cudaMemcpyDeviceToHost, g->stream));
+    return ENT_OK;
+  };
+  return run_bfs_typed<int32_t>(g, src, w->depth, parent_out ? w->parent : nullptr, g->stream,
+                                stats ? stats : &local, copies);
 }
 
 // The reference's source loop (bfs_gpu_opt.cuh:370-431: per source, reset,
@@ -2055,7 +2148,7 @@ static int bfs_many(ent_graph* g, const int32_t* src, int32_t n_src, void* const
     float ms = 0.f;
     cudaEventElapsedTime(&ms, ev[2 * (size_t)i], ev[2 * (size_t)i + 1]);
     fill_stats(h, ms, &st);
-    if (g->opts.loop == ENT_LOOP_GRAPH) g_kernel_launches += st.launches - 2;
+    if (g->opts.loop == ENT_LOOP_GRAPH) g_kernel_launches += st.launches - 1;  // the first was counted at launch
     if (stats) stats[i] = st;
     if (h.err && first_bad < 0) first_bad = i;
     if (bytes && st.levels > 255 && first_deep < 0) first_deep = i;

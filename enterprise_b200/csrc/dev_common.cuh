@@ -46,6 +46,39 @@ __device__ __forceinline__ unsigned long long lb_flag(unsigned long long w, uint
 // tile is always held by a running CTA and publishes within microseconds.
 constexpr int SPIN_LIMIT = 1 << 20;
 
+// One CTA's arrival at a grid-wide barrier (cooperative launch: every CTA is
+// resident) and its wait for all: `target` is the number of arrivals, counted
+// over the whole launch, after which it opens. `after` runs on thread 0 once it
+// has opened, before the other threads go on. The wait is bounded (seconds; a
+// wait this long means a bug): false when one ran out anywhere, and every CTA
+// then leaves.
+template <class F>
+__device__ bool grid_barrier(uint32_t* arrived, int32_t* err, uint32_t target, F after) {
+  __shared__ int s_ok;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    atomicAdd(arrived, 1u);
+    int ok = 1;
+    for (int spins = 0;; ++spins) {
+      uint32_t x;
+      asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(x) : "l"(arrived) : "memory");
+      if (x >= target) break;
+      if (spins > 64) __nanosleep(64);
+      if (spins >= SPIN_LIMIT * 4 || ((spins & 63) == 63 && *(volatile int32_t*)err)) {
+        *(volatile int32_t*)err = 1;
+        ok = 0;
+        break;
+      }
+    }
+    __threadfence();
+    s_ok = ok;
+    if (ok) after();
+  }
+  __syncthreads();
+  return s_ok != 0;
+}
+
 // Inclusive warp scan of K lanes' values (each lane holds v[k]).
 template <int K>
 __device__ __forceinline__ void warp_incl_scan(uint32_t (&v)[K]) {

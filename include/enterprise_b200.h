@@ -61,8 +61,10 @@ enum ent_policy {
 
 /* How the level loop is driven. */
 enum ent_loop {
-  ENT_LOOP_GRAPH = 0, /* whole traversal = one CUDA graph launch with a
-                         device-side while node (no host round trip)   */
+  ENT_LOOP_GRAPH = 0, /* whole traversal = one launch, no host round trip:
+                         a CUDA graph with a device-side while node, or on
+                         graphs of up to 2^23 vertices that are not
+                         road-like, without parents, one cooperative kernel */
   ENT_LOOP_HOST = 1   /* host launches each level and polls a flag     */
 };
 
