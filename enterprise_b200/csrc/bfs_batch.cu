@@ -101,9 +101,10 @@ struct BatchArgs {
   uint32_t* donebits;
   uint32_t* jfb[2];
   const uint32_t* lightbits;  // degree in [1, batch_small_max): bottom-up light tier
-  const int32_t* mid;         // batch_small_max <= degree < batch_large_min
+  const uint32_t* midbits;    // batch_small_max <= degree < batch_large_min
   const int32_t* large;       // degree >= batch_large_min
-  int32_t n_mid, n_large;
+  int32_t n_large;
+  int64_t mid_w0, mid_w1;     // midbits is empty outside these words
   int32_t* jf[2];
   int2* heavy[2];       // (vertex, chunk) per TD_CHUNK entries of each heavy frontier vertex
   const int32_t* src;   // [n_src], or the seed vertices of a seed list
@@ -449,57 +450,71 @@ __device__ void b_bu_mid(const BatchArgs& a, BatchCtl* c, const unsigned long lo
   const unsigned long long* ac = a.act[c->cur] + gl * WPT;
   const uint32_t* jfc = a.jfb[c->cur];
   const uint32_t sbit = 2u << (c->level - c->base);
-  for (int i = gw; i < a.n_mid; i += nw) {
-    const int v = a.mid[i];
-    if ((a.donebits[v >> 5] >> (v & 31)) & 1u) continue;
-    unsigned long long* xv = a.X + (size_t)v * W + gl * WPT;
-    unsigned long long need[WPT], acc[WPT];
-    bool any = false;
+  // A warp's share is `group` consecutive vertices, of which one word of
+  // completion bits tells the open ones: late levels, where nearly all are
+  // complete, took 58 us at s22 for a read per vertex and take 20 so. As large
+  // as leaves every warp MID_SHARES shares, for balance (whole words throughout:
+  // s20 x 1000 4.7 -> 5.7 ms; 4, 8, 16 and 32 shares: s22 x 256 3.80, 3.67,
+  // 3.66 and 3.73 ms, x 64 1.66, 1.67, 1.70 and 1.81; a read per vertex 4.00, 1.82).
+  constexpr int64_t MID_SHARES = 8;
+  const int64_t words = a.mid_w1 - a.mid_w0;
+  int lg = 5;  // log2 of the group
+  while (lg > 0 && (words << (5 - lg)) < MID_SHARES * nw) --lg;
+  const uint32_t group = lg == 5 ? FULL : (1u << (1 << lg)) - 1u;
+  for (int64_t i = gw; i < words << (5 - lg); i += nw) {
+    const int64_t wi = a.mid_w0 + (i >> (5 - lg));
+    const int sub = ((int)i & ((1 << (5 - lg)) - 1)) << lg;
+    for (uint32_t open = a.midbits[wi] & ~a.donebits[wi] & (group << sub); open; open &= open - 1) {
+      const int v = (int)(wi * 32 + __ffs(open) - 1);
+      unsigned long long* xv = a.X + (size_t)v * W + gl * WPT;
+      unsigned long long need[WPT], acc[WPT];
+      bool any = false;
 #pragma unroll
-    for (int j = 0; j < WPT; ++j) {
-      need[j] = ac[j] & ~xv[j];
-      acc[j] = 0;
-      any |= need[j] != 0;
-    }
-    if (!__any_sync(FULL, any)) {  // every source it still lacks has finished
-      if (lane == 0) bu_finish_vertex(a, c, v, nxt, sbit, false, true, a.deg[v], my_m, my_md);
-      continue;
-    }
-    const int64_t beg = a.off[v], end = a.off[v + 1];
-    int chk = 1, since = 0;
-    for (int64_t b0 = beg; b0 < end; b0 += 2 * NS) {
-      bu_gather2<WPT>(a, jfc, F, b0 + k, NS, end, gl * WPT, acc);
-      if (++since == chk) {
-        since = 0;
-        if (chk < 4) chk <<= 1;
-        unsigned long long r[WPT];
-        bool mine = true;
-#pragma unroll
-        for (int j = 0; j < WPT; ++j) r[j] = acc[j];
-        group_or<WPT>(r, G);
-#pragma unroll
-        for (int j = 0; j < WPT; ++j) mine &= (r[j] & need[j]) == need[j];
-        if (__all_sync(FULL, mine)) break;
+      for (int j = 0; j < WPT; ++j) {
+        need[j] = ac[j] & ~xv[j];
+        acc[j] = 0;
+        any |= need[j] != 0;
       }
-    }
-    group_or<WPT>(acc, G);
-    bool got = false, full = true;
+      if (!__any_sync(FULL, any)) {  // every source it still lacks has finished
+        if (lane == 0) bu_finish_vertex(a, c, v, nxt, sbit, false, true, a.deg[v], my_m, my_md);
+        continue;
+      }
+      const int64_t beg = a.off[v], end = a.off[v + 1];
+      int chk = 1, since = 0;
+      for (int64_t b0 = beg; b0 < end; b0 += 2 * NS) {
+        bu_gather2<WPT>(a, jfc, F, b0 + k, NS, end, gl * WPT, acc);
+        if (++since == chk) {
+          since = 0;
+          if (chk < 4) chk <<= 1;
+          unsigned long long r[WPT];
+          bool mine = true;
 #pragma unroll
-    for (int j = 0; j < WPT; ++j) {
-      const unsigned long long nw_ = acc[j] & need[j];
-      if (nw_) {
-        got = true;
-        if (k == 0) {
-          NB[(size_t)v * W + gl * WPT + j] = nw_;
-          xv[j] = xv[j] | nw_;
-          note_act(s_act + gl * WPT + j, nw_);
+          for (int j = 0; j < WPT; ++j) r[j] = acc[j];
+          group_or<WPT>(r, G);
+#pragma unroll
+          for (int j = 0; j < WPT; ++j) mine &= (r[j] & need[j]) == need[j];
+          if (__all_sync(FULL, mine)) break;
         }
       }
-      full &= (need[j] & ~nw_) == 0;
+      group_or<WPT>(acc, G);
+      bool got = false, full = true;
+#pragma unroll
+      for (int j = 0; j < WPT; ++j) {
+        const unsigned long long nw_ = acc[j] & need[j];
+        if (nw_) {
+          got = true;
+          if (k == 0) {
+            NB[(size_t)v * W + gl * WPT + j] = nw_;
+            xv[j] = xv[j] | nw_;
+            note_act(s_act + gl * WPT + j, nw_);
+          }
+        }
+        full &= (need[j] & ~nw_) == 0;
+      }
+      const bool gany = __any_sync(FULL, got);
+      const bool gfull = __all_sync(FULL, full);
+      if (lane == 0) bu_finish_vertex(a, c, v, nxt, sbit, gany, gfull, end - beg, my_m, my_md);
     }
-    const bool gany = __any_sync(FULL, got);
-    const bool gfull = __all_sync(FULL, full);
-    if (lane == 0) bu_finish_vertex(a, c, v, nxt, sbit, gany, gfull, end - beg, my_m, my_md);
   }
 }
 
@@ -511,7 +526,6 @@ template <int WPT>
 __device__ void b_bu_large(const BatchArgs& a, BatchCtl* c, const unsigned long long* F, unsigned long long* NB,
                            unsigned long long& my_m, unsigned long long& my_md, unsigned long long* s_act) {
   __shared__ unsigned long long s_acc[WMAX], s_need[WMAX];
-  __shared__ int s_skip;
   const int W = a.W, G = W / WPT, NS = BB / G;
   const int t = threadIdx.x, lane = t & 31, gl = t % G, k = t / G;
   const int nxt = c->cur ^ 1;
@@ -520,14 +534,13 @@ __device__ void b_bu_large(const BatchArgs& a, BatchCtl* c, const unsigned long 
   const uint32_t sbit = 2u << (c->level - c->base);
   for (int i = blockIdx.x; i < a.n_large; i += gridDim.x) {
     const int v = a.large[i];
+    if ((a.donebits[v >> 5] >> (v & 31)) & 1u) continue;  // set by this CTA only: the same for all its threads
     __syncthreads();
     if (t < W) {
       s_need[t] = ac[t] & ~a.X[(size_t)v * W + t];
       s_acc[t] = 0;
     }
-    if (t == 0) s_skip = (a.donebits[v >> 5] >> (v & 31)) & 1u;
     __syncthreads();
-    if (s_skip) continue;
     if (!__syncthreads_or(t < W && s_need[t] != 0)) {  // every source it still lacks has finished
       if (t == 0) bu_finish_vertex(a, c, v, nxt, sbit, false, true, a.deg[v], my_m, my_md);
       continue;
@@ -1489,7 +1502,7 @@ __global__ void __launch_bounds__(BB, 3) k_b_flush(BatchArgs a, int final_flush)
 
 // Static degree tiers of a graph for the bottom-up pass (degrees never change).
 __global__ void k_b_tiers(const int32_t* __restrict__ deg, int64_t V, int small_max, int large_min,
-                          uint32_t* __restrict__ lightbits, int32_t* __restrict__ mid, int32_t* __restrict__ large,
+                          uint32_t* __restrict__ lightbits, uint32_t* __restrict__ midbits, int32_t* __restrict__ large,
                           int32_t* __restrict__ counts) {
   const int lane = threadIdx.x & 31;
   const int64_t nth = (int64_t)gridDim.x * blockDim.x;
@@ -1497,8 +1510,15 @@ __global__ void k_b_tiers(const int32_t* __restrict__ deg, int64_t V, int small_
     const int64_t v = base + lane;
     const int d = v < V ? deg[v] : 0;
     const unsigned lb = __ballot_sync(FULL, d >= 1 && d < small_max);
-    if (lane == 0) lightbits[base >> 5] = lb;
-    wappend(d >= small_max && d < large_min, (int)v, mid, &counts[0]);
+    const unsigned mb = __ballot_sync(FULL, d >= small_max && d < large_min);
+    if (lane == 0) {
+      lightbits[base >> 5] = lb;
+      midbits[base >> 5] = mb;
+      if (mb) {
+        atomicMax(&counts[0], (int)(base >> 5) + 1);           // one past the last word with a mid vertex
+        atomicMax(&counts[2], (int)((V + 31) >> 5) - (int)(base >> 5));  // ... and the first, from the end
+      }
+    }
     wappend(d >= large_min, (int)v, large, &counts[1]);
   }
 }
@@ -1659,7 +1679,7 @@ int create_batch_workspace(ent_graph* g, int n_src, BatchWorkspace** out) {
   const size_t sz_heavy = al(sizeof(int2) * (g->E / TD_CHUNK + std::min(V, g->E / heavy_deg) + 1));
   const size_t sz_marks = al(sizeof(uint16_t) * V);
   const size_t sz_st = al(sizeof(unsigned long long) * w->cap_src) * 2 + 2 * al(sizeof(int32_t) * w->cap_src);
-  const size_t total = sz_x + sz_log + 4 * sz_bits + 4 * sz_q + 2 * sz_heavy + 3 * sz_mask + sz_src + sz_st + sz_marks + 256;
+  const size_t total = sz_x + sz_log + 5 * sz_bits + 3 * sz_q + 2 * sz_heavy + 3 * sz_mask + sz_src + sz_st + sz_marks + 256;
   cudaError_t e = cudaMalloc(&w->slab, total);
   if (e != cudaSuccess) { destroy_batch_workspace(w); return fail(ENT_ERR_OOM, "batch workspace (%zu bytes) failed", total); }
   // Initialise on the graph's stream and wait (see create_workspace in
@@ -1700,11 +1720,11 @@ int create_batch_workspace(ent_graph* g, int n_src, BatchWorkspace** out) {
   for (int i = 0; i < 2; ++i) { a.jf[i] = (int32_t*)p; p += sz_q; }
   for (int i = 0; i < 2; ++i) { a.heavy[i] = (int2*)p; p += sz_heavy; }
   uint32_t* lightbits = (uint32_t*)p; p += sz_bits;
-  int32_t* mid = (int32_t*)p; p += sz_q;
+  uint32_t* midbits = (uint32_t*)p; p += sz_bits;
   int32_t* large = (int32_t*)p; p += sz_q;
   int32_t* counts = (int32_t*)p; p += 256;
   a.lightbits = lightbits;
-  a.mid = mid;
+  a.midbits = midbits;
   a.large = large;
   a.mask = (const unsigned long long*)p; p += sz_mask;
   a.act[0] = (unsigned long long*)p; p += sz_mask;
@@ -1724,13 +1744,14 @@ int create_batch_workspace(ent_graph* g, int n_src, BatchWorkspace** out) {
   {
     const int blocks = (int)std::min<int64_t>((V + BB - 1) / BB, (int64_t)g->num_sms * 8);
     k_b_tiers<<<blocks, BB, 0, g->stream>>>(g->deg, V, g->opts.batch_small_max, g->opts.batch_large_min, lightbits,
-                                             mid, large, counts);
+                                             midbits, large, counts);
     g_kernel_launches++;
-    int32_t hc[2] = {0, 0};
+    int32_t hc[3] = {0, 0, 0};
     e = cudaMemcpyAsync(hc, counts, sizeof(hc), cudaMemcpyDeviceToHost, g->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(g->stream);
     if (e != cudaSuccess) { destroy_batch_workspace(w); return fail(ENT_ERR_CUDA, "tier build failed: %s", cudaGetErrorString(e)); }
-    a.n_mid = hc[0];
+    a.mid_w1 = hc[0];
+    a.mid_w0 = hc[0] ? Wd - hc[2] : 0;
     a.n_large = hc[1];
   }
   int occ = 0;
