@@ -9,9 +9,9 @@
 // that the barrier published, so no level ends in one CTA's chain.
 //
 // A phase is one of
-//   * a top-down level: rows split by degree over lane groups, CTAs and the
-//     whole grid (as in bfs_noalloc.cu); a claim queues its vertex by degree
-//     and sets its frontier bit, so that either direction can follow;
+//   * a top-down level: a warp takes up to 32 light rows together, heavy rows
+//     get as many warps each as there are for them; a claim queues its vertex
+//     by degree and sets its frontier bit, so that either direction can follow;
 //   * a bottom-up level: a warp per status word, as in k_expand;
 //   * a queue build, from the frontier bitmap, where a bottom-up level hands
 //     over to top-down;
@@ -22,6 +22,13 @@
 // barrier before; frontier bitmaps rotate the same way per level. All waits
 // are bounded: one that runs out sets the error bit and every CTA leaves.
 //
+// On large graphs the bottom-up levels are most of the time and want k_expand's
+// occupancy, twice this kernel's (R-MAT s24 0.355 -> 0.31 ms, ER 2^24 d32 2.43 ->
+// 1.69). The traversal then runs in parts: a head up to
+// the first bottom-up level, R_BU_LEVELS kernels of one level each (those not
+// needed leave at once; the last CTA of each takes the decision), and a tail
+// for whatever is left.
+//
 // Not here: parents, hub tables and runs with the small-frontier mode off stay
 // with the level kernels.
 #pragma once
@@ -31,17 +38,29 @@ constexpr int RW = RT / 32;
 constexpr int R_ILP = 4;          // row entries a lane has in flight together
 constexpr int R_BW = 3;           // bottom-up: status words a warp has in flight together
 constexpr int R_BILP = 2;         // ... and row entries of each per step
-constexpr int R_HEAVY = 256;      // degree from which a CTA takes a vertex's row
-constexpr int R_HUGE = 1 << 15;   // ... and from which all CTAs share it
+constexpr int R_HEAVY = 256;      // degree from which warps take a row alone, or share it
+constexpr int R_HUGE = 16384;     // ... and from which at least R_SHARE warps do
+constexpr int R_SHARE = 32;
 constexpr int R_SOLO = 2048;      // frontier up to which CTA 0 starts to run alone
 constexpr int R_SOLO_M = 16384;   // ... and its degree sum; it leaves above twice that
 constexpr int R_SOLO_CAP = 4096;  // frontier entries it keeps in shared memory
 constexpr int R_SOLO_LEVELS = 4096;  // levels it runs before it meets the others again
 
+enum { RK_TD, RK_BU, RK_QUEUE, RK_SOLO, RK_DONE };
+
+// What every CTA knows about the phase to come (thread 0 keeps it current).
+struct ResState {
+  int32_t kind, L, f, p;      // f: fb index of the frontier
+  int32_t n_l, n_h, n_g;
+  int32_t td_levels, bu_levels, narrow_levels, err;
+  int64_t n_f, m_f, n_vis, m_vis;
+};
+
 struct ResCtl {
-  uint32_t arrived;  // barrier arrivals of this launch
+  uint32_t arrived[2];  // barrier arrivals of the head (or the whole), and of the tail
   int32_t err;       // a wait ran out
-  int32_t pad[2];
+  uint32_t finished; // CTAs of a bottom-up kernel that are done
+  ResState state;    // between the kernels of a traversal in parts
   int32_t n[3][4];   // light, heavy, huge frontier vertices of a phase
   unsigned long long acc[3][2];  // vertices and degree sum that a phase found
   struct {
@@ -55,16 +74,6 @@ struct ResArgs {
   uint32_t* fb[3];
   int32_t* queue[2];  // light vertices from the front, heavy ones from the back (V entries)
   int32_t* huge[2];
-};
-
-enum { RK_TD, RK_BU, RK_QUEUE, RK_SOLO, RK_DONE };
-
-// What every CTA knows about the phase to come (thread 0 keeps it current).
-struct ResState {
-  int32_t kind, L, f, p;      // f: fb index of the frontier
-  int32_t n_l, n_h, n_g;
-  int32_t td_levels, bu_levels, narrow_levels, err;
-  int64_t n_f, m_f, n_vis, m_vis;
 };
 
 __device__ __forceinline__ int64_t ldcg64(const void* p) {
@@ -150,17 +159,47 @@ struct ResOut {
   int4* s_q;         // CTA 0 alone: entries in shared memory while they fit
 };
 
-// Queues vertex v (degree d, row start st) of a converged warp by degree;
-// n_light: the warp's light ones in all R_ILP rounds were counted at `base`.
-__device__ __forceinline__ void res_put_heavy(const LevelArgs& a, const ResOut& o, int v, int d) {
-  if (d >= R_HUGE) o.huge[atomicAdd(o.n + 2, 1)] = v;
-  else o.q[a.V - 1 - atomicAdd(o.n + 1, 1)] = v;
+// Where vertices queue by degree: 0 light, 1 heavy, 2 huge.
+__device__ __forceinline__ int res_class(int d) { return d < R_HEAVY ? 0 : (d < R_HUGE ? 1 : 2); }
+
+// Queues vertices of a converged warp, N per lane (cls < 0: none): one atomic
+// per class for all of them (one each for the heavy ones took 40 us on R-MAT
+// s24's second level, whose 23k finds are mostly hubs). put(i, at) stores the
+// lane's i-th light vertex at position `at`.
+template <int N, class Put>
+__device__ __forceinline__ void res_queue_up(const LevelArgs& a, const ResOut& o, const int (&v)[N],
+                                             const int (&cls)[N], Put put) {
+  const int lane = threadIdx.x & 31;
+  int cnt[3] = {0, 0, 0};
+#pragma unroll
+  for (int i = 0; i < N; ++i)
+#pragma unroll
+    for (int c = 0; c < 3; ++c) cnt[c] += __popc(__ballot_sync(FULL, cls[i] == c));
+  if (cnt[0] + cnt[1] + cnt[2] == 0) return;
+  const int mine = lane == 0 ? cnt[0] : (lane == 1 ? cnt[1] : (lane == 2 ? cnt[2] : 0));
+  int at = 0;
+  if (mine) at = atomicAdd(o.n + lane, mine);
+  int base[3];
+#pragma unroll
+  for (int c = 0; c < 3; ++c) base[c] = __shfl_sync(FULL, at, c);
+#pragma unroll
+  for (int i = 0; i < N; ++i)
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      const unsigned m = __ballot_sync(FULL, cls[i] == c);
+      const int pos = base[c] + __popc(m & lanemask_lt());
+      base[c] += __popc(m);
+      if (cls[i] == c) {
+        if (c == 0) put(i, pos);
+        else if (c == 1) o.q[a.V - 1 - pos] = v[i];
+        else o.huge[pos] = v[i];
+      }
+    }
 }
 
 template <class DT, bool SOLO>
 __device__ __forceinline__ void res_claim(const LevelArgs& a, const int (&v)[R_ILP], int ln, DT* depth, const ResOut& o,
                                           unsigned& my_n, unsigned long long& my_m) {
-  const int lane = threadIdx.x & 31;
   bool open[R_ILP], mine[R_ILP];
   int64_t st[R_ILP];
   int d[R_ILP], id[R_ILP];
@@ -184,9 +223,10 @@ __device__ __forceinline__ void res_claim(const LevelArgs& a, const int (&v)[R_I
       mine[i] = !(atomicOr(a.vis + (v[i] >> 5), b) & b);
     }
   }
-  int n_light = 0;
+  int cls[R_ILP];
 #pragma unroll
   for (int i = 0; i < R_ILP; ++i) {
+    cls[i] = mine[i] ? res_class(d[i]) : -1;
     if (mine[i]) {
       if (!SOLO) {  // alone, depths and bits are written later: off the level's chain
         depth[id[i]] = (DT)ln;
@@ -195,29 +235,13 @@ __device__ __forceinline__ void res_claim(const LevelArgs& a, const int (&v)[R_I
       my_n += 1;
       my_m += (unsigned)d[i];
     }
-    n_light += __popc(__ballot_sync(FULL, mine[i] && d[i] < R_HEAVY));
   }
-  if (__any_sync(FULL, mine[0] || mine[1] || mine[2] || mine[3])) {
-    int base = 0;
-    if (n_light) {
-      if (lane == 0) base = atomicAdd(o.n, n_light);
-      base = __shfl_sync(FULL, base, 0);
-    }
-#pragma unroll
-    for (int i = 0; i < R_ILP; ++i) {
-      const bool light = mine[i] && d[i] < R_HEAVY;
-      const unsigned m = __ballot_sync(FULL, light);
-      if (light) {
-        const int at = base + __popc(m & lanemask_lt());
-        if (SOLO && at < R_SOLO_CAP)
-          o.s_q[at] = make_int4(v[i], d[i], (int)(uint32_t)st[i], (int)(uint32_t)((uint64_t)st[i] >> 32));
-        else
-          o.q[at] = v[i];
-      }
-      base += __popc(m);
-      if (mine[i] && d[i] >= R_HEAVY) res_put_heavy(a, o, v[i], d[i]);  // few: an atomic each
-    }
-  }
+  res_queue_up<R_ILP>(a, o, v, cls, [&](int i, int at) {
+    if (SOLO && at < R_SOLO_CAP)
+      o.s_q[at] = make_int4(v[i], d[i], (int)(uint32_t)st[i], (int)(uint32_t)((uint64_t)st[i] >> 32));
+    else
+      o.q[at] = v[i];
+  });
 }
 
 // The concatenated rows of a warp's light vertices (lane: d entries from st).
@@ -277,14 +301,19 @@ __device__ void res_td(const LevelArgs& a, const ResArgs& r, const ResState& s, 
   const int32_t* q = r.queue[s.L & 1];
   const int ln = s.L + 1;
   const int64_t gw = (int64_t)blockIdx.x * RW + warp, nw = (int64_t)gridDim.x * RW;
-  for (int i = 0; i < s.n_g; ++i) {  // rows shared by all CTAs
-    const int u = __ldcg(r.huge[s.L & 1] + i);
-    res_slice(a, a.off[u] + gw * 32 * R_ILP, nw * 32 * R_ILP, a.off[u + 1], ln, depth, o, my_n, my_m);
-  }
-  for (int i = blockIdx.x; i < s.n_h; i += gridDim.x) {  // rows of one CTA
-    const int u = __ldcg(q + a.V - 1 - i);
-    res_slice(a, a.off[u] + warp * 32 * R_ILP, (int64_t)RW * 32 * R_ILP, a.off[u + 1], ln, depth, o, my_n, my_m);
-  }
+  // Long rows: `share` warps each, in turn over the rows. A CTA per row left
+  // R-MAT s24's second level (four rows of 24k entries in all) at 60 us and
+  // spent 2.1 ms on s22 top-down throughout; a list of equal chunks is as fast
+  // there but costs 100 us to make on levels whose next one is bottom-up.
+  const auto long_rows = [&](int n, int64_t share, auto row) {
+    for (int64_t k = gw; k < n * share; k += nw) {
+      const int u = row((int)(k % n));
+      const int64_t end = a.off[u + 1];
+      res_slice(a, a.off[u] + k / n * (32 * R_ILP), share * (32 * R_ILP), end, ln, depth, o, my_n, my_m);
+    }
+  };
+  if (s.n_g) long_rows(s.n_g, max((int64_t)R_SHARE, nw / s.n_g), [&](int i) { return __ldcg(r.huge[s.L & 1] + i); });
+  if (s.n_h) long_rows(s.n_h, max((int64_t)1, nw / s.n_h), [&](int i) { return __ldcg(q + a.V - 1 - i); });
   // up to 32 light rows per warp, spread over all warps
   const int k = (int)min((int64_t)32, (s.n_l + nw - 1) / nw);
   for (int64_t first = gw * k; first < s.n_l; first += nw * k) {
@@ -422,14 +451,8 @@ __device__ void res_queue(const LevelArgs& a, const ResArgs& r, const ResState& 
     while (__any_sync(FULL, bits != 0)) {
       const int v = bits ? (int)((w0 + lane) * 32 + __ffs(bits) - 1) : -1;
       bits &= bits - 1;
-      const int d = v >= 0 ? __ldg(a.deg + v) : 0;
-      const bool light = v >= 0 && d < R_HEAVY;
-      const unsigned m = __ballot_sync(FULL, light);
-      int base = 0;
-      if (lane == 0 && m) base = atomicAdd(o.n, __popc(m));
-      base = __shfl_sync(FULL, base, 0);
-      if (light) o.q[base + __popc(m & lanemask_lt())] = v;
-      if (v >= 0 && !light) res_put_heavy(a, o, v, d);
+      const int vs[1] = {v}, cls[1] = {v >= 0 ? res_class(__ldg(a.deg + v)) : -1};
+      res_queue_up<1>(a, o, vs, cls, [&](int, int at) { o.q[at] = v; });
     }
   }
 }
@@ -523,8 +546,13 @@ __device__ void res_solo(const LevelArgs& a, const ResArgs& r, const ResState& s
   }
 }
 
+enum { RP_ALL, RP_HEAD, RP_TAIL };  // the part of the traversal a launch runs
+// Bottom-up kernels between head and tail: R-MAT and uniform graphs take three
+// or four such levels, and one that is not needed costs 6 us.
+constexpr int R_BU_LEVELS = 4;
+
 template <class DT>
-__global__ void __launch_bounds__(RT, 1) k_resident(LevelArgs a, ResArgs r, int32_t src, DT* depth) {
+__global__ void __launch_bounds__(RT, 1) k_resident(LevelArgs a, ResArgs r, int32_t src, DT* depth, int part) {
   extern __shared__ int4 s_dyn[];
   int4(*s_q)[R_SOLO_CAP] = reinterpret_cast<int4(*)[R_SOLO_CAP]>(s_dyn);
   __shared__ ResState s_st;
@@ -532,42 +560,49 @@ __global__ void __launch_bounds__(RT, 1) k_resident(LevelArgs a, ResArgs r, int3
   ResCtl* c = r.rc;
   const int64_t tid = blockIdx.x * (int64_t)RT + threadIdx.x, nth = (int64_t)gridDim.x * RT;
   const int64_t W = (a.V + 31) >> 5;
-  const int32_t isrc = a.inv ? __ldg(a.inv + src) : src;
-  fill_unreached(depth, a.V, tid, nth, src);
-  for (int64_t i = tid; i < W; i += nth) {
-    const uint32_t x = i == (isrc >> 5) ? 1u << (isrc & 31) : 0u;
-    a.vis[i] = x;
-    r.fb[0][i] = x;
-    r.fb[1][i] = 0;
-    r.fb[2][i] = 0;
-  }
-  if (threadIdx.x == 0) {
-    const int d = a.deg[isrc];
-    ResState s;
-    s.L = s.f = s.p = 0;
-    s.td_levels = s.bu_levels = s.narrow_levels = s.err = 0;
-    s.n_f = s.n_vis = 1;
-    s.m_f = s.m_vis = d;
-    s.n_l = d < R_HEAVY;
-    s.n_g = d >= R_HUGE;
-    s.n_h = 1 - s.n_l - s.n_g;
-    s.kind = a.policy == ENT_POLICY_BU_ONLY ? RK_BU : res_td_kind(a, s);
-    s_st = s;
-    s_red[0] = s_red[1] = 0;
-    if (blockIdx.x == 0) {
-      if (s.n_l) r.queue[0][0] = isrc;
-      else if (s.n_h) r.queue[0][a.V - 1] = isrc;
-      else r.huge[0][0] = isrc;
-    }
-  }
+  uint32_t* arrived = &c->arrived[part == RP_TAIL];
   uint32_t target = 0;
-  if (!grid_barrier(&c->arrived, &c->err, target += gridDim.x, [] {})) {
-    if (tid == 0) atomicOr(&a.ctl->err, 2);
-    return;
+  if (threadIdx.x == 0) s_red[0] = s_red[1] = 0;
+  if (part == RP_TAIL) {
+    if (c->err) return;  // the head's status stands
+    if (threadIdx.x == 0) s_st = c->state;
+    __syncthreads();
+  } else {
+    const int32_t isrc = a.inv ? __ldg(a.inv + src) : src;
+    fill_unreached(depth, a.V, tid, nth, src);
+    for (int64_t i = tid; i < W; i += nth) {
+      const uint32_t x = i == (isrc >> 5) ? 1u << (isrc & 31) : 0u;
+      a.vis[i] = x;
+      r.fb[0][i] = x;
+      r.fb[1][i] = 0;
+      r.fb[2][i] = 0;
+    }
+    if (threadIdx.x == 0) {
+      const int d = a.deg[isrc];
+      ResState s;
+      s.L = s.f = s.p = 0;
+      s.td_levels = s.bu_levels = s.narrow_levels = s.err = 0;
+      s.n_f = s.n_vis = 1;
+      s.m_f = s.m_vis = d;
+      s.n_l = d < R_HEAVY;
+      s.n_g = d >= R_HUGE;
+      s.n_h = 1 - s.n_l - s.n_g;
+      s.kind = a.policy == ENT_POLICY_BU_ONLY ? RK_BU : res_td_kind(a, s);
+      s_st = s;
+      if (blockIdx.x == 0) {
+        if (s.n_l) r.queue[0][0] = isrc;
+        else if (s.n_h) r.queue[0][a.V - 1] = isrc;
+        else r.huge[0][0] = isrc;
+      }
+    }
+    if (!grid_barrier(arrived, &c->err, target += gridDim.x, [] {})) {
+      if (tid == 0) atomicOr(&a.ctl->err, 2);
+      return;
+    }
   }
   for (;;) {
     const ResState& s = s_st;  // thread 0 changes it inside the barrier only
-    if (s.kind == RK_DONE) break;
+    if (s.kind == RK_DONE || (part == RP_HEAD && s.kind == RK_BU)) break;
     int32_t* n_next = c->n[(s.p + 1) % 3];
     unsigned long long* acc = c->acc[(s.p + 1) % 3];
     if (tid < 3) c->n[(s.p + 2) % 3][tid] = 0;
@@ -602,12 +637,13 @@ __global__ void __launch_bounds__(RT, 1) k_resident(LevelArgs a, ResArgs r, int3
         s_red[0] = s_red[1] = 0;
       }
     }
-    if (!grid_barrier(&c->arrived, &c->err, target += gridDim.x, [&] { res_advance(a, r, s_st); })) {
+    if (!grid_barrier(arrived, &c->err, target += gridDim.x, [&] { res_advance(a, r, s_st); })) {
       if (tid == 0) atomicOr(&a.ctl->err, 2);
       return;
     }
   }
-  if (tid == 0) {
+  if (tid == 0 && part == RP_HEAD) c->state = s_st;
+  if (tid == 0 && part != RP_HEAD) {
     const ResState& s = s_st;
     BfsCtl* k = a.ctl;
     k->src = src;
@@ -619,7 +655,48 @@ __global__ void __launch_bounds__(RT, 1) k_resident(LevelArgs a, ResArgs r, int3
     k->narrow_levels = s.narrow_levels;
     k->iters = 0;
     k->narrow_calls = 0;
+    k->split_launches = part == RP_TAIL ? R_BU_LEVELS + 1 : 0;
     k->n_vis = s.n_vis;
     k->m_vis = s.m_vis;
   }
+}
+
+// One bottom-up level of a traversal in parts, if that is what comes next:
+// k_expand's sweep, the old frontier's bits cleared beside it, and the decision
+// by the last CTA to finish.
+template <class DT>
+__global__ void __launch_bounds__(BT, 8) k_res_bu_level(LevelArgs a, ResArgs r, DT* depth) {
+  __shared__ unsigned long long s_red[BT / 32];
+  __shared__ int s_last;
+  ResCtl* c = r.rc;
+  if (c->state.kind != RK_BU || c->err) return;
+  const int f = c->state.f, p = c->state.p, L = c->state.L;
+  {
+    uint32_t* old = r.fb[(f + 2) % 3];
+    const int64_t W = (a.V + 31) >> 5;
+    for (int64_t i = blockIdx.x * (int64_t)BT + threadIdx.x; i < W; i += (int64_t)gridDim.x * BT) old[i] = 0;
+  }
+  const Front is_front{r.fb[f], nullptr, 0, 0};
+  unsigned long long my_n = 0, my_m = 0;
+  bu_words<DT>(a, is_front, r.fb[(f + 1) % 3], L + 1, depth, nullptr, nullptr, my_n, my_m);
+  unsigned long long* acc = c->acc[(p + 1) % 3];
+  if (__syncthreads_or(my_n != 0)) {
+    unsigned long long x = block_sum(my_n, s_red);
+    if (threadIdx.x == 0) atomicAdd(&acc[0], x);
+    x = block_sum(my_m, s_red);
+    if (threadIdx.x == 0) atomicAdd(&acc[1], x);
+  }
+  if (threadIdx.x == 0) {
+    __threadfence();
+    s_last = atomicAdd(&c->finished, 1u) == gridDim.x - 1;
+  }
+  __syncthreads();
+  if (!s_last || threadIdx.x != 0) return;
+  __threadfence();
+  ResState s = c->state;
+  res_advance(a, r, s);
+  for (int i = 0; i < 3; ++i) c->n[(p + 2) % 3][i] = 0;
+  c->acc[(p + 2) % 3][0] = c->acc[(p + 2) % 3][1] = 0;
+  c->state = s;
+  c->finished = 0;
 }

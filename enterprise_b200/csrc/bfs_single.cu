@@ -47,9 +47,9 @@
 //    each queue entry carries the vertex's row start and degree, read while
 //    its visit was being claimed, so a level costs one adjacency read, one
 //    status probe and one claim on its critical path.
-//  * Graphs of up to 2^23 vertices run as one cooperative kernel instead
-//    (bfs_resident.cuh) unless they are road-like or parents are asked for;
-//    what follows is the rest.
+//  * Unless the graph is road-like or parents are asked for, a cooperative
+//    kernel goes from level to level instead (bfs_resident.cuh); what follows
+//    is the rest.
 //  * The whole traversal is one CUDA graph: a reset kernel (which also writes
 //    the loop state), then a while node whose body is two copies of
 //    [expand, inspect, narrow]; the inspector sets the loop condition and the
@@ -108,6 +108,7 @@ struct BfsCtl {
   int32_t narrow_levels;
   int32_t iters;      // inspector launches (level-loop iterations)
   int32_t narrow_runs;
+  int32_t split_launches;  // kernels after the first of a resident traversal in parts
   int32_t narrow_calls;  // launches of the small-frontier kernel, those that left at once included
   uint32_t n_spill;   // small-frontier entries that did not fit in shared memory
   uint32_t acc_maxd;  // maximum degree in the next frontier being classified
@@ -300,6 +301,7 @@ __device__ void init_state(const LevelArgs& a, int32_t caller_src, DT* depth, in
   c->iters = 0;
   c->narrow_runs = 0;
   c->narrow_calls = 0;
+  c->split_launches = 0;
   c->n_spill = 0;
   c->acc_maxd = 0;
   c->n_f = 1;
@@ -468,34 +470,15 @@ struct Front {
   }
 };
 
+// One bottom-up level over the status words of vertices that have rows. Finds
+// are counted in my_n and their degrees in my_m; hub_next may be null.
 template <class DT>
-__device__ void bu_expand(const LevelArgs& a, BfsCtl* c, int L, DT* depth, int32_t* parent, int32_t* s_hub,
-                          unsigned long long* s_red) {
-  const uint32_t* fbc = a.fb[L & 1];
-  uint32_t* fbn = a.fb[(L + 1) & 1];
-  unsigned long long* hub_next = a.hub[(L + 1) & 1];
-  if (a.hub_slots) {
-    const unsigned long long* ht = a.hub[L & 1];
-    for (int i = threadIdx.x; i < a.hub_slots; i += BT) {
-      const unsigned long long key = ht[i];
-      s_hub[i] = key ? (int)(uint32_t)key : -1;
-    }
-  }
-  // listing levels: this CTA's finds, appended to raw once at the end
-  __shared__ uint32_t s_lcnt, s_lbase, s_listing;
-  __shared__ int32_t s_list[LCAP];
-  if (threadIdx.x == 0) {
-    s_lcnt = 0;
-    s_listing = c->bu_list;  // read from shared memory where needed: no register held in the loop
-  }
-  __syncthreads();
-  const Front is_front{fbc, s_hub, a.hub_slots, a.hub_shift};
+__device__ __forceinline__ void bu_words(const LevelArgs& a, const Front& is_front, uint32_t* fbn, int ln, DT* depth,
+                                         int32_t* parent, unsigned long long* hub_next, unsigned long long& my_n,
+                                         unsigned long long& my_m) {
   const int lane = threadIdx.x & 31;
-  const int64_t gtid = blockIdx.x * (int64_t)BT + threadIdx.x, nth = (int64_t)gridDim.x * BT;
-  const int64_t gw = gtid >> 5, nw = nth >> 5;
-  const int ln = L + 1;
+  const int64_t gw = (blockIdx.x * (int64_t)BT + threadIdx.x) >> 5, nw = ((int64_t)gridDim.x * BT) >> 5;
   const int64_t W = (a.n_active + 31) >> 5;
-  unsigned long long my_n = 0, my_m = 0;
   // A warp owns one status word: 32 consecutive vertex ids.
   for (int64_t wi = gw; wi < W; wi += nw) {
     const uint32_t todo_mask = a.active[wi] & ~a.vis[wi];
@@ -563,7 +546,7 @@ __device__ void bu_expand(const LevelArgs& a, BfsCtl* c, int L, DT* depth, int32
       if (parent) parent[o] = out_id(a, pu);
       my_n++;
       my_m += (unsigned long long)d;
-      hub_insert(a, hub_next, (int)v, d);
+      if (hub_next) hub_insert(a, hub_next, (int)v, d);
     }
     const unsigned fm = __ballot_sync(FULL, found);
     if (lane == 0 && fm) {
@@ -572,6 +555,37 @@ __device__ void bu_expand(const LevelArgs& a, BfsCtl* c, int L, DT* depth, int32
       fbn[wi] = fm;
     }
   }
+}
+
+template <class DT>
+__device__ void bu_expand(const LevelArgs& a, BfsCtl* c, int L, DT* depth, int32_t* parent, int32_t* s_hub,
+                          unsigned long long* s_red) {
+  const uint32_t* fbc = a.fb[L & 1];
+  uint32_t* fbn = a.fb[(L + 1) & 1];
+  unsigned long long* hub_next = a.hub[(L + 1) & 1];
+  if (a.hub_slots) {
+    const unsigned long long* ht = a.hub[L & 1];
+    for (int i = threadIdx.x; i < a.hub_slots; i += BT) {
+      const unsigned long long key = ht[i];
+      s_hub[i] = key ? (int)(uint32_t)key : -1;
+    }
+  }
+  // listing levels: this CTA's finds, appended to raw once at the end
+  __shared__ uint32_t s_lcnt, s_lbase, s_listing;
+  __shared__ int32_t s_list[LCAP];
+  if (threadIdx.x == 0) {
+    s_lcnt = 0;
+    s_listing = c->bu_list;  // read from shared memory where needed: no register held in the loop
+  }
+  __syncthreads();
+  const Front is_front{fbc, s_hub, a.hub_slots, a.hub_shift};
+  const int lane = threadIdx.x & 31;
+  const int64_t gtid = blockIdx.x * (int64_t)BT + threadIdx.x, nth = (int64_t)gridDim.x * BT;
+  const int64_t gw = gtid >> 5, nw = nth >> 5;
+  const int ln = L + 1;
+  const int64_t W = (a.n_active + 31) >> 5;
+  unsigned long long my_n = 0, my_m = 0;
+  bu_words(a, is_front, fbn, ln, depth, parent, hub_next, my_n, my_m);
   if (s_listing) {
     // List this CTA's finds: re-read the next-frontier words its warps wrote
     // (kept out of the loop above, which runs at its register limit). Lane 0
@@ -1299,6 +1313,7 @@ struct BfsWorkspace {
   // the one-kernel traversal of small graphs (null rc: not for this workspace)
   ResArgs res = {};
   int grid_res = 0;
+  bool split = false;  // bottom-up levels as kernels of their own between its head and tail
   // traversals of one workspace run one after another, whatever streams they
   // are launched on: the end of the latest one, and its stream
   cudaEvent_t ev_order = nullptr;
@@ -1468,19 +1483,19 @@ static int pick_narrow_cluster(int limit, size_t smem) {
 
 constexpr size_t RES_SMEM = 2 * R_SOLO_CAP * sizeof(int4);
 
-// Whether this graph's traversals (without parents) run as one kernel,
-// k_resident, instead of the level kernels. Measured, level kernels -> one
-// kernel, ms: R-MAT s16 0.146 -> 0.068, s20 0.158 -> 0.101, s22 0.235 -> 0.16,
-// s23 0.272 -> 0.228; ER 2^22 d16 0.41 -> 0.29, 2^23 d16 0.70 -> 0.55. At 2^24
-// vertices the bottom-up levels outweigh the launches and want k_expand's
-// occupancy: R-MAT 0.340 -> 0.355, ER d32 1.89 -> 2.43. Graphs of low mean
-// degree (grids, roads) are deep, and their levels belong in the cluster of
+// Whether this graph's traversals (without parents) run as k_resident, in one
+// kernel or in parts, instead of the CUDA graph of level kernels. Measured,
+// level kernels -> resident, ms: R-MAT s16 0.146 -> 0.068, s20 0.158 -> 0.089,
+// s22 0.235 -> 0.150, s23 0.272 -> 0.205, s24 0.340 -> 0.310; ER 2^22 d16 0.41 ->
+// 0.285, 2^24 d32 1.89 -> 1.69. In parts from 2^22 vertices on (one kernel
+// there: R-MAT s22 0.150, in parts 0.161; s24 0.345 and 0.310). Graphs of low
+// mean degree (grids, roads) are deep, and their levels belong in the cluster of
 // k_narrow: a 300^2 grid 1.5 -> 2.1 ms, 1024^2 5.4 -> 13 ms.
-constexpr int64_t RES_MAX_V = 1 << 23;
+constexpr int64_t RES_SPLIT_V = 1 << 22;
 constexpr int64_t RES_MIN_DEGREE = 5;
 static bool resident_fits(const ent_graph* g, const BfsWorkspace* w) {
   const ent_bfs_opts& o = g->opts;
-  if (g->V > RES_MAX_V || g->E < RES_MIN_DEGREE * g->V || !g->perm) return false;
+  if (g->E < RES_MIN_DEGREE * g->V || !g->perm) return false;
   if (o.loop != ENT_LOOP_GRAPH || w->narrow_nc == 0 || o.hub_slots > 0 || o.fault_inject) return false;
   int n = 0;
   for (const void* f : {(const void*)k_resident<int32_t>, (const void*)k_resident<uint8_t>})
@@ -1596,6 +1611,7 @@ static int create_workspace(ent_graph* g, BfsWorkspace** out, bool force_graph =
     }
     // small graphs: fewer CTAs, cheaper barriers, and room for other streams' work
     const int64_t want = std::max<int64_t>((V + 4 * RT - 1) / (4 * RT), g->E / (8 * RT));
+    w->split = V > RES_SPLIT_V;
     w->grid_res = (int)std::max<int64_t>(1, std::min<int64_t>(g->num_sms, want));
   }
   if (force_graph) {  // else built on first use
@@ -1619,7 +1635,7 @@ static void fill_stats(const BfsCtl& h, float ms, ent_stats* stats) {
   stats->status = h.err;
   stats->device_ms = ms;
   stats->narrow_levels = h.narrow_levels;
-  stats->launches = 1 + 2 * h.iters + h.narrow_calls;
+  stats->launches = 1 + 2 * h.iters + h.narrow_calls + h.split_launches;
 }
 
 // One launch of the workspace's instantiated traversal graph on stream s.
@@ -1644,14 +1660,16 @@ static int launch_graph(ent_graph* g, BfsWorkspace* w, int32_t src, DT* depth, i
   return ENT_OK;
 }
 
-// One launch of the resident traversal on stream s (no parents).
+// The resident traversal on stream s (no parents): one kernel, or for large
+// graphs its level kernels between two.
 // ENT_ERR_UNSUPPORTED when the GPU cannot hold all its CTAs at once (part of
 // it set aside, by MPS or a partition): the level kernels take over.
 template <class DT>
 static int launch_resident(BfsWorkspace* w, int32_t src, DT* depth, cudaStream_t s) {
   LevelArgs a = w->args;
   a.use_cond = 0;
-  void* args[4] = {&a, &w->res, &src, &depth};
+  int part = w->split ? RP_HEAD : RP_ALL;
+  void* args[5] = {&a, &w->res, &src, &depth, &part};
   ENT_CUDA(cudaMemsetAsync(w->res.rc, 0, sizeof(ResCtl), s));
   const cudaError_t e =
       cudaLaunchCooperativeKernel((const void*)k_resident<DT>, dim3(w->grid_res), dim3(RT), args, RES_SMEM, s);
@@ -1661,6 +1679,11 @@ static int launch_resident(BfsWorkspace* w, int32_t src, DT* depth, cudaStream_t
     return ENT_ERR_UNSUPPORTED;
   }
   ENT_CUDA(e);
+  if (!w->split) return ENT_OK;
+  for (int i = 0; i < R_BU_LEVELS; ++i) k_res_bu_level<DT><<<w->grid_expand, BT, 0, s>>>(a, w->res, depth);
+  ENT_CUDA(cudaGetLastError());
+  part = RP_TAIL;
+  ENT_CUDA(cudaLaunchCooperativeKernel((const void*)k_resident<DT>, dim3(w->grid_res), dim3(RT), args, RES_SMEM, s));
   return ENT_OK;
 }
 

@@ -62,9 +62,9 @@ enum ent_policy {
 /* How the level loop is driven. */
 enum ent_loop {
   ENT_LOOP_GRAPH = 0, /* whole traversal = one launch, no host round trip:
-                         a CUDA graph with a device-side while node, or on
-                         graphs of up to 2^23 vertices that are not
-                         road-like, without parents, one cooperative kernel */
+                         a CUDA graph with a device-side while node, or,
+                         without parents and on graphs of mean degree 5 and
+                         more, cooperative kernels of many levels each      */
   ENT_LOOP_HOST = 1   /* host launches each level and polls a flag     */
 };
 

@@ -64,6 +64,29 @@ def test_direction_switches(eb, orc, alpha, beta, small_max):
                large_min=1024)
 
 
+@pytest.mark.parametrize("policy", [0, 2, 3])
+def test_in_parts(eb, orc, policy):
+    """Above 2^22 vertices the bottom-up levels are kernels of their own between
+    a head and a tail (eight bottom-up levels here when all are: the tail runs
+    what the kernels between do not)."""
+    with eb.Graph.er((1 << 22) + 37, 6, seed=0xA14) as g:
+        csr = g.download()
+        o = g.opts
+        o.policy = policy
+        g.opts = o
+        iso = int(np.flatnonzero(np.diff(csr.beg_pos) == 0)[0])
+        for s in [int(x) for x in eb.pick_sources(csr.beg_pos, 33, 2)] + [iso]:
+            d, _, st = g.bfs(s)
+            exp, _ = orc.bfs(csr.beg_pos, csr.csr, s)
+            np.testing.assert_array_equal(d, exp)
+            assert st.launches == 6 and st.levels == exp.max() + 1 == st.td_levels + st.bu_levels
+            if policy == 3:
+                assert st.bu_levels == st.levels
+            row = np.zeros(csr.vert_count, np.uint8)
+            g.bfs_many([s], [row])
+            np.testing.assert_array_equal(row, np.where(exp < 0, 255, exp).astype(np.uint8))
+
+
 def test_streams_in_turn(eb, orc):
     """Asynchronous traversals of one handle on two streams keep their order: each row is its own source's."""
     import torch
