@@ -31,6 +31,7 @@ CXX_FLAGS = ["-O3", "-std=c++17", "-fPIC", "-fopenmp", "-Wall", "-I" + INCLUDE, 
 
 SOURCES = [
     "host_graph.cpp",
+    "memory.cpp",
     "device_graph.cu",
     "bfs_single.cu",
     "bfs_batch.cu",

@@ -1548,9 +1548,10 @@ void destroy_batch_workspace(BatchWorkspace* w) {
   if (!w) return;
   if (w->exec) cudaGraphExecDestroy(w->exec);
   if (w->graph) cudaGraphDestroy(w->graph);
-  if (w->slab) cudaFree(w->slab);
-  if (w->ctl) cudaFree(w->ctl);
-  if (w->ctl_h) cudaFreeHost(w->ctl_h);
+  cudaDeviceSynchronize();  // its last run may still be on any stream
+  dev_free(w->slab);
+  dev_free(w->ctl);
+  host_slot_free(w->ctl_h);
   if (w->ev0) cudaEventDestroy(w->ev0);
   if (w->ev1) cudaEventDestroy(w->ev1);
   delete w;
@@ -1680,15 +1681,16 @@ int create_batch_workspace(ent_graph* g, int n_src, BatchWorkspace** out) {
   const size_t sz_marks = al(sizeof(uint16_t) * V);
   const size_t sz_st = al(sizeof(unsigned long long) * w->cap_src) * 2 + 2 * al(sizeof(int32_t) * w->cap_src);
   const size_t total = sz_x + sz_log + 5 * sz_bits + 3 * sz_q + 2 * sz_heavy + 3 * sz_mask + sz_src + sz_st + sz_marks + 256;
-  cudaError_t e = cudaMalloc(&w->slab, total);
+  cudaError_t e = dev_alloc(&w->slab, total);
   if (e != cudaSuccess) { destroy_batch_workspace(w); return fail(ENT_ERR_OOM, "batch workspace (%zu bytes) failed", total); }
   // Initialise on the graph's stream and wait (see create_workspace in
   // bfs_single.cu): the runs use other, non-blocking streams.
   e = cudaMemsetAsync(w->slab, 0, total, g->stream);
-  if (e == cudaSuccess) e = cudaMalloc(&w->ctl, sizeof(BatchCtl));
+  if (e == cudaSuccess) e = dev_alloc(&w->ctl, sizeof(BatchCtl));
   if (e == cudaSuccess) e = cudaMemsetAsync(w->ctl, 0, sizeof(BatchCtl), g->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(g->stream);
-  if (e == cudaSuccess) e = cudaMallocHost(&w->ctl_h, sizeof(BatchCtl));
+  static_assert(sizeof(BatchCtl) <= 512, "the control block's pinned copy is a host slot");
+  if (e == cudaSuccess && !(w->ctl_h = (BatchCtl*)host_slot(sizeof(BatchCtl)))) e = cudaErrorMemoryAllocation;
   if (e == cudaSuccess) e = cudaEventCreate(&w->ev0);
   if (e == cudaSuccess) e = cudaEventCreate(&w->ev1);
   if (e != cudaSuccess) { destroy_batch_workspace(w); return fail(ENT_ERR_OOM, "batch workspace setup failed"); }
@@ -2029,17 +2031,17 @@ static int batch_to_host(ent_graph* g, const int32_t* src, int32_t n_src, void* 
   DeviceGuard dg(g->device);
   const size_t need = (bytes ? 1 : sizeof(int32_t)) * (size_t)n_src * g->V;
   if (g->stage_cap < need) {
-    if (g->stage) cudaFree(g->stage);
+    dev_free(g->stage);
     g->stage = nullptr;
     g->stage_cap = 0;
-    ENT_CUDA(cudaMalloc(&g->stage, need));
+    ENT_CUDA(dev_alloc(&g->stage, need));
     g->stage_cap = need;
   }
   std::vector<ent_stats> local(stats ? 0 : n_src);
   int rc = run_bfs_batch(g, src, n_src, static_cast<int32_t*>(g->stage), g->stream, stats ? stats : local.data(), bytes);
   // a byte row past depth 254 still holds the other sources' complete rows
   if (rc != ENT_OK && !(bytes && rc == ENT_ERR_UNSUPPORTED)) return rc;
-  if (depth_out) ENT_CUDA(cudaMemcpyAsync(depth_out, g->stage, need, cudaMemcpyDeviceToHost, g->stream));
+  if (depth_out) ENT_CUDA(to_host(depth_out, g->stage, need, g->stream));
   ENT_CUDA(cudaStreamSynchronize(g->stream));
   return rc;
 }
@@ -2180,8 +2182,8 @@ static void multi_free(ent_multi* m) {
   if (m->graph) cudaGraphDestroy(m->graph);
   for (MultiUnion& mu : m->unions) {
     destroy_batch_workspace(mu.w);
-    if (mu.depth) cudaFree(mu.depth);
-    if (mu.seeds) cudaFree(mu.seeds);
+    dev_free(mu.depth);
+    dev_free(mu.seeds);
     if (mu.u) ent_graph_destroy(mu.u);
   }
   if (m->ev0) cudaEventDestroy(m->ev0);
@@ -2309,9 +2311,9 @@ int ent_multi_create(ent_graph* const* graphs, int32_t n_graphs, const int32_t* 
         h[mu.n_seed + j] = i;
       }
     }
-    e = cudaMalloc(&mu.seeds, sizeof(int32_t) * h.size());
+    e = dev_alloc(&mu.seeds, sizeof(int32_t) * h.size());
     if (e == cudaSuccess) e = cudaMemcpy(mu.seeds, h.data(), sizeof(int32_t) * h.size(), cudaMemcpyHostToDevice);
-    if (e == cudaSuccess) e = cudaMalloc(&mu.depth, sizeof(int32_t) * (size_t)mu.slots * mu.u->V);
+    if (e == cudaSuccess) e = dev_alloc(&mu.depth, sizeof(int32_t) * (size_t)mu.slots * mu.u->V);
     if (e != cudaSuccess) { multi_free(m); return fail(ENT_ERR_OOM, "multi seed list or output allocation failed"); }
     mu.w->args.src = mu.seeds;
     mu.w->args.seed_slot = mu.seeds + mu.n_seed;
@@ -2360,12 +2362,12 @@ int ent_multi_depths(ent_multi* m, int32_t k, int32_t* depth_out) {
   int max_pitch = 0;
   ENT_CUDA(cudaDeviceGetAttribute(&max_pitch, cudaDevAttrMaxPitch, m->device));
   if (pitch <= (size_t)max_pitch) {
-    ENT_CUDA(cudaMemcpy2D(depth_out, width, mu.depth + p.v0, pitch, width, m->n_src[k], cudaMemcpyDeviceToHost));
+    ENT_CUDA(rows_to_host(depth_out, mu.depth + p.v0, width, pitch, m->n_src[k], m->stream));
   } else {
     for (int32_t i = 0; i < m->n_src[k]; ++i)
-      ENT_CUDA(cudaMemcpy(depth_out + (size_t)i * m->vcount[k], mu.depth + (size_t)i * mu.u->V + p.v0, width,
-                          cudaMemcpyDeviceToHost));
+      ENT_CUDA(to_host(depth_out + (size_t)i * m->vcount[k], mu.depth + (size_t)i * mu.u->V + p.v0, width, m->stream));
   }
+  ENT_CUDA(cudaStreamSynchronize(m->stream));
   return ENT_OK;
 }
 

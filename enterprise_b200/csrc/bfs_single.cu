@@ -1338,17 +1338,17 @@ void destroy_bfs_workspace(BfsWorkspace* w) {
     if (w->exec[k]) cudaGraphExecDestroy(w->exec[k]);
     if (w->graph[k]) cudaGraphDestroy(w->graph[k]);
   }
-  if (w->slab) cudaFree(w->slab);
-  if (w->ctl) cudaFree(w->ctl);
-  if (w->ctl_h) cudaFreeHost(w->ctl_h);
-  if (w->depth) cudaFree(w->depth);
-  if (w->parent) cudaFree(w->parent);
+  cudaDeviceSynchronize();  // its last traversal may still be on any stream
+  dev_free(w->slab);
+  dev_free(w->ctl);
+  host_slot_free(w->ctl_h);
+  dev_free(w->depth);
+  dev_free(w->parent);
   if (w->ev0) cudaEventDestroy(w->ev0);
   if (w->ev1) cudaEventDestroy(w->ev1);
   if (w->ev_order) cudaEventDestroy(w->ev_order);
-  if (w->depth_b) cudaFree(w->depth_b);
-  for (int i = 0; i < 2; ++i)
-    if (w->depth8[i]) cudaFree(w->depth8[i]);
+  dev_free(w->depth_b);
+  for (int i = 0; i < 2; ++i) dev_free(w->depth8[i]);
   if (w->copy_stream) cudaStreamDestroy(w->copy_stream);
   if (w->many_ctl_h) cudaFreeHost(w->many_ctl_h);
   for (cudaEvent_t e : w->many_ev) cudaEventDestroy(e);
@@ -1524,18 +1524,19 @@ static int create_workspace(ent_graph* g, BfsWorkspace** out, bool force_graph =
   size_t sz_hub = al(sizeof(unsigned long long) * (hub > 0 ? hub : 1));
   size_t sz_tiles = al(sizeof(unsigned long long) * tiles * KS);
   size_t total = 4 * sz_bits + 9 * sz_q + 2 * sz_hub + sz_tiles + al(sizeof(ResCtl));
-  cudaError_t e = cudaMalloc(&w->slab, total);
+  cudaError_t e = dev_alloc(&w->slab, total);
   if (e != cudaSuccess) { destroy_bfs_workspace(w); return fail(ENT_ERR_OOM, "workspace allocation (%zu bytes) failed", total); }
   // Initialise on the graph's stream and wait: the traversal runs on
   // non-blocking streams, which a plain cudaMemset (legacy stream, async to
   // the host) would not be ordered against.
   e = cudaMemsetAsync(w->slab, 0, total, g->stream);
-  if (e == cudaSuccess) e = cudaMalloc(&w->ctl, sizeof(BfsCtl));
+  if (e == cudaSuccess) e = dev_alloc(&w->ctl, sizeof(BfsCtl));
   if (e == cudaSuccess) e = cudaMemsetAsync(w->ctl, 0, sizeof(BfsCtl), g->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(g->stream);
-  if (e == cudaSuccess) e = cudaMallocHost(&w->ctl_h, sizeof(BfsCtl));
-  if (e == cudaSuccess) e = cudaMalloc(&w->depth, sizeof(int32_t) * V);
-  if (e == cudaSuccess) e = cudaMalloc(&w->parent, sizeof(int32_t) * V);
+  static_assert(sizeof(BfsCtl) <= 512, "the control block's pinned copy is a host slot");
+  if (e == cudaSuccess && !(w->ctl_h = (BfsCtl*)host_slot(sizeof(BfsCtl)))) e = cudaErrorMemoryAllocation;
+  if (e == cudaSuccess) e = dev_alloc(&w->depth, sizeof(int32_t) * V);
+  if (e == cudaSuccess) e = dev_alloc(&w->parent, sizeof(int32_t) * V);
   if (e == cudaSuccess) e = cudaEventCreate(&w->ev0);
   if (e == cudaSuccess) e = cudaEventCreate(&w->ev1);
   if (e == cudaSuccess) e = cudaEventCreateWithFlags(&w->ev_order, cudaEventDisableTiming);
@@ -2059,9 +2060,9 @@ int ent_bfs(ent_graph* g, int32_t src, int32_t* depth_out, int32_t* parent_out, 
   // the copies are queued behind the traversal, before its statistics are waited for
   const auto copies = [&]() -> int {
     if (depth_out)
-      ENT_CUDA(cudaMemcpyAsync(depth_out, w->depth, sizeof(int32_t) * g->V, cudaMemcpyDeviceToHost, g->stream));
+      ENT_CUDA(to_host(depth_out, w->depth, sizeof(int32_t) * g->V, g->stream));
     if (parent_out)
-      ENT_CUDA(cudaMemcpyAsync(parent_out, w->parent, sizeof(int32_t) * g->V, cudaMemcpyDeviceToHost, g->stream));
+      ENT_CUDA(to_host(parent_out, w->parent, sizeof(int32_t) * g->V, g->stream));
     return ENT_OK;
   };
   return run_bfs_typed<int32_t>(g, src, w->depth, parent_out ? w->parent : nullptr, g->stream,
@@ -2091,12 +2092,12 @@ static int bfs_many(ent_graph* g, const int32_t* src, int32_t n_src, void* const
   }
   if (n_src == 0) return ENT_OK;
   BfsWorkspace* w = g->ws;
-  if (!bytes && !w->depth_b && cudaMalloc(&w->depth_b, sizeof(int32_t) * g->V) != cudaSuccess) {
+  if (!bytes && !w->depth_b && dev_alloc(&w->depth_b, sizeof(int32_t) * g->V) != cudaSuccess) {
     w->depth_b = nullptr;
     return fail(ENT_ERR_OOM, "second depth buffer (%lld bytes) failed", (long long)(sizeof(int32_t) * g->V));
   }
   for (int i = 0; bytes && i < 2; ++i)
-    if (!w->depth8[i] && cudaMalloc(&w->depth8[i], (size_t)g->V) != cudaSuccess) {
+    if (!w->depth8[i] && dev_alloc(&w->depth8[i], (size_t)g->V) != cudaSuccess) {
       w->depth8[i] = nullptr;
       return fail(ENT_ERR_OOM, "byte depth buffer (%lld bytes) failed", (long long)g->V);
     }

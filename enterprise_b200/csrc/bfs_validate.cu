@@ -260,7 +260,7 @@ extern "C" int ent_validate(ent_graph* g, int32_t src, const int32_t* depth_dev,
   constexpr int NW = 6;
   unsigned long long h[NW];
   if (!g->val) {
-    const cudaError_t ea = cudaMalloc(&g->val, 256 + sizeof(int32_t) * (g->perm ? V : 0));
+    const cudaError_t ea = dev_alloc(&g->val, 256 + sizeof(int32_t) * (g->perm ? V : 0));
     if (ea != cudaSuccess) {
       g->val = nullptr;
       return fail(ENT_ERR_OOM, "validation scratch: %s", cudaGetErrorString(ea));

@@ -89,6 +89,30 @@ struct DeviceGuard {
                          __LINE__);                                                         \
   } while (0)
 
+// Device memory of the library's own, from a pool (memory.cpp), on the current
+// device and ready for any stream. dev_free: no work may still use the memory.
+cudaError_t dev_alloc(void** out, size_t bytes);
+void dev_free(void* ptr);
+template <class T>
+cudaError_t dev_alloc(T** out, size_t bytes) { return dev_alloc(reinterpret_cast<void**>(out), bytes); }
+// cudaMalloc, for memory whose address a caller may get (it can be shared with
+// peers and other processes, which pool memory cannot); frees what the pool
+// keeps before it fails.
+cudaError_t dev_malloc(void** out, size_t bytes);
+template <class T>
+cudaError_t dev_malloc(T** out, size_t bytes) { return dev_malloc(reinterpret_cast<void**>(out), bytes); }
+// A page-locked block of at most 512 bytes, for copies from any device; null
+// when there is no memory. host_slot_free: no copy may still use it.
+void* host_slot(size_t bytes);
+void host_slot_free(void* p);
+// Copies on stream s between the device and host memory of any kind. Pageable
+// memory has been read, or holds the data, when the call returns (after the
+// stream got there); page-locked memory is copied asynchronously.
+cudaError_t to_device(void* dst, const void* src, size_t bytes, cudaStream_t s);
+cudaError_t to_host(void* dst, const void* src, size_t bytes, cudaStream_t s);
+// `rows` rows of `width` bytes, `pitch` apart on the device, to a contiguous host array.
+cudaError_t rows_to_host(void* dst, const void* src, size_t width, size_t pitch, size_t rows, cudaStream_t s);
+
 int graph_alloc(ent_graph* g, int64_t V, int64_t E);
 int graph_finish(ent_graph* g);  // computes deg, creates stream
 int run_bfs_single(ent_graph* g, int32_t src, int32_t* depth_dev, int32_t* parent_dev, cudaStream_t stream,

@@ -22,8 +22,10 @@ ErParams make_er_params(int64_t n, double mean_degree, uint64_t seed);
 int graph_alloc(ent_graph* g, int64_t V, int64_t E) {
   g->V = V;
   g->E = E;
-  ENT_CUDA(cudaMalloc(&g->off, sizeof(int64_t) * (V + 1)));
-  ENT_CUDA(cudaMalloc(&g->adj, sizeof(int32_t) * (E > 0 ? E : 1)));
+  // one allocation: offsets, then (256-byte aligned) the column ids
+  const size_t at = (sizeof(int64_t) * (V + 1) + 255) & ~(size_t)255;
+  ENT_CUDA(dev_malloc(&g->off, at + sizeof(int32_t) * (E > 0 ? E : 1)));
+  g->adj = reinterpret_cast<int32_t*>(reinterpret_cast<char*>(g->off) + at);
   return ENT_OK;
 }
 
@@ -162,7 +164,7 @@ static cudaError_t build_traversal_order(ent_graph* g) {
   const size_t sz_a = 3 * sz_v, sz_b = al(sizeof(int32_t) * E);
   const size_t t_cub = al(std::max(std::max(t_sort, t_scan), t_seg));
   char* tmp = nullptr;
-  e = cudaMalloc(&tmp, 256 + std::max(sz_a, sz_b) + t_cub);
+  e = dev_alloc(&tmp, 256 + std::max(sz_a, sz_b) + t_cub);
   if (e != cudaSuccess) return e;
   int64_t* n_active = (int64_t*)tmp;  // [0], and [1]: some row is not sorted
   uint32_t* key = (uint32_t*)(tmp + 256);
@@ -188,7 +190,7 @@ static cudaError_t build_traversal_order(ent_graph* g) {
   const cudaError_t e2 = cudaStreamSynchronize(s);
   g->n_active = h[0];
   g->rows_sorted = h[1] == 0;
-  cudaFree(tmp);
+  dev_free(tmp);
   return e != cudaSuccess ? e : e2;
 }
 
@@ -197,7 +199,7 @@ int graph_finish(ent_graph* g) {
   if (!g->stream) ENT_CUDA(cudaStreamCreateWithFlags(&g->stream, cudaStreamNonBlocking));
   const int64_t V = g->V, E = g->E;
   const TravLayout l = trav_layout(V, E);
-  ENT_CUDA(cudaMalloc(&g->slab, l.total));
+  ENT_CUDA(dev_alloc(&g->slab, l.total));
   char* p = (char*)g->slab;
   g->lead = (int4*)(p + l.lead);
   g->deg = (int32_t*)(p + l.deg);
@@ -237,11 +239,11 @@ static void graph_free(ent_graph* g) {
   if (g->ws) destroy_bfs_workspace(g->ws);
   if (g->bws) destroy_batch_workspace(g->bws);
   if (g->lanes) destroy_deep_lanes(g->lanes);
-  if (g->stage) cudaFree(g->stage);
-  if (g->val) cudaFree(g->val);
-  if (g->slab) cudaFree(g->slab);
+  cudaDeviceSynchronize();  // nothing of the graph's may still be in use
+  dev_free(g->stage);
+  dev_free(g->val);
+  dev_free(g->slab);
   if (g->off) cudaFree(g->off);
-  if (g->adj) cudaFree(g->adj);
   if (g->stream) cudaStreamDestroy(g->stream);
   delete g;
 }
@@ -345,10 +347,11 @@ static int build_on_device(Draw draw, uint64_t n_draws, int64_t V, int gpu, ent_
   int64_t* d_nsel = nullptr;
   int rc = ENT_OK;
   auto cleanup = [&]() {
-    if (k0) cudaFree(k0);
-    if (k1) cudaFree(k1);
-    if (tmp) cudaFree(tmp);
-    if (d_nsel) cudaFree(d_nsel);
+    cudaStreamSynchronize(s);
+    dev_free(k0);
+    dev_free(k1);
+    dev_free(tmp);
+    dev_free(d_nsel);
   };
 #define GEN_CUDA(call)                                                                          \
   do {                                                                                          \
@@ -361,9 +364,9 @@ static int build_on_device(Draw draw, uint64_t n_draws, int64_t V, int gpu, ent_
       return rc;                                                                                \
     }                                                                                           \
   } while (0)
-  GEN_CUDA(cudaMalloc(&k0, sizeof(uint64_t) * std::max<int64_t>(n_keys, 1)));
-  GEN_CUDA(cudaMalloc(&k1, sizeof(uint64_t) * std::max<int64_t>(n_keys, 1)));
-  GEN_CUDA(cudaMalloc(&d_nsel, sizeof(int64_t)));
+  GEN_CUDA(dev_alloc(&k0, sizeof(uint64_t) * std::max<int64_t>(n_keys, 1)));
+  GEN_CUDA(dev_alloc(&k1, sizeof(uint64_t) * std::max<int64_t>(n_keys, 1)));
+  GEN_CUDA(dev_alloc(&d_nsel, sizeof(int64_t)));
   int blocks = nsm * 16;
   k_gen_keys<<<blocks, 256, 0, s>>>(draw, n_draws, kc, k0);
   g_kernel_launches++;
@@ -372,7 +375,7 @@ static int build_on_device(Draw draw, uint64_t n_draws, int64_t V, int gpu, ent_
   GEN_CUDA(cub::DeviceRadixSort::SortKeys(nullptr, tmp_bytes, db, n_keys, 0, end_bit, s));
   GEN_CUDA(cub::DeviceSelect::Unique(nullptr, tmp2, k0, k1, d_nsel, n_keys, s));
   tmp_bytes = std::max(tmp_bytes, tmp2);
-  GEN_CUDA(cudaMalloc(&tmp, tmp_bytes));
+  GEN_CUDA(dev_alloc(&tmp, tmp_bytes));
   GEN_CUDA(cub::DeviceRadixSort::SortKeys(tmp, tmp_bytes, db, n_keys, 0, end_bit, s));
   uint64_t* sorted = db.Current();
   uint64_t* uniq = db.Alternate();
@@ -470,9 +473,9 @@ int ent_graph_create(const int64_t* beg, const int32_t* csr, int64_t V, int64_t 
   // CSR next run on this non-blocking stream.
   cudaError_t e1 = cudaStreamCreateWithFlags(&g->stream, cudaStreamNonBlocking);
   if (e1 == cudaSuccess)
-    e1 = cudaMemcpyAsync(g->off, beg, sizeof(int64_t) * (V + 1), cudaMemcpyHostToDevice, g->stream);
+    e1 = to_device(g->off, beg, sizeof(int64_t) * (V + 1), g->stream);
   cudaError_t e2 = (E > 0 && e1 == cudaSuccess)
-                       ? cudaMemcpyAsync(g->adj, csr, sizeof(int32_t) * E, cudaMemcpyHostToDevice, g->stream)
+                       ? to_device(g->adj, csr, sizeof(int32_t) * E, g->stream)
                        : cudaSuccess;
   if (e1 == cudaSuccess && e2 == cudaSuccess) e1 = cudaStreamSynchronize(g->stream);
   if (e1 != cudaSuccess || e2 != cudaSuccess) {
@@ -563,11 +566,11 @@ int ent_graph_from_edges(const int64_t* src, const int64_t* dst, int64_t n, int6
   cudaStream_t s = nullptr;
   cudaError_t e = cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking);
   const size_t bytes = sizeof(int64_t) * (size_t)std::max<int64_t>(n, 1);
-  if (e == cudaSuccess) e = cudaMalloc(&d_src, bytes);
-  if (e == cudaSuccess) e = cudaMalloc(&d_dst, bytes);
-  if (e == cudaSuccess) e = cudaMalloc(&d_bad, sizeof(bad));
-  if (e == cudaSuccess && n > 0) e = cudaMemcpyAsync(d_src, src, sizeof(int64_t) * n, cudaMemcpyHostToDevice, s);
-  if (e == cudaSuccess && n > 0) e = cudaMemcpyAsync(d_dst, dst, sizeof(int64_t) * n, cudaMemcpyHostToDevice, s);
+  if (e == cudaSuccess) e = dev_alloc(&d_src, bytes);
+  if (e == cudaSuccess) e = dev_alloc(&d_dst, bytes);
+  if (e == cudaSuccess) e = dev_alloc(&d_bad, sizeof(bad));
+  if (e == cudaSuccess && n > 0) e = to_device(d_src, src, sizeof(int64_t) * n, s);
+  if (e == cudaSuccess && n > 0) e = to_device(d_dst, dst, sizeof(int64_t) * n, s);
   if (e == cudaSuccess) e = cudaMemcpyAsync(d_bad, &bad, sizeof(bad), cudaMemcpyHostToDevice, s);
   if (e == cudaSuccess && n > 0) {
     int nsm = 148;
@@ -586,9 +589,10 @@ int ent_graph_from_edges(const int64_t* src, const int64_t* dst, int64_t n, int6
   } else {
     rc = build_on_device(ListDraw{d_src, d_dst}, (uint64_t)n, V, gpu, out);
   }
-  if (d_src) cudaFree(d_src);
-  if (d_dst) cudaFree(d_dst);
-  if (d_bad) cudaFree(d_bad);
+  if (s) cudaStreamSynchronize(s);
+  dev_free(d_src);
+  dev_free(d_dst);
+  dev_free(d_bad);
   if (s) cudaStreamDestroy(s);
   return rc;
 }
@@ -610,7 +614,7 @@ int ent_device_alloc(int32_t gpu, size_t bytes, void** out) {
     return fail(ENT_ERR_INVALID_ARG, "no GPU %d (%d present)", gpu, n);
   DeviceGuard dg(gpu);
   void* p = nullptr;
-  if (cudaMalloc(&p, bytes ? bytes : 1) != cudaSuccess)
+  if (dev_malloc(&p, bytes ? bytes : 1) != cudaSuccess)
     return fail(ENT_ERR_OOM, "device allocation of %zu bytes on GPU %d failed", bytes, gpu);
   *out = p;
   return ENT_OK;
@@ -626,8 +630,10 @@ int ent_graph_download(const ent_graph* g, int64_t* beg, int32_t* csr) {
   clear_error();
   if (!g || !beg || (!csr && g->E > 0)) return fail(ENT_ERR_INVALID_ARG, "null argument");
   DeviceGuard dg(g->device);
-  ENT_CUDA(cudaMemcpy(beg, g->off, sizeof(int64_t) * (g->V + 1), cudaMemcpyDeviceToHost));
-  if (g->E > 0) ENT_CUDA(cudaMemcpy(csr, g->adj, sizeof(int32_t) * g->E, cudaMemcpyDeviceToHost));
+  // on the legacy stream, as a plain copy is, and waited for
+  ENT_CUDA(to_host(beg, g->off, sizeof(int64_t) * (g->V + 1), nullptr));
+  if (g->E > 0) ENT_CUDA(to_host(csr, g->adj, sizeof(int32_t) * g->E, nullptr));
+  ENT_CUDA(cudaStreamSynchronize(nullptr));
   return ENT_OK;
 }
 

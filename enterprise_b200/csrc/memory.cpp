@@ -1,0 +1,257 @@
+// Device memory from a pool, and host copies through page-locked staging.
+//
+// cudaMalloc and cudaFree map and unmap memory and wait for the device: 0.3 to
+// 0.5 ms each at tens of MB, with outliers of tens of ms, and building a graph
+// and traversing it once made 15 of each (R-MAT s18 edge list: 11 of 19 ms).
+// dev_alloc takes memory from a pool of the library's own that keeps up to
+// POOL_KEEP bytes of what was given back for the next allocation. Whatever is
+// above goes back to the device at once, and all of it when an allocation of
+// this library fails.
+//
+// A copy between the device and pageable host memory runs through the driver's
+// own staging on one host thread (about 10 GB/s, first touch of fresh pages
+// included). Here two page-locked chunks take turns: the DMA of one overlaps
+// the copying of the other by several threads.
+#include <algorithm>
+#include <cuda_runtime.h>
+#include <mutex>
+#include <omp.h>
+#include <string.h>
+#include <vector>
+
+#include "dev_graph.h"
+
+namespace ent {
+namespace {
+
+constexpr uint64_t POOL_KEEP = 512ull << 20;  // per device
+constexpr size_t CHUNK = 4 << 20;             // bytes per staging chunk
+constexpr size_t STAGED_MIN = 1 << 20;        // shorter copies go to the driver
+constexpr int COPY_THREADS = 8;
+
+struct DevicePool {
+  cudaMemPool_t pool = nullptr;
+  cudaStream_t stream = nullptr;  // orders the pool's own allocations and frees
+  bool tried = false;
+};
+std::mutex g_mu;
+std::vector<DevicePool> g_pools;      // by device
+std::vector<char*> g_idle;            // page-locked pairs of chunks not in use
+int g_pairs = 0;                      // ... and all of them
+constexpr int MAX_PAIRS = 2;          // 16 MB; further copies at the same time go to the driver
+
+// Small page-locked blocks (a traversal's status words): a slot of an arena, for
+// a call of cudaHostAlloc and cudaFreeHost each takes as long as a small graph's
+// whole build. Arenas stay; their number follows the most slots in use at once.
+constexpr size_t SLOT = 512, ARENA = 64 << 10;
+std::vector<char*> g_slots;           // free ones
+
+// The current device's pool; pool null where it cannot have one.
+DevicePool device_pool() {
+  int dev = 0;
+  cudaGetDevice(&dev);
+  std::lock_guard<std::mutex> lk(g_mu);
+  if ((int)g_pools.size() <= dev) g_pools.resize(dev + 1);
+  DevicePool& p = g_pools[dev];
+  if (!p.tried) {
+    p.tried = true;
+    int ok = 0;
+    cudaMemPoolProps props = {};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = dev;
+    uint64_t keep = POOL_KEEP;
+    if (cudaDeviceGetAttribute(&ok, cudaDevAttrMemoryPoolsSupported, dev) != cudaSuccess || !ok ||
+        cudaStreamCreateWithFlags(&p.stream, cudaStreamNonBlocking) != cudaSuccess ||
+        cudaMemPoolCreate(&p.pool, &props) != cudaSuccess ||
+        cudaMemPoolSetAttribute(p.pool, cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess) {
+      cudaGetLastError();
+      p.pool = nullptr;
+    }
+  }
+  return p;
+}
+
+struct Staging {
+  char* buf = nullptr;  // two chunks
+  cudaEvent_t done[2] = {nullptr, nullptr};
+  Staging() {
+    {
+      std::lock_guard<std::mutex> lk(g_mu);
+      if (!g_idle.empty()) {
+        buf = g_idle.back();
+        g_idle.pop_back();
+      } else if (g_pairs < MAX_PAIRS) {
+        if (cudaHostAlloc((void**)&buf, 2 * CHUNK, cudaHostAllocPortable) == cudaSuccess) {
+          ++g_pairs;
+        } else {
+          buf = nullptr;
+          cudaGetLastError();
+        }
+      }
+    }
+    for (cudaEvent_t& e : done)
+      if (buf && cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess) {
+        e = nullptr;
+        cudaGetLastError();
+      }
+  }
+  bool ok() const { return buf && done[0] && done[1]; }
+  ~Staging() {
+    for (cudaEvent_t e : done)
+      if (e) {
+        cudaEventSynchronize(e);  // no DMA may still use the chunk
+        cudaEventDestroy(e);
+      }
+    if (!buf) return;
+    std::lock_guard<std::mutex> lk(g_mu);
+    g_idle.push_back(buf);
+  }
+};
+
+// memcpy by several threads (first touch of the destination's pages included).
+void copy_host(char* dst, const char* src, size_t n) {
+  const int t = (int)std::min<size_t>(std::min(COPY_THREADS, omp_get_max_threads()), n / (256 << 10) + 1);
+  if (t <= 1) {
+    memcpy(dst, src, n);
+    return;
+  }
+#pragma omp parallel for num_threads(t) schedule(static)
+  for (int i = 0; i < t; ++i) {
+    const size_t a = n * i / t, b = n * (i + 1) / t;
+    memcpy(dst + a, src + a, b - a);
+  }
+}
+
+bool pageable(const void* host) {
+  cudaPointerAttributes at;
+  if (cudaPointerGetAttributes(&at, host) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  return at.type == cudaMemoryTypeUnregistered;
+}
+
+}  // namespace
+
+cudaError_t dev_alloc(void** out, size_t bytes) {
+  *out = nullptr;
+  bytes = std::max<size_t>(bytes, 1);
+  const DevicePool p = device_pool();
+  if (!p.pool) return cudaMalloc(out, bytes);
+  cudaError_t e = cudaMallocFromPoolAsync(out, bytes, p.pool, p.stream);
+  if (e == cudaErrorMemoryAllocation) {
+    cudaGetLastError();
+    cudaMemPoolTrimTo(p.pool, 0);
+    e = cudaMallocFromPoolAsync(out, bytes, p.pool, p.stream);
+  }
+  // usable on any stream once the pool's stream has reached it
+  if (e == cudaSuccess) e = cudaStreamSynchronize(p.stream);
+  if (e != cudaSuccess) *out = nullptr;
+  return e;
+}
+
+cudaError_t dev_malloc(void** out, size_t bytes) {
+  cudaError_t e = cudaMalloc(out, bytes);
+  if (e != cudaErrorMemoryAllocation) return e;
+  cudaGetLastError();
+  const DevicePool p = device_pool();
+  if (p.pool) cudaMemPoolTrimTo(p.pool, 0);
+  return cudaMalloc(out, bytes);
+}
+
+void dev_free(void* ptr) {
+  if (!ptr) return;
+  const DevicePool p = device_pool();
+  if (p.pool) cudaFreeAsync(ptr, p.stream);
+  else cudaFree(ptr);
+}
+
+void* host_slot(size_t bytes) {
+  if (bytes > SLOT) return nullptr;
+  std::lock_guard<std::mutex> lk(g_mu);
+  if (g_slots.empty()) {
+    char* a = nullptr;
+    if (cudaHostAlloc((void**)&a, ARENA, cudaHostAllocPortable) != cudaSuccess) {
+      cudaGetLastError();
+      return nullptr;
+    }
+    for (size_t at = 0; at < ARENA; at += SLOT) g_slots.push_back(a + at);
+  }
+  char* p = g_slots.back();
+  g_slots.pop_back();
+  return p;
+}
+
+void host_slot_free(void* p) {
+  if (!p) return;
+  std::lock_guard<std::mutex> lk(g_mu);
+  g_slots.push_back((char*)p);
+}
+
+cudaError_t to_device(void* dst, const void* src, size_t bytes, cudaStream_t s) {
+  if (bytes < STAGED_MIN || !pageable(src)) return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, s);
+  Staging st;
+  if (!st.ok()) return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, s);
+  cudaError_t e = cudaSuccess;
+  for (size_t at = 0, k = 0; at < bytes && e == cudaSuccess; at += CHUNK, ++k) {
+    const size_t n = std::min(CHUNK, bytes - at);
+    char* buf = st.buf + (k & 1) * CHUNK;
+    if (k >= 2) e = cudaEventSynchronize(st.done[k & 1]);
+    if (e != cudaSuccess) break;
+    copy_host(buf, (const char*)src + at, n);
+    e = cudaMemcpyAsync((char*)dst + at, buf, n, cudaMemcpyHostToDevice, s);
+    if (e == cudaSuccess) e = cudaEventRecord(st.done[k & 1], s);
+  }
+  return e;
+}
+
+cudaError_t rows_to_host(void* dst, const void* src, size_t width, size_t pitch, size_t rows, cudaStream_t s) {
+  if (width == 0 || rows == 0) return cudaSuccess;
+  const size_t bytes = width * rows;
+  const auto direct = [&] {
+    return pitch == width ? cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, s)
+                          : cudaMemcpy2DAsync(dst, width, src, pitch, width, rows, cudaMemcpyDeviceToHost, s);
+  };
+  // whole rows per chunk, or one run of bytes; other shapes go to the driver
+  const bool flat = pitch == width;
+  if (bytes < STAGED_MIN || (!flat && width > CHUNK) || !pageable(dst)) return direct();
+  Staging st;
+  if (!st.ok()) return direct();
+  const size_t unit = flat ? 1 : width, per = flat ? CHUNK : CHUNK / width * width;
+  struct Part {
+    size_t at = 0, n = 0;
+  } part[2];
+  cudaError_t e = cudaSuccess;
+  size_t at = 0;
+  for (size_t k = 0;; ++k) {
+    Part& p = part[k & 1];
+    if (p.n) {  // the DMA of two turns ago: copy it out (the other chunk's is in flight)
+      e = cudaEventSynchronize(st.done[k & 1]);
+      if (e != cudaSuccess) break;
+      copy_host((char*)dst + p.at, st.buf + (k & 1) * CHUNK, p.n);
+      p.n = 0;
+    }
+    if (at < bytes) {
+      const size_t n = std::min(per, bytes - at);
+      char* buf = st.buf + (k & 1) * CHUNK;
+      e = flat ? cudaMemcpyAsync(buf, (const char*)src + at, n, cudaMemcpyDeviceToHost, s)
+               : cudaMemcpy2DAsync(buf, width, (const char*)src + at / unit * pitch, pitch, width, n / unit,
+                                   cudaMemcpyDeviceToHost, s);
+      if (e == cudaSuccess) e = cudaEventRecord(st.done[k & 1], s);
+      if (e != cudaSuccess) break;
+      p.at = at;
+      p.n = n;
+      at += n;
+    } else if (!part[0].n && !part[1].n) {
+      break;
+    }
+  }
+  return e;
+}
+
+cudaError_t to_host(void* dst, const void* src, size_t bytes, cudaStream_t s) {
+  return rows_to_host(dst, src, bytes, bytes, 1, s);
+}
+
+}  // namespace ent

@@ -445,7 +445,7 @@ int ent_server_create(ent_graph* const* graphs, int32_t n_graphs, const ent_serv
     int64_t rows = o.rows_per_graph > 0 ? o.rows_per_graph : (budget / n_graphs) / (g.V * 4);
     rows = std::max<int64_t>(1, std::min<int64_t>(rows, 1 << 16));
     g.rows = (int32_t)rows;
-    cudaError_t e = cudaMalloc(&g.pool, sizeof(int32_t) * (size_t)g.rows * g.V);
+    cudaError_t e = dev_malloc(&g.pool, sizeof(int32_t) * (size_t)g.rows * g.V);
     if (e != cudaSuccess) {
       free_server(s);
       return fail(ENT_ERR_OOM, "graph %d: depth pool of %d rows does not fit", k, g.rows);
