@@ -1035,11 +1035,13 @@ __device__ __forceinline__ void narrow_append(const LevelArgs& a, BfsCtl* c, boo
 //    shared-memory entries) and arrives.
 // Every CTA takes the same decisions from the same counts, so all reach the
 // same barriers; there are no spin waits.
-// A vertex's depth is written when its entry is expanded, not when it is
-// claimed: the caller's id it is stored under is read beside the entry's row,
-// off the level's critical path (a frontier handed over gets its depths from
-// the inspector).
-template <class DT>
+// A vertex's depth is written when it is claimed, or (LATE) when its entry is
+// expanded: in a traversal order of its own, the caller's id it is stored under is then
+// read beside the entry's row, off the level's critical path (a frontier handed
+// over gets its depths from the inspector).
+// LATE: depths are written at the expansion. In caller order that pays only where
+// the depths outgrow L2's share (4096^2 grid 32.7 -> 32.2 ms; 1024^2 5.45 -> 5.50).
+template <class DT, bool LATE>
 __global__ void __launch_bounds__(NT, 1) k_narrow(LevelArgs a) {
   extern __shared__ int4 s_q[];  // [2][NQCAP]
   __shared__ uint32_t s_cnt[2], s_flag[2];
@@ -1122,6 +1124,7 @@ __global__ void __launch_bounds__(NT, 1) k_narrow(LevelArgs a) {
 
     if (!coord) {
       const NarrowOut o{s_q + nxt * NQCAP, &s_cnt[nxt], &s_m[nxt], &s_flag[nxt], spill};
+      [[maybe_unused]] const int ln = L + 1;
       int k = (int)((n_all + nwt - 1) / nwt);
       if (k > 32) k = 32;
       for (int first = gw * k; first < (int)n_all; first += nwt * k) {
@@ -1134,14 +1137,15 @@ __global__ void __launch_bounds__(NT, 1) k_narrow(LevelArgs a) {
           if (r + step <= nc - 1 && (uint32_t)i >= e_end) r += step;
         }
         const uint32_t base = __shfl_sync(FULL, incl, (r + 31) & 31);  // end of CTA r-1 (unused for r = 0)
-        int u = -1, d = 0, out = -1;
+        int u = -1, d = 0;
+        [[maybe_unused]] int out = -1;
         int64_t st = 0;
         if (lane < k && i < (int)n_all) {
           const int4 e = *(cl.map_shared_rank(s_q + cur * NQCAP, r) + (i - (r ? (int)base : 0)));
           u = e.x;
           d = e.y;
           st = (int64_t)(((uint64_t)(uint32_t)e.w << 32) | (uint32_t)e.z);
-          out = out_id(a, u);
+          if constexpr (LATE) out = out_id(a, u);
         }
         int dincl = d;
 #pragma unroll
@@ -1193,7 +1197,8 @@ __global__ void __launch_bounds__(NT, 1) k_narrow(LevelArgs a) {
                 // the next level walks this row: start its first sector towards L2 now
                 // (an empty row may start one past the array: nothing to fetch)
                 if (o1 > o0) asm volatile("prefetch.global.L2 [%0];" ::"l"(a.adj + o0));
-                if (parent) parent[out_id(a, x)] = out_id(a, uj[q]);
+                if constexpr (!LATE) depth[x] = (DT)ln;
+                if (parent) parent[LATE ? out_id(a, x) : x] = LATE ? out_id(a, uj[q]) : uj[q];
               }
             }
           }
@@ -1201,7 +1206,9 @@ __global__ void __launch_bounds__(NT, 1) k_narrow(LevelArgs a) {
           for (int q = 0; q < NROUND; ++q)
             if (r0 + 32 * q < total) narrow_append(a, c, mine[q], v[q], vd[q], vst[q], o);
         }
-        if (out >= 0) depth[out] = (DT)L;
+        if constexpr (LATE) {
+          if (out >= 0) depth[out] = (DT)L;
+        }
       }
       bar1_arrive();  // this warp's appends are complete
       cluster_arrive_relaxed();
@@ -1285,7 +1292,13 @@ __global__ void __launch_bounds__(NT, 1) k_narrow(LevelArgs a) {
 // levels, mostly evicted since, and the copy engine would otherwise read it
 // from DRAM that the next traversal keeps busy (s24, 64 sources: 36.2 against
 // 44.9 ms with every row copied; one prefetch per 128-byte line).
-__global__ void __launch_bounds__(256) k_row_to_l2(const uint8_t* __restrict__ p, int64_t n) {
+// Beside it the traversal's control block is saved for its statistics: read
+// back by a copy of its own, it would wait in the copy engine behind the
+// previous row, and the next traversal with it (16 rows at s24: 6.17 -> 6.00 ms).
+__global__ void __launch_bounds__(256) k_row_to_l2(const uint8_t* __restrict__ p, int64_t n, const BfsCtl* ctl,
+                                                   BfsCtl* save) {
+  if (blockIdx.x == 0 && threadIdx.x < sizeof(BfsCtl) / 4)
+    reinterpret_cast<uint32_t*>(save)[threadIdx.x] = reinterpret_cast<const uint32_t*>(ctl)[threadIdx.x];
   const int64_t step = (int64_t)gridDim.x * blockDim.x * 128;
   for (int64_t i = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) * 128; i < n; i += step)
     asm volatile("prefetch.global.L2::evict_last [%0];" ::"l"(p + i));
@@ -1323,6 +1336,7 @@ struct BfsWorkspace {
   int32_t* depth_b = nullptr;
   uint8_t* depth8[2] = {nullptr, nullptr};  // byte depths (ent_bfs_many_u8)
   cudaStream_t copy_stream = nullptr;
+  BfsCtl* many_ctl = nullptr;    // one per source, on the device and its pinned copy
   BfsCtl* many_ctl_h = nullptr;
   int32_t many_cap = 0;
   std::vector<cudaEvent_t> many_ev;          // [2i], [2i+1] bracket traversal i
@@ -1350,12 +1364,16 @@ void destroy_bfs_workspace(BfsWorkspace* w) {
   dev_free(w->depth_b);
   for (int i = 0; i < 2; ++i) dev_free(w->depth8[i]);
   if (w->copy_stream) cudaStreamDestroy(w->copy_stream);
+  dev_free(w->many_ctl);
   if (w->many_ctl_h) cudaFreeHost(w->many_ctl_h);
   for (cudaEvent_t e : w->many_ev) cudaEventDestroy(e);
   for (cudaEvent_t e : w->many_sync)
     if (e) cudaEventDestroy(e);
   delete w;
 }
+
+// Which k_narrow a graph gets (see there).
+static bool narrow_late(const LevelArgs& a) { return a.perm || a.V > (1 << 22); }
 
 template <class DT>
 static int build_graph(ent_graph* g, BfsWorkspace* w) {
@@ -1417,7 +1435,7 @@ static int build_graph(ent_graph* g, BfsWorkspace* w) {
     prev = n_inspect;
     if (w->narrow_nc > 0) {
       cudaGraphNode_t n_narrow;
-      bp.func = (void*)k_narrow<DT>;
+      bp.func = narrow_late(w->args) ? (void*)k_narrow<DT, true> : (void*)k_narrow<DT, false>;
       bp.gridDim = dim3(w->narrow_nc);
       bp.blockDim = dim3(NT);
       bp.sharedMemBytes = (unsigned)w->smem_narrow;
@@ -1448,19 +1466,20 @@ static cudaError_t launch_narrow(const BfsWorkspace* w, const LevelArgs& la, cud
   at[0].val.clusterDim.z = 1;
   cfg.attrs = at;
   cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, k_narrow<DT>, la);
+  return narrow_late(w->args) ? cudaLaunchKernelEx(&cfg, k_narrow<DT, true>, la)
+                      : cudaLaunchKernelEx(&cfg, k_narrow<DT, false>, la);
 }
 
 // Largest cluster (<= limit CTAs, 0 = no limit) of the small-frontier kernel
 // that can be resident on this GPU; 0 if none.
 static int pick_narrow_cluster(int limit, size_t smem) {
-  if (cudaFuncSetAttribute(k_narrow<int32_t>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
-      cudaFuncSetAttribute(k_narrow<int32_t>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
-      cudaFuncSetAttribute(k_narrow<uint8_t>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
-      cudaFuncSetAttribute(k_narrow<uint8_t>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
-    cudaGetLastError();
-    return 0;
-  }
+  for (const void* f : {(const void*)k_narrow<int32_t, true>, (const void*)k_narrow<int32_t, false>,
+                        (const void*)k_narrow<uint8_t, true>, (const void*)k_narrow<uint8_t, false>})
+    if (cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
+        cudaFuncSetAttribute(f, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
+      cudaGetLastError();
+      return 0;
+    }
   for (int nc = NC_MAX; nc >= 1; nc >>= 1) {
     if (limit > 0 && nc > limit) continue;
     cudaLaunchConfig_t cfg = {};
@@ -1475,7 +1494,7 @@ static int pick_narrow_cluster(int limit, size_t smem) {
     cfg.attrs = at;
     cfg.numAttrs = 1;
     int n = 0;
-    if (cudaOccupancyMaxActiveClusters(&n, k_narrow<int32_t>, &cfg) == cudaSuccess && n >= 1) return nc;
+    if (cudaOccupancyMaxActiveClusters(&n, k_narrow<int32_t, true>, &cfg) == cudaSuccess && n >= 1) return nc;
     cudaGetLastError();
   }
   return 0;
@@ -2104,11 +2123,17 @@ static int bfs_many(ent_graph* g, const int32_t* src, int32_t n_src, void* const
   if (!w->copy_stream) ENT_CUDA(cudaStreamCreateWithFlags(&w->copy_stream, cudaStreamNonBlocking));
   if (w->many_cap < n_src) {
     if (w->many_ctl_h) cudaFreeHost(w->many_ctl_h);
+    dev_free(w->many_ctl);
     w->many_ctl_h = nullptr;
+    w->many_ctl = nullptr;
     w->many_cap = 0;
     if (cudaMallocHost(&w->many_ctl_h, sizeof(BfsCtl) * n_src) != cudaSuccess) {
       w->many_ctl_h = nullptr;
       return fail(ENT_ERR_OOM, "pinned control copies failed");
+    }
+    if (dev_alloc(&w->many_ctl, sizeof(BfsCtl) * n_src) != cudaSuccess) {
+      w->many_ctl = nullptr;
+      return fail(ENT_ERR_OOM, "control copies failed");
     }
     w->many_cap = n_src;
   }
@@ -2143,15 +2168,18 @@ static int bfs_many(ent_graph* g, const int32_t* src, int32_t n_src, void* const
                : run_bfs_typed<int32_t>(g, src[i], (int32_t*)buf[b], nullptr, s, nullptr);
     if (rc != ENT_OK) break;
     ce = cudaEventRecord(ev[2 * (size_t)i + 1], s);
-    if (ce == cudaSuccess)
-      ce = cudaMemcpyAsync(&w->many_ctl_h[i], w->ctl, sizeof(BfsCtl), cudaMemcpyDeviceToHost, s);
-    if (ce == cudaSuccess && depth_out && depth_out[i]) {
+    const bool row = depth_out && depth_out[i];
+    if (ce == cudaSuccess) {  // the row towards L2 (bytes, and only if it is copied), and the control block
+      const int64_t n = row && bytes ? g->V : 0;
+      k_row_to_l2<<<(unsigned)std::max<int64_t>(1, (n + 128 * 256 - 1) / (128 * 256)), 256, 0, s>>>(
+          (const uint8_t*)buf[b], n, w->ctl, w->many_ctl + i);
+      g_kernel_launches += 1;
+      ce = cudaGetLastError();
+    }
+    if (ce == cudaSuccess && row) {
       cudaEvent_t ready = ev[2 * (size_t)i + 1];
       if (bytes) {
-        k_row_to_l2<<<(unsigned)((g->V + 128 * 256 - 1) / (128 * 256)), 256, 0, s>>>((const uint8_t*)buf[b], g->V);
-        g_kernel_launches += 1;
-        ce = cudaGetLastError();
-        if (ce == cudaSuccess) ce = cudaEventRecord(w->many_sync[2], s);
+        ce = cudaEventRecord(w->many_sync[2], s);
         ready = w->many_sync[2];
       }
       if (ce == cudaSuccess) ce = cudaStreamWaitEvent(cs, ready, 0);
@@ -2161,6 +2189,8 @@ static int bfs_many(ent_graph* g, const int32_t* src, int32_t n_src, void* const
     }
     if (ce == cudaSuccess) done = i + 1;
   }
+  if (done > 0 && ce == cudaSuccess)
+    ce = cudaMemcpyAsync(w->many_ctl_h, w->many_ctl, sizeof(BfsCtl) * done, cudaMemcpyDeviceToHost, s);
   const cudaError_t se = cudaStreamSynchronize(s);
   const cudaError_t sc = cudaStreamSynchronize(cs);
   if (rc == ENT_OK && ce == cudaSuccess) ce = se != cudaSuccess ? se : sc;

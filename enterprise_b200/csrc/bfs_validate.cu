@@ -103,11 +103,14 @@ __device__ __forceinline__ int64_t first_below(const int32_t* deg, int64_t n, in
 // entries (whole calls, with the traversal: 1.90 -> 1.00 and 18.3 -> 1.12 ms).
 __global__ void __launch_bounds__(VT) k_val_rows(const int64_t* __restrict__ off, const int32_t* __restrict__ rows,
                                                  const int32_t* __restrict__ deg, int64_t n_active,
-                                                 const uint32_t* __restrict__ dt, unsigned long long* broken) {
+                                                 const uint32_t* __restrict__ dt, int short_rows,
+                                                 unsigned long long* broken) {
   __shared__ int64_t s_bound[2];
   __shared__ unsigned s_mn[VT / 32], s_mx[VT / 32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  if (warp < 2) {
+  if (short_rows) {  // in any order
+    if (threadIdx.x < 2) s_bound[threadIdx.x] = 0;
+  } else if (warp < 2) {
     const int64_t b = first_below(deg, n_active, warp == 0 ? VAL_CTA : VAL_WARP);
     if (lane == 0) s_bound[warp] = b;
   }
@@ -199,8 +202,8 @@ __global__ void __launch_bounds__(VT) k_val_vertex(const int64_t* __restrict__ o
                                                    const int32_t* __restrict__ parent, int32_t* __restrict__ dt,
                                                    unsigned long long* words) {
   for (int64_t v = blockIdx.x * (int64_t)VT + threadIdx.x; v < V; v += (int64_t)gridDim.x * VT) {
-    const int dv = depth[v], i = inv[v], p = parent ? parent[v] : -1;
-    dt[i] = dv;
+    const int dv = depth[v], i = inv ? inv[v] : (int)v, p = parent ? parent[v] : -1;
+    if (inv) dt[i] = dv;
     if (dv < -1 || (dv == 0 && v != src) || (dv > 0 && i >= n_active)) words[3] = 1;
     if (v == src) {
       if (dv != 0) words[4] = 1;
@@ -282,14 +285,15 @@ extern "C" int ent_validate(ent_graph* g, int32_t src, const int32_t* depth_dev,
   };
   cudaError_t e = cudaMemsetAsync(words, 0xFF, 2 * sizeof(unsigned long long), s);
   if (e == cudaSuccess) e = cudaMemsetAsync(words + 2, 0, (NW - 2) * sizeof(unsigned long long), s);
-  const bool fast = g->perm != nullptr;               // else the rows are in caller order, of any lengths
+  const bool fast = g->perm || g->road;               // else the rows are in caller order, of any lengths
   const bool fast_parent = fast && g->rows_sorted;
   if (e == cudaSuccess && fast) {
     k_val_vertex<<<grid, VT, 0, s>>>(g->off, g->adj, g->inv, V, g->n_active, src, depth_dev,
                                      fast_parent ? parent_dev : nullptr, dt, words);
     e = launched();
     if (e == cudaSuccess) {
-      k_val_rows<<<grid, VT, 0, s>>>(g->toff, g->trav, g->deg, g->n_active, (const uint32_t*)dt, words + 3);
+      k_val_rows<<<grid, VT, 0, s>>>(g->toff, g->trav, g->deg, g->n_active,
+                                       (const uint32_t*)(g->perm ? dt : depth_dev), g->road, words + 3);
       e = launched();
     }
     if (e == cudaSuccess) e = read_words();

@@ -24,7 +24,8 @@ void destroy_deep_lanes(DeepLanes* l);
 // hubs, which most probes hit, share a few cache lines of every per-vertex
 // array. Caller ids appear only where sources come in and results go out.
 //   perm int32[V]     caller id of each traversal id (null: caller order, when
-//                     E >= 2^31 or E == 0; toff and trav are then off and adj)
+//                     E >= 2^31 or E == 0 and on road-like graphs; toff and trav
+//                     are then off and adj)
 //   inv  int32[V]     traversal id of each caller id
 //   toff int64[V+1]   row offsets
 //   trav int32[E]     the rows, ascending: the highest-degree neighbours first.
@@ -51,7 +52,8 @@ struct ent_graph {
   uint32_t* active = nullptr;
   int4* lead = nullptr;
   int64_t n_active = 0;  // vertices with a row are traversal ids [0, n_active); V in caller order
-  bool rows_sorted = false;  // every adj row is ascending (known with an order of its own)
+  bool road = false;         // low mean degree and no hub: keeps the caller's order
+  bool rows_sorted = false;  // every adj row is ascending (known with an order of its own, and for road-like graphs)
   cudaStream_t stream = nullptr;
   ent_bfs_opts opts;
   std::mutex mu;
