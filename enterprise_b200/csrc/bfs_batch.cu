@@ -994,7 +994,7 @@ __global__ void __launch_bounds__(BB) k_b_commit(BatchArgs a) {
 // ----------------------------------------------------------- flush --------
 // Converts log slots [first, last] (levels base+first .. base+last) into the
 // source-major depth rows and recycles the slots in the same pass. A CTA takes
-// a span of 1024 vertices (caller ids) and walks the W word columns in groups of
+// units of consecutive vertices (caller ids) and walks the W word columns in groups of
 // CG = min(W, 4), VS = 1024 / CG vertices per pass.
 // Decode (thread per vertex): the slots of a vertex are disjoint bit sets, so
 // the vertex's CG words of every slot fold into a found mask and four bit
@@ -1141,8 +1141,7 @@ __device__ __forceinline__ void settle_pattern(const FlushState& fs, int cg) {
 // reached vertices and their degrees; without, the caller has counted the
 // tile's vertices under the shared mask.
 template <int CG, bool BYTES, bool STATS>
-__device__ __forceinline__ void write_rows(const BatchArgs& a, const FlushState& fs, int64_t v0, int sub, int nsub,
-                                           int cg) {
+__device__ __forceinline__ void write_rows(const BatchArgs& a, const FlushState& fs, int64_t v0, int nsub, int cg) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   for (int r0 = warp * 4; r0 < 64 * CG; r0 += BB / 32 * 4) {
     const int s0 = cg * 64 + r0;
@@ -1156,7 +1155,7 @@ __device__ __forceinline__ void write_rows(const BatchArgs& a, const FlushState&
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       rv[j] = s0 + j < fs.nsrc;
-      ofs[j] = rv[j] ? (size_t)(fs.row_map ? fs.row_map[s0 + j] : s0 + j) * a.V + v0 + sub : 0;
+      ofs[j] = rv[j] ? (size_t)(fs.row_map ? fs.row_map[s0 + j] : s0 + j) * a.V + v0 : 0;
       rb[j] = fs.base - (fs.joined && rv[j] ? a.join[s0 + j] : 0);
       if (BYTES && rv[j] && rb[j] > 239) wide = true;
       plain &= rb[j] == 0;
@@ -1170,7 +1169,7 @@ __device__ __forceinline__ void write_rows(const BatchArgs& a, const FlushState&
         for (int t = 0; t < 4; ++t) wv[t] = fs.tile[tile_word<CG>(vi + t, c4)];
         if constexpr (BYTES) byte_transpose4(wv[0], wv[1], wv[2], wv[3], x[0], x[1], x[2], x[3]);
         int4 dg = make_int4(0, 0, 0, 0);
-        if constexpr (STATS) dg = *reinterpret_cast<const int4*>(fs.s_deg + sub + vi);
+        if constexpr (STATS) dg = *reinterpret_cast<const int4*>(fs.s_deg + vi);
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
           if (!rv[j]) continue;
@@ -1205,7 +1204,7 @@ __device__ __forceinline__ void write_rows(const BatchArgs& a, const FlushState&
       bool deep = false;  // a depth above 254 met in byte rows
       for (int vi = lane; vi < nsub; vi += 32) {
         const uint32_t wv = fs.tile[tile_word<CG>(vi, c4)];
-        const int dg = STATS ? fs.s_deg[sub + vi] : 0;
+        const int dg = STATS ? fs.s_deg[vi] : 0;
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
           if (!rv[j]) continue;
@@ -1246,34 +1245,44 @@ __device__ __forceinline__ void write_rows(const BatchArgs& a, const FlushState&
   }
 }
 
+// All of a CTA's units: VS consecutive vertices (caller ids) each, in turn over
+// the CTAs, so that CTAs running side by side write neighbouring segments of
+// every row at about the same time (units of 1024
+// vertices, a column group at a time: s22 x 256 flush 1.30 ms, 1.18 so, batch
+// 3.69 -> 3.56; ER 2^20 x 256 batch 1.57 -> 1.44; byte rows of s20 x 1000 equal).
 template <int CG, bool BYTES>
-__device__ void flush_span(const BatchArgs& a, const FlushState& fs, int64_t v0, int nv) {
-  constexpr int VS = 1024 / CG;  // vertices per pass
+__device__ void flush_units(const BatchArgs& a, const FlushState& fs, int* s_deg) {
+  constexpr int VS = 1024 / CG;  // vertices per unit
   constexpr int Q = VS / BB;     // ... and per thread
   const int lane = threadIdx.x & 31;
   // the slots decoded: [first, last]
   const uint32_t decoded = ((2u << fs.last) - 1u) & ~((1u << fs.first) - 1u);
-  // The thread's vertices of this pass (traversal ids) and their slot marks.
-  // Both reads for the next pass are issued during this one: the ids before
+  // The thread's vertices of this unit (traversal ids) and their slot marks.
+  // Both reads for the next unit are issued during this one: the ids before
   // the decode, the marks (gathered at those ids) before the rows are written.
   int iv[Q], next_iv[Q];
   uint32_t mk[Q];
-  const auto load_ids = [&](int sub, int (&id)[Q]) {
+  const int64_t units = (a.V + VS - 1) / VS;
+  const auto load_ids = [&](int64_t unit, int (&id)[Q]) {
 #pragma unroll
     for (int q = 0; q < Q; ++q) {
-      const int vi = sub + (int)threadIdx.x + q * BB;
-      id[q] = vi < nv ? (a.inv ? __ldg(a.inv + v0 + vi) : (int)(v0 + vi)) : -1;
+      const int64_t v = unit * VS + threadIdx.x + q * BB;
+      id[q] = v < a.V ? (a.inv ? __ldg(a.inv + v) : (int)v) : -1;
     }
   };
   const auto load_marks = [&](const int (&id)[Q]) {
 #pragma unroll
     for (int q = 0; q < Q; ++q) mk[q] = id[q] >= 0 ? a.smask[id[q]] : 0u;
   };
-  load_ids(0, iv);
+  load_ids(blockIdx.x, iv);
   load_marks(iv);
-  for (int sub = 0; sub < nv; sub += VS) {
-    const int nsub = min(VS, nv - sub);
-    load_ids(sub + VS, next_iv);
+  for (int64_t unit = blockIdx.x; unit < units; unit += gridDim.x) {
+    const int64_t v0 = unit * VS;
+    const int nsub = (int)min((int64_t)VS, a.V - v0);
+    load_ids(unit + gridDim.x, next_iv);
+    __syncthreads();  // the previous unit's rows have been written
+    for (int i = threadIdx.x; i < VS; i += BB)
+      s_deg[i] = i < nsub ? (int)(a.coff[v0 + i + 1] - a.coff[v0 + i]) : 0;
     for (int cg = 0; cg < a.W; cg += CG) {
       if (cg * 64 >= fs.nsrc) break;  // words of no source: never set, so already zero
       __syncthreads();  // the previous tile has been written out
@@ -1341,7 +1350,7 @@ __device__ void flush_span(const BatchArgs& a, const FlushState& fs, int64_t v0,
           for (int cc = 0; cc < CG; ++cc) any |= f[cc];
           if (eq && any) {
             pn += 1;
-            pe += (unsigned)fs.s_deg[sub + vi];
+            pe += (unsigned)s_deg[vi];  // this thread's own entry
           } else if (any) {
             mis = true;
             if (atomicExch(fs.s_claim, 1) == 0)
@@ -1379,9 +1388,9 @@ __device__ void flush_span(const BatchArgs& a, const FlushState& fs, int64_t v0,
           atomicAdd(fs.s_pn + cg / CG, n);
           atomicAdd(fs.s_pe + cg / CG, ((unsigned long long)ehi << 16) + elo);
         }
-        write_rows<CG, BYTES, false>(a, fs, v0, sub, nsub, cg);
+        write_rows<CG, BYTES, false>(a, fs, v0, nsub, cg);
       } else {
-        write_rows<CG, BYTES, true>(a, fs, v0, sub, nsub, cg);
+        write_rows<CG, BYTES, true>(a, fs, v0, nsub, cg);
         __syncthreads();
         if (odd >= BB / 4) {  // most vertices differ: take the proposed mask from here on
           settle_pattern<CG>(fs, cg);
@@ -1399,7 +1408,7 @@ __device__ void flush_span(const BatchArgs& a, const FlushState& fs, int64_t v0,
 // Runs after a level when the log window is full (flush_now) or sources
 // joined (clear_done), and once at the end (final_flush). Joined sources void
 // the completion bits, which are cleared. A flush writes the window's depth
-// rows and per-source statistics and recycles the slots (flush_span); a window
+// rows and per-source statistics and recycles the slots (flush_units); a window
 // flush then moves the window by K-1 levels.
 __global__ void __launch_bounds__(BB, 3) k_b_flush(BatchArgs a, int final_flush) {
   extern __shared__ __align__(16) unsigned char s_flush[];
@@ -1445,23 +1454,15 @@ __global__ void __launch_bounds__(BB, 3) k_b_flush(BatchArgs a, int final_flush)
     if (threadIdx.x == 0) *fs.s_claim = 0;
     int* s_deg = reinterpret_cast<int*>(s_flush + TILE_BYTES);
     for (int i = threadIdx.x; i < NSRC; i += BB) { fs.s_cnt[i] = 0; fs.s_edg[i] = 0; }
-    const int64_t units = (a.V + 1023) / 1024;
-    for (int64_t u = blockIdx.x; u < units; u += gridDim.x) {
-      const int64_t v0 = u * 1024;
-      const int nv = (int)min((int64_t)1024, a.V - v0);
-      __syncthreads();
-      for (int i = threadIdx.x; i < 1024; i += BB)
-        s_deg[i] = i < nv ? (int)(a.coff[v0 + i + 1] - a.coff[v0 + i]) : 0;
-      __syncthreads();
-      if (bytes) {
-        if (a.W == 1) flush_span<1, true>(a, fs, v0, nv);
-        else if (a.W == 2) flush_span<2, true>(a, fs, v0, nv);
-        else flush_span<4, true>(a, fs, v0, nv);
-      } else {
-        if (a.W == 1) flush_span<1, false>(a, fs, v0, nv);
-        else if (a.W == 2) flush_span<2, false>(a, fs, v0, nv);
-        else flush_span<4, false>(a, fs, v0, nv);
-      }
+    __syncthreads();
+    if (bytes) {
+      if (a.W == 1) flush_units<1, true>(a, fs, s_deg);
+      else if (a.W == 2) flush_units<2, true>(a, fs, s_deg);
+      else flush_units<4, true>(a, fs, s_deg);
+    } else {
+      if (a.W == 1) flush_units<1, false>(a, fs, s_deg);
+      else if (a.W == 2) flush_units<2, false>(a, fs, s_deg);
+      else flush_units<4, false>(a, fs, s_deg);
     }
     __syncthreads();
     for (int cg = 0; cg < a.W; cg += a.W >= 4 ? 4 : a.W) {
@@ -1763,7 +1764,7 @@ int create_batch_workspace(ent_graph* g, int n_src, BatchWorkspace** out) {
   // launch can run side by side
   const int64_t want = std::max<int64_t>(1, (V + BB * 8 - 1) / (BB * 8));
   w->grid = (int)std::min<int64_t>((int64_t)g->num_sms * occ, want);
-  w->grid_flush = (int)std::min<int64_t>((int64_t)g->num_sms * 3, std::max<int64_t>(1, (V + 1023) / 1024));
+  w->grid_flush = (int)std::min<int64_t>((int64_t)g->num_sms * 3, (V * std::min(W, 4) + 1023) / 1024);
   // tile and degrees; per source: reached vertices, their degree sum
   // per word: its part of the shared mask, its counts; and the proposed mask
   w->smem_flush = FLUSH_TILE_BYTES + (size_t)W * 64 * (4 + 8) + (size_t)W * (8 + 8 + 4) + 4 * 8 + 16;
