@@ -175,11 +175,11 @@ __device__ __forceinline__ bool row_has(const int64_t* off, const int32_t* rows,
 }
 
 __device__ __forceinline__ int parent_code(const int64_t* off, const int32_t* rows_sorted, int64_t V, int32_t v,
-                                           const int32_t* depth, int dv, int p) {
+                                           const int32_t* depth, int dv, int p, bool symmetric = false) {
   if (dv == -1) return p != -1 ? -2 : 0;
   if (p < 0 || p >= V) return -3;
   if (depth[p] != dv - 1) return -4;
-  return row_has(off, rows_sorted, p, v) ? 0 : -5;
+  return (symmetric ? row_has(off, rows_sorted, v, p) : row_has(off, rows_sorted, p, v)) ? 0 : -5;
 }
 
 __global__ void __launch_bounds__(VT) k_val_parent(const int64_t* __restrict__ off,
@@ -195,12 +195,15 @@ __global__ void __launch_bounds__(VT) k_val_parent(const int64_t* __restrict__ o
 
 // The rules that need no row, over caller ids: depths of their own, the rules
 // of the source, and (with parents and sorted rows) the parent certificate;
-// and the depths by traversal id, for k_val_rows.
+// and the depths by traversal id, for k_val_rows. Where every edge is known to
+// be there both ways, the vertex looks for its parent in its own row, which
+// lies beside its neighbour thread's, instead of for itself in the parent's
+// row, a random one: a traversal of ER 2^22 x 16 with its certificates 1018 us, 890 so.
 __global__ void __launch_bounds__(VT) k_val_vertex(const int64_t* __restrict__ off, const int32_t* __restrict__ adj,
                                                    const int32_t* __restrict__ inv, int64_t V, int64_t n_active,
                                                    int32_t src, const int32_t* __restrict__ depth,
-                                                   const int32_t* __restrict__ parent, int32_t* __restrict__ dt,
-                                                   unsigned long long* words) {
+                                                   const int32_t* __restrict__ parent, bool symmetric,
+                                                   int32_t* __restrict__ dt, unsigned long long* words) {
   for (int64_t v = blockIdx.x * (int64_t)VT + threadIdx.x; v < V; v += (int64_t)gridDim.x * VT) {
     const int dv = depth[v], i = inv ? inv[v] : (int)v, p = parent ? parent[v] : -1;
     if (inv) dt[i] = dv;
@@ -209,7 +212,7 @@ __global__ void __launch_bounds__(VT) k_val_vertex(const int64_t* __restrict__ o
       if (dv != 0) words[4] = 1;
       if (parent && (p != src || dv != 0)) words[5] = 1;
     } else if (parent) {
-      const int code = parent_code(off, adj, V, (int32_t)v, depth, dv, p);
+      const int code = parent_code(off, adj, V, (int32_t)v, depth, dv, p, symmetric);
       if (code) report(words + 1, v, code);
     }
   }
@@ -289,7 +292,7 @@ extern "C" int ent_validate(ent_graph* g, int32_t src, const int32_t* depth_dev,
   const bool fast_parent = fast && g->rows_sorted;
   if (e == cudaSuccess && fast) {
     k_val_vertex<<<grid, VT, 0, s>>>(g->off, g->adj, g->inv, V, g->n_active, src, depth_dev,
-                                     fast_parent ? parent_dev : nullptr, dt, words);
+                                     fast_parent ? parent_dev : nullptr, g->symmetric, dt, words);
     e = launched();
     if (e == cudaSuccess) {
       k_val_rows<<<grid, VT, 0, s>>>(g->toff, g->trav, g->deg, g->n_active,

@@ -53,6 +53,7 @@ struct ent_graph {
   int4* lead = nullptr;
   int64_t n_active = 0;  // vertices with a row are traversal ids [0, n_active); V in caller order
   bool road = false;         // low mean degree and no hub: keeps the caller's order
+  bool symmetric = false;  // every edge is there both ways (rows built here from undirected edges)
   bool rows_sorted = false;  // every adj row is ascending (known with an order of its own, and for road-like graphs)
   cudaStream_t stream = nullptr;
   ent_bfs_opts opts;

@@ -435,6 +435,7 @@ static int build_on_device(Draw draw, uint64_t n_draws, int64_t V, int gpu, ent_
     return rc;
   }
   k_offsets_from_keys<<<blocks, 256, 0, s>>>(uniq, n_uniq, kc, g->off, V);
+  g->symmetric = true;  // k_gen_keys writes both directions of a draw
   k_adj_from_keys<<<blocks, 256, 0, s>>>(uniq, n_uniq, (1ull << kc.b) - 1, g->adj);
   g_kernel_launches += 2;
   GEN_CUDA(cudaGetLastError());

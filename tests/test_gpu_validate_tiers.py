@@ -31,3 +31,24 @@ def test_certificates_at_row_tiers(eb, orc, degree):
             dc, pc = g.validate(s, depth, bad)
             assert dc == (0, -1)
             assert pc == orc.check_parents(csr.beg_pos, csr.csr, s, depth, bad), (v, value)
+
+
+@pytest.mark.parametrize("build", ["rmat", "er", "edges"])
+def test_parent_certificates_of_graphs_built_here(eb, orc, build):
+    """Rows with every edge both ways: a parent of the right depth that is no
+    neighbour is found at the vertex, as from the parent's row."""
+    rng = np.random.RandomState(3)
+    g = {"rmat": lambda: eb.Graph.rmat(12, 8, seed=9), "er": lambda: eb.Graph.er(5003, 9.0, seed=9),
+         "edges": lambda: eb.Graph.from_edges(rng.randint(0, 5003, 20000), rng.randint(0, 5003, 20000), 5003)}[build]()
+    with g:
+        csr = g.download()
+        s = int(np.argmax(np.diff(csr.beg_pos)))
+        depth, parent, _ = g.bfs(s, parents=True)
+        assert g.validate(s, depth, parent) == ((0, -1), (0, -1))
+        for v in np.flatnonzero(depth >= 2)[:: max(1, (depth >= 2).sum() // 12)]:
+            row = csr.csr[csr.beg_pos[v]:csr.beg_pos[v + 1]]
+            level = np.flatnonzero(depth == depth[v] - 1)
+            for p in [level[-1], level[0], row[0], row[-1], np.setdiff1d(level, row)[0], int(v)]:
+                bad = parent.copy()
+                bad[v] = p
+                assert g.validate(s, depth, bad)[1] == orc.check_parents(csr.beg_pos, csr.csr, s, depth, bad), (v, p)
