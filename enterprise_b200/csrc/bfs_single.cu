@@ -1328,9 +1328,8 @@ struct BfsWorkspace {
   int grid_res = 0;
   bool split = false;  // bottom-up levels as kernels of their own between its head and tail
   // traversals of one workspace run one after another, whatever streams they
-  // are launched on: the end of the latest one, and its stream
+  // are launched on: the end of the latest one
   cudaEvent_t ev_order = nullptr;
-  cudaStream_t last_stream = nullptr;
   // ent_bfs_many: a second depth buffer, a copy stream and pinned per-source
   // copies of the control block (created on first use)
   int32_t* depth_b = nullptr;
@@ -1736,7 +1735,7 @@ static int run_bfs_typed(ent_graph* g, int32_t src, DT* depth, int32_t* parent, 
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusActive;
   if (cudaStreamIsCapturing(s, &cap) != cudaSuccess) cudaGetLastError();
   const bool capturing = cap != cudaStreamCaptureStatusNone;  // the launches below refuse it
-  if (!capturing && w->last_stream && w->last_stream != s) ENT_CUDA(cudaStreamWaitEvent(s, w->ev_order, 0));
+  if (!capturing) ENT_CUDA(cudaStreamWaitEvent(s, w->ev_order, 0));
   if (stats) ENT_CUDA(cudaEventRecord(w->ev0, s));
   if (g->opts.loop == ENT_LOOP_GRAPH) {
     int rc = ENT_ERR_UNSUPPORTED;
@@ -1765,10 +1764,7 @@ static int run_bfs_typed(ent_graph* g, int32_t src, DT* depth, int32_t* parent, 
       if (it > w->V + 2) return fail(ENT_ERR_INTERNAL, "level loop did not terminate");
     }
   }
-  if (!capturing) {
-    ENT_CUDA(cudaEventRecord(w->ev_order, s));
-    w->last_stream = s;
-  }
+  if (!capturing) ENT_CUDA(cudaEventRecord(w->ev_order, s));
   if (stats) {
     ENT_CUDA(cudaEventRecord(w->ev1, s));
     ENT_CUDA(cudaMemcpyAsync(w->ctl_h, w->ctl, sizeof(BfsCtl), cudaMemcpyDeviceToHost, s));

@@ -211,9 +211,9 @@ int ent_graph_from_edges(const int64_t* src, const int64_t* dst, int64_t n_edges
 int64_t ent_graph_vert_count(const ent_graph* g);
 int64_t ent_graph_edge_count(const ent_graph* g);
 int32_t ent_graph_device(const ent_graph* g);  /* the graph's GPU */
-/* Device bytes held by the graph's resident arrays (offsets, the two column
- * arrays, degrees, the active bitmap and the lead entries; traversal
- * workspaces come on top). The reference prints its allocation total as
+/* Device bytes held by the graph's resident arrays (offsets and columns in the
+ * caller's and in traversal order, the two id maps, degrees, the active bitmap
+ * and the lead entries; traversal workspaces come on top). The reference prints its allocation total as
  * "GPU alloc space: N bytes" (allocator.cuh:149). */
 int64_t ent_graph_device_bytes(const ent_graph* g);
 /* Device buffers for callers without a CUDA runtime of their own (a
