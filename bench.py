@@ -349,8 +349,7 @@ def run_ours(args, rank, world, dist):
         "gteps_reference_convention": {
             "value": round(amean_ref, 3) if amean_ref is not None else None,
             "rule": "arithmetic mean over sources with more than 2 levels",
-            "time": "includes the on-device depth/status reset (the reference times without it); the reset "
-                    "(k_reset) is about 2% of kernel time per the committed s24 launch list"},
+            "time": "includes the on-device depth/status reset (the reference times without it)"},
         "gteps_arithmetic_mean": round(amean, 3),
         "gteps_graph500": round(value / 2, 3),
         "ms_per_bfs_median": round(float(np.median(mean_per_src)), 4),
@@ -365,7 +364,7 @@ def run_ours(args, rank, world, dist):
             "traffic_basis": traffic_basis,
             "physical_gbs": round(physical, 1) if physical else None,
             "physical_frac": round(physical / peak, 4) if physical else None,
-            "unit_of_work": "one BFS (one CUDA-graph launch: reset + [expand, inspect] x levels); "
+            "unit_of_work": "one BFS (resident head, four bottom-up launches, resident tail; reset in the head); "
                             "algorithmic bytes 4*m_c + 8*n_c + 4*V; physical = ncu DRAM bytes per traversal "
                             "over the same mean traversal time",
         },
@@ -531,7 +530,7 @@ def run_batched(args, rank=0, no_multi=False):
         out["batch_256_vs_sequential_256"] = round(out["sequential_256"]["ms"] / out["batch_256"]["ms"], 3)
         # roofline of the batch from ncu-measured DRAM bytes (algorithmic sums would count the
         # shared CSR reads once per source), scaled from the profiled graph by directed entries
-        prof = "bfs_batch_rmat_s21_256_graph.md"
+        prof = "bfs_batch_rmat_s21_256_ordered.md"
         tb, e_prof = profiled_traffic(prof, "dram_bytes_per_batch"), profiled_traffic(prof, "directed_entries")
         if tb and e_prof:
             traffic = tb * g.edge_count / e_prof
