@@ -6,7 +6,7 @@
 // dev_alloc takes memory from a pool of the library's own that keeps up to
 // POOL_KEEP bytes of what was given back for the next allocation. Whatever is
 // above goes back to the device at once, and all of it when an allocation of
-// this library fails.
+// this library fails. Blocks of POOL_MAX and more bypass it.
 //
 // A copy between the device and pageable host memory runs through the driver's
 // own staging on one host thread (about 10 GB/s, first touch of fresh pages
@@ -28,6 +28,11 @@ constexpr uint64_t POOL_KEEP = 512ull << 20;  // per device
 constexpr size_t CHUNK = 4 << 20;             // bytes per staging chunk
 constexpr size_t STAGED_MIN = 1 << 20;        // shorter copies go to the driver
 constexpr int COPY_THREADS = 8;
+// Larger blocks come from the device and go back to it: the pool would keep none
+// of them, and maps and unmaps them far more slowly (making R-MAT s22 58 ms at
+// best and up to 750, 29 so; s24 246 and up to seconds, 116 so; from 32 MB on
+// s20 10 -> 25).
+constexpr size_t POOL_MAX = 256ull << 20;
 
 struct DevicePool {
   cudaMemPool_t pool = nullptr;
@@ -36,6 +41,7 @@ struct DevicePool {
 };
 std::mutex g_mu;
 std::vector<DevicePool> g_pools;      // by device
+std::vector<void*> g_large;           // blocks that did
 std::vector<char*> g_idle;            // page-locked pairs of chunks not in use
 int g_pairs = 0;                      // ... and all of them
 constexpr int MAX_PAIRS = 2;          // 16 MB; further copies at the same time go to the driver
@@ -137,6 +143,14 @@ bool pageable(const void* host) {
 cudaError_t dev_alloc(void** out, size_t bytes) {
   *out = nullptr;
   bytes = std::max<size_t>(bytes, 1);
+  if (bytes >= POOL_MAX) {
+    const cudaError_t e = dev_malloc(out, bytes);
+    if (e == cudaSuccess) {
+      std::lock_guard<std::mutex> lk(g_mu);
+      g_large.push_back(*out);
+    }
+    return e;
+  }
   const DevicePool p = device_pool();
   if (!p.pool) return cudaMalloc(out, bytes);
   cudaError_t e = cudaMallocFromPoolAsync(out, bytes, p.pool, p.stream);
@@ -162,6 +176,16 @@ cudaError_t dev_malloc(void** out, size_t bytes) {
 
 void dev_free(void* ptr) {
   if (!ptr) return;
+  bool large = false;
+  {
+    std::lock_guard<std::mutex> lk(g_mu);
+    const auto it = std::find(g_large.begin(), g_large.end(), ptr);
+    if ((large = it != g_large.end())) g_large.erase(it);
+  }
+  if (large) {
+    cudaFree(ptr);
+    return;
+  }
   const DevicePool p = device_pool();
   if (p.pool) cudaFreeAsync(ptr, p.stream);
   else cudaFree(ptr);
