@@ -2359,7 +2359,9 @@ int ent_multi_create(ent_graph* const* graphs, int32_t n_graphs, const int32_t* 
       }
     }
     e = dev_alloc(&mu.seeds, sizeof(int32_t) * h.size());
-    if (e == cudaSuccess) e = cudaMemcpy(mu.seeds, h.data(), sizeof(int32_t) * h.size(), cudaMemcpyHostToDevice);
+    // on the plan's stream, ahead of the kernels that read it: a plain copy of a pageable list may
+    // return before it has landed, and nothing orders the legacy stream before this one
+    if (e == cudaSuccess) e = to_device(mu.seeds, h.data(), sizeof(int32_t) * h.size(), m->stream);
     if (e == cudaSuccess) e = dev_alloc(&mu.depth, sizeof(int32_t) * (size_t)mu.slots * mu.u->V);
     if (e != cudaSuccess) { multi_free(m); return fail(ENT_ERR_OOM, "multi seed list or output allocation failed"); }
     mu.w->args.src = mu.seeds;
