@@ -1583,6 +1583,9 @@ struct BatchWorkspace {
   cudaGraphExec_t exec = nullptr;
   cudaGraph_t graph = nullptr;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
+  // runs of one workspace follow one another, whatever streams they are
+  // launched on: the end of the latest one
+  cudaEvent_t ev_order = nullptr;
   std::vector<unsigned long long> h_edges, h_verts;
   std::vector<int32_t> h_maxd;
   size_t x_bytes = 0, small_bytes = 0, stats_bytes = 0;
@@ -1601,6 +1604,7 @@ void destroy_batch_workspace(BatchWorkspace* w) {
   host_slot_free(w->ctl_h);
   if (w->ev0) cudaEventDestroy(w->ev0);
   if (w->ev1) cudaEventDestroy(w->ev1);
+  if (w->ev_order) cudaEventDestroy(w->ev_order);
   delete w;
 }
 
@@ -1740,6 +1744,7 @@ int create_batch_workspace(ent_graph* g, int n_src, BatchWorkspace** out) {
   if (e == cudaSuccess && !(w->ctl_h = (BatchCtl*)host_slot(sizeof(BatchCtl)))) e = cudaErrorMemoryAllocation;
   if (e == cudaSuccess) e = cudaEventCreate(&w->ev0);
   if (e == cudaSuccess) e = cudaEventCreate(&w->ev1);
+  if (e == cudaSuccess) e = cudaEventCreateWithFlags(&w->ev_order, cudaEventDisableTiming);
   if (e != cudaSuccess) { destroy_batch_workspace(w); return fail(ENT_ERR_OOM, "batch workspace setup failed"); }
   char* p = (char*)w->slab;
   BatchArgs& a = w->args;
@@ -2029,11 +2034,14 @@ int run_bfs_batch(ent_graph* g, const int32_t* src, int32_t n_src, int32_t* dept
   if (rc != ENT_OK) return rc;
   BatchWorkspace* w = g->bws;
   cudaStream_t s = stream ? stream : g->stream;
+  const bool captured = capturing(s);  // the launch below refuses it
+  if (!captured) ENT_CUDA(cudaStreamWaitEvent(s, w->ev_order, 0));
   rc = stage_request(g, w, src, n_src, depth_dev, s, nullptr, bytes);
   if (rc != ENT_OK) return rc;
   ENT_CUDA(cudaEventRecord(w->ev0, s));
   ENT_CUDA(cudaGraphLaunch(w->exec, s));
   ENT_CUDA(cudaEventRecord(w->ev1, s));
+  if (!captured) ENT_CUDA(cudaEventRecord(w->ev_order, s));
   if (stats) return read_batch_stats(g, w, n_src, s, stats);
   g_kernel_launches += 2;
   return ENT_OK;
@@ -2118,6 +2126,7 @@ int ent_bfs_batch_trace(ent_graph* g, const int32_t* src, int32_t n_src, int32_t
   int rc = ensure_batch(g, n_src);
   if (rc != ENT_OK) return rc;
   BatchWorkspace* w = g->bws;
+  ENT_CUDA(cudaStreamWaitEvent(g->stream, w->ev_order, 0));
   rc = stage_request(g, w, src, n_src, depth_dev, g->stream, nullptr, false);
   if (rc != ENT_OK) return rc;
   return host_batch_loop(w, g->E, w->args, g->stream, out, max_levels, n_levels, nullptr);

@@ -1732,14 +1732,12 @@ static int run_bfs_typed(ent_graph* g, int32_t src, DT* depth, int32_t* parent, 
   }
   BfsWorkspace* w = g->ws;
   cudaStream_t s = stream ? stream : g->stream;
-  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusActive;
-  if (cudaStreamIsCapturing(s, &cap) != cudaSuccess) cudaGetLastError();
-  const bool capturing = cap != cudaStreamCaptureStatusNone;  // the launches below refuse it
-  if (!capturing) ENT_CUDA(cudaStreamWaitEvent(s, w->ev_order, 0));
+  const bool captured = capturing(s);  // the launches below refuse it
+  if (!captured) ENT_CUDA(cudaStreamWaitEvent(s, w->ev_order, 0));
   if (stats) ENT_CUDA(cudaEventRecord(w->ev0, s));
   if (g->opts.loop == ENT_LOOP_GRAPH) {
     int rc = ENT_ERR_UNSUPPORTED;
-    if (w->res.rc && !parent && !capturing) rc = launch_resident(w, src, depth, s);
+    if (w->res.rc && !parent && !captured) rc = launch_resident(w, src, depth, s);
     if (rc == ENT_ERR_UNSUPPORTED) rc = launch_graph(g, w, src, depth, parent, s);
     if (rc != ENT_OK) return rc;
   } else {
@@ -1764,7 +1762,7 @@ static int run_bfs_typed(ent_graph* g, int32_t src, DT* depth, int32_t* parent, 
       if (it > w->V + 2) return fail(ENT_ERR_INTERNAL, "level loop did not terminate");
     }
   }
-  if (!capturing) ENT_CUDA(cudaEventRecord(w->ev_order, s));
+  if (!captured) ENT_CUDA(cudaEventRecord(w->ev_order, s));
   if (stats) {
     ENT_CUDA(cudaEventRecord(w->ev1, s));
     ENT_CUDA(cudaMemcpyAsync(w->ctl_h, w->ctl, sizeof(BfsCtl), cudaMemcpyDeviceToHost, s));

@@ -83,6 +83,14 @@ struct DeviceGuard {
   }
 };
 
+// Whether stream s is being captured into a graph (events of other streams
+// then have no place in it).
+inline bool capturing(cudaStream_t s) {
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusActive;
+  if (cudaStreamIsCapturing(s, &cap) != cudaSuccess) cudaGetLastError();
+  return cap != cudaStreamCaptureStatusNone;
+}
+
 #define ENT_CUDA(call)                                                                      \
   do {                                                                                      \
     cudaError_t _e = (call);                                                                \

@@ -26,3 +26,47 @@ def test_plan_seeds_land_before_they_are_read(eb, orc):
                 plan.run()
                 for k in range(2):
                     np.testing.assert_array_equal(plan.depths(k), np.stack(exp[turn][k]))
+
+
+@pytest.mark.parametrize("bytes_", [False, True])
+def test_batches_on_streams_in_turn(eb, orc, bytes_):
+    """Asynchronous batches of one handle on two streams, of other sources and
+    another number of them each, keep their order: each writes its own rows."""
+    import torch
+    csr = eb.Csr.rmat(14, 16, seed=0xB3)
+    lists = [eb.pick_sources(csr.beg_pos, 50 + i, 60 + 3 * i) for i in range(8)]
+    with eb.Graph.from_csr(csr) as g:
+        call = g.bfs_batch_device_u8 if bytes_ else g.bfs_batch_device
+        rows = [torch.full((len(ss), csr.vert_count), 7, dtype=torch.uint8 if bytes_ else torch.int32, device="cuda")
+                for ss in lists]
+        streams = [torch.cuda.Stream(), torch.cuda.Stream()]
+        call(lists[-1], rows[-1].data_ptr())  # the workspace is as wide as the widest batch from here on
+        torch.cuda.synchronize()
+        for i, ss in enumerate(lists):
+            call(ss, rows[i].data_ptr(), stream=streams[i % 2].cuda_stream, stats=False)
+        torch.cuda.synchronize()
+        for ss, r in zip(lists, rows):
+            got = r.cpu().numpy()
+            for s, d in zip(ss, got):
+                exp = orc.bfs(csr.beg_pos, csr.csr, int(s))[0]
+                np.testing.assert_array_equal(d, np.where(exp < 0, 255, exp).astype(np.uint8) if bytes_ else exp)
+
+
+def test_batch_trace_after_an_asynchronous_batch(eb, orc):
+    import torch
+    csr = eb.Csr.rmat(16, 16, seed=0xB4)
+    ss, st = eb.pick_sources(csr.beg_pos, 60, 128), eb.pick_sources(csr.beg_pos, 61, 70)
+    with eb.Graph.from_csr(csr) as g:
+        rows = torch.full((len(ss), csr.vert_count), 7, dtype=torch.int32, device="cuda")
+        traced = torch.full((len(st), csr.vert_count), 7, dtype=torch.int32, device="cuda")
+        stream = torch.cuda.Stream()
+        g.bfs_batch_device(ss, rows.data_ptr())
+        torch.cuda.synchronize()
+        for _ in range(4):
+            g.bfs_batch_device(ss, rows.data_ptr(), stream=stream.cuda_stream, stats=False)
+        g.trace_batch(st, traced.data_ptr())
+        torch.cuda.synchronize()
+        for got, src in ((rows, ss), (traced, st)):
+            got = got.cpu().numpy()
+            for s, d in zip(src, got):
+                np.testing.assert_array_equal(d, orc.bfs(csr.beg_pos, csr.csr, int(s))[0])
