@@ -1991,6 +1991,7 @@ int ent_bfs_trace(ent_graph* g, int32_t src, ent_level_trace* out, int32_t max_l
   for (int i = 0; i < 3; ++i) ENT_CUDA(cudaEventCreate(&e[i]));
   LevelArgs la = w->args;
   la.use_cond = 0;
+  ENT_CUDA(cudaStreamWaitEvent(s, w->ev_order, 0));  // a traversal may still run on a caller's stream
   ENT_CUDA(cudaEventRecord(w->ev0, s));
   k_reset<int32_t><<<w->grid_reset, BT, 0, s>>>(la, src, w->depth, nullptr);
   g_kernel_launches += 1;

@@ -70,3 +70,26 @@ def test_batch_trace_after_an_asynchronous_batch(eb, orc):
             got = got.cpu().numpy()
             for s, d in zip(src, got):
                 np.testing.assert_array_equal(d, orc.bfs(csr.beg_pos, csr.csr, int(s))[0])
+
+
+@pytest.mark.parametrize("loop", ["graph", "host"])
+def test_trace_after_an_asynchronous_traversal(eb, orc, loop):
+    import torch
+    csr = eb.Csr.rmat(18, 16, seed=0xB5)
+    a, b = (int(s) for s in eb.pick_sources(csr.beg_pos, 62, 2))
+    with eb.Graph.from_csr(csr) as g:
+        o = g.opts
+        o.loop = eb.LOOP[loop]
+        g.opts = o
+        row = torch.full((csr.vert_count,), 7, dtype=torch.int32, device="cuda")
+        stream = torch.cuda.Stream()
+        g.bfs_device(a, row.data_ptr())
+        torch.cuda.synchronize()
+        for _ in range(8):
+            g.bfs_device(a, row.data_ptr(), stream=stream.cuda_stream, stats=False)
+        levels, st = g.trace(b)
+        torch.cuda.synchronize()
+        np.testing.assert_array_equal(row.cpu().numpy(), orc.bfs(csr.beg_pos, csr.csr, a)[0])
+        exp = orc.bfs(csr.beg_pos, csr.csr, b)[0]
+        assert (st.traversed_edges, st.reached_vertices) == orc.report(csr.beg_pos, exp) and st.levels == exp.max() + 1
+        assert sum(r["frontier_vertices"] for r in levels) <= st.reached_vertices
