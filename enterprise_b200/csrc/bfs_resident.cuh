@@ -20,7 +20,8 @@
 // Phase p reads the counts n[p % 3] and acc[p % 3], fills those of p + 1 and
 // clears those of p + 2, which no CTA reads any more once it is past the
 // barrier before; frontier bitmaps rotate the same way per level. All waits
-// are bounded: one that runs out sets the error bit and every CTA leaves.
+// are bounded: one that runs out sets the error word and every CTA leaves; the
+// traversal's status, an error from its start on, is then never cleared.
 //
 // On large graphs the bottom-up levels are most of the time and want k_expand's
 // occupancy, twice this kernel's (R-MAT s24 0.355 -> 0.31 ms, ER 2^24 d32 2.43 ->
@@ -564,10 +565,13 @@ __global__ void __launch_bounds__(RT, 1) k_resident(LevelArgs a, ResArgs r, int3
   uint32_t target = 0;
   if (threadIdx.x == 0) s_red[0] = s_red[1] = 0;
   if (part == RP_TAIL) {
-    if (c->err) return;  // the head's status stands
+    if (c->err) return;  // the head's error status stands
     if (threadIdx.x == 0) s_st = c->state;
     __syncthreads();
   } else {
+    // Until its end says otherwise the traversal has failed: whichever wait runs
+    // out, and whichever CTAs notice, the host does not read the last one's status.
+    if (tid == 0) a.ctl->err = 2;
     const int32_t isrc = a.inv ? __ldg(a.inv + src) : src;
     fill_unreached(depth, a.V, tid, nth, src);
     for (int64_t i = tid; i < W; i += nth) {
@@ -595,10 +599,9 @@ __global__ void __launch_bounds__(RT, 1) k_resident(LevelArgs a, ResArgs r, int3
         else r.huge[0][0] = isrc;
       }
     }
-    if (!grid_barrier(arrived, &c->err, target += gridDim.x, [] {})) {
-      if (tid == 0) atomicOr(&a.ctl->err, 2);
-      return;
-    }
+    // test hook: a CTA that never arrives (the others' waits run out)
+    if (a.fault_inject && part == RP_ALL && blockIdx.x == gridDim.x - 1) return;
+    if (!grid_barrier(arrived, &c->err, target += gridDim.x, [] {})) return;
   }
   for (;;) {
     const ResState& s = s_st;  // thread 0 changes it inside the barrier only
@@ -637,11 +640,10 @@ __global__ void __launch_bounds__(RT, 1) k_resident(LevelArgs a, ResArgs r, int3
         s_red[0] = s_red[1] = 0;
       }
     }
-    if (!grid_barrier(arrived, &c->err, target += gridDim.x, [&] { res_advance(a, r, s_st); })) {
-      if (tid == 0) atomicOr(&a.ctl->err, 2);
-      return;
-    }
+    if (!grid_barrier(arrived, &c->err, target += gridDim.x, [&] { res_advance(a, r, s_st); })) return;
   }
+  // test hook: a CTA that gave up just as the head's last barrier opened for the others
+  if (a.fault_inject && part == RP_HEAD && threadIdx.x == 0 && blockIdx.x == gridDim.x - 1) c->err = 1;
   if (tid == 0 && part == RP_HEAD) c->state = s_st;
   if (tid == 0 && part != RP_HEAD) {
     const ResState& s = s_st;

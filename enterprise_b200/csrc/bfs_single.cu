@@ -1514,7 +1514,7 @@ constexpr int64_t RES_MIN_DEGREE = 5;
 static bool resident_fits(const ent_graph* g, const BfsWorkspace* w) {
   const ent_bfs_opts& o = g->opts;
   if (g->E < RES_MIN_DEGREE * g->V || !g->perm) return false;
-  if (o.loop != ENT_LOOP_GRAPH || w->narrow_nc == 0 || o.hub_slots > 0 || o.fault_inject) return false;
+  if (o.loop != ENT_LOOP_GRAPH || w->narrow_nc == 0 || o.hub_slots > 0) return false;
   int n = 0;
   for (const void* f : {(const void*)k_resident<int32_t>, (const void*)k_resident<uint8_t>})
     if (cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)RES_SMEM) != cudaSuccess ||

@@ -97,9 +97,10 @@ typedef struct ent_bfs_opts {
   int32_t narrow_max_degree;
   int32_t narrow_cluster;  /* CTAs in the cluster (1..16), 0 = largest that fits */
   int32_t fault_inject;    /* test hook, 0 in use. 1: the first tile of each frontier
-                              classification never publishes its prefix, so the
-                              tiles that wait for it run out their bounded spin
-                              (about a second) and the traversal returns
+                              classification never publishes its prefix, and a
+                              block of a cooperative kernel leaves early, so
+                              those that wait for it run out their bounded spin
+                              (seconds) and the traversal returns
                               ENT_ERR_TIMEOUT with the context still usable */
   /* Batches on deep graphs (grids, road-like graphs): their thousands of small
      levels would cost a grid-wide bitwise batch two launches each, and sources
