@@ -58,6 +58,7 @@ constexpr int NA_HEAVY = 256;     // degree from which a CTA takes a vertex's ro
 constexpr int NA_HUGE = 1 << 15;  // ... and from which all CTAs share it
 constexpr int NA_HUGE_CAP = 1024; // listed ones per level (more are rows of one CTA)
 constexpr int NA_SOLO = 1024;     // light frontier vertices up to which CTA 0 runs alone
+constexpr int NA_SOLO_M = 4096;   // ... and the sum of their degrees; it leaves above twice that
 constexpr int NA_SOLO_CAP = 2048; // frontier entries it keeps in shared memory
 constexpr int NA_SOLO_LEVELS = 4096;  // levels it runs before it meets the others again
 
@@ -65,7 +66,7 @@ struct NaCtl {
   uint32_t arrived;   // barrier arrivals, all barriers of a launch together
   int32_t err;        // a wait ran out
   int32_t level[2];   // per phase (mod 2): the level CTA 0 reached running alone
-  int32_t n[3][4];    // per phase (mod 3): light, heavy, huge frontier vertices
+  int32_t n[3][4];    // per phase (mod 3): light, heavy, huge frontier vertices; degree sum of the light
   int32_t huge[2][NA_HUGE_CAP];
 };
 constexpr size_t NA_BYTES = (NA_OFF_CTL + sizeof(NaCtl) + 255) / 256 * 256;
@@ -94,9 +95,12 @@ struct NaOut {
 };
 
 // Claims the neighbours v[] (negative: none) of frontier vertices for `ln` and
-// queues the won ones by degree. One warp, converged.
+// queues the won ones by degree. One warp, converged. my_m: the lane's sum of the
+// light ones' degrees (CTA 0 alone adds them beside the count instead: the sums
+// at the level's end would lengthen its chain).
 template <bool SOLO>
-__device__ __forceinline__ void na_claim(const NaArgs& a, const int (&v)[NA_ILP], int ln, const NaOut& o) {
+__device__ __forceinline__ void na_claim(const NaArgs& a, const int (&v)[NA_ILP], int ln, const NaOut& o,
+                                         unsigned& my_m) {
   const int lane = threadIdx.x & 31;
   bool open[NA_ILP], mine[NA_ILP];
   int64_t st[NA_ILP];
@@ -120,14 +124,23 @@ __device__ __forceinline__ void na_claim(const NaArgs& a, const int (&v)[NA_ILP]
     }
   }
   int n_light = 0;
+  unsigned m_light = 0;
 #pragma unroll
   for (int i = 0; i < NA_ILP; ++i) {
     if (mine[i]) a.depth[v[i]] = ln;
-    n_light += __popc(__ballot_sync(FULL, mine[i] && d[i] > 0 && d[i] < NA_HEAVY));
+    const bool light = mine[i] && d[i] > 0 && d[i] < NA_HEAVY;
+    n_light += __popc(__ballot_sync(FULL, light));
+    m_light += light ? d[i] : 0;
   }
   int base = 0;
   if (n_light) {
-    if (lane == 0) base = atomicAdd(SOLO ? o.s_n : o.n, n_light);
+    if (SOLO) {
+      m_light = __reduce_add_sync(FULL, m_light);
+      if (lane < 2) base = atomicAdd(o.s_n + 3 * lane, lane ? (int)m_light : n_light);
+    } else {
+      if (lane == 0) base = atomicAdd(o.n, n_light);
+      my_m += m_light;
+    }
     base = __shfl_sync(FULL, base, 0);
   }
 #pragma unroll
@@ -153,7 +166,7 @@ __device__ __forceinline__ void na_claim(const NaArgs& a, const int (&v)[NA_ILP]
 // The concatenated rows of a warp's light vertices (lane: one row of d entries
 // from st, d = 0: none), NA_ILP rounds of 32 entries together.
 template <bool SOLO>
-__device__ __forceinline__ void na_rows(const NaArgs& a, int d, int64_t st, int ln, const NaOut& o) {
+__device__ __forceinline__ void na_rows(const NaArgs& a, int d, int64_t st, int ln, const NaOut& o, unsigned& my_m) {
   const int lane = threadIdx.x & 31;
   int incl = d;
 #pragma unroll
@@ -180,14 +193,14 @@ __device__ __forceinline__ void na_rows(const NaArgs& a, int d, int64_t st, int 
         if (k < total) v[i] = __ldg(a.adj + sj + (k - ej));
       }
     }
-    na_claim<SOLO>(a, v, ln, o);
+    na_claim<SOLO>(a, v, ln, o, my_m);
   }
 }
 
 // Entries first, first + step, ... below end of one long row, 32 * NA_ILP
 // consecutive ones per warp and turn.
 __device__ __forceinline__ void na_slice(const NaArgs& a, int64_t first, int64_t step, int64_t end, int ln,
-                                         const NaOut& o) {
+                                         const NaOut& o, unsigned& my_m) {
   const int lane = threadIdx.x & 31;
   for (int64_t e0 = first; e0 < end; e0 += step) {
     int v[NA_ILP];
@@ -196,14 +209,18 @@ __device__ __forceinline__ void na_slice(const NaArgs& a, int64_t first, int64_t
       const int64_t e = e0 + 32 * i + lane;
       v[i] = e < end ? __ldg(a.adj + e) : -1;
     }
-    na_claim<false>(a, v, ln, o);
+    na_claim<false>(a, v, ln, o, my_m);
   }
 }
 
 // CTA 0 alone, from level L on: runs levels while all frontier vertices are
-// light and fit, at most NA_SOLO_LEVELS, and leaves the next frontier in the
-// queues, its counts in `out` and its level in *level.
-__device__ void na_solo(const NaArgs& a, int L, int n, int4 (*s_q)[NA_SOLO_CAP], int32_t (*s_n)[3], int32_t* out,
+// light and fit and their rows are few, at most NA_SOLO_LEVELS, and leaves the
+// next frontier in the queues, its counts in `out` and its level in *level. It
+// walks about 1.2 entries a ns: without the bound on the rows a band graph of
+// 1000-vertex levels took 147 us a level at degree 200 and 19 at 20, and 12 and 8
+// so. The bound costs 2% where it never applies (700 x 700 grid 4.12 -> 4.20 ms,
+// R-MAT s18 221 -> 225 us; sums at the level's end cost the grid 3%).
+__device__ void na_solo(const NaArgs& a, int L, int n, int4 (*s_q)[NA_SOLO_CAP], int32_t (*s_n)[4], int32_t* out,
                         int32_t* level) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   constexpr int NWARP = NA_T / 32;
@@ -213,14 +230,15 @@ __device__ void na_solo(const NaArgs& a, int L, int n, int4 (*s_q)[NA_SOLO_CAP],
     const int64_t st = a.off[u];
     s_q[L & 1][i] = make_int4(u, (int)(a.off[u + 1] - st), (int)(uint32_t)st, (int)(uint32_t)((uint64_t)st >> 32));
   }
-  if (tid < 3) s_n[0][tid] = s_n[1][tid] = 0;
+  if (tid < 4) s_n[0][tid] = s_n[1][tid] = 0;
   __syncthreads();
-  int n2 = 0, n3 = 0;
+  int n2 = 0, n3 = 0, m = 0;
   for (int run = 0;; ++run) {
     const int cur = L & 1, nxt = cur ^ 1;
     const NaOut o{a.queue[nxt], nullptr, a.ctl->huge[nxt], s_q[nxt], s_n[nxt]};
     // up to 32 rows per warp, spread over all warps
     const int k = min(32, (n + NWARP - 1) / NWARP);
+    unsigned unused = 0;
     for (int first = warp * k; first < n; first += NWARP * k) {
       int d = 0;
       int64_t st = 0;
@@ -229,15 +247,16 @@ __device__ void na_solo(const NaArgs& a, int L, int n, int4 (*s_q)[NA_SOLO_CAP],
         d = e.y;
         st = (int64_t)(((uint64_t)(uint32_t)e.w << 32) | (uint32_t)e.z);
       }
-      na_rows<true>(a, d, st, L + 1, o);
+      na_rows<true>(a, d, st, L + 1, o, unused);
     }
     __syncthreads();
     n = s_n[nxt][0];
     n2 = s_n[nxt][1];
     n3 = s_n[nxt][2];
     ++L;
-    if (n == 0 || n > NA_SOLO_CAP || n2 || n3 || run + 1 >= NA_SOLO_LEVELS) break;
-    if (tid < 3) s_n[cur][tid] = 0;  // takes the counts of the level after
+    m = s_n[nxt][3];
+    if (n == 0 || n > NA_SOLO_CAP || m > 2 * NA_SOLO_M || n2 || n3 || run + 1 >= NA_SOLO_LEVELS) break;
+    if (tid < 4) s_n[cur][tid] = 0;  // takes the counts of the level after
     __syncthreads();
   }
   // hand over: stored entries to the queue (the rest are there), counts
@@ -247,6 +266,7 @@ __device__ void na_solo(const NaArgs& a, int L, int n, int4 (*s_q)[NA_SOLO_CAP],
     out[0] = n;
     out[1] = n2;
     out[2] = n3;
+    out[3] = m;
     *level = L;
   }
 }
@@ -266,7 +286,9 @@ __device__ void na_solo(const NaArgs& a, int L, int n, int4 (*s_q)[NA_SOLO_CAP],
 __global__ void __launch_bounds__(NA_T, 1) k_na_run(NaArgs a) {
   extern __shared__ int4 s_dyn[];
   int4(*s_q)[NA_SOLO_CAP] = reinterpret_cast<int4(*)[NA_SOLO_CAP]>(s_dyn);
-  __shared__ int32_t s_n[2][3];
+  __shared__ int32_t s_n[2][4];
+  __shared__ unsigned s_m;
+  if (threadIdx.x == 0) s_m = 0;
   NaCtl* c = a.ctl;
   const int64_t tid = blockIdx.x * (int64_t)NA_T + threadIdx.x, nth = (int64_t)gridDim.x * NA_T;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -279,6 +301,7 @@ __global__ void __launch_bounds__(NA_T, 1) k_na_run(NaArgs a) {
     if (d > 0 && d < NA_HEAVY) {
       a.queue[0][0] = a.src;
       c->n[0][0] = 1;
+      c->n[0][3] = (int32_t)d;
     } else if (d >= NA_HEAVY) {
       a.queue[0][NOALLOC_MAX_VERTICES - 1] = a.src;
       c->n[0][1] = 1;
@@ -292,8 +315,8 @@ __global__ void __launch_bounds__(NA_T, 1) k_na_run(NaArgs a) {
     int32_t* next = c->n[(p + 1) % 3];
     const int n_l = __ldcg(cnt), n_h = __ldcg(cnt + 1), n_g = min(__ldcg(cnt + 2), NA_HUGE_CAP);
     if (n_l + n_h + n_g == 0) return;
-    if (tid < 3) c->n[(p + 2) % 3][tid] = 0;
-    if (n_l <= NA_SOLO && n_h + n_g == 0) {
+    if (tid < 4) c->n[(p + 2) % 3][tid] = 0;
+    if (n_l <= NA_SOLO && __ldcg(cnt + 3) <= NA_SOLO_M && n_h + n_g == 0) {
       if (blockIdx.x == 0) na_solo(a, L, n_l, s_q, s_n, next, &c->level[p & 1]);
       if (!grid_barrier(&c->arrived, &c->err, target += gridDim.x, [] {})) return;
       L = __ldcg(&c->level[p & 1]);
@@ -302,15 +325,16 @@ __global__ void __launch_bounds__(NA_T, 1) k_na_run(NaArgs a) {
     const int32_t* q = a.queue[L & 1];
     const NaOut o{a.queue[(L + 1) & 1], next, c->huge[(L + 1) & 1], nullptr, nullptr};
     const int64_t gw = (int64_t)blockIdx.x * NWARP + warp, nw = (int64_t)gridDim.x * NWARP;
+    unsigned my_m = 0;
     for (int i = 0; i < n_g; ++i) {  // rows shared by all CTAs
       const int u = __ldcg(c->huge[L & 1] + i);
       const int64_t beg = a.off[u], end = a.off[u + 1];
-      na_slice(a, beg + gw * 32 * NA_ILP, nw * 32 * NA_ILP, end, L + 1, o);
+      na_slice(a, beg + gw * 32 * NA_ILP, nw * 32 * NA_ILP, end, L + 1, o, my_m);
     }
     for (int i = blockIdx.x; i < n_h; i += gridDim.x) {  // rows of one CTA
       const int u = __ldcg(q + NOALLOC_MAX_VERTICES - 1 - i);
       const int64_t beg = a.off[u], end = a.off[u + 1];
-      na_slice(a, beg + warp * 32 * NA_ILP, NWARP * 32 * NA_ILP, end, L + 1, o);
+      na_slice(a, beg + warp * 32 * NA_ILP, NWARP * 32 * NA_ILP, end, L + 1, o, my_m);
     }
     // up to 32 light rows per warp, spread over all warps
     const int k = (int)min((int64_t)32, (n_l + nw - 1) / nw);
@@ -322,7 +346,14 @@ __global__ void __launch_bounds__(NA_T, 1) k_na_run(NaArgs a) {
         st = a.off[u];
         d = (int)(a.off[u + 1] - st);
       }
-      na_rows<false>(a, d, st, L + 1, o);
+      na_rows<false>(a, d, st, L + 1, o, my_m);
+    }
+    my_m = __reduce_add_sync(FULL, my_m);
+    if (lane == 0 && my_m) atomicAdd(&s_m, my_m);
+    __syncthreads();
+    if (threadIdx.x == 0 && s_m) {
+      atomicAdd(next + 3, (int)s_m);
+      s_m = 0;
     }
     ++L;
     if (!grid_barrier(&c->arrived, &c->err, target += gridDim.x, [] {})) return;
