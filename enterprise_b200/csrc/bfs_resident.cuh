@@ -30,8 +30,8 @@
 // needed leave at once; the last CTA of each takes the decision), and a tail
 // for whatever is left.
 //
-// Not here: parents, hub tables and runs with the small-frontier mode off stay
-// with the level kernels.
+// Not here: parents, hub tables, runs with the small-frontier mode off and graphs
+// of many small levels (meshes, bands) stay with the level kernels.
 #pragma once
 
 constexpr int RT = 1024;          // threads per CTA, one per SM (64 registers a thread)
@@ -53,9 +53,14 @@ enum { RK_TD, RK_BU, RK_QUEUE, RK_SOLO, RK_DONE };
 struct ResState {
   int32_t kind, L, f, p;      // f: fb index of the frontier
   int32_t n_l, n_h, n_g;
-  int32_t td_levels, bu_levels, narrow_levels, err;
+  int32_t td_levels, bu_levels, narrow_levels, mid_levels, err;
   int64_t n_f, m_f, n_vis, m_vis;
 };
+
+// Frontiers, by degree sum, that the cluster of k_narrow takes in less time.
+constexpr int64_t RES_MID_MIN = 64, RES_MID_MAX = 40000;
+__device__ __forceinline__ int res_mid(int64_t m_f) { return m_f >= RES_MID_MIN && m_f <= RES_MID_MAX; }
+
 
 struct ResCtl {
   uint32_t arrived[2];  // barrier arrivals of the head (or the whole), and of the tail
@@ -66,7 +71,7 @@ struct ResCtl {
   unsigned long long acc[3][2];  // vertices and degree sum that a phase found
   struct {
     int64_t n_f, m_f, n_vis, m_vis;
-    int32_t level, pad;
+    int32_t level, mid_levels;
   } solo[2];         // where CTA 0 got to alone, by phase parity
 };
 
@@ -105,6 +110,7 @@ __device__ void res_advance(const LevelArgs& a, const ResArgs& r, ResState& s) {
     s.m_vis = ldcg64(&so->m_vis);
     s.td_levels += L - s.L;
     s.narrow_levels += L - s.L;
+    s.mid_levels += __ldcg(&so->mid_levels);
     s.L = L;
   } else if (kind != RK_QUEUE) {
     n_next = ldcg64(&c->acc[q][0]);
@@ -112,6 +118,7 @@ __device__ void res_advance(const LevelArgs& a, const ResArgs& r, ResState& s) {
     s.n_vis += n_next;
     s.m_vis += m_next;
     s.L += 1;
+    s.mid_levels += res_mid(s.m_f);
     if (kind == RK_TD) s.td_levels += 1;
     else s.bu_levels += 1;
   }
@@ -477,9 +484,10 @@ __device__ void res_solo(const LevelArgs& a, const ResArgs& r, const ResState& s
   if (tid < 3) s_n[0][tid] = s_n[1][tid] = 0;
   if (tid < 2) s_m[tid] = s_v[tid] = 0;
   __syncthreads();
-  int n2 = 0, n3 = 0;
+  int n2 = 0, n3 = 0, mid = 0;
   for (int run = 0;; ++run) {
     const int cur = L & 1, nxt = cur ^ 1;
+    mid += res_mid(m_f);
     const ResOut o{nullptr, r.queue[nxt], r.huge[nxt], s_n[nxt], s_q[nxt]};
     const int k = min(32, (cnt + RW - 1) / RW);
     unsigned my_n = 0;
@@ -544,6 +552,7 @@ __device__ void res_solo(const LevelArgs& a, const ResArgs& r, const ResState& s
     so->n_vis = n_vis;
     so->m_vis = m_vis;
     so->level = L;
+    so->mid_levels = mid;
   }
 }
 
@@ -585,7 +594,7 @@ __global__ void __launch_bounds__(RT, 1) k_resident(LevelArgs a, ResArgs r, int3
       const int d = a.deg[isrc];
       ResState s;
       s.L = s.f = s.p = 0;
-      s.td_levels = s.bu_levels = s.narrow_levels = s.err = 0;
+      s.td_levels = s.bu_levels = s.narrow_levels = s.mid_levels = s.err = 0;
       s.n_f = s.n_vis = 1;
       s.m_f = s.m_vis = d;
       s.n_l = d < R_HEAVY;
@@ -655,11 +664,13 @@ __global__ void __launch_bounds__(RT, 1) k_resident(LevelArgs a, ResArgs r, int3
     k->td_levels = s.td_levels;
     k->bu_levels = s.bu_levels;
     k->narrow_levels = s.narrow_levels;
+    k->mid_levels = s.mid_levels;
     k->iters = 0;
     k->narrow_calls = 0;
     k->split_launches = part == RP_TAIL ? R_BU_LEVELS + 1 : 0;
     k->n_vis = s.n_vis;
     k->m_vis = s.m_vis;
+    k->m_f = s.m_f;
   }
 }
 

@@ -109,6 +109,7 @@ struct BfsCtl {
   int32_t iters;      // inspector launches (level-loop iterations)
   int32_t narrow_runs;
   int32_t split_launches;  // kernels after the first of a resident traversal in parts
+  int32_t mid_levels;      // levels of a resident traversal that suit the cluster of k_narrow better
   int32_t narrow_calls;  // launches of the small-frontier kernel, those that left at once included
   uint32_t n_spill;   // small-frontier entries that did not fit in shared memory
   uint32_t acc_maxd;  // maximum degree in the next frontier being classified
@@ -1511,6 +1512,15 @@ constexpr size_t RES_SMEM = 2 * R_SOLO_CAP * sizeof(int4);
 // k_narrow: a 300^2 grid 1.5 -> 2.1 ms, 1024^2 5.4 -> 13 ms.
 constexpr int64_t RES_SPLIT_V = 1 << 22;
 constexpr int64_t RES_MIN_DEGREE = 5;
+// Nor do graphs of higher mean degree that turn out to have many levels of
+// RES_MID_MIN to RES_MID_MAX entries (meshes, bands): in the cluster such a level
+// takes 3 to 5 us, here 4 to 12. us a traversal, caller's order and level
+// kernels, resident, this order and level kernels: mesh 80^3 1158, 2923, 1166; 200 levels of 200
+// vertices, degree 40: 812, 2421, 717; 192 levels of 1000, degree 20: 1173, 1451,
+// 979. Larger levels are faster here (192 of 5000, degree 16: 3043, 2012, 2603;
+// mesh 160^3 8.25, 5.55, 8.12 ms), and a path's are equal.
+constexpr int32_t RES_DEEP = 12;    // such levels from which a graph counts as deep
+constexpr int32_t RES_PROBE = 128;  // levels that a probe runs at most
 static bool resident_fits(const ent_graph* g, const BfsWorkspace* w) {
   const ent_bfs_opts& o = g->opts;
   if (g->E < RES_MIN_DEGREE * g->V || !g->perm) return false;
@@ -1523,6 +1533,56 @@ static bool resident_fits(const ent_graph* g, const BfsWorkspace* w) {
       return false;
     }
   return true;
+}
+
+// The resident traversal on stream s (no parents): one kernel, or for large
+// graphs its level kernels between two.
+// ENT_ERR_UNSUPPORTED when the GPU cannot hold all its CTAs at once (part of
+// it set aside, by MPS or a partition): the level kernels take over.
+template <class DT>
+static int launch_resident(BfsWorkspace* w, int32_t src, DT* depth, cudaStream_t s, int32_t max_levels = 0) {
+  LevelArgs a = w->args;
+  if (max_levels > 0) a.max_levels = max_levels;
+  a.use_cond = 0;
+  int part = w->split ? RP_HEAD : RP_ALL;
+  void* args[5] = {&a, &w->res, &src, &depth, &part};
+  ENT_CUDA(cudaMemsetAsync(w->res.rc, 0, sizeof(ResCtl), s));
+  const cudaError_t e =
+      cudaLaunchCooperativeKernel((const void*)k_resident<DT>, dim3(w->grid_res), dim3(RT), args, RES_SMEM, s);
+  if (e == cudaErrorCooperativeLaunchTooLarge) {
+    cudaGetLastError();
+    w->res.rc = nullptr;
+    return ENT_ERR_UNSUPPORTED;
+  }
+  ENT_CUDA(e);
+  if (!w->split) return ENT_OK;
+  for (int i = 0; i < R_BU_LEVELS; ++i) k_res_bu_level<DT><<<w->grid_expand, BT, 0, s>>>(a, w->res, depth);
+  ENT_CUDA(cudaGetLastError());
+  part = RP_TAIL;
+  ENT_CUDA(cudaLaunchCooperativeKernel((const void*)k_resident<DT>, dim3(w->grid_res), dim3(RT), args, RES_SMEM, s));
+  return ENT_OK;
+}
+
+// Notes what a resident traversal says of the graph: whether most of its levels
+// are better run by the level kernels, which have it from here on. A frontier
+// still growing past that size when a probe was cut off speaks against it.
+static void note_depth(ent_graph* g, const BfsCtl& h) {
+  g->deep = h.mid_levels >= RES_DEEP && 2 * h.mid_levels >= h.level && h.m_f <= RES_MID_MAX;
+}
+
+// The same before a traversal that the host does not wait for: from a vertex of
+// the highest degree, RES_PROBE levels at most, on the graph's stream.
+static int probe_depth(ent_graph* g, BfsWorkspace* w) {
+  ENT_CUDA(cudaStreamWaitEvent(g->stream, w->ev_order, 0));
+  const int rc = launch_resident<int32_t>(w, g->top, w->depth, g->stream, RES_PROBE);
+  if (rc != ENT_OK) return rc == ENT_ERR_UNSUPPORTED ? ENT_OK : rc;
+  ENT_CUDA(cudaMemcpyAsync(w->ctl_h, w->ctl, sizeof(BfsCtl), cudaMemcpyDeviceToHost, g->stream));
+  ENT_CUDA(cudaStreamSynchronize(g->stream));
+  g_kernel_launches += 1 + w->ctl_h->split_launches;
+  if (w->ctl_h->err & ~4)  // 4: cut off
+    return fail(ENT_ERR_TIMEOUT, "device traversal reported error flags 0x%x", w->ctl_h->err);
+  note_depth(g, *w->ctl_h);
+  return ENT_OK;
 }
 
 static int create_workspace(ent_graph* g, BfsWorkspace** out, bool force_graph = false, int32_t cluster = 0) {
@@ -1679,33 +1739,6 @@ static int launch_graph(ent_graph* g, BfsWorkspace* w, int32_t src, DT* depth, i
   return ENT_OK;
 }
 
-// The resident traversal on stream s (no parents): one kernel, or for large
-// graphs its level kernels between two.
-// ENT_ERR_UNSUPPORTED when the GPU cannot hold all its CTAs at once (part of
-// it set aside, by MPS or a partition): the level kernels take over.
-template <class DT>
-static int launch_resident(BfsWorkspace* w, int32_t src, DT* depth, cudaStream_t s) {
-  LevelArgs a = w->args;
-  a.use_cond = 0;
-  int part = w->split ? RP_HEAD : RP_ALL;
-  void* args[5] = {&a, &w->res, &src, &depth, &part};
-  ENT_CUDA(cudaMemsetAsync(w->res.rc, 0, sizeof(ResCtl), s));
-  const cudaError_t e =
-      cudaLaunchCooperativeKernel((const void*)k_resident<DT>, dim3(w->grid_res), dim3(RT), args, RES_SMEM, s);
-  if (e == cudaErrorCooperativeLaunchTooLarge) {
-    cudaGetLastError();
-    w->res.rc = nullptr;
-    return ENT_ERR_UNSUPPORTED;
-  }
-  ENT_CUDA(e);
-  if (!w->split) return ENT_OK;
-  for (int i = 0; i < R_BU_LEVELS; ++i) k_res_bu_level<DT><<<w->grid_expand, BT, 0, s>>>(a, w->res, depth);
-  ENT_CUDA(cudaGetLastError());
-  part = RP_TAIL;
-  ENT_CUDA(cudaLaunchCooperativeKernel((const void*)k_resident<DT>, dim3(w->grid_res), dim3(RT), args, RES_SMEM, s));
-  return ENT_OK;
-}
-
 int launch_bfs_single(BfsWorkspace* w, int32_t src, int32_t* depth_dev, cudaStream_t s) {
   g_kernel_launches += 1;  // reset; the level kernels are counted by bfs_single_stats
   return launch_graph(nullptr, w, src, depth_dev, nullptr, s);  // int32 graph: built with the workspace
@@ -1733,11 +1766,17 @@ static int run_bfs_typed(ent_graph* g, int32_t src, DT* depth, int32_t* parent, 
   BfsWorkspace* w = g->ws;
   cudaStream_t s = stream ? stream : g->stream;
   const bool captured = capturing(s);  // the launches below refuse it
+  bool resident = false;
   if (!captured) ENT_CUDA(cudaStreamWaitEvent(s, w->ev_order, 0));
   if (stats) ENT_CUDA(cudaEventRecord(w->ev0, s));
   if (g->opts.loop == ENT_LOOP_GRAPH) {
+    if (w->res.rc && !parent && !captured && g->deep < 0 && !stats) {
+      const int rcode = probe_depth(g, w);
+      if (rcode != ENT_OK) return rcode;
+    }
     int rc = ENT_ERR_UNSUPPORTED;
-    if (w->res.rc && !parent && !captured) rc = launch_resident(w, src, depth, s);
+    resident = w->res.rc && !parent && !captured && g->deep != 1;
+    if (resident) rc = launch_resident(w, src, depth, s);
     if (rc == ENT_ERR_UNSUPPORTED) rc = launch_graph(g, w, src, depth, parent, s);
     if (rc != ENT_OK) return rc;
   } else {
@@ -1772,6 +1811,8 @@ static int run_bfs_typed(ent_graph* g, int32_t src, DT* depth, int32_t* parent, 
     float ms = 0.f;
     cudaEventElapsedTime(&ms, w->ev0, w->ev1);
     fill_stats(*w->ctl_h, ms, stats);
+    // a source in the bulk of the graph speaks for it
+    if (resident && g->deep < 0 && !w->ctl_h->err && w->ctl_h->n_vis * 4 >= w->V) note_depth(g, *w->ctl_h);
     if (g->opts.loop == ENT_LOOP_GRAPH) g_kernel_launches += stats->launches;
     if (w->ctl_h->err) return fail(ENT_ERR_TIMEOUT, "device traversal reported error flags 0x%x", w->ctl_h->err);
   } else if (g->opts.loop == ENT_LOOP_GRAPH) {

@@ -64,7 +64,8 @@ enum ent_loop {
   ENT_LOOP_GRAPH = 0, /* whole traversal = one launch, no host round trip:
                          a CUDA graph with a device-side while node, or,
                          without parents and on graphs of mean degree 5 and
-                         more, cooperative kernels of many levels each      */
+                         more whose levels do not prove many and small,
+                         cooperative kernels of many levels each            */
   ENT_LOOP_HOST = 1   /* host launches each level and polls a flag     */
 };
 
