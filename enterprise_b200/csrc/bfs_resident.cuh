@@ -37,8 +37,7 @@
 constexpr int RT = 1024;          // threads per CTA, one per SM (64 registers a thread)
 constexpr int RW = RT / 32;
 constexpr int R_ILP = 4;          // row entries a lane has in flight together
-constexpr int R_BW = 3;           // bottom-up: status words a warp has in flight together
-constexpr int R_BILP = 2;         // ... and row entries of each per step
+constexpr int R_BW_WORDS = 4;     // bottom-up: words a warp up to which it takes them two by two
 constexpr int R_HEAVY = 256;      // degree from which warps take a row alone, or share it
 constexpr int R_HUGE = 16384;     // ... and from which at least R_SHARE warps do
 constexpr int R_SHARE = 32;
@@ -337,9 +336,10 @@ __device__ void res_td(const LevelArgs& a, const ResArgs& r, const ResState& s, 
 }
 
 // One bottom-up level over the words of vertices that have rows (bu_expand
-// with nothing to list).
-template <class DT>
-__device__ void res_bu(const LevelArgs& a, const ResArgs& r, const ResState& s, DT* depth, unsigned& my_n,
+// with nothing to list), BW words of a warp in flight together, and ILP row
+// entries of each vertex per step.
+template <class DT, int BW, int ILP>
+__device__ void res_bu_words(const LevelArgs& a, const ResArgs& r, const ResState& s, DT* depth, unsigned& my_n,
                        unsigned long long& my_m) {
   const uint32_t* fbc = r.fb[s.f];
   uint32_t* fbn = r.fb[(s.f + 1) % 3];
@@ -348,24 +348,23 @@ __device__ void res_bu(const LevelArgs& a, const ResArgs& r, const ResState& s, 
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int64_t gw = (int64_t)blockIdx.x * RW + warp, nw = (int64_t)gridDim.x * RW;
   const int64_t W = (a.n_active + 31) >> 5;
-  // R_BW words at a time through every stage together: a CTA of 64-register
+  // BW words at a time through every stage together: a CTA of 64-register
   // threads holds half the warps of k_expand, so each has to keep more reads in
-  // flight (R-MAT s24, whole traversal: 1 word 0.43 ms, 2 0.38, 3 0.355, 4 0.35;
-  // ER 2^23 d16: 0.65, 0.58, 0.55, 0.59).
-  for (int64_t w0 = gw; w0 < W; w0 += R_BW * nw) {
-    uint32_t vis[R_BW], mask[R_BW];
-    int4 ld[R_BW];
-    int d[R_BW], id[R_BW];
-    bool todo[R_BW];  // still to be found
-    bool found[R_BW];
+  // flight.
+  for (int64_t w0 = gw; w0 < W; w0 += BW * nw) {
+    uint32_t vis[BW], mask[BW];
+    int4 ld[BW];
+    int d[BW], id[BW];
+    bool todo[BW];  // still to be found
+    bool found[BW];
 #pragma unroll
-    for (int t = 0; t < R_BW; ++t) {
+    for (int t = 0; t < BW; ++t) {
       const int64_t wi = w0 + t * nw;
       vis[t] = wi < W ? __ldcg(a.vis + wi) : 0u;
       mask[t] = wi < W ? a.active[wi] & ~vis[t] : 0u;
     }
 #pragma unroll
-    for (int t = 0; t < R_BW; ++t) {
+    for (int t = 0; t < BW; ++t) {
       ld[t] = make_int4(-1, -1, -1, -1);
       d[t] = id[t] = 0;
       todo[t] = (mask[t] >> lane) & 1u;
@@ -377,47 +376,70 @@ __device__ void res_bu(const LevelArgs& a, const ResArgs& r, const ResState& s, 
       }
     }
 #pragma unroll
-    for (int t = 0; t < R_BW; ++t) {
+    for (int t = 0; t < BW; ++t) {
       found[t] = todo[t] && is_front(ld[t].x);
       todo[t] &= !found[t];
     }
 #pragma unroll
-    for (int t = 0; t < R_BW; ++t)
+    for (int t = 0; t < BW; ++t)
       if (todo[t] && d[t] > 1) {
         found[t] = is_front(ld[t].y) | (ld[t].z >= 0 && is_front(ld[t].z)) | (ld[t].w >= 0 && is_front(ld[t].w));
         todo[t] = !found[t];
       }
-    uint32_t e0[R_BW];
+    uint32_t e0[BW];
 #pragma unroll
-    for (int t = 0; t < R_BW; ++t) {
+    for (int t = 0; t < BW; ++t) {
       todo[t] &= d[t] > 4;  // shorter rows have been looked through
       e0[t] = 0;
       if (todo[t]) e0[t] = (uint32_t)__ldcs(a.off + (w0 + t * nw) * 32 + lane);
     }
-    // light rows: R_BILP entries of each word per step
-    for (int k = 4;; k += R_BILP) {
+    // light rows: ILP entries of each word per step
+    for (int k = 4;; k += ILP) {
       bool more = false;
-      int u[R_BW][R_BILP];
+      int u[BW][ILP];
 #pragma unroll
-      for (int t = 0; t < R_BW; ++t) {
+      for (int t = 0; t < BW; ++t) {
         const bool go = todo[t] && d[t] < a.small_max && k < d[t];
         more |= go;
 #pragma unroll
-        for (int i = 0; i < R_BILP; ++i) u[t][i] = go && k + i < d[t] ? __ldg(a.adj + e0[t] + k + i) : -1;
+        for (int i = 0; i < ILP; ++i) u[t][i] = go && k + i < d[t] ? __ldg(a.adj + e0[t] + k + i) : -1;
       }
       if (!more) break;
 #pragma unroll
-      for (int t = 0; t < R_BW; ++t) {
+      for (int t = 0; t < BW; ++t) {
         bool f = false;
 #pragma unroll
-        for (int i = 0; i < R_BILP; ++i) f |= u[t][i] >= 0 && is_front(u[t][i]);
+        for (int i = 0; i < ILP; ++i) f |= u[t][i] >= 0 && is_front(u[t][i]);
         if (f) found[t] = true, todo[t] = false;
       }
     }
-    // heavy rows: the warp together
+    // Heavy rows: the warp together, four rows at a time while there are four.
+    // In the order by degree whole words hold them, and a row at a time took 32
+    // trips for rows just above small_max (ER 2^19, mean degree 40: 145 -> 100 us a
+    // traversal, 29: 216 -> 184).
 #pragma unroll
-    for (int t = 0; t < R_BW; ++t) {
+    for (int t = 0; t < BW; ++t) {
       unsigned heavy = __ballot_sync(FULL, todo[t] && d[t] >= a.small_max);
+      while (__popc(heavy) >= 4) {  // four rows at a time, eight lanes each
+        const unsigned h1 = heavy & (heavy - 1), h2 = h1 & (h1 - 1), h3 = h2 & (h2 - 1);
+        const int sub = lane >> 3;
+        const int j = __ffs(sub == 0 ? heavy : (sub == 1 ? h1 : (sub == 2 ? h2 : h3))) - 1;
+        heavy = h3 & (h3 - 1);
+        const uint32_t beg = __shfl_sync(FULL, e0[t], j);
+        const int n = __shfl_sync(FULL, d[t], j);
+        bool hit = false;
+        for (int b0 = lane & 7;; b0 += 32) {
+          int u[4];
+#pragma unroll
+          for (int i = 0; i < 4; ++i) u[i] = !hit && b0 + 8 * i < n ? __ldg(a.adj + beg + b0 + 8 * i) : -1;
+          bool f = false;
+#pragma unroll
+          for (int i = 0; i < 4; ++i) f |= u[i] >= 0 && is_front(u[i]);
+          hit |= ((__ballot_sync(FULL, f) >> (8 * sub)) & 0xFFu) != 0;
+          if (__all_sync(FULL, hit || b0 + 32 - (lane & 7) >= n)) break;
+        }
+        if (__reduce_or_sync(FULL, hit ? 1u << j : 0u) >> lane & 1u) found[t] = true;
+      }
       while (heavy) {
         const int j = __ffs(heavy) - 1;
         heavy &= heavy - 1;
@@ -433,7 +455,7 @@ __device__ void res_bu(const LevelArgs& a, const ResArgs& r, const ResState& s, 
       }
     }
 #pragma unroll
-    for (int t = 0; t < R_BW; ++t) {
+    for (int t = 0; t < BW; ++t) {
       if (found[t]) {
         st_keep(depth + id[t], (DT)(s.L + 1));
         my_n += 1;
@@ -447,6 +469,18 @@ __device__ void res_bu(const LevelArgs& a, const ResArgs& r, const ResState& s, 
       }
     }
   }
+}
+
+// Three words of a warp and three entries a step; on small graphs, where a warp
+// has few words and its last group would be mostly empty, two and four. us a
+// traversal, words x entries 3 x 2, 3 x 3, 2 x 4: ER 2^19 of mean degree 16 108, 105,
+// 100, of 29 184, 180, 172; R-MAT s16 66.6, 65.6, 63.5; ER 2^22 d16 291, 283, 301;
+// ER 3M d6 305, 303, 323; R-MAT s22 155, 153, 153.
+template <class DT>
+__device__ void res_bu(const LevelArgs& a, const ResArgs& r, const ResState& s, DT* depth, unsigned& my_n,
+                       unsigned long long& my_m) {
+  if ((a.n_active + 31) >> 5 <= (int64_t)gridDim.x * RW * R_BW_WORDS) res_bu_words<DT, 2, 4>(a, r, s, depth, my_n, my_m);
+  else res_bu_words<DT, 3, 3>(a, r, s, depth, my_n, my_m);
 }
 
 // Queues the frontier in fb[s.f], left by a bottom-up level (vertices with rows).
