@@ -1,11 +1,11 @@
-// The whole single-source traversal as one cooperative kernel, for graphs that
-// the level kernels of bfs_single.cu cannot keep busy (included there).
+// The whole single-source traversal as one kernel, for graphs that the level
+// kernels of bfs_single.cu cannot keep busy (included there).
 //
 // On a small graph the level loop costs more than the levels: a level is three
 // kernel nodes and half a while-node iteration, about 20 us whatever it does
 // (R-MAT s12: 124 us a traversal, 16 us of them in kernels; s20: 138 us). Here
-// the CTAs stay resident and go from level to level through a grid-wide
-// barrier, and every CTA takes the level's decision by itself from the counts
+// the CTAs stay resident and go from level to level together (a Crew,
+// dev_common.cuh), and each takes the level's decision by itself from the counts
 // that the barrier published, so no level ends in one CTA's chain.
 //
 // A phase is one of
@@ -15,8 +15,10 @@
 //   * a bottom-up level: a warp per status word, as in k_expand;
 //   * a queue build, from the frontier bitmap, where a bottom-up level hands
 //     over to top-down;
-//   * a run of small top-down levels by CTA 0 alone, its frontier in shared
-//     memory (counted as small-frontier levels), while the others wait.
+//   * a run of small top-down levels by the leader alone, its frontier in shared
+//     memory (counted as small-frontier levels), while the others wait;
+//   * where other work holds some SMs, a wait for more members before a long phase,
+//     or the fills of CTAs that had not started.
 // Phase p reads the counts n[p % 3] and acc[p % 3], fills those of p + 1 and
 // clears those of p + 2, which no CTA reads any more once it is past the
 // barrier before; frontier bitmaps rotate the same way per level. All waits
@@ -25,8 +27,8 @@
 //
 // On large graphs the bottom-up levels are most of the time and want k_expand's
 // occupancy, twice this kernel's (R-MAT s24 0.355 -> 0.31 ms, ER 2^24 d32 2.43 ->
-// 1.69). The traversal then runs in parts: a head up to
-// the first bottom-up level, R_BU_LEVELS kernels of one level each (those not
+// 1.69). The traversal then runs in parts: a head up to the first bottom-up
+// level, R_BU_LEVELS kernels of one level each (those not
 // needed leave at once; the last CTA of each takes the decision), and a tail
 // for whatever is left.
 //
@@ -41,16 +43,17 @@ constexpr int R_BW_WORDS = 4;     // bottom-up: words a warp up to which it take
 constexpr int R_HEAVY = 256;      // degree from which warps take a row alone, or share it
 constexpr int R_HUGE = 16384;     // ... and from which at least R_SHARE warps do
 constexpr int R_SHARE = 32;
-constexpr int R_SOLO = 2048;      // frontier up to which CTA 0 starts to run alone
+constexpr int R_SOLO = 2048;      // frontier up to which the leader starts to run alone
 constexpr int R_SOLO_M = 16384;   // ... and its degree sum; it leaves above twice that
 constexpr int R_SOLO_CAP = 4096;  // frontier entries it keeps in shared memory
 constexpr int R_SOLO_LEVELS = 4096;  // levels it runs before it meets the others again
 
-enum { RK_TD, RK_BU, RK_QUEUE, RK_SOLO, RK_DONE };
+enum { RK_TD, RK_BU, RK_QUEUE, RK_SOLO, RK_DONE, RK_GATHER, RK_FILL };
 
-// What every CTA knows about the phase to come (thread 0 keeps it current).
+// What every member knows about the phase to come (thread 0 keeps it current).
 struct ResState {
   int32_t kind, L, f, p;      // f: fb index of the frontier
+  int32_t then;               // RK_GATHER, RK_FILL: the kind of the phase after
   int32_t n_l, n_h, n_g;
   int32_t td_levels, bu_levels, narrow_levels, mid_levels, err;
   int64_t n_f, m_f, n_vis, m_vis;
@@ -62,7 +65,7 @@ __device__ __forceinline__ int res_mid(int64_t m_f) { return m_f >= RES_MID_MIN 
 
 
 struct ResCtl {
-  uint32_t arrived[2];  // barrier arrivals of the head (or the whole), and of the tail
+  Crew<ResState> crew[2];  // of the head (or the whole), and of the tail
   int32_t err;       // a wait ran out
   uint32_t finished; // CTAs of a bottom-up kernel that are done
   ResState state;    // between the kernels of a traversal in parts
@@ -71,7 +74,7 @@ struct ResCtl {
   struct {
     int64_t n_f, m_f, n_vis, m_vis;
     int32_t level, mid_levels;
-  } solo[2];         // where CTA 0 got to alone, by phase parity
+  } solo[2];         // where the leader got to alone, by phase parity
 };
 
 struct ResArgs {
@@ -159,11 +162,11 @@ __device__ void res_advance(const LevelArgs& a, const ResArgs& r, ResState& s) {
 
 // Where the claims of a top-down phase go, and what they add up to.
 struct ResOut {
-  uint32_t* fb;      // the next frontier's bits (not while CTA 0 runs alone)
+  uint32_t* fb;      // the next frontier's bits (not while the leader runs alone)
   int32_t* q;
   int32_t* huge;
-  int32_t* n;        // counts: global, or CTA 0's own in shared memory
-  int4* s_q;         // CTA 0 alone: entries in shared memory while they fit
+  int32_t* n;        // counts: global, or the leader's own in shared memory
+  int4* s_q;         // the leader alone: entries in shared memory while they fit
 };
 
 // Where vertices queue by degree: 0 light, 1 heavy, 2 huge.
@@ -302,12 +305,12 @@ __device__ __forceinline__ void res_slice(const LevelArgs& a, int64_t first, int
 }
 
 template <class DT>
-__device__ void res_td(const LevelArgs& a, const ResArgs& r, const ResState& s, DT* depth, const ResOut& o,
-                       unsigned& my_n, unsigned long long& my_m) {
+__device__ void res_td(const LevelArgs& a, const ResArgs& r, const ResState& s, const CrewSeat& seat, DT* depth,
+                       const ResOut& o, unsigned& my_n, unsigned long long& my_m) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int32_t* q = r.queue[s.L & 1];
   const int ln = s.L + 1;
-  const int64_t gw = (int64_t)blockIdx.x * RW + warp, nw = (int64_t)gridDim.x * RW;
+  const int64_t gw = (int64_t)seat.rank * RW + warp, nw = (int64_t)seat.size * RW;
   // Long rows: `share` warps each, in turn over the rows. A CTA per row left
   // R-MAT s24's second level (four rows of 24k entries in all) at 60 us and
   // spent 2.1 ms on s22 top-down throughout; a list of equal chunks is as fast
@@ -339,19 +342,19 @@ __device__ void res_td(const LevelArgs& a, const ResArgs& r, const ResState& s, 
 // with nothing to list), BW words of a warp in flight together, and ILP row
 // entries of each vertex per step.
 template <class DT, int BW, int ILP>
-__device__ void res_bu_words(const LevelArgs& a, const ResArgs& r, const ResState& s, DT* depth, unsigned& my_n,
-                       unsigned long long& my_m) {
+__device__ void res_bu_words(const LevelArgs& a, const ResArgs& r, const ResState& s, const CrewSeat& seat, DT* depth,
+                             unsigned& my_n, unsigned long long& my_m) {
   const uint32_t* fbc = r.fb[s.f];
   uint32_t* fbn = r.fb[(s.f + 1) % 3];
   // read through L1: the barrier before this phase made it current
   const auto is_front = [&](int u) { return (__ldca(fbc + (u >> 5)) >> (u & 31)) & 1u; };
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int64_t gw = (int64_t)blockIdx.x * RW + warp, nw = (int64_t)gridDim.x * RW;
-  const int64_t W = (a.n_active + 31) >> 5;
+  const int gw = seat.rank * RW + warp, nw = seat.size * RW;
+  const int W = (int)((a.n_active + 31) >> 5);  // below 2^26: ids are int32
   // BW words at a time through every stage together: a CTA of 64-register
   // threads holds half the warps of k_expand, so each has to keep more reads in
   // flight.
-  for (int64_t w0 = gw; w0 < W; w0 += BW * nw) {
+  for (int w0 = gw; w0 < W; w0 += BW * nw) {
     uint32_t vis[BW], mask[BW];
     int4 ld[BW];
     int d[BW], id[BW];
@@ -359,7 +362,7 @@ __device__ void res_bu_words(const LevelArgs& a, const ResArgs& r, const ResStat
     bool found[BW];
 #pragma unroll
     for (int t = 0; t < BW; ++t) {
-      const int64_t wi = w0 + t * nw;
+      const int wi = w0 + t * nw;
       vis[t] = wi < W ? __ldcg(a.vis + wi) : 0u;
       mask[t] = wi < W ? a.active[wi] & ~vis[t] : 0u;
     }
@@ -369,10 +372,10 @@ __device__ void res_bu_words(const LevelArgs& a, const ResArgs& r, const ResStat
       d[t] = id[t] = 0;
       todo[t] = (mask[t] >> lane) & 1u;
       if (todo[t]) {
-        const int64_t v = (w0 + t * nw) * 32 + lane;
+        const int v = (w0 + t * nw) * 32 + lane;
         ld[t] = __ldcs(a.lead + v);
         d[t] = __ldcs(a.deg + v);
-        id[t] = a.perm ? __ldcs(a.perm + v) : (int)v;
+        id[t] = a.perm ? __ldcs(a.perm + v) : v;
       }
     }
 #pragma unroll
@@ -462,7 +465,7 @@ __device__ void res_bu_words(const LevelArgs& a, const ResArgs& r, const ResStat
         my_m += (unsigned)d[t];
       }
       const unsigned fm = __ballot_sync(FULL, found[t]);
-      const int64_t wi = w0 + t * nw;
+      const int wi = w0 + t * nw;
       if (lane == 0 && fm) {  // this warp is the only writer of word wi during the level
         a.vis[wi] = vis[t] | fm;
         fbn[wi] = fm;
@@ -477,16 +480,19 @@ __device__ void res_bu_words(const LevelArgs& a, const ResArgs& r, const ResStat
 // 100, of 29 184, 180, 172; R-MAT s16 66.6, 65.6, 63.5; ER 2^22 d16 291, 283, 301;
 // ER 3M d6 305, 303, 323; R-MAT s22 155, 153, 153.
 template <class DT>
-__device__ void res_bu(const LevelArgs& a, const ResArgs& r, const ResState& s, DT* depth, unsigned& my_n,
-                       unsigned long long& my_m) {
-  if ((a.n_active + 31) >> 5 <= (int64_t)gridDim.x * RW * R_BW_WORDS) res_bu_words<DT, 2, 4>(a, r, s, depth, my_n, my_m);
-  else res_bu_words<DT, 3, 3>(a, r, s, depth, my_n, my_m);
+__device__ void res_bu(const LevelArgs& a, const ResArgs& r, const ResState& s, const CrewSeat& seat, DT* depth,
+                       unsigned& my_n, unsigned long long& my_m) {
+  if ((a.n_active + 31) >> 5 <= (int64_t)seat.size * RW * R_BW_WORDS)
+    res_bu_words<DT, 2, 4>(a, r, s, seat, depth, my_n, my_m);
+  else
+    res_bu_words<DT, 3, 3>(a, r, s, seat, depth, my_n, my_m);
 }
 
 // Queues the frontier in fb[s.f], left by a bottom-up level (vertices with rows).
-__device__ void res_queue(const LevelArgs& a, const ResArgs& r, const ResState& s, const ResOut& o) {
+__device__ void res_queue(const LevelArgs& a, const ResArgs& r, const ResState& s, const CrewSeat& seat,
+                          const ResOut& o) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int64_t gw = (int64_t)blockIdx.x * RW + warp, nw = (int64_t)gridDim.x * RW;
+  const int64_t gw = (int64_t)seat.rank * RW + warp, nw = (int64_t)seat.size * RW;
   const int64_t W = (a.n_active + 31) >> 5;
   for (int64_t w0 = gw * 32; w0 < W; w0 += nw * 32) {
     uint32_t bits = w0 + lane < W ? __ldcg(r.fb[s.f] + w0 + lane) : 0u;
@@ -499,7 +505,7 @@ __device__ void res_queue(const LevelArgs& a, const ResArgs& r, const ResState& 
   }
 }
 
-// CTA 0 alone: top-down levels while the frontier is light and small, at most
+// The leader alone: top-down levels while the frontier is light and small, at most
 // R_SOLO_LEVELS and no further than the direction rule allows; leaves the next
 // frontier queued, its bits set in fbn, its counts in `n` and the totals in so.
 template <class DT, class Solo>
@@ -595,27 +601,62 @@ enum { RP_ALL, RP_HEAD, RP_TAIL };  // the part of the traversal a launch runs
 // or four such levels, and one that is not needed costs 6 us.
 constexpr int R_BU_LEVELS = 4;
 
+// The row entries, about, of a phase to come.
+__device__ __forceinline__ int64_t res_work(const LevelArgs& a, const ResState& s, int kind) {
+  switch (kind) {
+    case RK_TD: return s.m_f;
+    case RK_BU: return 2 * (a.n_active - s.n_vis);
+    case RK_QUEUE: return a.n_active / 16;
+    default: return 0;
+  }
+}
+
+// A small crew waits for more members before a long phase.
+__device__ __forceinline__ void res_gather(const LevelArgs& a, ResState& s, const CrewSeat& seat, int part) {
+  if ((part == RP_HEAD && s.kind == RK_BU) || s.kind == RK_DONE || !crew_short(seat, res_work(a, s, s.kind))) return;
+  s.then = s.kind;
+  s.kind = RK_GATHER;
+}
+
+// The traversal's end, for the host (one thread).
+__device__ void res_finish(const LevelArgs& a, const ResState& s, int32_t src, int part) {
+  BfsCtl* k = a.ctl;
+  k->src = src;
+  k->level = s.L;
+  k->done = 1;
+  k->err = s.err;
+  k->td_levels = s.td_levels;
+  k->bu_levels = s.bu_levels;
+  k->narrow_levels = s.narrow_levels;
+  k->mid_levels = s.mid_levels;
+  k->iters = 0;
+  k->narrow_calls = 0;
+  k->split_launches = part == RP_TAIL ? R_BU_LEVELS + 1 : 0;
+  k->n_vis = s.n_vis;
+  k->m_vis = s.m_vis;
+  k->m_f = s.m_f;
+}
+
 template <class DT>
 __global__ void __launch_bounds__(RT, 1) k_resident(LevelArgs a, ResArgs r, int32_t src, DT* depth, int part) {
   extern __shared__ int4 s_dyn[];
   int4(*s_q)[R_SOLO_CAP] = reinterpret_cast<int4(*)[R_SOLO_CAP]>(s_dyn);
   __shared__ ResState s_st;
+  __shared__ CrewSeat s_seat;
   __shared__ unsigned long long s_red[2];
   ResCtl* c = r.rc;
-  const int64_t tid = blockIdx.x * (int64_t)RT + threadIdx.x, nth = (int64_t)gridDim.x * RT;
+  Crew<ResState>* crew = &c->crew[part == RP_TAIL];
   const int64_t W = (a.V + 31) >> 5;
-  uint32_t* arrived = &c->arrived[part == RP_TAIL];
-  uint32_t target = 0;
   if (threadIdx.x == 0) s_red[0] = s_red[1] = 0;
-  if (part == RP_TAIL) {
-    if (c->err) return;  // the head's error status stands
-    if (threadIdx.x == 0) s_st = c->state;
-    __syncthreads();
-  } else {
-    // Until its end says otherwise the traversal has failed: whichever wait runs
-    // out, and whichever CTAs notice, the host does not read the last one's status.
-    if (tid == 0) a.ctl->err = 2;
-    const int32_t isrc = a.inv ? __ldg(a.inv + src) : src;
+  if (part == RP_TAIL && c->err) return;  // the head's error status stands
+  if (part == RP_TAIL && c->state.kind == RK_DONE) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) res_finish(a, c->state, src, part);
+    return;
+  }
+  const int32_t isrc = part == RP_TAIL ? 0 : (a.inv ? __ldg(a.inv + src) : src);
+  // one CTA's share of the fills
+  const auto fill = [&](uint32_t share) {
+    const int64_t tid = (int64_t)share * RT + threadIdx.x, nth = (int64_t)gridDim.x * RT;
     fill_unreached(depth, a.V, tid, nth, src);
     for (int64_t i = tid; i < W; i += nth) {
       const uint32_t x = i == (isrc >> 5) ? 1u << (isrc & 31) : 0u;
@@ -624,36 +665,73 @@ __global__ void __launch_bounds__(RT, 1) k_resident(LevelArgs a, ResArgs r, int3
       r.fb[1][i] = 0;
       r.fb[2][i] = 0;
     }
-    if (threadIdx.x == 0) {
-      const int d = a.deg[isrc];
+  };
+  // what a founder does before the first phase, of which it knows the state
+  const auto begin = [&](uint32_t rank) {
+    if (threadIdx.x == 32) {
       ResState s;
-      s.L = s.f = s.p = 0;
-      s.td_levels = s.bu_levels = s.narrow_levels = s.mid_levels = s.err = 0;
-      s.n_f = s.n_vis = 1;
-      s.m_f = s.m_vis = d;
-      s.n_l = d < R_HEAVY;
-      s.n_g = d >= R_HUGE;
-      s.n_h = 1 - s.n_l - s.n_g;
-      s.kind = a.policy == ENT_POLICY_BU_ONLY ? RK_BU : res_td_kind(a, s);
+      if (part == RP_TAIL) {
+        s = c->state;
+      } else {
+        const int d = a.deg[isrc];
+        s.L = s.f = s.p = s.then = 0;
+        s.td_levels = s.bu_levels = s.narrow_levels = s.mid_levels = s.err = 0;
+        s.n_f = s.n_vis = 1;
+        s.m_f = s.m_vis = d;
+        s.n_l = d < R_HEAVY;
+        s.n_g = d >= R_HUGE;
+        s.n_h = 1 - s.n_l - s.n_g;
+        s.kind = a.policy == ENT_POLICY_BU_ONLY ? RK_BU : res_td_kind(a, s);
+        if (rank == 0) {
+          if (s.n_l) r.queue[0][0] = isrc;
+          else if (s.n_h) r.queue[0][a.V - 1] = isrc;
+          else r.huge[0][0] = isrc;
+          // Until its end says otherwise the traversal has failed: whichever wait
+          // runs out, and whichever CTAs notice, the host does not read the last
+          // one's status.
+          a.ctl->err = 2;
+        }
+      }
       s_st = s;
-      if (blockIdx.x == 0) {
-        if (s.n_l) r.queue[0][0] = isrc;
-        else if (s.n_h) r.queue[0][a.V - 1] = isrc;
-        else r.huge[0][0] = isrc;
+    }
+    if (part != RP_TAIL) fill(rank);
+  };
+  // what every member concludes from an opened barrier
+  const auto advance = [&] {
+    ResState& s = s_st;
+    if (s.kind >= RK_GATHER) {
+      s.p += 1;
+      s.kind = s.then;
+      return;
+    }
+    res_advance(a, r, s);
+    if (s_seat.size < gridDim.x) res_gather(a, s, s_seat, part);
+  };
+  const int in = crew_join(crew, &c->err, s_seat, s_st, begin, advance);
+  if (!in) return;
+  const int rank = s_seat.rank;
+  if (in == 1 && s_seat.size < gridDim.x) {  // a small crew
+    if (threadIdx.x == 0) {
+      ResState& s = s_st;
+      if (part == RP_TAIL) {
+        res_gather(a, s, s_seat, part);
+      } else {  // some shares are nobody's
+        s.then = s.kind;
+        s.kind = RK_FILL;
       }
     }
-    // test hook: a CTA that never arrives (the others' waits run out)
-    if (a.fault_inject && part == RP_ALL && blockIdx.x == gridDim.x - 1) return;
-    if (!grid_barrier(arrived, &c->err, target += gridDim.x, [] {})) return;
+    __syncthreads();
   }
   for (;;) {
     const ResState& s = s_st;  // thread 0 changes it inside the barrier only
     if (s.kind == RK_DONE || (part == RP_HEAD && s.kind == RK_BU)) break;
+    const CrewSeat seat = s_seat;
+    const int64_t tid = (int64_t)rank * RT + threadIdx.x, nth = (int64_t)seat.size * RT;
     int32_t* n_next = c->n[(s.p + 1) % 3];
     unsigned long long* acc = c->acc[(s.p + 1) % 3];
     if (tid < 3) c->n[(s.p + 2) % 3][tid] = 0;
     if (tid < 2) c->acc[(s.p + 2) % 3][tid] = 0;
-    if (s.kind != RK_QUEUE) {  // the bits of the frontier before this one
+    if (s.kind != RK_QUEUE && s.kind < RK_DONE) {  // the bits of the frontier before this one
       uint32_t* old = r.fb[(s.f + 2) % 3];
       for (int64_t i = tid; i < W; i += nth) old[i] = 0;
     }
@@ -662,10 +740,13 @@ __global__ void __launch_bounds__(RT, 1) k_resident(LevelArgs a, ResArgs r, int3
     uint32_t* fbn = r.fb[(s.f + 1) % 3];
     const int nq = s.kind == RK_QUEUE ? s.L & 1 : (s.L + 1) & 1;
     const ResOut o{fbn, r.queue[nq], r.huge[nq], n_next, nullptr};
-    if (s.kind == RK_TD) res_td(a, r, s, depth, o, my_n, my_m);
-    else if (s.kind == RK_BU) res_bu(a, r, s, depth, my_n, my_m);
-    else if (s.kind == RK_QUEUE) res_queue(a, r, s, o);
-    else if (blockIdx.x == 0) res_solo(a, r, s, depth, fbn, n_next, &c->solo[s.p & 1], s_q);
+    if (s.kind == RK_TD) res_td(a, r, s, seat, depth, o, my_n, my_m);
+    else if (s.kind == RK_BU) res_bu(a, r, s, seat, depth, my_n, my_m);
+    else if (s.kind == RK_QUEUE) res_queue(a, r, s, seat, o);
+    else if (s.kind == RK_GATHER) crew_gather(crew, seat, res_work(a, s, s.then));
+    else if (s.kind == RK_FILL)
+      for (uint32_t i = s_seat.size + rank; i < gridDim.x; i += s_seat.size) fill(i);
+    else if (rank == 0) res_solo(a, r, s, depth, fbn, n_next, &c->solo[s.p & 1], s_q);
     if (s.kind <= RK_BU) {
       const unsigned wn = __reduce_add_sync(FULL, my_n);
       if (wn) {
@@ -683,29 +764,19 @@ __global__ void __launch_bounds__(RT, 1) k_resident(LevelArgs a, ResArgs r, int3
         s_red[0] = s_red[1] = 0;
       }
     }
-    if (!grid_barrier(arrived, &c->err, target += gridDim.x, [&] { res_advance(a, r, s_st); })) return;
+    // test hook: a CTA that never arrives (the others' waits run out)
+    if (a.fault_inject && part == RP_ALL && rank > 0 && rank == (int)s_seat.size - 1) return;
+    if (!crew_barrier(crew, &c->err, s_seat, s_st, advance)) {
+      crew_close(crew, s_seat);
+      return;
+    }
   }
+  crew_close(crew, s_seat);
+  const int64_t tid = (int64_t)rank * RT + threadIdx.x;
   // test hook: a CTA that gave up just as the head's last barrier opened for the others
-  if (a.fault_inject && part == RP_HEAD && threadIdx.x == 0 && blockIdx.x == gridDim.x - 1) c->err = 1;
+  if (a.fault_inject && part == RP_HEAD && threadIdx.x == 0 && rank == (int)s_seat.size - 1) c->err = 1;
   if (tid == 0 && part == RP_HEAD) c->state = s_st;
-  if (tid == 0 && part != RP_HEAD) {
-    const ResState& s = s_st;
-    BfsCtl* k = a.ctl;
-    k->src = src;
-    k->level = s.L;
-    k->done = 1;
-    k->err = s.err;
-    k->td_levels = s.td_levels;
-    k->bu_levels = s.bu_levels;
-    k->narrow_levels = s.narrow_levels;
-    k->mid_levels = s.mid_levels;
-    k->iters = 0;
-    k->narrow_calls = 0;
-    k->split_launches = part == RP_TAIL ? R_BU_LEVELS + 1 : 0;
-    k->n_vis = s.n_vis;
-    k->m_vis = s.m_vis;
-    k->m_f = s.m_f;
-  }
+  if (tid == 0 && part != RP_HEAD) res_finish(a, s_st, src, part);
 }
 
 // One bottom-up level of a traversal in parts, if that is what comes next:

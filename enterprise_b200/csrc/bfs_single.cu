@@ -47,7 +47,7 @@
 //    each queue entry carries the vertex's row start and degree, read while
 //    its visit was being claimed, so a level costs one adjacency read, one
 //    status probe and one claim on its critical path.
-//  * Unless the graph is road-like or parents are asked for, a cooperative
+//  * Unless the graph is road-like or deep, or parents are asked for, a resident
 //    kernel goes from level to level instead (bfs_resident.cuh); what follows
 //    is the rest.
 //  * The whole traversal is one CUDA graph: a reset kernel (which also writes
@@ -1506,8 +1506,8 @@ constexpr size_t RES_SMEM = 2 * R_SOLO_CAP * sizeof(int4);
 // kernel or in parts, instead of the CUDA graph of level kernels. Measured,
 // level kernels -> resident, ms: R-MAT s16 0.146 -> 0.068, s20 0.158 -> 0.089,
 // s22 0.235 -> 0.150, s23 0.272 -> 0.205, s24 0.340 -> 0.310; ER 2^22 d16 0.41 ->
-// 0.285, 2^24 d32 1.89 -> 1.69. In parts from 2^22 vertices on (one kernel
-// there: R-MAT s22 0.150, in parts 0.161; s24 0.345 and 0.310). Graphs of low
+// 0.285, 2^24 d32 1.89 -> 1.69. In parts above 2^22 vertices (R-MAT s22 as one
+// kernel 0.150, in parts 0.161; s24 0.345 and 0.310). Graphs of low
 // mean degree (grids, roads) are deep, and their levels belong in the cluster of
 // k_narrow: a 300^2 grid 1.5 -> 2.1 ms, 1024^2 5.4 -> 13 ms.
 constexpr int64_t RES_SPLIT_V = 1 << 22;
@@ -1537,29 +1537,18 @@ static bool resident_fits(const ent_graph* g, const BfsWorkspace* w) {
 
 // The resident traversal on stream s (no parents): one kernel, or for large
 // graphs its level kernels between two.
-// ENT_ERR_UNSUPPORTED when the GPU cannot hold all its CTAs at once (part of
-// it set aside, by MPS or a partition): the level kernels take over.
 template <class DT>
 static int launch_resident(BfsWorkspace* w, int32_t src, DT* depth, cudaStream_t s, int32_t max_levels = 0) {
   LevelArgs a = w->args;
   if (max_levels > 0) a.max_levels = max_levels;
   a.use_cond = 0;
-  int part = w->split ? RP_HEAD : RP_ALL;
-  void* args[5] = {&a, &w->res, &src, &depth, &part};
   ENT_CUDA(cudaMemsetAsync(w->res.rc, 0, sizeof(ResCtl), s));
-  const cudaError_t e =
-      cudaLaunchCooperativeKernel((const void*)k_resident<DT>, dim3(w->grid_res), dim3(RT), args, RES_SMEM, s);
-  if (e == cudaErrorCooperativeLaunchTooLarge) {
-    cudaGetLastError();
-    w->res.rc = nullptr;
-    return ENT_ERR_UNSUPPORTED;
-  }
-  ENT_CUDA(e);
+  k_resident<DT><<<w->grid_res, RT, RES_SMEM, s>>>(a, w->res, src, depth, w->split ? RP_HEAD : RP_ALL);
+  ENT_CUDA(cudaGetLastError());
   if (!w->split) return ENT_OK;
   for (int i = 0; i < R_BU_LEVELS; ++i) k_res_bu_level<DT><<<w->grid_expand, BT, 0, s>>>(a, w->res, depth);
+  k_resident<DT><<<w->grid_res, RT, RES_SMEM, s>>>(a, w->res, src, depth, RP_TAIL);
   ENT_CUDA(cudaGetLastError());
-  part = RP_TAIL;
-  ENT_CUDA(cudaLaunchCooperativeKernel((const void*)k_resident<DT>, dim3(w->grid_res), dim3(RT), args, RES_SMEM, s));
   return ENT_OK;
 }
 
@@ -1575,7 +1564,7 @@ static void note_depth(ent_graph* g, const BfsCtl& h) {
 static int probe_depth(ent_graph* g, BfsWorkspace* w) {
   ENT_CUDA(cudaStreamWaitEvent(g->stream, w->ev_order, 0));
   const int rc = launch_resident<int32_t>(w, g->top, w->depth, g->stream, RES_PROBE);
-  if (rc != ENT_OK) return rc == ENT_ERR_UNSUPPORTED ? ENT_OK : rc;
+  if (rc != ENT_OK) return rc;
   ENT_CUDA(cudaMemcpyAsync(w->ctl_h, w->ctl, sizeof(BfsCtl), cudaMemcpyDeviceToHost, g->stream));
   ENT_CUDA(cudaStreamSynchronize(g->stream));
   g_kernel_launches += 1 + w->ctl_h->split_launches;
@@ -1691,7 +1680,7 @@ static int create_workspace(ent_graph* g, BfsWorkspace** out, bool force_graph =
     // small graphs: fewer CTAs, cheaper barriers, and room for other streams' work
     const int64_t want = std::max<int64_t>((V + 4 * RT - 1) / (4 * RT), g->E / (8 * RT));
     w->split = V > RES_SPLIT_V;
-    w->grid_res = (int)std::max<int64_t>(1, std::min<int64_t>(g->num_sms, want));
+    w->grid_res = (int)std::max<int64_t>(1, std::min<int64_t>(std::min(g->num_sms, CREW_MAX), want));
   }
   if (force_graph) {  // else built on first use
     int rcode = build_graph<int32_t>(g, w);
@@ -1774,10 +1763,8 @@ static int run_bfs_typed(ent_graph* g, int32_t src, DT* depth, int32_t* parent, 
       const int rcode = probe_depth(g, w);
       if (rcode != ENT_OK) return rcode;
     }
-    int rc = ENT_ERR_UNSUPPORTED;
     resident = w->res.rc && !parent && !captured && g->deep != 1;
-    if (resident) rc = launch_resident(w, src, depth, s);
-    if (rc == ENT_ERR_UNSUPPORTED) rc = launch_graph(g, w, src, depth, parent, s);
+    const int rc = resident ? launch_resident(w, src, depth, s) : launch_graph(g, w, src, depth, parent, s);
     if (rc != ENT_OK) return rc;
   } else {
     LevelArgs la = w->args;

@@ -46,37 +46,214 @@ __device__ __forceinline__ unsigned long long lb_flag(unsigned long long w, uint
 // tile is always held by a running CTA and publishes within microseconds.
 constexpr int SPIN_LIMIT = 1 << 20;
 
-// One CTA's arrival at a grid-wide barrier (cooperative launch: every CTA is
-// resident) and its wait for all: `target` is the number of arrivals, counted
-// over the whole launch, after which it opens. `after` runs on thread 0 once it
-// has opened, before the other threads go on. The wait is bounded (seconds; a
-// wait this long means a bug): false when one ran out anywhere, and every CTA
-// then leaves.
-template <class F>
-__device__ bool grid_barrier(uint32_t* arrived, int32_t* err, uint32_t target, F after) {
-  __shared__ int s_ok;
+// A crew: the CTAs of one ordinary launch that go from phase to phase of some
+// work together. A CTA takes part from the phase after the one in which it
+// started, and none is waited for that has not started. So the work begins as
+// soon as one SM is free and grows onto the others as they come free, where a
+// cooperative launch begins when all its CTAs fit at once. Beside a server with
+// eight deep queries in flight, whose clusters hold some SMs for milliseconds at a
+// time, an R-MAT s16 traversal took 5.7 ms when launched so and takes 81 us (66 on
+// an idle GPU), s24 7.0 and 0.49 ms, and the server kept a third of its queries
+// and keeps all. On an idle GPU the seats cost 1 to 3 us a traversal.
+//
+// Ranks are given in the order of starting. Rank 0 leads. It founds the crew with
+// those that have started within a moment, nearly always the whole grid; from then
+// on, before it arrives at the barrier that ends a phase, it admits those that
+// have started since and leaves them the phase's state. They wait for that
+// barrier too (without an arrival) and draw the same conclusions from it as
+// everyone. While the size is the whole grid none of this costs anything.
+//
+// State is what every member knows about the phase; its `p` counts phases. Posts
+// and sizes alternate between two places: the leader writes one again two
+// barriers later, and those who read it have arrived at the barrier between.
+constexpr int CREW_MAX = 256;  // CTAs of a launch at most
+constexpr uint32_t CREW_FOUNDED = 1u << 31;
+constexpr uint32_t CREW_DISMISSED = 1u << 30;  // more arrivals than any launch has
+template <class State>
+struct Crew {  // zeroed before the launch
+  unsigned long long arrived;  // arrivals, all barriers of the launch together; << 32: members of the first phase
+  uint32_t joined;    // CTAs that have started, and CREW_FOUNDED
+  uint32_t closed;    // the work is over: CTAs that have not been admitted leave
+  uint32_t size[2];   // members of a phase, by its parity
+  struct {
+    State state;
+    uint32_t target, size;
+  } post[2];
+  uint32_t when[CREW_MAX];  // by rank: 1 + the post it was admitted with, or 0
+};
+struct CrewSeat {  // one CTA's, in shared memory
+  uint32_t rank, size;  // of the phase that is running
+  uint32_t target;      // arrivals at which its barrier opens
+};
+
+__device__ __forceinline__ uint32_t ld_acquire32(const uint32_t* p) {
+  uint32_t x;
+  asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(x) : "l"(p) : "memory");
+  return x;
+}
+__device__ __forceinline__ void st_release32(uint32_t* p, uint32_t x) {
+  asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(x) : "memory");
+}
+
+// One thread's wait until test() holds, bounded (`limit` polls of half a
+// microsecond; one that runs out means a bug): false when it ran out here, or
+// when *err says that another did.
+template <class Test>
+__device__ __forceinline__ bool crew_wait(int32_t* err, int limit, Test test) {
+  for (int spins = 0;; ++spins) {
+    if (test()) return true;
+    if (spins > 64) __nanosleep(64);
+    if (spins >= limit || ((spins & 63) == 63 && *(volatile int32_t*)err)) {
+      *(volatile int32_t*)err = 1;
+      return false;
+    }
+  }
+}
+
+// Thread 0, once a phase's barrier has opened: the next phase's size and target
+// (s.p still counts the one that ended).
+template <class State>
+__device__ __forceinline__ void crew_next(Crew<State>* c, CrewSeat& seat, const State& s) {
+  if (seat.size < gridDim.x) seat.size = __ldcg(&c->size[(s.p + 1) & 1]);
+  seat.target += seat.size;
+}
+
+// Takes a seat: 0, there is nothing left to do; 1, a founder, whose own share
+// begin(rank) of what comes before the first phase is done and visible, like that
+// of the other founders (ranks from seat.size on have had none); 2, a member of
+// the phase that begins, its state in s. advance(): thread 0's conclusions from an
+// opened barrier, s.p included.
+template <class State, class Begin, class F>
+__device__ int crew_join(Crew<State>* c, int32_t* err, CrewSeat& seat, State& s, Begin begin, F advance) {
+  __shared__ int s_in;
+  if (threadIdx.x == 0) {
+    const uint32_t ticket = atomicAdd(&c->joined, 1u);
+    seat.rank = ticket & ~CREW_FOUNDED;
+    s_in = ticket & CREW_FOUNDED ? 2 : 1;
+    if (ticket == gridDim.x - 1) atomicAdd(&c->arrived, (unsigned long long)gridDim.x << 32);  // all are there
+  }
   __syncthreads();
+  const uint32_t rank = seat.rank;
+  if (s_in == 1) {
+    begin(rank);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      __threadfence();
+      atomicAdd(&c->arrived, 1ull);
+      uint32_t n = 0;  // founders, once known
+      const auto all = [&] {
+        const unsigned long long now = ld_acquire(&c->arrived);
+        n = (uint32_t)(now >> 32);
+        return n != 0 && (uint32_t)now >= n;
+      };
+      if (rank == 0) {  // the CTAs of an idle GPU start within a microsecond or two
+        for (const long long t0 = clock64(); !all() && clock64() - t0 < 4096;) {
+        }
+        if (n == 0) {
+          const uint32_t there = atomicOr(&c->joined, CREW_FOUNDED);
+          if (there < gridDim.x) atomicAdd(&c->arrived, (unsigned long long)there << 32);
+        }
+      }
+      const bool ok = crew_wait(err, SPIN_LIMIT * 4, all);
+      __threadfence();
+      seat.size = n;
+      seat.target = 2 * n;
+      s_in = ok;
+    }
+  } else if (threadIdx.x == 0) {
+    uint32_t w = 0;
+    // as long as a phase of the others lasts, and they may still be few
+    bool in = crew_wait(err, SPIN_LIMIT * 64, [&] {
+      w = ld_acquire32(&c->when[rank]);
+      return w != 0 || ld_acquire32(&c->closed) != 0;
+    });
+    in = in && w != 0;
+    if (in) {
+      const auto& post = c->post[w - 1];
+      s = post.state;
+      seat.target = post.target;
+      in = crew_wait(err, SPIN_LIMIT * 4, [&] { return (uint32_t)ld_acquire(&c->arrived) >= seat.target; });
+      __threadfence();
+      seat.size = post.size;
+      seat.target += seat.size;
+      if (in) advance();
+    }
+    s_in = in ? 2 : 0;
+  }
+  __syncthreads();
+  return s_in;
+}
+
+// Ends a phase: every member's work of it is visible to all, and thread 0 has
+// run advance(). False when a wait ran out anywhere, or when the leader dismissed
+// the others; the CTA then leaves.
+template <class State, class F>
+__device__ bool crew_barrier(Crew<State>* c, int32_t* err, CrewSeat& seat, const State& s, F advance) {
+  __shared__ int s_ok;
+  __shared__ uint32_t s_joined;
+  __syncthreads();
+  if (seat.rank == 0 && seat.size < gridDim.x) {
+    if (threadIdx.x == 0) {
+      s_joined = *(volatile uint32_t*)&c->joined & ~CREW_FOUNDED;
+      auto& post = c->post[s.p & 1];
+      post.state = s;
+      post.target = seat.target;
+      post.size = s_joined;
+      c->size[(s.p + 1) & 1] = s_joined;
+      __threadfence();
+    }
+    __syncthreads();
+    for (uint32_t r = seat.size + threadIdx.x; r < s_joined; r += blockDim.x)
+      st_release32(&c->when[r], 1 + (s.p & 1));
+  }
   if (threadIdx.x == 0) {
     __threadfence();
-    atomicAdd(arrived, 1u);
-    int ok = 1;
-    for (int spins = 0;; ++spins) {
-      uint32_t x;
-      asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(x) : "l"(arrived) : "memory");
-      if (x >= target) break;
-      if (spins > 64) __nanosleep(64);
-      if (spins >= SPIN_LIMIT * 4 || ((spins & 63) == 63 && *(volatile int32_t*)err)) {
-        *(volatile int32_t*)err = 1;
-        ok = 0;
-        break;
-      }
-    }
+    atomicAdd(&c->arrived, 1ull);
+    const uint32_t target = seat.target;
+    uint32_t now = 0;
+    bool ok = crew_wait(err, SPIN_LIMIT * 4, [&] {
+      now = (uint32_t)ld_acquire(&c->arrived);
+      return now >= target;
+    });
     __threadfence();
+    ok = ok && now < CREW_DISMISSED;
     s_ok = ok;
-    if (ok) after();
+    if (ok) {
+      crew_next(c, seat, s);
+      advance();
+    }
   }
   __syncthreads();
   return s_ok != 0;
+}
+
+// Whether a phase of `work` row entries is worth waiting for more members (a CTA
+// walks about one entry a nanosecond): a phase of its own then, in which the
+// leader waits for them, up to a quarter of what they would save.
+__device__ __forceinline__ bool crew_short(const CrewSeat& seat, int64_t work) {
+  return work / seat.size - work / gridDim.x > 4096;
+}
+template <class State>
+__device__ void crew_gather(Crew<State>* c, const CrewSeat& seat, int64_t work) {
+  if (seat.rank != 0 || threadIdx.x != 0) return;
+  const int64_t limit = min((work / seat.size - work / gridDim.x) / 2, (int64_t)1 << 30);  // cycles, two a nanosecond
+  for (const long long t0 = clock64(); clock64() - t0 < limit && (*(volatile uint32_t*)&c->joined & ~CREW_FOUNDED) < gridDim.x;)
+    __nanosleep(100);
+}
+
+// Sends every other member away, from the barrier of the running phase: their SMs
+// are free for other work while the leader goes on alone (its thread 0 calls
+// this). It meets nobody at a barrier again.
+template <class State>
+__device__ __forceinline__ void crew_dismiss(Crew<State>* c) {
+  st_release32(&c->closed, 1u);
+  atomicAdd(&c->arrived, (unsigned long long)CREW_DISMISSED);
+}
+
+// The leader's last word, whichever way it leaves.
+template <class State>
+__device__ __forceinline__ void crew_close(Crew<State>* c, const CrewSeat& seat) {
+  if (seat.rank == 0 && threadIdx.x == 0) st_release32(&c->closed, 1u);
 }
 
 // Inclusive warp scan of K lanes' values (each lane holds v[k]).

@@ -65,7 +65,9 @@ enum ent_loop {
                          a CUDA graph with a device-side while node, or,
                          without parents and on graphs of mean degree 5 and
                          more whose levels do not prove many and small,
-                         cooperative kernels of many levels each            */
+                         kernels of many levels each, whose blocks hold the
+                         SMs they were given until the traversal ends (they
+                         take those that are free, and wait for none)       */
   ENT_LOOP_HOST = 1   /* host launches each level and polls a flag     */
 };
 
@@ -99,7 +101,7 @@ typedef struct ent_bfs_opts {
   int32_t narrow_cluster;  /* CTAs in the cluster (1..16), 0 = largest that fits */
   int32_t fault_inject;    /* test hook, 0 in use. 1: the first tile of each frontier
                               classification never publishes its prefix, and a
-                              block of a cooperative kernel leaves early, so
+                              block of a resident kernel leaves early, so
                               those that wait for it run out their bounded spin
                               (seconds) and the traversal returns
                               ENT_ERR_TIMEOUT with the context still usable */
@@ -299,7 +301,10 @@ int ent_bfs_trace(ent_graph* g, int32_t src, ent_level_trace* out, int32_t max_l
  * driver-API plug-in) gets one more lookup, once, in that context.
  * All calls share the array: calls whose work overlaps on one GPU race and
  * give wrong results, so serialise them. Synchronous on `stream` (NULL = the
- * default stream). */
+ * default stream). One kernel runs the traversal, on the SMs that are free when
+ * it starts and those that come free; it waits for none. Each of its blocks (up
+ * to one per SM) holds its SM while the frontier is large or has been so within
+ * the last 64 levels; longer runs of small levels keep one SM. */
 #define ENT_NOALLOC_MAX_VERTICES (1 << 20)
 int ent_bfs_noalloc(const int64_t* beg_pos_dev, const int32_t* csr_dev, int64_t vert_count,
                     int32_t src, int32_t* depth_dev, void* stream);
