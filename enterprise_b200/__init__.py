@@ -209,6 +209,7 @@ def lib() -> C.CDLL:
         "ent_graph_device_bytes": (C.c_int64, [_P]),
         "ent_device_alloc": (C.c_int, [C.c_int32, C.c_size_t, C.POINTER(_P)]),
         "ent_device_free": (C.c_int, [_P]),
+        "ent_release_memory": (C.c_int, [C.c_int32]),
         "ent_graph_from_edges": (C.c_int, [_I64P, _I64P, C.c_int64, C.c_int64, C.c_int32, C.POINTER(_P)]),
         "ent_graph_load": (C.c_int, [C.c_char_p, C.c_char_p, C.c_int32, C.POINTER(_P)]),
         "ent_graph_download": (C.c_int, [_P, _I64P, _I32P]),
@@ -276,6 +277,12 @@ def _i64p(a: np.ndarray):
 def kernel_launch_count() -> int:
     """Kernels launched by the native library in this process."""
     return int(lib().ent_kernel_launch_count())
+
+
+def release_memory(gpu: int = 0) -> None:
+    """Gives the device memory that the library keeps for its next allocations
+    (at most 512 MB) back to the GPU."""
+    _check(lib().ent_release_memory(gpu))
 
 
 def host_register(arr: np.ndarray) -> None:

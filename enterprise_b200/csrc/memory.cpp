@@ -6,7 +6,8 @@
 // dev_alloc takes memory from a pool of the library's own that keeps up to
 // POOL_KEEP bytes of what was given back for the next allocation. Whatever is
 // above goes back to the device at once, and all of it when an allocation of
-// this library fails. Blocks of POOL_MAX and more bypass it.
+// this library fails or ent_release_memory is called. Blocks of POOL_MAX and more
+// bypass it.
 //
 // A copy between the device and pageable host memory runs through the driver's
 // own staging on one host thread (about 10 GB/s, first touch of fresh pages
@@ -41,7 +42,7 @@ struct DevicePool {
 };
 std::mutex g_mu;
 std::vector<DevicePool> g_pools;      // by device
-std::vector<void*> g_large;           // blocks that did
+std::vector<void*> g_large;           // blocks that bypassed the pools
 std::vector<char*> g_idle;            // page-locked pairs of chunks not in use
 int g_pairs = 0;                      // ... and all of them
 constexpr int MAX_PAIRS = 2;          // 16 MB; further copies at the same time go to the driver
@@ -279,3 +280,18 @@ cudaError_t to_host(void* dst, const void* src, size_t bytes, cudaStream_t s) {
 }
 
 }  // namespace ent
+
+extern "C" int ent_release_memory(int32_t gpu) {
+  using namespace ent;
+  clear_error();
+  int n = 0;
+  if (cudaGetDeviceCount(&n) != cudaSuccess || gpu < 0 || gpu >= n)
+    return fail(ENT_ERR_INVALID_ARG, "no GPU %d (%d present)", gpu, n);
+  cudaMemPool_t pool = nullptr;
+  {
+    std::lock_guard<std::mutex> lk(g_mu);
+    if ((size_t)gpu < g_pools.size()) pool = g_pools[gpu].pool;
+  }
+  if (pool) ENT_CUDA(cudaMemPoolTrimTo(pool, 0));
+  return ENT_OK;
+}
