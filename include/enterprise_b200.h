@@ -226,9 +226,9 @@ int64_t ent_graph_device_bytes(const ent_graph* g);
 int ent_device_alloc(int32_t gpu, size_t bytes, void** out);
 int ent_device_free(void* ptr);
 /* The library keeps up to 512 MB per GPU of device memory that destroyed graphs
- * and finished calls gave back, for the next ones, and gives all of it back to
- * the GPU when an allocation of its own would fail. For other allocators of the
- * process: this call gives it back at once. */
+ * and finished calls gave back, for the next ones. An allocation of this process
+ * that finds too little free memory gets it (the driver takes it out of the
+ * pool); for other processes this call gives it back at once. */
 int ent_release_memory(int32_t gpu);
 /* Copies the device CSR to caller host arrays (V+1 and E entries). */
 int ent_graph_download(const ent_graph* g, int64_t* beg_pos, int32_t* csr);

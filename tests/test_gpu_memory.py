@@ -33,3 +33,19 @@ def test_release_memory(eb):
     for gpu in (-1, 1000):
         with pytest.raises(eb.EntError):
             eb.release_memory(gpu)
+
+
+def test_other_allocators_get_what_is_kept(eb):
+    import torch
+    eb.release_memory()
+    _fill_the_pool(eb)
+    held = []
+    try:
+        while _free() > 170 * MB:
+            held.append(torch.empty(min(_free() - 160 * MB, 16 << 30), dtype=torch.uint8, device="cuda"))
+        held.append(torch.empty(300 * MB, dtype=torch.uint8, device="cuda"))
+    finally:
+        held.clear()
+        torch.cuda.empty_cache()
+    with eb.Graph.rmat(12, 16, seed=1) as g:
+        assert g.bfs(0)[2].status == 0
