@@ -32,8 +32,13 @@
 // needed leave at once; the last CTA of each takes the decision), and a tail
 // for whatever is left.
 //
-// Not here: parents, hub tables, runs with the small-frontier mode off and graphs
-// of many small levels (meshes, bands) stay with the level kernels.
+// With parents (PAR) a claim also stores the caller's id of the vertex in whose row
+// it was found, and a bottom-up find its neighbour's: instantiations of their own,
+// so that traversals without them keep their registers.
+//
+// Not here: hub tables, runs with the small-frontier mode off, parents of small
+// graphs, and graphs of many small levels (meshes, bands) stay with the level
+// kernels.
 #pragma once
 
 constexpr int RT = 1024;          // threads per CTA, one per SM (64 registers a thread)
@@ -82,6 +87,7 @@ struct ResArgs {
   uint32_t* fb[3];
   int32_t* queue[2];  // light vertices from the front, heavy ones from the back (V entries)
   int32_t* huge[2];
+  int32_t* parent;    // PAR
 };
 
 __device__ __forceinline__ int64_t ldcg64(const void* p) {
@@ -167,6 +173,7 @@ struct ResOut {
   int32_t* huge;
   int32_t* n;        // counts: global, or the leader's own in shared memory
   int4* s_q;         // the leader alone: entries in shared memory while they fit
+  int32_t* parent;   // PAR
 };
 
 // Where vertices queue by degree: 0 light, 1 heavy, 2 huge.
@@ -207,9 +214,10 @@ __device__ __forceinline__ void res_queue_up(const LevelArgs& a, const ResOut& o
     }
 }
 
-template <class DT, bool SOLO>
-__device__ __forceinline__ void res_claim(const LevelArgs& a, const int (&v)[R_ILP], int ln, DT* depth, const ResOut& o,
-                                          unsigned& my_n, unsigned long long& my_m) {
+// from (PAR): the caller's id of the vertex in whose row each v was found.
+template <class DT, bool SOLO, bool PAR>
+__device__ __forceinline__ void res_claim(const LevelArgs& a, const int (&v)[R_ILP], const int (&from)[R_ILP], int ln,
+                                          DT* depth, const ResOut& o, unsigned& my_n, unsigned long long& my_m) {
   bool open[R_ILP], mine[R_ILP];
   int64_t st[R_ILP];
   int d[R_ILP], id[R_ILP];
@@ -227,8 +235,8 @@ __device__ __forceinline__ void res_claim(const LevelArgs& a, const int (&v)[R_I
         d[i] = (int)(__ldg(a.off + v[i] + 1) - st[i]);
       } else {
         d[i] = __ldg(a.deg + v[i]);
-        id[i] = out_id(a, v[i]);
       }
+      if (!SOLO || PAR) id[i] = out_id(a, v[i]);
       const uint32_t b = 1u << (v[i] & 31);
       mine[i] = !(atomicOr(a.vis + (v[i] >> 5), b) & b);
     }
@@ -242,6 +250,7 @@ __device__ __forceinline__ void res_claim(const LevelArgs& a, const int (&v)[R_I
         depth[id[i]] = (DT)ln;
         red_or(o.fb + (v[i] >> 5), 1u << (v[i] & 31));
       }
+      if (PAR) o.parent[id[i]] = from[i];
       my_n += 1;
       my_m += (unsigned)d[i];
     }
@@ -254,10 +263,11 @@ __device__ __forceinline__ void res_claim(const LevelArgs& a, const int (&v)[R_I
   });
 }
 
-// The concatenated rows of a warp's light vertices (lane: d entries from st).
-template <class DT, bool SOLO>
-__device__ __forceinline__ void res_rows(const LevelArgs& a, int d, int64_t st, int ln, DT* depth, const ResOut& o,
-                                         unsigned& my_n, unsigned long long& my_m) {
+// The concatenated rows of a warp's light vertices (lane: d entries from st, of
+// the vertex with the caller's id `own`).
+template <class DT, bool SOLO, bool PAR>
+__device__ __forceinline__ void res_rows(const LevelArgs& a, int d, int64_t st, int own, int ln, DT* depth,
+                                         const ResOut& o, unsigned& my_n, unsigned long long& my_m) {
   const int lane = threadIdx.x & 31;
   int incl = d;
 #pragma unroll
@@ -267,10 +277,10 @@ __device__ __forceinline__ void res_rows(const LevelArgs& a, int d, int64_t st, 
   }
   const int total = __shfl_sync(FULL, incl, 31), excl = incl - d;
   for (int r0 = 0; r0 < total; r0 += 32 * R_ILP) {
-    int v[R_ILP];
+    int v[R_ILP], from[R_ILP];
 #pragma unroll
     for (int i = 0; i < R_ILP; ++i) {
-      v[i] = -1;
+      v[i] = from[i] = -1;
       if (r0 + 32 * i < total) {  // warp-uniform
         const int k = r0 + 32 * i + lane;
         int j = 0;
@@ -281,30 +291,33 @@ __device__ __forceinline__ void res_rows(const LevelArgs& a, int d, int64_t st, 
         }
         const int64_t sj = __shfl_sync(FULL, st, j);
         const int ej = __shfl_sync(FULL, excl, j);
+        if (PAR) from[i] = __shfl_sync(FULL, own, j);
         if (k < total) v[i] = __ldg(a.adj + sj + (k - ej));
       }
     }
-    res_claim<DT, SOLO>(a, v, ln, depth, o, my_n, my_m);
+    res_claim<DT, SOLO, PAR>(a, v, from, ln, depth, o, my_n, my_m);
   }
 }
 
 // Entries first, first + step, ... of one long row, 32 * R_ILP per warp and turn.
-template <class DT>
-__device__ __forceinline__ void res_slice(const LevelArgs& a, int64_t first, int64_t step, int64_t end, int ln,
-                                          DT* depth, const ResOut& o, unsigned& my_n, unsigned long long& my_m) {
+template <class DT, bool PAR>
+__device__ __forceinline__ void res_slice(const LevelArgs& a, int64_t first, int64_t step, int64_t end, int own,
+                                          int ln, DT* depth, const ResOut& o, unsigned& my_n,
+                                          unsigned long long& my_m) {
   const int lane = threadIdx.x & 31;
   for (int64_t e0 = first; e0 < end; e0 += step) {
-    int v[R_ILP];
+    int v[R_ILP], from[R_ILP];
 #pragma unroll
     for (int i = 0; i < R_ILP; ++i) {
       const int64_t e = e0 + 32 * i + lane;
       v[i] = e < end ? __ldg(a.adj + e) : -1;
+      from[i] = own;
     }
-    res_claim<DT, false>(a, v, ln, depth, o, my_n, my_m);
+    res_claim<DT, false, PAR>(a, v, from, ln, depth, o, my_n, my_m);
   }
 }
 
-template <class DT>
+template <class DT, bool PAR>
 __device__ void res_td(const LevelArgs& a, const ResArgs& r, const ResState& s, const CrewSeat& seat, DT* depth,
                        const ResOut& o, unsigned& my_n, unsigned long long& my_m) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -319,7 +332,8 @@ __device__ void res_td(const LevelArgs& a, const ResArgs& r, const ResState& s, 
     for (int64_t k = gw; k < n * share; k += nw) {
       const int u = row((int)(k % n));
       const int64_t end = a.off[u + 1];
-      res_slice(a, a.off[u] + k / n * (32 * R_ILP), share * (32 * R_ILP), end, ln, depth, o, my_n, my_m);
+      res_slice<DT, PAR>(a, a.off[u] + k / n * (32 * R_ILP), share * (32 * R_ILP), end, PAR ? out_id(a, u) : -1, ln,
+                         depth, o, my_n, my_m);
     }
   };
   if (s.n_g) long_rows(s.n_g, max((int64_t)R_SHARE, nw / s.n_g), [&](int i) { return __ldcg(r.huge[s.L & 1] + i); });
@@ -327,21 +341,22 @@ __device__ void res_td(const LevelArgs& a, const ResArgs& r, const ResState& s, 
   // up to 32 light rows per warp, spread over all warps
   const int k = (int)min((int64_t)32, (s.n_l + nw - 1) / nw);
   for (int64_t first = gw * k; first < s.n_l; first += nw * k) {
-    int d = 0;
+    int d = 0, own = -1;
     int64_t st = 0;
     if (lane < k && first + lane < s.n_l) {
       const int u = __ldcg(q + first + lane);
       st = a.off[u];
       d = a.deg[u];
+      if (PAR) own = out_id(a, u);
     }
-    res_rows<DT, false>(a, d, st, ln, depth, o, my_n, my_m);
+    res_rows<DT, false, PAR>(a, d, st, own, ln, depth, o, my_n, my_m);
   }
 }
 
 // One bottom-up level over the words of vertices that have rows (bu_expand
 // with nothing to list), BW words of a warp in flight together, and ILP row
 // entries of each vertex per step.
-template <class DT, int BW, int ILP>
+template <class DT, bool PAR, int BW, int ILP>
 __device__ void res_bu_words(const LevelArgs& a, const ResArgs& r, const ResState& s, const CrewSeat& seat, DT* depth,
                              unsigned& my_n, unsigned long long& my_m) {
   const uint32_t* fbc = r.fb[s.f];
@@ -360,6 +375,7 @@ __device__ void res_bu_words(const LevelArgs& a, const ResArgs& r, const ResStat
     int d[BW], id[BW];
     bool todo[BW];  // still to be found
     bool found[BW];
+    [[maybe_unused]] int by[BW];  // the neighbour that found it
 #pragma unroll
     for (int t = 0; t < BW; ++t) {
       const int wi = w0 + t * nw;
@@ -382,12 +398,15 @@ __device__ void res_bu_words(const LevelArgs& a, const ResArgs& r, const ResStat
     for (int t = 0; t < BW; ++t) {
       found[t] = todo[t] && is_front(ld[t].x);
       todo[t] &= !found[t];
+      by[t] = ld[t].x;
     }
 #pragma unroll
     for (int t = 0; t < BW; ++t)
       if (todo[t] && d[t] > 1) {
-        found[t] = is_front(ld[t].y) | (ld[t].z >= 0 && is_front(ld[t].z)) | (ld[t].w >= 0 && is_front(ld[t].w));
+        const bool fy = is_front(ld[t].y), fz = ld[t].z >= 0 && is_front(ld[t].z);
+        found[t] = fy | fz | (ld[t].w >= 0 && is_front(ld[t].w));
         todo[t] = !found[t];
+        by[t] = fy ? ld[t].y : (fz ? ld[t].z : ld[t].w);
       }
     uint32_t e0[BW];
 #pragma unroll
@@ -412,7 +431,11 @@ __device__ void res_bu_words(const LevelArgs& a, const ResArgs& r, const ResStat
       for (int t = 0; t < BW; ++t) {
         bool f = false;
 #pragma unroll
-        for (int i = 0; i < ILP; ++i) f |= u[t][i] >= 0 && is_front(u[t][i]);
+        for (int i = 0; i < ILP; ++i) {
+          const bool fi = u[t][i] >= 0 && is_front(u[t][i]);
+          f |= fi;
+          if (PAR && fi) by[t] = u[t][i];
+        }
         if (f) found[t] = true, todo[t] = false;
       }
     }
@@ -431,17 +454,33 @@ __device__ void res_bu_words(const LevelArgs& a, const ResArgs& r, const ResStat
         const uint32_t beg = __shfl_sync(FULL, e0[t], j);
         const int n = __shfl_sync(FULL, d[t], j);
         bool hit = false;
+        int hit_by = -1;  // PAR
         for (int b0 = lane & 7;; b0 += 32) {
           int u[4];
 #pragma unroll
           for (int i = 0; i < 4; ++i) u[i] = !hit && b0 + 8 * i < n ? __ldg(a.adj + beg + b0 + 8 * i) : -1;
           bool f = false;
 #pragma unroll
-          for (int i = 0; i < 4; ++i) f |= u[i] >= 0 && is_front(u[i]);
-          hit |= ((__ballot_sync(FULL, f) >> (8 * sub)) & 0xFFu) != 0;
+          for (int i = 0; i < 4; ++i) {
+            const bool fi = u[i] >= 0 && is_front(u[i]);
+            f |= fi;
+            if (PAR && fi) u[0] = u[i];
+          }
+          const unsigned hits = (__ballot_sync(FULL, f) >> (8 * sub)) & 0xFFu;  // none once the row is found
+          if (PAR) {
+            const int x = __shfl_sync(FULL, u[0], hits ? 8 * sub + __ffs(hits) - 1 : lane);
+            if (hits) hit_by = x;
+          }
+          hit |= hits != 0;
           if (__all_sync(FULL, hit || b0 + 32 - (lane & 7) >= n)) break;
         }
         if (__reduce_or_sync(FULL, hit ? 1u << j : 0u) >> lane & 1u) found[t] = true;
+        if (PAR)
+#pragma unroll
+          for (int r4 = 0; r4 < 4; ++r4) {
+            const int row = __shfl_sync(FULL, hit ? j : -1, 8 * r4), x = __shfl_sync(FULL, hit_by, 8 * r4);
+            if (lane == row) by[t] = x;
+          }
       }
       while (heavy) {
         const int j = __ffs(heavy) - 1;
@@ -452,7 +491,13 @@ __device__ void res_bu_words(const LevelArgs& a, const ResArgs& r, const ResStat
         for (int b0 = 0; b0 < n && !hit; b0 += 64) {
           const int e = b0 + lane;
           const int u0 = e < n ? __ldg(a.adj + beg + e) : -1, u1 = e + 32 < n ? __ldg(a.adj + beg + e + 32) : -1;
-          hit = __any_sync(FULL, (u0 >= 0 && is_front(u0)) || (u1 >= 0 && is_front(u1)));
+          const bool f0 = u0 >= 0 && is_front(u0), f1 = u1 >= 0 && is_front(u1);
+          const unsigned hits = __ballot_sync(FULL, f0 || f1);
+          hit = hits != 0;
+          if (PAR && hit) {
+            const int x = __shfl_sync(FULL, f0 ? u0 : u1, __ffs(hits) - 1);
+            if (lane == j) by[t] = x;
+          }
         }
         if (lane == j) found[t] = hit;
       }
@@ -461,6 +506,7 @@ __device__ void res_bu_words(const LevelArgs& a, const ResArgs& r, const ResStat
     for (int t = 0; t < BW; ++t) {
       if (found[t]) {
         st_keep(depth + id[t], (DT)(s.L + 1));
+        if (PAR) st_keep(r.parent + id[t], out_id(a, by[t]));
         my_n += 1;
         my_m += (unsigned)d[t];
       }
@@ -479,13 +525,13 @@ __device__ void res_bu_words(const LevelArgs& a, const ResArgs& r, const ResStat
 // traversal, words x entries 3 x 2, 3 x 3, 2 x 4: ER 2^19 of mean degree 16 108, 105,
 // 100, of 29 184, 180, 172; R-MAT s16 66.6, 65.6, 63.5; ER 2^22 d16 291, 283, 301;
 // ER 3M d6 305, 303, 323; R-MAT s22 155, 153, 153.
-template <class DT>
+template <class DT, bool PAR>
 __device__ void res_bu(const LevelArgs& a, const ResArgs& r, const ResState& s, const CrewSeat& seat, DT* depth,
                        unsigned& my_n, unsigned long long& my_m) {
   if ((a.n_active + 31) >> 5 <= (int64_t)seat.size * RW * R_BW_WORDS)
-    res_bu_words<DT, 2, 4>(a, r, s, seat, depth, my_n, my_m);
+    res_bu_words<DT, PAR, 2, 4>(a, r, s, seat, depth, my_n, my_m);
   else
-    res_bu_words<DT, 3, 3>(a, r, s, seat, depth, my_n, my_m);
+    res_bu_words<DT, PAR, 3, 3>(a, r, s, seat, depth, my_n, my_m);
 }
 
 // Queues the frontier in fb[s.f], left by a bottom-up level (vertices with rows).
@@ -508,7 +554,7 @@ __device__ void res_queue(const LevelArgs& a, const ResArgs& r, const ResState& 
 // The leader alone: top-down levels while the frontier is light and small, at most
 // R_SOLO_LEVELS and no further than the direction rule allows; leaves the next
 // frontier queued, its bits set in fbn, its counts in `n` and the totals in so.
-template <class DT, class Solo>
+template <class DT, bool PAR, class Solo>
 __device__ void res_solo(const LevelArgs& a, const ResArgs& r, const ResState& s0, DT* depth, uint32_t* fbn, int32_t* n,
                          Solo* so, int4 (*s_q)[R_SOLO_CAP]) {
   __shared__ int32_t s_n[2][3];
@@ -528,7 +574,7 @@ __device__ void res_solo(const LevelArgs& a, const ResArgs& r, const ResState& s
   for (int run = 0;; ++run) {
     const int cur = L & 1, nxt = cur ^ 1;
     mid += res_mid(m_f);
-    const ResOut o{nullptr, r.queue[nxt], r.huge[nxt], s_n[nxt], s_q[nxt]};
+    const ResOut o{nullptr, r.queue[nxt], r.huge[nxt], s_n[nxt], s_q[nxt], r.parent};
     const int k = min(32, (cnt + RW - 1) / RW);
     unsigned my_n = 0;
     unsigned long long my_m = 0;
@@ -541,7 +587,7 @@ __device__ void res_solo(const LevelArgs& a, const ResArgs& r, const ResState& s
         st = (int64_t)(((uint64_t)(uint32_t)e.w << 32) | (uint32_t)e.z);
         id = out_id(a, e.x);
       }
-      res_rows<DT, true>(a, d, st, L + 1, depth, o, my_n, my_m);
+      res_rows<DT, true, PAR>(a, d, st, id, L + 1, depth, o, my_n, my_m);
       if (id >= 0) depth[id] = (DT)L;
     }
     my_n = __reduce_add_sync(FULL, my_n);
@@ -637,7 +683,7 @@ __device__ void res_finish(const LevelArgs& a, const ResState& s, int32_t src, i
   k->m_f = s.m_f;
 }
 
-template <class DT>
+template <class DT, bool PAR>
 __global__ void __launch_bounds__(RT, 1) k_resident(LevelArgs a, ResArgs r, int32_t src, DT* depth, int part) {
   extern __shared__ int4 s_dyn[];
   int4(*s_q)[R_SOLO_CAP] = reinterpret_cast<int4(*)[R_SOLO_CAP]>(s_dyn);
@@ -658,6 +704,7 @@ __global__ void __launch_bounds__(RT, 1) k_resident(LevelArgs a, ResArgs r, int3
   const auto fill = [&](uint32_t share) {
     const int64_t tid = (int64_t)share * RT + threadIdx.x, nth = (int64_t)gridDim.x * RT;
     fill_unreached(depth, a.V, tid, nth, src);
+    if (PAR) fill_neg1(r.parent, a.V, tid, nth, src, src);
     for (int64_t i = tid; i < W; i += nth) {
       const uint32_t x = i == (isrc >> 5) ? 1u << (isrc & 31) : 0u;
       a.vis[i] = x;
@@ -739,14 +786,14 @@ __global__ void __launch_bounds__(RT, 1) k_resident(LevelArgs a, ResArgs r, int3
     unsigned long long my_m = 0;
     uint32_t* fbn = r.fb[(s.f + 1) % 3];
     const int nq = s.kind == RK_QUEUE ? s.L & 1 : (s.L + 1) & 1;
-    const ResOut o{fbn, r.queue[nq], r.huge[nq], n_next, nullptr};
-    if (s.kind == RK_TD) res_td(a, r, s, seat, depth, o, my_n, my_m);
-    else if (s.kind == RK_BU) res_bu(a, r, s, seat, depth, my_n, my_m);
+    const ResOut o{fbn, r.queue[nq], r.huge[nq], n_next, nullptr, r.parent};
+    if (s.kind == RK_TD) res_td<DT, PAR>(a, r, s, seat, depth, o, my_n, my_m);
+    else if (s.kind == RK_BU) res_bu<DT, PAR>(a, r, s, seat, depth, my_n, my_m);
     else if (s.kind == RK_QUEUE) res_queue(a, r, s, seat, o);
     else if (s.kind == RK_GATHER) crew_gather(crew, seat, res_work(a, s, s.then));
     else if (s.kind == RK_FILL)
       for (uint32_t i = s_seat.size + rank; i < gridDim.x; i += s_seat.size) fill(i);
-    else if (rank == 0) res_solo(a, r, s, depth, fbn, n_next, &c->solo[s.p & 1], s_q);
+    else if (rank == 0) res_solo<DT, PAR>(a, r, s, depth, fbn, n_next, &c->solo[s.p & 1], s_q);
     if (s.kind <= RK_BU) {
       const unsigned wn = __reduce_add_sync(FULL, my_n);
       if (wn) {
@@ -782,7 +829,7 @@ __global__ void __launch_bounds__(RT, 1) k_resident(LevelArgs a, ResArgs r, int3
 // One bottom-up level of a traversal in parts, if that is what comes next:
 // k_expand's sweep, the old frontier's bits cleared beside it, and the decision
 // by the last CTA to finish.
-template <class DT>
+template <class DT, bool PAR>
 __global__ void __launch_bounds__(BT, 8) k_res_bu_level(LevelArgs a, ResArgs r, DT* depth) {
   __shared__ unsigned long long s_red[BT / 32];
   __shared__ int s_last;
@@ -796,7 +843,7 @@ __global__ void __launch_bounds__(BT, 8) k_res_bu_level(LevelArgs a, ResArgs r, 
   }
   const Front is_front{r.fb[f], nullptr, 0, 0};
   unsigned long long my_n = 0, my_m = 0;
-  bu_words<DT>(a, is_front, r.fb[(f + 1) % 3], L + 1, depth, nullptr, nullptr, my_n, my_m);
+  bu_words<DT>(a, is_front, r.fb[(f + 1) % 3], L + 1, depth, PAR ? r.parent : nullptr, nullptr, my_n, my_m);
   unsigned long long* acc = c->acc[(p + 1) % 3];
   if (__syncthreads_or(my_n != 0)) {
     unsigned long long x = block_sum(my_n, s_red);

@@ -1502,7 +1502,7 @@ static int pick_narrow_cluster(int limit, size_t smem) {
 
 constexpr size_t RES_SMEM = 2 * R_SOLO_CAP * sizeof(int4);
 
-// Whether this graph's traversals (without parents) run as k_resident, in one
+// Whether this graph's traversals run as k_resident, in one
 // kernel or in parts, instead of the CUDA graph of level kernels. Measured,
 // level kernels -> resident, ms: R-MAT s16 0.146 -> 0.068, s20 0.158 -> 0.089,
 // s22 0.235 -> 0.150, s23 0.272 -> 0.205, s24 0.340 -> 0.310; ER 2^22 d16 0.41 ->
@@ -1511,6 +1511,12 @@ constexpr size_t RES_SMEM = 2 * R_SOLO_CAP * sizeof(int4);
 // mean degree (grids, roads) are deep, and their levels belong in the cluster of
 // k_narrow: a 300^2 grid 1.5 -> 2.1 ms, 1024^2 5.4 -> 13 ms.
 constexpr int64_t RES_SPLIT_V = 1 << 22;
+// With parents only above this size. The order by degree made the level kernels
+// slower there on uniform graphs, for every find's caller id and its parent's are
+// read and both results stored apart: ER 2^20 d16 228 -> 244 us, 2^22 d16 440 ->
+// 473; resident 168 and 324 (R-MAT s20 183, 175, 94; s24 522, 420, 362). Up to it
+// they lose 3% at most.
+constexpr int64_t RES_PARENTS_V = 1 << 18;
 constexpr int64_t RES_MIN_DEGREE = 5;
 // Nor do graphs of higher mean degree that turn out to have many levels of
 // RES_MID_MIN to RES_MID_MAX entries (meshes, bands): in the cluster such a level
@@ -1526,7 +1532,8 @@ static bool resident_fits(const ent_graph* g, const BfsWorkspace* w) {
   if (g->E < RES_MIN_DEGREE * g->V || !g->perm) return false;
   if (o.loop != ENT_LOOP_GRAPH || w->narrow_nc == 0 || o.hub_slots > 0) return false;
   int n = 0;
-  for (const void* f : {(const void*)k_resident<int32_t>, (const void*)k_resident<uint8_t>})
+  for (const void* f : {(const void*)k_resident<int32_t, false>, (const void*)k_resident<uint8_t, false>,
+                        (const void*)k_resident<int32_t, true>})
     if (cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)RES_SMEM) != cudaSuccess ||
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, f, RT, RES_SMEM) != cudaSuccess || n < 1) {
       cudaGetLastError();
@@ -1535,21 +1542,31 @@ static bool resident_fits(const ent_graph* g, const BfsWorkspace* w) {
   return true;
 }
 
-// The resident traversal on stream s (no parents): one kernel, or for large
-// graphs its level kernels between two.
-template <class DT>
-static int launch_resident(BfsWorkspace* w, int32_t src, DT* depth, cudaStream_t s, int32_t max_levels = 0) {
+// The resident traversal on stream s: one kernel, or for large graphs its level
+// kernels between two.
+template <class DT, bool PAR>
+static int launch_resident_as(BfsWorkspace* w, int32_t src, DT* depth, int32_t* parent, cudaStream_t s,
+                              int32_t max_levels) {
   LevelArgs a = w->args;
   if (max_levels > 0) a.max_levels = max_levels;
   a.use_cond = 0;
-  ENT_CUDA(cudaMemsetAsync(w->res.rc, 0, sizeof(ResCtl), s));
-  k_resident<DT><<<w->grid_res, RT, RES_SMEM, s>>>(a, w->res, src, depth, w->split ? RP_HEAD : RP_ALL);
+  ResArgs r = w->res;
+  r.parent = parent;
+  ENT_CUDA(cudaMemsetAsync(r.rc, 0, sizeof(ResCtl), s));
+  k_resident<DT, PAR><<<w->grid_res, RT, RES_SMEM, s>>>(a, r, src, depth, w->split ? RP_HEAD : RP_ALL);
   ENT_CUDA(cudaGetLastError());
   if (!w->split) return ENT_OK;
-  for (int i = 0; i < R_BU_LEVELS; ++i) k_res_bu_level<DT><<<w->grid_expand, BT, 0, s>>>(a, w->res, depth);
-  k_resident<DT><<<w->grid_res, RT, RES_SMEM, s>>>(a, w->res, src, depth, RP_TAIL);
+  for (int i = 0; i < R_BU_LEVELS; ++i) k_res_bu_level<DT, PAR><<<w->grid_expand, BT, 0, s>>>(a, r, depth);
+  k_resident<DT, PAR><<<w->grid_res, RT, RES_SMEM, s>>>(a, r, src, depth, RP_TAIL);
   ENT_CUDA(cudaGetLastError());
   return ENT_OK;
+}
+template <class DT>
+static int launch_resident(BfsWorkspace* w, int32_t src, DT* depth, int32_t* parent, cudaStream_t s,
+                           int32_t max_levels = 0) {
+  if constexpr (sizeof(DT) == 4)  // byte depths come without parents
+    if (parent) return launch_resident_as<DT, true>(w, src, depth, parent, s, max_levels);
+  return launch_resident_as<DT, false>(w, src, depth, nullptr, s, max_levels);
 }
 
 // Notes what a resident traversal says of the graph: whether most of its levels
@@ -1563,7 +1580,7 @@ static void note_depth(ent_graph* g, const BfsCtl& h) {
 // the highest degree, RES_PROBE levels at most, on the graph's stream.
 static int probe_depth(ent_graph* g, BfsWorkspace* w) {
   ENT_CUDA(cudaStreamWaitEvent(g->stream, w->ev_order, 0));
-  const int rc = launch_resident<int32_t>(w, g->top, w->depth, g->stream, RES_PROBE);
+  const int rc = launch_resident<int32_t>(w, g->top, w->depth, nullptr, g->stream, RES_PROBE);
   if (rc != ENT_OK) return rc;
   ENT_CUDA(cudaMemcpyAsync(w->ctl_h, w->ctl, sizeof(BfsCtl), cudaMemcpyDeviceToHost, g->stream));
   ENT_CUDA(cudaStreamSynchronize(g->stream));
@@ -1759,12 +1776,13 @@ static int run_bfs_typed(ent_graph* g, int32_t src, DT* depth, int32_t* parent, 
   if (!captured) ENT_CUDA(cudaStreamWaitEvent(s, w->ev_order, 0));
   if (stats) ENT_CUDA(cudaEventRecord(w->ev0, s));
   if (g->opts.loop == ENT_LOOP_GRAPH) {
-    if (w->res.rc && !parent && !captured && g->deep < 0 && !stats) {
+    const bool fits = w->res.rc && !captured && (!parent || w->V > RES_PARENTS_V);
+    if (fits && g->deep < 0 && !stats) {
       const int rcode = probe_depth(g, w);
       if (rcode != ENT_OK) return rcode;
     }
-    resident = w->res.rc && !parent && !captured && g->deep != 1;
-    const int rc = resident ? launch_resident(w, src, depth, s) : launch_graph(g, w, src, depth, parent, s);
+    resident = fits && g->deep != 1;
+    const int rc = resident ? launch_resident(w, src, depth, parent, s) : launch_graph(g, w, src, depth, parent, s);
     if (rc != ENT_OK) return rc;
   } else {
     LevelArgs la = w->args;

@@ -63,8 +63,9 @@ enum ent_policy {
 enum ent_loop {
   ENT_LOOP_GRAPH = 0, /* whole traversal = one launch, no host round trip:
                          a CUDA graph with a device-side while node, or,
-                         without parents and on graphs of mean degree 5 and
-                         more whose levels do not prove many and small,
+                         on graphs of mean degree 5 and more whose levels do
+                         not prove many and small (with parents: of more than
+                         2^18 vertices),
                          kernels of many levels each, whose blocks hold the
                          SMs they were given until the traversal ends (they
                          take those that are free, and wait for none)       */

@@ -49,11 +49,14 @@ def test_time_of_uniform_rows(eb):
     import torch
     with eb.Graph.er(1 << 20, 40, seed=3) as g:
         d = torch.empty(g.vert_count, dtype=torch.int32, device="cuda")
-        p = torch.empty_like(d)
         srcs = eb.pick_sources(g.download().beg_pos, 83, 8)
 
-        def median(parents):
-            t = [g.bfs_device(int(s), d.data_ptr(), parents).device_ms for _ in range(3) for s in srcs]
+        def median():
+            t = [g.bfs_device(int(s), d.data_ptr()).device_ms for _ in range(3) for s in srcs]
             return float(np.median(t[len(srcs):]))
 
-        assert median(0) < 0.85 * median(p.data_ptr())
+        resident = median()
+        o = g.opts
+        o.narrow_max_frontier = 0  # the level kernels
+        g.opts = o
+        assert resident < 0.85 * median()
