@@ -466,16 +466,18 @@ __device__ void res_bu_words(const LevelArgs& a, const ResArgs& r, const ResStat
             f |= fi;
             if (PAR && fi) u[0] = u[i];
           }
-          const unsigned hits = (__ballot_sync(FULL, f) >> (8 * sub)) & 0xFFu;  // none once the row is found
-          if (PAR) {
+          const unsigned any = __ballot_sync(FULL, f);
+          const unsigned hits = (any >> (8 * sub)) & 0xFFu;  // none once the row is found
+          if (PAR && any) {
             const int x = __shfl_sync(FULL, u[0], hits ? 8 * sub + __ffs(hits) - 1 : lane);
             if (hits) hit_by = x;
           }
           hit |= hits != 0;
           if (__all_sync(FULL, hit || b0 + 32 - (lane & 7) >= n)) break;
         }
-        if (__reduce_or_sync(FULL, hit ? 1u << j : 0u) >> lane & 1u) found[t] = true;
-        if (PAR)
+        const unsigned rows = __reduce_or_sync(FULL, hit ? 1u << j : 0u);
+        if (rows >> lane & 1u) found[t] = true;
+        if (PAR && rows)
 #pragma unroll
           for (int r4 = 0; r4 < 4; ++r4) {
             const int row = __shfl_sync(FULL, hit ? j : -1, 8 * r4), x = __shfl_sync(FULL, hit_by, 8 * r4);

@@ -1512,11 +1512,12 @@ constexpr size_t RES_SMEM = 2 * R_SOLO_CAP * sizeof(int4);
 // k_narrow: a 300^2 grid 1.5 -> 2.1 ms, 1024^2 5.4 -> 13 ms.
 constexpr int64_t RES_SPLIT_V = 1 << 22;
 // With parents only above this size. The order by degree made the level kernels
-// slower there on uniform graphs, for every find's caller id and its parent's are
+// slower on uniform graphs there, for every find's caller id and its parent's are
 // read and both results stored apart: ER 2^20 d16 228 -> 244 us, 2^22 d16 440 ->
-// 473; resident 168 and 324 (R-MAT s20 183, 175, 94; s24 522, 420, 362). Up to it
-// they lose 3% at most.
-constexpr int64_t RES_PARENTS_V = 1 << 18;
+// 473; resident 168 and 324 (R-MAT s20 183, 175, 94; s24 522, 420, 362). Below, the
+// level kernels lose up to 11% (ER 2^19 d16 178 -> 196), but resident traversals with
+// parents up to 25% at mean degrees just below small_max (d29 178 -> 224).
+constexpr int64_t RES_PARENTS_V = 3 << 18;
 constexpr int64_t RES_MIN_DEGREE = 5;
 // Nor do graphs of higher mean degree that turn out to have many levels of
 // RES_MID_MIN to RES_MID_MAX entries (meshes, bands): in the cluster such a level

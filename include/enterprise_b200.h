@@ -65,7 +65,7 @@ enum ent_loop {
                          a CUDA graph with a device-side while node, or,
                          on graphs of mean degree 5 and more whose levels do
                          not prove many and small (with parents: of more than
-                         2^18 vertices),
+                         786432 vertices),
                          kernels of many levels each, whose blocks hold the
                          SMs they were given until the traversal ends (they
                          take those that are free, and wait for none)       */

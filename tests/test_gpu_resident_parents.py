@@ -1,5 +1,5 @@
-"""GPU test of traversals with parents as resident kernels, which graphs above 2^18
-vertices take: every place where a parent is stored (claims of light, heavy and
+"""GPU test of traversals with parents as resident kernels, which graphs of more than
+786432 vertices take: every place where a parent is stored (claims of light, heavy and
 huge rows, of one CTA alone, bottom-up finds by lead entry, by lane, by four rows
 and by one row of a warp), in one kernel and in parts. Depths equal the oracle's,
 and every parent is an edge one level up."""
@@ -8,7 +8,7 @@ import pytest
 
 pytestmark = pytest.mark.gpu
 
-LIMIT = 1 << 18
+LIMIT = 3 << 18
 
 
 def _check(eb, orc, csr, srcs, launches, **opts):
@@ -31,8 +31,8 @@ def _check(eb, orc, csr, srcs, launches, **opts):
 @pytest.mark.parametrize("small_max", [4, 32])
 @pytest.mark.parametrize("kind", ["rmat", "er", "uniform"])
 def test_one_kernel(eb, orc, kind, small_max, policy):
-    csr = {"rmat": lambda: eb.Csr.rmat(19, 8, seed=0xF1), "er": lambda: eb.Csr.er(LIMIT + 1, 9.0, seed=0xF2),
-           "uniform": lambda: eb.Csr.er(LIMIT + 77, 40.0, seed=0xF3)}[kind]()
+    csr = {"rmat": lambda: eb.Csr.rmat(20, 8, seed=0xF1), "er": lambda: eb.Csr.er(LIMIT + 1, 9.0, seed=0xF2),
+           "uniform": lambda: eb.Csr.er(LIMIT + 77, 36.0, seed=0xF3)}[kind]()
     _check(eb, orc, csr, eb.pick_sources(csr.beg_pos, 101, 2), 1, small_max=small_max, large_min=1024, policy=policy)
 
 
@@ -46,8 +46,8 @@ def test_long_rows_and_chains(eb, orc, hub, policy):
     chain = np.arange(at, at + 300)
     rest = LIMIT - at - 300 + 50
     r0 = at + 300
-    src = np.concatenate([np.zeros(hub, np.int64), kids, [hub], chain[:-1], rng.randint(0, rest, 4 * LIMIT) + r0, [r0]])
-    dst = np.concatenate([kids, kids + hub, [at], chain[1:], rng.randint(0, rest, 4 * LIMIT) + r0, [at + 299]])
+    src = np.concatenate([np.zeros(hub, np.int64), kids, [hub], chain[:-1], rng.randint(0, rest, 3 * LIMIT) + r0, [r0]])
+    dst = np.concatenate([kids, kids + hub, [at], chain[1:], rng.randint(0, rest, 3 * LIMIT) + r0, [at + 299]])
     csr = eb.Csr.from_edges(src, dst, LIMIT + 60)
     _check(eb, orc, csr, [0, 1, at + 150, r0 + 5, LIMIT + 59], 1, policy=policy)
 
