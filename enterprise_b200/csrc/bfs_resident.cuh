@@ -682,7 +682,6 @@ __device__ void res_finish(const LevelArgs& a, const ResState& s, int32_t src, i
   k->split_launches = part == RP_TAIL ? R_BU_LEVELS + 1 : 0;
   k->n_vis = s.n_vis;
   k->m_vis = s.m_vis;
-  k->m_f = s.m_f;
 }
 
 template <class DT, bool PAR>

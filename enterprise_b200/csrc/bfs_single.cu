@@ -58,6 +58,7 @@
 //    classification whose wait ran out ends the traversal with an error bit
 //    instead of handing on inconsistent queues.
 #include <algorithm>
+#include <atomic>
 #include <type_traits>
 #include <vector>
 #include <string.h>
@@ -1328,6 +1329,8 @@ struct BfsWorkspace {
   ResArgs res = {};
   int grid_res = 0;
   bool split = false;  // bottom-up levels as kernels of their own between its head and tail
+  struct DepthNote* note = nullptr;  // page-locked; note_left: its copies have been queued
+  bool note_left = false;
   // traversals of one workspace run one after another, whatever streams they
   // are launched on: the end of the latest one
   cudaEvent_t ev_order = nullptr;
@@ -1356,6 +1359,7 @@ void destroy_bfs_workspace(BfsWorkspace* w) {
   dev_free(w->slab);
   dev_free(w->ctl);
   host_slot_free(w->ctl_h);
+  host_slot_free(w->note);
   dev_free(w->depth);
   dev_free(w->parent);
   if (w->ev0) cudaEventDestroy(w->ev0);
@@ -1521,13 +1525,12 @@ constexpr int64_t RES_PARENTS_V = 3 << 18;
 constexpr int64_t RES_MIN_DEGREE = 5;
 // Nor do graphs of higher mean degree that turn out to have many levels of
 // RES_MID_MIN to RES_MID_MAX entries (meshes, bands): in the cluster such a level
-// takes 3 to 5 us, here 4 to 12. us a traversal, caller's order and level
-// kernels, resident, this order and level kernels: mesh 80^3 1158, 2923, 1166; 200 levels of 200
-// vertices, degree 40: 812, 2421, 717; 192 levels of 1000, degree 20: 1173, 1451,
-// 979. Larger levels are faster here (192 of 5000, degree 16: 3043, 2012, 2603;
-// mesh 160^3 8.25, 5.55, 8.12 ms), and a path's are equal.
+// takes 3 to 5 us, here 4 to 12. us a traversal (caller's order and level kernels,
+// resident, this order and level kernels): mesh 80^3 1158, 2923, 1166; 200 levels
+// of 200 vertices, degree 40: 812, 2421, 717; 192 levels of 1000, degree 20: 1173,
+// 1451, 979. Larger levels are faster here (192 of 5000, degree 16: 3043, 2012,
+// 2603; mesh 160^3 8.25, 5.55, 8.12 ms), and a path's are equal.
 constexpr int32_t RES_DEEP = 12;    // such levels from which a graph counts as deep
-constexpr int32_t RES_PROBE = 128;  // levels that a probe runs at most
 static bool resident_fits(const ent_graph* g, const BfsWorkspace* w) {
   const ent_bfs_opts& o = g->opts;
   if (g->E < RES_MIN_DEGREE * g->V || !g->perm) return false;
@@ -1546,10 +1549,8 @@ static bool resident_fits(const ent_graph* g, const BfsWorkspace* w) {
 // The resident traversal on stream s: one kernel, or for large graphs its level
 // kernels between two.
 template <class DT, bool PAR>
-static int launch_resident_as(BfsWorkspace* w, int32_t src, DT* depth, int32_t* parent, cudaStream_t s,
-                              int32_t max_levels) {
+static int launch_resident_as(BfsWorkspace* w, int32_t src, DT* depth, int32_t* parent, cudaStream_t s) {
   LevelArgs a = w->args;
-  if (max_levels > 0) a.max_levels = max_levels;
   a.use_cond = 0;
   ResArgs r = w->res;
   r.parent = parent;
@@ -1563,33 +1564,39 @@ static int launch_resident_as(BfsWorkspace* w, int32_t src, DT* depth, int32_t* 
   return ENT_OK;
 }
 template <class DT>
-static int launch_resident(BfsWorkspace* w, int32_t src, DT* depth, int32_t* parent, cudaStream_t s,
-                           int32_t max_levels = 0) {
+static int launch_resident(BfsWorkspace* w, int32_t src, DT* depth, int32_t* parent, cudaStream_t s) {
   if constexpr (sizeof(DT) == 4)  // byte depths come without parents
-    if (parent) return launch_resident_as<DT, true>(w, src, depth, parent, s, max_levels);
-  return launch_resident_as<DT, false>(w, src, depth, nullptr, s, max_levels);
+    if (parent) return launch_resident_as<DT, true>(w, src, depth, parent, s);
+  return launch_resident_as<DT, false>(w, src, depth, nullptr, s);
 }
 
-// Notes what a resident traversal says of the graph: whether most of its levels
-// are better run by the level kernels, which have it from here on. A frontier
-// still growing past that size when a probe was cut off speaks against it.
+// Notes what a resident traversal says of the graph, if its source lies in the
+// bulk of it: whether most of the levels are better run by the level kernels,
+// which have it from here on.
 static void note_depth(ent_graph* g, const BfsCtl& h) {
-  g->deep = h.mid_levels >= RES_DEEP && 2 * h.mid_levels >= h.level && h.m_f <= RES_MID_MAX;
+  if (g->deep >= 0 || h.err || h.n_vis * 4 < g->V) return;
+  g->deep = h.mid_levels >= RES_DEEP && 2 * h.mid_levels >= h.level;
 }
 
-// The same before a traversal that the host does not wait for: from a vertex of
-// the highest degree, RES_PROBE levels at most, on the graph's stream.
-static int probe_depth(ent_graph* g, BfsWorkspace* w) {
-  ENT_CUDA(cudaStreamWaitEvent(g->stream, w->ev_order, 0));
-  const int rc = launch_resident<int32_t>(w, g->top, w->depth, nullptr, g->stream, RES_PROBE);
-  if (rc != ENT_OK) return rc;
-  ENT_CUDA(cudaMemcpyAsync(w->ctl_h, w->ctl, sizeof(BfsCtl), cudaMemcpyDeviceToHost, g->stream));
-  ENT_CUDA(cudaStreamSynchronize(g->stream));
-  g_kernel_launches += 1 + w->ctl_h->split_launches;
-  if (w->ctl_h->err & ~4)  // 4: cut off
-    return fail(ENT_ERR_TIMEOUT, "device traversal reported error flags 0x%x", w->ctl_h->err);
-  note_depth(g, *w->ctl_h);
+// The same from a traversal that the host does not wait for: its control block is
+// copied behind it, then a flag, which the next call looks at.
+struct DepthNote {
+  BfsCtl ctl;
+  volatile int32_t there;
+};
+static int leave_note(BfsWorkspace* w, cudaStream_t s) {
+  if (w->note_left) return ENT_OK;
+  w->note->there = 0;
+  ENT_CUDA(cudaMemcpyAsync(&w->note->ctl, w->ctl, sizeof(BfsCtl), cudaMemcpyDeviceToHost, s));
+  ENT_CUDA(cudaMemcpyAsync((void*)&w->note->there, &w->ctl->done, sizeof(int32_t), cudaMemcpyDeviceToHost, s));
+  w->note_left = true;
   return ENT_OK;
+}
+static void take_note(ent_graph* g, BfsWorkspace* w) {
+  if (!w->note_left || !w->note->there) return;
+  std::atomic_thread_fence(std::memory_order_acquire);
+  note_depth(g, w->note->ctl);
+  w->note_left = false;
 }
 
 static int create_workspace(ent_graph* g, BfsWorkspace** out, bool force_graph = false, int32_t cluster = 0) {
@@ -1618,8 +1625,9 @@ static int create_workspace(ent_graph* g, BfsWorkspace** out, bool force_graph =
   if (e == cudaSuccess) e = dev_alloc(&w->ctl, sizeof(BfsCtl));
   if (e == cudaSuccess) e = cudaMemsetAsync(w->ctl, 0, sizeof(BfsCtl), g->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(g->stream);
-  static_assert(sizeof(BfsCtl) <= 512, "the control block's pinned copy is a host slot");
+  static_assert(sizeof(DepthNote) <= 512, "the control block's pinned copies are host slots");
   if (e == cudaSuccess && !(w->ctl_h = (BfsCtl*)host_slot(sizeof(BfsCtl)))) e = cudaErrorMemoryAllocation;
+  if (e == cudaSuccess && !(w->note = (DepthNote*)host_slot(sizeof(DepthNote)))) e = cudaErrorMemoryAllocation;
   if (e == cudaSuccess) e = dev_alloc(&w->depth, sizeof(int32_t) * V);
   if (e == cudaSuccess) e = dev_alloc(&w->parent, sizeof(int32_t) * V);
   if (e == cudaSuccess) e = cudaEventCreate(&w->ev0);
@@ -1777,13 +1785,10 @@ static int run_bfs_typed(ent_graph* g, int32_t src, DT* depth, int32_t* parent, 
   if (!captured) ENT_CUDA(cudaStreamWaitEvent(s, w->ev_order, 0));
   if (stats) ENT_CUDA(cudaEventRecord(w->ev0, s));
   if (g->opts.loop == ENT_LOOP_GRAPH) {
-    const bool fits = w->res.rc && !captured && (!parent || w->V > RES_PARENTS_V);
-    if (fits && g->deep < 0 && !stats) {
-      const int rcode = probe_depth(g, w);
-      if (rcode != ENT_OK) return rcode;
-    }
-    resident = fits && g->deep != 1;
-    const int rc = resident ? launch_resident(w, src, depth, parent, s) : launch_graph(g, w, src, depth, parent, s);
+    take_note(g, w);
+    resident = w->res.rc && !captured && (!parent || w->V > RES_PARENTS_V) && g->deep != 1;
+    int rc = resident ? launch_resident(w, src, depth, parent, s) : launch_graph(g, w, src, depth, parent, s);
+    if (rc == ENT_OK && resident && g->deep < 0 && !stats) rc = leave_note(w, s);
     if (rc != ENT_OK) return rc;
   } else {
     LevelArgs la = w->args;
@@ -1817,8 +1822,7 @@ static int run_bfs_typed(ent_graph* g, int32_t src, DT* depth, int32_t* parent, 
     float ms = 0.f;
     cudaEventElapsedTime(&ms, w->ev0, w->ev1);
     fill_stats(*w->ctl_h, ms, stats);
-    // a source in the bulk of the graph speaks for it
-    if (resident && g->deep < 0 && !w->ctl_h->err && w->ctl_h->n_vis * 4 >= w->V) note_depth(g, *w->ctl_h);
+    if (resident) note_depth(g, *w->ctl_h);
     if (g->opts.loop == ENT_LOOP_GRAPH) g_kernel_launches += stats->launches;
     if (w->ctl_h->err) return fail(ENT_ERR_TIMEOUT, "device traversal reported error flags 0x%x", w->ctl_h->err);
   } else if (g->opts.loop == ENT_LOOP_GRAPH) {
@@ -2210,6 +2214,10 @@ static int bfs_many(ent_graph* g, const int32_t* src, int32_t n_src, void* const
                : run_bfs_typed<int32_t>(g, src[i], (int32_t*)buf[b], nullptr, s, nullptr);
     if (rc != ENT_OK) break;
     ce = cudaEventRecord(ev[2 * (size_t)i + 1], s);
+    if (ce == cudaSuccess && g->deep < 0 && w->note_left && i < 3) {  // which kernels the rest is for
+      ce = cudaStreamSynchronize(s);
+      take_note(g, w);
+    }
     const bool row = depth_out && depth_out[i];
     if (ce == cudaSuccess) {  // the row towards L2 (bytes, and only if it is copied), and the control block
       const int64_t n = row && bytes ? g->V : 0;

@@ -61,7 +61,6 @@ struct ent_graph {
   ent::BfsWorkspace* ws = nullptr;
   ent::BatchWorkspace* bws = nullptr;
   ent::DeepLanes* lanes = nullptr;
-  int32_t top = 0;            // caller id of a vertex of the highest degree (known with an order of its own)
   int32_t deep = -1;          // whether traversals have many small levels (-1: not yet known)
   int32_t probe_levels = -1;  // depth of the graph as probed by its first auto-mode batch (-1: not yet)
   void* stage = nullptr;      // device rows of batches whose results go to host memory

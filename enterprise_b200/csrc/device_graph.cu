@@ -207,7 +207,6 @@ static cudaError_t build_traversal_order(ent_graph* g) {
   }
   g_kernel_launches += 3;
   if (e == cudaSuccess) e = cudaMemcpyAsync(h, n_active, sizeof(h), cudaMemcpyDeviceToHost, s);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(&g->top, g->perm, sizeof(g->top), cudaMemcpyDeviceToHost, s);
   const cudaError_t e2 = cudaStreamSynchronize(s);
   g->n_active = h[0];
   g->rows_sorted = h[1] == 0;

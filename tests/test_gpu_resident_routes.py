@@ -1,7 +1,7 @@
 """GPU test of which graphs of mean degree 5 and more leave the resident kernels
 for the level loop: those whose traversals show many small levels (meshes,
-bands), known after the first traversal that the host waits for or after a probe
-before the first that it does not. Depths equal the oracle's on both routes; the
+bands), known once a first traversal has ended, whether the host waited for it or
+not, and within a source list after its first sources. Depths equal the oracle's on both routes; the
 launches of the statistics tell the routes apart."""
 import numpy as np
 import pytest
