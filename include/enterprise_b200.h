@@ -79,17 +79,21 @@ typedef struct ent_bfs_opts {
   double beta;           /* Beamer: BU->TD when n_f < V / beta (shrinking) */
   double ref_ratio;      /* reference rule ratio (0.3, inspector.cuh:497)  */
   int32_t small_max;     /* degree <  small_max -> thread tier (ref 32)    */
-  int32_t large_min;     /* degree >  large_min -> CTA tier (ref 1024)     */
+  int32_t large_min;     /* degree >  large_min -> CTA tier (ref 1024); level
+                            kernels only                                   */
   int32_t hub_slots;     /* shared-memory hub cache slots, power of two,
                             0 disables (ref 1536/1920, comm.h:176-177)     */
-  int32_t chunk_edges;   /* edges per CTA chunk of a large TD vertex       */
-  int32_t blocks_per_sm; /* resident CTAs per SM for the level kernels,
-                            0 = occupancy maximum                          */
+  int32_t chunk_edges;   /* edges per CTA chunk of a large TD vertex; level
+                            kernels only                                   */
+  int32_t blocks_per_sm; /* resident CTAs per SM for the level kernels and the
+                            bottom-up kernels of a resident traversal in
+                            parts, 0 = occupancy maximum                   */
   /* batched (bitwise multi-source) traversal */
   double batch_alpha;      /* bottom-up when frontier edges*alpha > unfinished edges */
   int32_t batch_small_max; /* bottom-up: degree < this -> lane group per vertex     */
   int32_t batch_large_min; /* bottom-up: degree >= this -> CTA per vertex           */
-  int32_t batch_heavy;     /* top-down: degree >= min(this, 512) -> warps share the vertex */
+  int32_t batch_heavy;     /* top-down: degree >= min(this, 512) -> warps share the vertex
+                              (values of 512 and more act the same)                  */
   /* small-frontier ("narrow") mode of the single-source traversal: while the
      top-down frontier stays small, one thread-block cluster runs level after
      level inside a single launch. Entered when the frontier has at most
