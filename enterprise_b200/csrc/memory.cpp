@@ -11,6 +11,9 @@
 // free and 420 kept: 300 MB by cudaMalloc succeed). Blocks of POOL_MAX and more
 // bypass it.
 //
+// Programs with CUDA contexts of their own (driver-API plug-ins) get memory from
+// the device there, and page-locked memory made in the same context.
+//
 // A copy between the device and pageable host memory runs through the driver's
 // own staging on one host thread (about 10 GB/s, first touch of fresh pages
 // included). Here two page-locked chunks take turns: the DMA of one overlaps
@@ -40,38 +43,103 @@ constexpr size_t POOL_MAX = 256ull << 20;
 struct DevicePool {
   cudaMemPool_t pool = nullptr;
   cudaStream_t stream = nullptr;  // orders the pool's own allocations and frees
-  bool tried = false;
+  uint64_t ctx = 0;               // the primary context it was made in
 };
 std::mutex g_mu;
 std::vector<DevicePool> g_pools;      // by device
 std::vector<void*> g_large;           // blocks that bypassed the pools
-std::vector<char*> g_idle;            // page-locked pairs of chunks not in use
-int g_pairs = 0;                      // ... and all of them
+// What is kept belongs to the CUDA context it was made in and ends with it: it is
+// used in that context only, by an id that no later context has again.
+struct Chunks {
+  uint64_t ctx = 0;
+  char* idle[2];  // page-locked pairs of chunks not in use
+  int n_idle = 0;
+  int n = 0;      // ... and all of them
+};
+std::vector<Chunks> g_chunks;
 constexpr int MAX_PAIRS = 2;          // 16 MB; further copies at the same time go to the driver
 
 // Small page-locked blocks (a traversal's status words): a slot of an arena, for
 // a call of cudaHostAlloc and cudaFreeHost each takes as long as a small graph's
 // whole build. Arenas stay; their number follows the most slots in use at once.
 constexpr size_t SLOT = 512, ARENA = 64 << 10;
-std::vector<char*> g_slots;           // free ones
+struct Arena {
+  uint64_t ctx;
+  char* base;
+  std::vector<char*> free;
+};
+std::vector<Arena> g_arenas;
+
+// The current context's id (0: unknown), and whether it is its device's primary
+// one. Only that one has a pool: memory of another context goes with it, and a
+// pool's would stay.
+struct Context {
+  uint64_t id = 0;
+  bool primary = true;
+};
+Context context() {
+  typedef int (*GetCurrent)(void**);
+  typedef int (*GetId)(void*, unsigned long long*);
+  typedef int (*GetState)(int, unsigned*, int*);
+  typedef int (*Retain)(void**, int);
+  typedef int (*Release)(int);
+  static const auto entry = [](const char* name) {
+    void* fn = nullptr;
+    cudaDriverEntryPointQueryResult q = cudaDriverEntryPointSymbolNotFound;
+    if (cudaGetDriverEntryPoint(name, &fn, cudaEnableDefault, &q) != cudaSuccess || q != cudaDriverEntryPointSuccess) {
+      cudaGetLastError();
+      fn = nullptr;
+    }
+    return fn;
+  };
+  static const auto current = (GetCurrent)entry("cuCtxGetCurrent");
+  static const auto id_of = (GetId)entry("cuCtxGetId");
+  static const auto state = (GetState)entry("cuDevicePrimaryCtxGetState");
+  static const auto retain = (Retain)entry("cuDevicePrimaryCtxRetain");
+  static const auto release = (Release)entry("cuDevicePrimaryCtxRelease");
+  static std::mutex mu;
+  static std::vector<Context> known;
+  Context c;
+  void* ctx = nullptr;
+  unsigned long long id = 0;
+  if (!current || !id_of || !state || !retain || !release) return c;
+  if (current(&ctx) != 0) return c;
+  if (!ctx && (cudaFree(nullptr) != cudaSuccess || current(&ctx) != 0 || !ctx)) return c;  // binds the primary one
+  if (id_of(ctx, &id) != 0) return c;
+  c.id = id + 1;
+  std::lock_guard<std::mutex> lk(mu);
+  for (const Context& k : known)
+    if (k.id == c.id) return k;
+  int dev = 0, active = 0;
+  unsigned flags = 0;
+  cudaGetDevice(&dev);
+  void* p = nullptr;
+  if (state(dev, &flags, &active) == 0 && active && retain(&p, dev) == 0) release(dev);
+  c.primary = p == ctx;
+  known.push_back(c);
+  return c;
+}
 
 // The current device's pool; pool null where it cannot have one.
 DevicePool device_pool() {
+  const Context c = context();
+  if (!c.primary) return {};
   int dev = 0;
   cudaGetDevice(&dev);
   std::lock_guard<std::mutex> lk(g_mu);
   if ((int)g_pools.size() <= dev) g_pools.resize(dev + 1);
   DevicePool& p = g_pools[dev];
-  if (!p.tried) {
-    p.tried = true;
+  if (!p.stream || p.ctx != c.id) {
+    p = DevicePool{};
+    p.ctx = c.id;
     int ok = 0;
     cudaMemPoolProps props = {};
     props.allocType = cudaMemAllocationTypePinned;
     props.location.type = cudaMemLocationTypeDevice;
     props.location.id = dev;
     uint64_t keep = POOL_KEEP;
-    if (cudaDeviceGetAttribute(&ok, cudaDevAttrMemoryPoolsSupported, dev) != cudaSuccess || !ok ||
-        cudaStreamCreateWithFlags(&p.stream, cudaStreamNonBlocking) != cudaSuccess ||
+    if (cudaDeviceGetAttribute(&ok, cudaDevAttrMemoryPoolsSupported, dev) != cudaSuccess ||
+        cudaStreamCreateWithFlags(&p.stream, cudaStreamNonBlocking) != cudaSuccess || !ok ||
         cudaMemPoolCreate(&p.pool, &props) != cudaSuccess ||
         cudaMemPoolSetAttribute(p.pool, cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess) {
       cudaGetLastError();
@@ -83,16 +151,25 @@ DevicePool device_pool() {
 
 struct Staging {
   char* buf = nullptr;  // two chunks
+  uint64_t ctx = 0;
   cudaEvent_t done[2] = {nullptr, nullptr};
+  static Chunks& of(uint64_t ctx) {
+    for (Chunks& c : g_chunks)
+      if (c.ctx == ctx) return c;
+    g_chunks.emplace_back();
+    g_chunks.back().ctx = ctx;
+    return g_chunks.back();
+  }
   Staging() {
+    ctx = context().id;
     {
       std::lock_guard<std::mutex> lk(g_mu);
-      if (!g_idle.empty()) {
-        buf = g_idle.back();
-        g_idle.pop_back();
-      } else if (g_pairs < MAX_PAIRS) {
+      Chunks& c = of(ctx);
+      if (c.n_idle > 0) {
+        buf = c.idle[--c.n_idle];
+      } else if (c.n < MAX_PAIRS) {
         if (cudaHostAlloc((void**)&buf, 2 * CHUNK, cudaHostAllocPortable) == cudaSuccess) {
-          ++g_pairs;
+          ++c.n;
         } else {
           buf = nullptr;
           cudaGetLastError();
@@ -114,7 +191,8 @@ struct Staging {
       }
     if (!buf) return;
     std::lock_guard<std::mutex> lk(g_mu);
-    g_idle.push_back(buf);
+    Chunks& c = of(ctx);
+    c.idle[c.n_idle++] = buf;
   }
 };
 
@@ -143,19 +221,22 @@ bool pageable(const void* host) {
 
 }  // namespace
 
+// Memory from the device itself, which dev_free gives back to it.
+static cudaError_t alloc_large(void** out, size_t bytes) {
+  const cudaError_t e = dev_malloc(out, bytes);
+  if (e == cudaSuccess) {
+    std::lock_guard<std::mutex> lk(g_mu);
+    g_large.push_back(*out);
+  }
+  return e;
+}
+
 cudaError_t dev_alloc(void** out, size_t bytes) {
   *out = nullptr;
   bytes = std::max<size_t>(bytes, 1);
-  if (bytes >= POOL_MAX) {
-    const cudaError_t e = dev_malloc(out, bytes);
-    if (e == cudaSuccess) {
-      std::lock_guard<std::mutex> lk(g_mu);
-      g_large.push_back(*out);
-    }
-    return e;
-  }
+  if (bytes >= POOL_MAX) return alloc_large(out, bytes);
   const DevicePool p = device_pool();
-  if (!p.pool) return cudaMalloc(out, bytes);
+  if (!p.pool) return alloc_large(out, bytes);
   cudaError_t e = cudaMallocFromPoolAsync(out, bytes, p.pool, p.stream);
   if (e == cudaErrorMemoryAllocation) {
     cudaGetLastError();
@@ -196,24 +277,34 @@ void dev_free(void* ptr) {
 
 void* host_slot(size_t bytes) {
   if (bytes > SLOT) return nullptr;
+  const uint64_t ctx = context().id;
   std::lock_guard<std::mutex> lk(g_mu);
-  if (g_slots.empty()) {
-    char* a = nullptr;
-    if (cudaHostAlloc((void**)&a, ARENA, cudaHostAllocPortable) != cudaSuccess) {
+  Arena* a = nullptr;
+  for (Arena& x : g_arenas)
+    if (x.ctx == ctx && !x.free.empty()) a = &x;
+  if (!a) {
+    char* base = nullptr;
+    if (cudaHostAlloc((void**)&base, ARENA, cudaHostAllocPortable) != cudaSuccess) {
       cudaGetLastError();
       return nullptr;
     }
-    for (size_t at = 0; at < ARENA; at += SLOT) g_slots.push_back(a + at);
+    g_arenas.push_back({ctx, base, {}});
+    a = &g_arenas.back();
+    for (size_t at = 0; at < ARENA; at += SLOT) a->free.push_back(base + at);
   }
-  char* p = g_slots.back();
-  g_slots.pop_back();
+  char* p = a->free.back();
+  a->free.pop_back();
   return p;
 }
 
 void host_slot_free(void* p) {
   if (!p) return;
   std::lock_guard<std::mutex> lk(g_mu);
-  g_slots.push_back((char*)p);
+  for (auto a = g_arenas.rbegin(); a != g_arenas.rend(); ++a)  // an address may be a dead context's too: the latest
+    if ((char*)p >= a->base && (char*)p < a->base + ARENA) {
+      a->free.push_back((char*)p);
+      return;
+    }
 }
 
 cudaError_t to_device(void* dst, const void* src, size_t bytes, cudaStream_t s) {
