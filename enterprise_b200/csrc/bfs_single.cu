@@ -47,9 +47,9 @@
 //    each queue entry carries the vertex's row start and degree, read while
 //    its visit was being claimed, so a level costs one adjacency read, one
 //    status probe and one claim on its critical path.
-//  * Unless the graph is road-like or deep, or parents are asked for, a resident
-//    kernel goes from level to level instead (bfs_resident.cuh); what follows
-//    is the rest.
+//  * Unless the graph is road-like or deep, or parents of a smaller graph are asked
+//    for, resident kernels go from level to level instead (bfs_resident.cuh); what
+//    follows is the rest.
 //  * The whole traversal is one CUDA graph: a reset kernel (which also writes
 //    the loop state), then a while node whose body is two copies of
 //    [expand, inspect, narrow]; the inspector sets the loop condition and the
@@ -1041,8 +1041,9 @@ __device__ __forceinline__ void narrow_append(const LevelArgs& a, BfsCtl* c, boo
 // expanded: in a traversal order of its own, the caller's id it is stored under is then
 // read beside the entry's row, off the level's critical path (a frontier handed
 // over gets its depths from the inspector).
-// LATE: depths are written at the expansion. In caller order that pays only where
-// the depths outgrow L2's share (4096^2 grid 32.7 -> 32.2 ms; 1024^2 5.45 -> 5.50).
+// LATE: depths are written at the expansion. In caller order it makes little
+// difference (one comparison each: 4096^2 grid 32.7 -> 32.2 ms, 1024^2 5.45 -> 5.50;
+// between whole runs the former isn't above the noise).
 template <class DT, bool LATE>
 __global__ void __launch_bounds__(NT, 1) k_narrow(LevelArgs a) {
   extern __shared__ int4 s_q[];  // [2][NQCAP]
