@@ -54,7 +54,9 @@ constexpr int SPIN_LIMIT = 1 << 20;
 // eight deep queries in flight, whose clusters hold some SMs for milliseconds at a
 // time, an R-MAT s16 traversal took 5.7 ms when launched so and takes 81 us (66 on
 // an idle GPU), s24 7.0 and 0.49 ms, and the server kept a third of its queries
-// and keeps all. On an idle GPU the seats cost 1 to 3 us a traversal.
+// and keeps all. On an idle GPU the seats cost 0 to 3 us a launch: R-MAT s12 47.4 us
+// a traversal (46.9 as a cooperative launch), s20 83.3 (81-84), s22 136 (133), s24, whose
+// traversals have two such launches, 337 (328).
 //
 // Ranks are given in the order of starting. Rank 0 leads. It founds the crew with
 // those that have started within a moment, nearly always the whole grid; from then
